@@ -221,3 +221,66 @@ def tolerance(case):
     if case["kind"] == "decode":
         return {"rel": 5e-3, "max": 2.5e-2}
     return {"rel": 1.1e-3, "max": 3.2e-3}
+
+
+# ---------------------------------------------------------------------------------------------- the same in 64 bits
+def _expand(wq, scales):
+    """The weights in 64 bits with the values that the decode stage gives them: (q - 7) * s rounded once to fp16."""
+    n, words = wq.shape
+    shifts = torch.arange(0, 32, 4, dtype=torch.int32, device="cuda")
+    q = (wq.view(torch.int32).unsqueeze(-1) >> shifts) & 15
+    w = (q - 7).view(n, words // 4, 32).double() * scales.double().unsqueeze(-1)
+    return w.to(torch.float16).double().view(n, words * 8)
+
+
+def _rmsnorm(x, weight, eps):
+    return x * torch.rsqrt((x * x).mean(dim=-1, keepdim=True) + eps) * weight.double()
+
+
+def _rotate(v, cos, sin):
+    a, b = v[..., :64], v[..., 64:]
+    return torch.cat((a * cos - b * sin, b * cos + a * sin), dim=-1)
+
+
+def _exact_decode(case, seed):
+    cfg = decoder.DecoderConfig(hidden=case["hidden"], heads=case["heads"], inter=case["inter"], layers=case["layers"],
+                                vocab=case["vocab"])
+    h, pos, batch = cfg.hidden, case["pos"], case["batch"]
+    embed = torch.randn((cfg.vocab, h), dtype=torch.float16, device="cuda", generator=_generator(seed, 2)) * 0.02
+    g = _generator(seed, 3)
+    shape = (batch, (pos + 1 + 63) // 64 * 64, cfg.heads, 128)
+    kc, vc = ([torch.empty(shape, dtype=torch.float16, device="cuda").normal_(generator=g) for _ in range(cfg.layers)] for _ in "kv")
+    tokens = torch.randint(0, cfg.vocab, (batch,), dtype=torch.int32, device="cuda", generator=g)
+    angle = pos * cfg.theta ** (-torch.arange(64, dtype=torch.float64, device="cuda") * 2.0 / 128)
+    cos, sin = torch.cos(angle), torch.sin(angle)
+    x = embed[tokens.long()].double()
+    for i in range(cfg.layers):
+        layer = decoder.synth_layer_torch(cfg, seed * 64 + i, "cuda")
+        w = {name: _expand(layer[name][0], layer[name][1] * 0.1) for name in ("qkv", "o", "gu", "down")}
+        qkv = (_rmsnorm(x, layer["norm1"], cfg.eps) @ w["qkv"].t()).view(batch, 3, cfg.heads, 128)
+        q, k, v = _rotate(qkv[:, 0], cos, sin), _rotate(qkv[:, 1], cos, sin), qkv[:, 2]
+        attn = torch.empty((batch, cfg.heads, 128), dtype=torch.float64, device="cuda")
+        for b in range(batch):
+            keys = torch.cat((kc[i][b, :pos].double(), k[b:b + 1]))
+            values = torch.cat((vc[i][b, :pos].double(), v[b:b + 1]))
+            p = torch.softmax(torch.einsum("hd,thd->ht", q[b], keys) / 128 ** 0.5, dim=-1)
+            attn[b] = torch.einsum("ht,thd->hd", p, values)
+        x = x + attn.view(batch, h) @ w["o"].t()
+        gate, up = (_rmsnorm(x, layer["norm2"], cfg.eps) @ w["gu"].t()).chunk(2, dim=1)
+        x = x + (torch.nn.functional.silu(gate) * up) @ w["down"].t()
+    ones = torch.ones(h, dtype=torch.float16, device="cuda")
+    return {"logits": _rmsnorm(x, ones, cfg.eps) @ embed.double().t(), "k": k, "v": v}
+
+
+def exact(case, seed):
+    kind = case["kind"]
+    if kind == "decode":
+        return _exact_decode(case, seed)
+    n, k = case["n"], case["k"]
+    if kind == "dequantize":
+        return _expand(*synth.make_weights_torch(n, k, seed, "cuda")).to(torch.float16)
+    x = _activations(case["m"], k, seed).double()
+    if kind == "chain":
+        return [x @ _expand(*synth.make_weights_torch(n, k, seed * 64 + i, "cuda")).t() for i in range(case["sets"])]
+    y = x @ _expand(*synth.make_weights_torch(n, k, seed, "cuda")).t()
+    return y.cpu() if kind == "host" else y
