@@ -115,29 +115,25 @@ int matmul_impl(Family fam, const char* who, const void* x, const void* wq, cons
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (M == 0 || N == 0) return B200_OK;
   if (K == 0) return zero_output(y, M, N, s);
-  bool use_gemv = fam == kGemv || (fam == kAuto && M <= 16);
-  // 9..16 batch rows: the skinny kernel stages all of x in every CTA (and restages it in K blocks once 16 rows x K
-  // no longer fit beside its ring); the weight-stationary kernel streams x through a ring instead.  Measured on
-  // B200 it is the faster one wherever its K split is in use (N up to about 8192: 9.8 against 12.1 us at
-  // N = K = 4096, 16.4 against 29.5 at K = 11008) and always when x does not fit; with many row tiles the skinny
-  // kernel wins (24.8 against 39 us at N = 22016).
-  if (fam == kAuto && M >= 9 && M <= 16 && (N <= 8192 || M * K * 2 > 160 * 1024) && K % 256 == 0 && options().gemm_ws_max_m >= M) {
-    rc = launch_gemm_ws(static_cast<const __half*>(x), static_cast<const uint32_t*>(wq), static_cast<const __half*>(scales),
-                        static_cast<__half*>(y), M, N, K, s);
-    if (rc != B200_ENOTREADY) return rc;
-  }
+  const bool use_gemv = fam == kGemv || (fam == kAuto && M <= 16);
   auto xh = static_cast<const __half*>(x);
   auto wh = static_cast<const uint32_t*>(wq);
   auto sh = static_cast<const __half*>(scales);
   auto yh = static_cast<__half*>(y);
-  if (use_gemv) return launch_gemv(xh, wh, sh, yh, M, N, K, s);
-  // Mid-sized batches (up to 128 rows): the weights stream once whatever the batch, which the prefill kernel's
-  // 256-token tiles would waste (measured at M = 64: 23.7 against 51 us at N = 12288, 46 against 51 at N = 22016).
-  if (fam == kGemmWs || (fam == kAuto && M <= options().gemm_ws_max_m)) {
+  // 9..128 rows, and 5..8 where K is long: the weight-stationary kernel, whose weights stream once whatever the batch.
+  // Measured on B200, skinny / weight-stationary kernel in us at 4, 8 and 16 rows: N = K = 4096 6.0 / 6.1, 7.7 / 6.4,
+  // 11.1 / 6.5; N = 22016 16.5 / 17.9, 17.9 / 18.1, 24.4 / 18.4; N = 4096, K = 11008 11.8 / 12.2, 18.9 / 12.3, 29.3 / 12.5;
+  // N = 1280, K = 8192 6.6 / 5.9, 9.7 / 6.0, 17.0 / 6.1 (the skinny kernel stages all of x in every CTA, and its
+  // arithmetic grows from 8 columns on).  At 5..8 rows and a shorter K the skinny kernel is the better one inside a
+  // decode step, where two of its CTAs fit an SM and it starts beside the kernel before it (8 layers of hidden
+  // 2048 at 5 rows: 413 us with it, 440 without).  The prefill kernel's 256-token tiles would be waste up to 128 rows.
+  // (A variant of the skinny kernel asked for by option keeps its rows.)
+  if (fam == kGemmWs || (fam == kAuto && (M >= 9 || (M >= 5 && K >= 8192)) && M <= options().gemm_ws_max_m && (M > 16 || options().gemv_variant == 0))) {
     rc = launch_gemm_ws(xh, wh, sh, yh, M, N, K, s);
     if (rc != B200_ENOTREADY) return rc;
     if (fam == kGemmWs) return fail(B200_EINVAL, "%s: the weight-stationary kernel takes 1 <= M <= 128, K %% 256 == 0, 16-byte aligned scales", who);
   }
+  if (use_gemv) return launch_gemv(xh, wh, sh, yh, M, N, K, s);
   return launch_gemm(xh, wh, sh, yh, M, N, K, s);
 }
 

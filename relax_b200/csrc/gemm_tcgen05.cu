@@ -176,7 +176,7 @@ q4f16_gemm_tcgen05_kernel(const __grid_constant__ GemmParams p) {
   volatile int* abort_flag = &sm.abort_flag;
 
   const int tid = threadIdx.x;
-  const int warp = tid >> 5;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // warp-uniform, and known to be
   const int lane = tid & 31;
   const int num_kb = (p.K + BK - 1) / BK;
 
@@ -195,7 +195,7 @@ q4f16_gemm_tcgen05_kernel(const __grid_constant__ GemmParams p) {
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  const uint32_t tmem_base = sm.tmem_base;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, sm.tmem_base, 0);
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer: x
@@ -236,9 +236,8 @@ q4f16_gemm_tcgen05_kernel(const __grid_constant__ GemmParams p) {
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
     {
-      // The whole warp walks the loop (waits, cursors, descriptor arithmetic are warp-uniform, so the compiler can
-      // keep them on the uniform datapath); only the tcgen05 instructions themselves are issued by one lane.
-      const bool leader = lane == 0;
+      // The whole warp walks the loop, converged (waits, cursors and descriptor arithmetic are warp-uniform); the
+      // tcgen05 wrappers elect the lane that issues.
       constexpr uint32_t idesc = umma_idesc_f16_f32(BM, BN);
       // The issue of a tcgen05.mma holds this thread until the tensor core takes the instruction, so the time of
       // this loop's own instructions ADDS to the MMAs' time (measured with a micro-benchmark, and a lone thread
@@ -256,7 +255,7 @@ q4f16_gemm_tcgen05_kernel(const __grid_constant__ GemmParams p) {
         tc_fence_after_sync();
       };
       auto release_and_advance = [&]() {
-        if (leader) umma_commit(&sm.empty[sb]);
+        umma_commit(&sm.empty[sb]);
         sb = sb + 1 == SB ? 0 : sb + 1;
         pb ^= (uint32_t)(sb == 0);
       };
@@ -277,12 +276,12 @@ q4f16_gemm_tcgen05_kernel(const __grid_constant__ GemmParams p) {
             for (int k16 = 0; k16 < BK / 16; ++k16) {
               // advancing 16 fp16 along K inside the swizzled 128-byte row = +32 bytes = +2 in the
               // descriptor's 16-byte address units
-              if (leader) umma_f16_ss(tmem_base + (uint32_t)h * BN, da + (uint64_t)(2 * k16), db + (uint64_t)(2 * k16), idesc, k16 != 0);
+              umma_f16_ss(tmem_base + (uint32_t)h * BN, da + (uint64_t)(2 * k16), db + (uint64_t)(2 * k16), idesc, k16 != 0);
             }
           }
           if (num_kb == 1) {
-            if (leader) umma_commit(&sm.acc_full[0]);
-            if (nhalf == 2 && leader) umma_commit(&sm.acc_full[1]);
+            umma_commit(&sm.acc_full[0]);
+            if (nhalf == 2) umma_commit(&sm.acc_full[1]);
           }
           release_and_advance();
         }
@@ -297,12 +296,12 @@ q4f16_gemm_tcgen05_kernel(const __grid_constant__ GemmParams p) {
             const uint64_t db = dconst | (uint64_t)(b_base + sb * b_step);
 #pragma unroll
             for (int k16 = 0; k16 < BK / 16; ++k16) {
-              if (leader) umma_f16_ss(tmem_base, da0 + (uint64_t)(2 * k16), db + (uint64_t)(2 * k16), idesc, 1);
-              if (leader) umma_f16_ss(tmem_base + (uint32_t)BN, da1 + (uint64_t)(2 * k16), db + (uint64_t)(2 * k16), idesc, 1);
+              umma_f16_ss(tmem_base, da0 + (uint64_t)(2 * k16), db + (uint64_t)(2 * k16), idesc, 1);
+              umma_f16_ss(tmem_base + (uint32_t)BN, da1 + (uint64_t)(2 * k16), db + (uint64_t)(2 * k16), idesc, 1);
             }
             if (kb == num_kb - 1) {
-              if (leader) umma_commit(&sm.acc_full[0]);
-              if (leader) umma_commit(&sm.acc_full[1]);
+              umma_commit(&sm.acc_full[0]);
+              umma_commit(&sm.acc_full[1]);
             }
             release_and_advance();
           }
@@ -313,13 +312,13 @@ q4f16_gemm_tcgen05_kernel(const __grid_constant__ GemmParams p) {
             const uint64_t db = dconst | (uint64_t)(b_base + sb * b_step);
 #pragma unroll
             for (int k16 = 0; k16 < BK / 16; ++k16)
-              if (leader) umma_f16_ss(tmem_base, da + (uint64_t)(2 * k16), db + (uint64_t)(2 * k16), idesc, 1);
-            if (kb == num_kb - 1 && leader) umma_commit(&sm.acc_full[0]);
+              umma_f16_ss(tmem_base, da + (uint64_t)(2 * k16), db + (uint64_t)(2 * k16), idesc, 1);
+            if (kb == num_kb - 1) umma_commit(&sm.acc_full[0]);
             release_and_advance();
           }
         }
         // a skipped half still takes part in the hand-shake so that the parities stay in step
-        if (nhalf == 1 && leader) umma_commit(&sm.acc_full[1]);
+        if (nhalf == 1) umma_commit(&sm.acc_full[1]);
       }
     }
   } else if ((warp >= 4 && warp < 8) || warp >= 24) {

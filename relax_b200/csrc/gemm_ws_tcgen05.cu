@@ -1,41 +1,47 @@
 // Weight-stationary q4f16 matmul on the 5th-generation tensor cores for mid-sized batches
-// (M <= 128; the dispatcher gives it 17..128 rows, and 9..16 where it beats the skinny kernel):
-// y[M,N] = x[M,K] . decode(Wq,S)^T.
+// (M <= 128; the dispatcher gives it 9..128 rows, and 5..8 with a long K): y[M,N] = x[M,K] . decode(Wq,S)^T.
 //
-// Decode at batch 16..128 is still bound by streaming the weights once, so the roles of the prefill
-// kernel are swapped: the MMA's M dimension is 128 WEIGHT rows (A operand = dequantised weights), its
-// N dimension is the batch (B operand = x, 16..128 columns).  A CTA owns 128 weight rows and a slice
-// of K; the `ksplit` CTAs of a thread-block cluster that share a row tile add their fp32 partial
-// tiles through distributed shared memory in rank order (deterministic), so small N still fills
-// the GPU (N = 4096: 32 row tiles x 4 K slices = 128 CTAs) without atomics or a scratch buffer.
+// Decode at these batches is still bound by streaming the weights once, so the roles of a plain GEMM are swapped:
+// the MMA's M dimension is 128 WEIGHT rows (A operand), its N dimension is the batch (B operand = x, 16..128 columns).
 //
-//   warps 0,2,3 TMA producers: x (WK K blocks of {64 k, NB batch rows} per load, 128-byte swizzle), packed
-//               weights (256 k per load: whole 128-byte lines of 128 rows, 128-byte swizzle), scales
-//               {8 groups = 256 k, 128 rows}; the first ring-full of weights is requested during set-up
-//   warps 8-23  dequantisers, two groups of 8 warps that take alternate 256-k spans (a group's load ->
-//               convert -> store -> fence -> arrive chain is latency bound; two chains in flight double
-//               the rate): thread (row, half) turns 4 packed words of one scale group into 32 fp16
-//               (exact q-7, one HMUL2 by the scale: the reference's rounding) and stores them as its
-//               part of row `row` of the K-major SWIZZLE_128B operand tile
-//   warp 1      one thread issues tcgen05.mma kind::f16 (M=128, N=NB, K=16) four times per K block;
-//               fp32 accumulator [128 rows x NB] in TMEM.  An MMA of N <= 128 takes 60-64 clocks, so this
-//               thread has about 250 clocks per K block: its loop is kept to a few dozen instructions
-//               (one wait each on the weight and the x stage per WK K blocks, descriptors advanced by
-//               32-bit adds, ring cursors without divisions); a lone thread runs some 10-15 clocks per
-//               instruction, and a longer loop is what the whole kernel then waits for
-//   warps 4-7   epilogue: tcgen05.ld -> this CTA's partial tile in shared memory; after the cluster
-//               barrier CTA r adds up batch columns r, r+ksplit, ... over all ranks (every thread of
-//               the CTA takes part, all of a column's remote loads in flight together) and stores fp16
+// The A operand lives in TENSOR MEMORY: a dequantiser thread turns the packed words of one row into registers and
+// stores them with tcgen05.st; the MMA reads them from there.  Shared memory then carries the packed words and x only
+// (no 16 KB of stores and 16 KB of operand reads per 64 k), no proxy fence stands between conversion and MMA, and
+// the room goes to the rings.
+//
+// Work: a tile is 128 weight rows over the whole K.  The CTAs of a cluster share tiles: CTA r takes the r-th slice of
+// K of every tile of the cluster's list (tile = cluster, cluster + clusters, ...), so the kernel starts once however
+// many tiles there are (a second wave of CTAs cost 7 us), and x of a slice stays in shared memory for all tiles where
+// it fits.  The accumulator is double-buffered: the next tile's MMAs run while the epilogue drains this one's.  The
+// partial tiles are exchanged by 16-byte stores into the owners' shared memory (owner o of a tile: batch columns
+// [o * cw, (o + 1) * cw)) and added up there in rank order: deterministic, no atomics, no scratch in global memory.
+//
+//   warps 0,2,3 TMA producers: x (two K blocks of {64 k, NB batch rows} per load, 128-byte swizzle), packed weights
+//               (256 k per load: whole 128-byte lines of 128 rows, 128-byte swizzle), scales {8 groups = 256 k,
+//               128 rows}; the first ring-full of weights is requested during set-up
+//   warps 8-23  dequantisers, four groups of 4 warps; a group takes one half (two K blocks) of every second 256-k
+//               span and owns one slot of the A ring (its wait -> load -> convert -> store -> arrive chain is
+//               latency bound, so it moves 128 k per trip); thread = weight row (= TMEM lane): 8 packed words -> 64 fp16
+//               (exact q-7, one HMUL2 by the scale: the reference's rounding) -> 32 columns, twice
+//   warp 1      issues tcgen05.mma kind::f16 (M=128, N=NB, K=16), eight per pair of K blocks
+//   warps 4-7, 24-27  epilogue: tcgen05.ld -> owners' inboxes -> sum over the K slices -> fp16 stores (or, with one
+//               slice, straight to y); two warps per TMEM quadrant share the columns
+//
+// What bounds it (measured at a batch of 64): 0.56 us per 256-k span and CTA, of which 0.37-0.39 us is the delivery of
+// the span's 18 KB (a copy of the kernel without the conversion) and the rest the conversion's 16 instructions per packed
+// word; the MMAs (45 clocks each or less) are hidden.  Before, with A in shared memory, the MMAs issued under a
+// branch on one lane and a grid of one tile per CTA: M = 64, N = 22016, K = 4096 46.1 -> 20.2 us; N = 12288
+// 23.3 -> 12.9; N = K = 4096 11.0 -> 9.0; N = 4096, K = 11008 18.9 -> 13.6; M = 128, N = 22016 49.5 -> 25.0; M = 16,
+// N = K = 4096 9.7 -> 6.5.
 //
 // Launched with programmatic dependent launch: set-up and the weight loads run ahead of the previous
 // kernel's end; the loads of x and the stores of y wait for it.
 //
 // Every mbarrier wait is bounded; a wait that runs out raises a block-wide abort flag and a device
-// error word, all loops then run through without waiting (cluster barriers are still reached by
+// error word, all loops then run through without waiting (the cluster barriers are still reached by
 // every thread), TMEM is freed and the kernel ends.
+#include <atomic>
 #include <cooperative_groups.h>
-
-#include <type_traits>
 
 #include "internal.h"
 #include "q4_common.cuh"
@@ -52,40 +58,40 @@ namespace cg = cooperative_groups;
 using namespace ptx;
 
 constexpr int BR = 128;            // weight rows per tile (UMMA M)
-constexpr int BK = 64;             // k per MMA stage (one 128-byte swizzled row of fp16)
+constexpr int BK = 64;             // k per K block (one 128-byte swizzled row of fp16)
 constexpr int kMaxNB = 128;        // batch columns (UMMA N), multiple of 16
-constexpr int kMaxStages = 8;
-constexpr int kWBytes = BR * BK * 2;          // 16384: one dequantised K block
-constexpr int kRawBytes = BR * 128;           // 16384: 128 rows x 32 words = 256 k = four K blocks, one 128-byte line per row
+constexpr int kMaxXStages = 32;    // x stages (two K blocks each)
+constexpr int kMaxRawStages = 8;
+constexpr int kASlots = 4;         // A ring: slots of two K blocks (64 TMEM columns), one per dequantiser group
+constexpr int kRawBytes = BR * 128;           // 16384: 128 rows x 32 words = 256 k, one 128-byte line per row
 constexpr int kScBytes = BR * 16;             // 2048:  128 rows x 8 scales  = 256 k
-constexpr int kDequantWarps = 8;           // per group
-constexpr int kDequantGroups = 2;          // alternate 256-k spans
-constexpr int kNumThreads = 256 + kDequantGroups * kDequantWarps * 32;   // 768
+constexpr int kDequantWarps = 16;
+constexpr int kNumThreads = 256 + kDequantWarps * 32 + 128;   // 896: warps 24-27 are a second set of epilogue warps
+constexpr uint32_t kTmemCols = 512;           // accumulators at 0 and 128, A ring at 256..511
+constexpr uint32_t kTmemA = 256;
 constexpr uint64_t kWaitNs = 4000000000ull;   // 4 s
 
-// A single thread sustains only ~2 tiled TMA loads per microsecond whatever their size, so every
-// load carries several K blocks (3-D boxes: the K block is the outer coordinate) and the three
-// kinds of load are issued by three different warps.
 struct WsParams {
-  CUtensorMap tm_x;    // fp16   {64, M, K/64},    box {64, NB, WK},   SWIZZLE_128B: [K block][batch row][128 B]
+  CUtensorMap tm_x;    // fp16   {64, M, K/64},    box {64, NB, 2},    SWIZZLE_128B: [K block][batch row][128 B]
   CUtensorMap tm_w;    // uint32 {K/8, N},         box {32, 128},      SWIZZLE_128B: [row][128 B] (whole lines: 64-byte pieces
                        //                                                    halve the rate the weights arrive at)
   CUtensorMap tm_s;    // fp16   {K/32, N},        box {8, 128}
   __half* y;
   int M, N, K;
-  int NB;              // batch columns of the MMA: M rounded up to 16
-  int WK;              // K blocks per stage of the x ring and of the dequantised-weight ring (4 or 2): the kernel's template value
-  int SX, SW, SR;      // ring depths: x loads, dequantised stages, packed 256-k spans (weights + scales)
+  int NB;              // batch columns of the MMA: M rounded up to 16 (32 with 8 slices)
+  int SX, SR;          // ring depths: x stages, packed 256-k spans (weights + scales; even)
+  int x_resident;      // the x ring holds a whole slice: loaded once, kept for every tile
   int ksplit;          // CTAs per cluster = K slices
-  int kb_total;        // K / 64
-  uint32_t tmem_cols;  // power of two >= max(32, NB)
+  int tiles;           // ceil(N / 128)
+  int cw;              // batch columns per owner: NB / ksplit, a multiple of 4
 };
 
 struct Bars {
-  uint64_t x_full[kMaxStages], x_empty[kMaxStages];
-  uint64_t w_full[kMaxStages], w_empty[kMaxStages];
-  uint64_t r_full[kMaxStages], r_empty[kMaxStages];
-  uint64_t acc_full;
+  uint64_t x_full[kMaxXStages], x_empty[kMaxXStages];
+  uint64_t r_full[kMaxRawStages], r_empty[kMaxRawStages];
+  uint64_t a_full[kASlots], a_empty[kASlots];
+  uint64_t acc_full[2], acc_empty[2];
+  uint64_t inbox_full, inbox_free;
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -98,19 +104,16 @@ __device__ __forceinline__ void wait_or_abort(uint64_t* bar, uint32_t parity, vo
     atomicExch(&g_gemm_ws_error, code);
   }
 }
-
-// Same for the roles that are off the critical path (TMA producers, epilogue warps): they sleep
-// between polls, so their polling does not take issue slots from the dequantisers.
-__device__ __forceinline__ void wait_or_abort_relaxed(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int code) {
+__device__ __forceinline__ void wait_or_abort_cluster(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int code) {
+  if (mbar_try_wait_cluster(bar, parity)) return;
   if (*abort_flag) return;
-  if (!mbar_wait_ns_relaxed(bar, parity, kWaitNs)) {
+  if (!mbar_wait_cluster_ns(bar, parity, kWaitNs)) {
     *abort_flag = 1;
     atomicExch(&g_gemm_ws_error, code);
   }
 }
 
-// Position in a ring of `n` stages without divisions (the ring depths are run-time values and a
-// single issuing thread cannot afford integer divisions per K block): stage index + wrap parity.
+// Position in a ring of `n` stages without divisions: stage index + wrap parity.
 struct Ring {
   int s = 0;
   uint32_t phase = 0;      // number of completed wraps, mod 2
@@ -128,287 +131,296 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const void* tmap, in
       : "memory");
 }
 
-// Shared memory (1024-aligned base): x ring [SX][WK][NB][128 B] | w ring [SW][WK][16 KB] | raw ring [SR][16 KB]
-// | scale ring [SR][2 KB] | barriers.  After the main loop the x ring is reused for this CTA's
-// partial tile [batch column][weight row] fp32 (NB * 512 B <= SX * WK * NB * 128 B since SX * WK >= 4).
-// WK: K blocks per stage of the x ring and of the dequantised ring (2 or 4).  PAIRED: nibble order of the packed
-// words (q4_common.cuh).
-template <int WK, bool PAIRED>
+// Shared memory (1024-aligned base): x ring [SX][2][NB][128 B] | raw ring [SR][16 KB] | scale ring [SR][2 KB] |
+// inbox [ksplit source ranks][cw / 4][128 rows][4 columns] fp32 (ksplit > 1; a warp's 16-byte stores are then 512
+// contiguous bytes: with rows 80 bytes apart, so 16-byte pieces on the SM-to-SM network, the exchange of a tile of 64
+// columns took 3900 clocks instead of 1400) | barriers.
+// PAIRED: nibble order of the packed words (q4_common.cuh).
+template <bool PAIRED>
 __global__ void __launch_bounds__(kNumThreads, 1)
 q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
   extern __shared__ unsigned char smem_unaligned[];
   unsigned char* base = smem_unaligned + ((1024u - (smem_u32(smem_unaligned) & 1023u)) & 1023u);
-  const int xstage = WK * p.NB * 128;
+  const int xstage = 2 * p.NB * 128;
   unsigned char* x_ring = base;
-  unsigned char* w_ring = x_ring + (size_t)p.SX * xstage;
-  constexpr int wstage = WK * kWBytes;
-  unsigned char* raw_ring = w_ring + (size_t)p.SW * wstage;
+  unsigned char* raw_ring = x_ring + (size_t)p.SX * xstage;
   unsigned char* sc_ring = raw_ring + (size_t)p.SR * kRawBytes;
-  Bars& bar = *reinterpret_cast<Bars*>(sc_ring + (size_t)p.SR * kScBytes);
-  float* part = reinterpret_cast<float*>(x_ring);
+  float* inbox = reinterpret_cast<float*>(sc_ring + (size_t)p.SR * kScBytes);
+  Bars& bar = *reinterpret_cast<Bars*>(inbox + (p.ksplit > 1 ? (size_t)BR * p.NB : 0));
   volatile int* abort_flag = &bar.abort_flag;
   cg::cluster_group cluster = cg::this_cluster();
 
   const int tid = threadIdx.x;
-  const int warp = tid >> 5;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // warp-uniform, and known to be
   const int lane = tid & 31;
   const int krank = (int)cluster.block_rank();          // K slice of this CTA (gridDim.x == ksplit)
-  const int row0 = blockIdx.y * BR;
-  // K blocks of 64, handed out in units of 4 (= one 256-k span), the first slices one unit longer
-  const int units = p.kb_total >> 2;
+  const int tile0 = blockIdx.y, tstep = gridDim.y;
+  // 256-k spans, the first slices one span longer (every slice has at least one)
+  const int units = p.K >> 8;
   const int ubase = units / p.ksplit, uextra = units % p.ksplit;
-  const int u0 = krank * ubase + min(krank, uextra);
-  const int kb0 = u0 * 4;
-  const int num_kb = (ubase + (krank < uextra ? 1 : 0)) * 4;
+  const int span0 = krank * ubase + min(krank, uextra);
+  const int nspans = ubase + (krank < uextra ? 1 : 0);
+  const int npairs = 2 * nspans;
 
-  const int nspans = num_kb >> 2;
   if (tid == 0) {
     bar.abort_flag = 0;
-    for (int i = 0; i < kMaxStages; ++i) {
-      mbar_init(&bar.x_full[i], 1); mbar_init(&bar.x_empty[i], 1);
-      mbar_init(&bar.w_full[i], kDequantWarps); mbar_init(&bar.w_empty[i], 1);
-    }
-    mbar_init(&bar.acc_full, 1);
+    for (int i = 0; i < p.SX; ++i) { mbar_init(&bar.x_full[i], 1); mbar_init(&bar.x_empty[i], 1); }
+    for (int i = 0; i < kASlots; ++i) { mbar_init(&bar.a_full[i], 4); mbar_init(&bar.a_empty[i], 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&bar.acc_full[i], 1); mbar_init(&bar.acc_empty[i], 8); }
+    mbar_init(&bar.inbox_full, 1);
+    mbar_init(&bar.inbox_free, p.ksplit > 1 ? 8 * (p.ksplit - 1) : 1);
     mbar_fence_init();
   }
   if (tid == 64) {
     // The weights depend on nothing: the thread that will stream them sets up the packed ring's barriers itself
-    // and fills the ring at once, ahead of the rest of the set-up (barriers, TMEM allocation, the block-wide sync).
-    for (int i = 0; i < kMaxStages; ++i) { mbar_init(&bar.r_full[i], 2); mbar_init(&bar.r_empty[i], kDequantWarps); }
+    // and fills the ring at once, ahead of the rest of the set-up (barriers, TMEM allocation, the cluster-wide sync).
+    for (int i = 0; i < p.SR; ++i) { mbar_init(&bar.r_full[i], 2); mbar_init(&bar.r_empty[i], kDequantWarps / 2); }
     mbar_fence_init();
     for (int i = 0; i < p.SR && i < nspans; ++i) {
-      const int gk = kb0 + 4 * i;
       mbar_arrive_expect_tx(&bar.r_full[i], kRawBytes);
-      tma_load_2d(raw_ring + (size_t)i * kRawBytes, &p.tm_w, (gk >> 2) * 32, row0, &bar.r_full[i]);
+      tma_load_2d(raw_ring + (size_t)i * kRawBytes, &p.tm_w, (span0 + i) * 32, tile0 * BR, &bar.r_full[i]);
       mbar_arrive_expect_tx(&bar.r_full[i], kScBytes);
-      tma_load_2d(sc_ring + (size_t)i * kScBytes, &p.tm_s, (gk >> 2) * 8, row0, &bar.r_full[i]);
+      tma_load_2d(sc_ring + (size_t)i * kScBytes, &p.tm_s, (span0 + i) * 8, tile0 * BR, &bar.r_full[i]);
     }
   }
   if (warp == 1) {
-    tmem_alloc(&bar.tmem_base, p.tmem_cols);
+    tmem_alloc(&bar.tmem_base, kTmemCols);
     tmem_relinquish();
   }
+  __syncwarp();
   tc_fence_before_sync();
-  __syncthreads();
+  if (p.ksplit > 1) cluster.sync();      // the peers' barriers are initialised before anything arrives on them
+  else __syncthreads();
   tc_fence_after_sync();
-  const uint32_t tmem_base = bar.tmem_base;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, bar.tmem_base, 0);
   pdl_launch_dependents();
 
   if (warp == 0) {
-    // ------------------------------------------------------------------ TMA producer: x (WK K blocks per load)
+    // ------------------------------------------------------------------ TMA producer: x (two K blocks per load)
     if (lane == 0) {
       prefetch_tmap(&p.tm_x);
       pdl_wait();                                     // x may be the previous kernel's output
       Ring rx;
-      for (int kb = 0; kb < num_kb; kb += WK, rx.next(p.SX)) {
-        // (not the sleeping wait: a nanosleep lasts far longer than the time a stage takes, and a ring of two or
-        // three stages then runs at the pace of the sleeps)
-        if (rx.wrapped) wait_or_abort(&bar.x_empty[rx.s], rx.phase ^ 1, abort_flag, 1);
-        mbar_arrive_expect_tx(&bar.x_full[rx.s], xstage);
-        tma_load_3d(x_ring + (size_t)rx.s * xstage, &p.tm_x, 0, 0, kb0 + kb, &bar.x_full[rx.s]);
+      for (int tile = tile0; tile < p.tiles; tile += tstep) {
+        for (int pr = 0; pr < npairs; ++pr, rx.next(p.SX)) {
+          // (not a sleeping wait: a nanosleep lasts far longer than the time a stage takes)
+          if (rx.wrapped) wait_or_abort(&bar.x_empty[rx.s], rx.phase ^ 1, abort_flag, 1);
+          mbar_arrive_expect_tx(&bar.x_full[rx.s], xstage);
+          tma_load_3d(x_ring + (size_t)rx.s * xstage, &p.tm_x, 0, 0, span0 * 4 + 2 * pr, &bar.x_full[rx.s]);
+        }
+        if (p.x_resident) break;                      // one trip: the stages stay
       }
     }
   } else if (warp == 2 || warp == 3) {
     // ------------------------------------------------------------------ TMA producers: packed weights (warp 2), scales (warp 3), 256 k per load
     if (lane == 0) {
-      // the first SR spans were requested during set-up: the cursor starts one trip round the ring later
+      const int first = min(p.SR, nspans);            // requested during set-up
       Ring rr;
-      rr.phase = 1;
-      rr.wrapped = true;
-      for (int kb = 4 * p.SR; kb < num_kb; kb += 4, rr.next(p.SR)) {
-        const int s = rr.s;
-        const int gk = kb0 + kb;
-        if (rr.wrapped) wait_or_abort(&bar.r_empty[s], rr.phase ^ 1, abort_flag, 3);
-        if (warp == 2) {
-          mbar_arrive_expect_tx(&bar.r_full[s], kRawBytes);
-          tma_load_2d(raw_ring + (size_t)s * kRawBytes, &p.tm_w, (gk >> 2) * 32, row0, &bar.r_full[s]);
-        } else {
-          mbar_arrive_expect_tx(&bar.r_full[s], kScBytes);
-          tma_load_2d(sc_ring + (size_t)s * kScBytes, &p.tm_s, (gk >> 2) * 8, row0, &bar.r_full[s]);
+      for (int tile = tile0; tile < p.tiles; tile += tstep) {
+        for (int sp = 0; sp < nspans; ++sp, rr.next(p.SR)) {
+          if (tile == tile0 && sp < first) continue;
+          const int s = rr.s;
+          if (rr.wrapped) wait_or_abort(&bar.r_empty[s], rr.phase ^ 1, abort_flag, 3);
+          if (warp == 2) {
+            mbar_arrive_expect_tx(&bar.r_full[s], kRawBytes);
+            tma_load_2d(raw_ring + (size_t)s * kRawBytes, &p.tm_w, (span0 + sp) * 32, tile * BR, &bar.r_full[s]);
+          } else {
+            mbar_arrive_expect_tx(&bar.r_full[s], kScBytes);
+            tma_load_2d(sc_ring + (size_t)s * kScBytes, &p.tm_s, (span0 + sp) * 8, tile * BR, &bar.r_full[s]);
+          }
         }
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      const uint32_t idesc = umma_idesc_f16_f32(BR, p.NB);
-      // descriptor = constant fields | (shared-memory address >> 4) in bits 0-13: stepping through the rings
-      // adds to the low word only (every address is below 256 KB, so nothing carries out of the field)
-      const uint64_t dconst = umma_desc_k128(0);
-      const uint32_t a0 = (smem_u32(w_ring) & 0x3FFFFu) >> 4, b0 = (smem_u32(x_ring) & 0x3FFFFu) >> 4;
-      const uint32_t a_step = (uint32_t)wstage >> 4, b_step = (uint32_t)xstage >> 4, b_kb = (uint32_t)(p.NB * 128) >> 4;
-      const uint32_t SW = (uint32_t)p.SW, SX = (uint32_t)p.SX;
-      uint32_t ws = 0, wphase = 0, xs = 0, xphase = 0;
-      // The issue of a tcgen05.mma holds this thread until the tensor core takes it (the time of the loop and
-      // the time of the MMAs add up, measured), and a lone thread spends 10-15 clocks per instruction, more on a
-      // taken branch: the loop is straight-line code, one branch for both waits, cursors advanced by selects.
-      auto stage = [&](uint32_t acc_first) {
-        uint64_t* wf = &bar.w_full[ws];
+    // The whole warp walks the loop, converged: its values are warp-uniform and the tcgen05 wrappers elect the lane
+    // that issues (see there).  Straight-line code per pair of K blocks, one branch for both waits, cursors advanced
+    // by selects, descriptors by 32-bit adds (every shared-memory address is below 256 KB, so nothing carries out of
+    // the address field).
+    const uint32_t idesc = umma_idesc_f16_f32(BR, p.NB);
+    const uint64_t dconst = umma_desc_k128(0);
+    const uint32_t b0 = (smem_u32(x_ring) & 0x3FFFFu) >> 4;
+    const uint32_t b_step = (uint32_t)xstage >> 4, b_kb = (uint32_t)(p.NB * 128) >> 4;
+    const uint32_t SX = (uint32_t)p.SX;
+    const bool resident = p.x_resident != 0;
+    uint32_t as = 0, aphase = 0, xs = 0, xphase = 0, it = 0;
+    for (int tile = tile0; tile < p.tiles; tile += tstep, ++it) {
+      const uint32_t buf = it & 1;
+      if (it >= 2) wait_or_abort(&bar.acc_empty[buf], ((it >> 1) - 1) & 1, abort_flag, 4);
+      const uint32_t td = tmem_base + buf * 128;
+      if (resident) xs = xphase = 0;
+      for (int pr = 0; pr < npairs; ++pr) {
+        uint64_t* af = &bar.a_full[as];
         uint64_t* xf = &bar.x_full[xs];
-        const bool ready = mbar_try_wait(wf, wphase) & mbar_try_wait(xf, xphase);
+        const bool ready = mbar_try_wait(af, aphase) & mbar_try_wait(xf, xphase);
         if (!ready) {
-          wait_or_abort(wf, wphase, abort_flag, 6);
+          wait_or_abort(af, aphase, abort_flag, 6);
           wait_or_abort(xf, xphase, abort_flag, 5);
         }
         tc_fence_after_sync();
-        const uint64_t da = dconst | (uint64_t)(a0 + ws * a_step);
+        const uint32_t ta = tmem_base + kTmemA + as * 64;
         const uint64_t db = dconst | (uint64_t)(b0 + xs * b_step);
 #pragma unroll
-        for (int j = 0; j < WK; ++j) {
+        for (int j = 0; j < 2; ++j) {
 #pragma unroll
           for (int k16 = 0; k16 < 4; ++k16) {
-            // +16 k inside the swizzled 128-byte row = +32 bytes = +2 in the descriptor's 16-byte units
-            umma_f16_ss(tmem_base, da + (uint64_t)(j * (kWBytes >> 4) + 2 * k16), db + (uint64_t)(j * b_kb + 2 * k16), idesc,
-                        (j | k16) == 0 ? acc_first : 1u);
+            // +16 k = +8 columns of A, +32 bytes inside the swizzled 128-byte row of x (+2 in 16-byte units)
+            umma_f16_ts(td, ta + j * 32 + k16 * 8, db + (uint64_t)(j * b_kb + 2 * k16), idesc,
+                        (j | k16) == 0 ? (uint32_t)(pr != 0) : 1u);
           }
         }
-        umma_commit(&bar.x_empty[xs]);
-        umma_commit(&bar.w_empty[ws]);
-        ws = ws + 1 == SW ? 0 : ws + 1;
-        wphase ^= (uint32_t)(ws == 0);
+        if (!resident) umma_commit(&bar.x_empty[xs]);
+        umma_commit(&bar.a_empty[as]);
+        as = as + 1 == kASlots ? 0 : as + 1;
+        aphase ^= (uint32_t)(as == 0);
         xs = xs + 1 == SX ? 0 : xs + 1;
         xphase ^= (uint32_t)(xs == 0);
-      };
-      if (num_kb > 0) stage(0);
-      for (int kb = WK; kb < num_kb; kb += WK) stage(1);
-      umma_commit(&bar.acc_full);
+      }
+      umma_commit(&bar.acc_full[buf]);
     }
-  } else if (warp >= 8) {
+  } else if (warp >= 8 && warp < 24) {
     // ------------------------------------------------------------------ dequantisers
-    const int t = (tid - 256) & 255;
-    const int grp = (tid - 256) >> 8;               // this group converts the spans whose index is grp mod 2
-    const int r = t & 127;                          // weight row inside the tile
-    const int half = t >> 7;                        // which 32-k half (= scale group) of each K block
+    // Pair n of K blocks of the CTA's whole run goes to slot n % 4: group `grp` fills slot grp with the half grp % 2 of
+    // the spans whose running index has the parity grp / 2.
+    const int grp = (warp - 8) >> 2;
+    const int half = grp & 1;
+    const int r = (warp & 3) * 32 + lane;           // weight row inside the tile = TMEM lane (a warp reaches quadrant warp % 4)
     const int r8 = r & 7;
+    const uint32_t tslot = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + kTmemA + (uint32_t)grp * 64;
+    uint32_t off[4];                                // the four 16-byte chunks of the half span; 128-byte swizzle: chunk ^ (row % 8)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) off[j] = (uint32_t)(r * 128 + (((4 * half + j) ^ r8) << 4));
     const Q4Consts qc = q4_consts();
-    Ring rr, rw;
-    for (int it = 0; it * 4 < num_kb; ++it, rr.next(p.SR)) {
-      if ((it & 1) != grp) {                        // the other group's span: keep the ring cursors in step
-#pragma unroll
-        for (int j0 = 0; j0 < 4; j0 += WK) rw.next(p.SW);
-        continue;
-      }
-      const int s = rr.s;
-      wait_or_abort(&bar.r_full[s], rr.phase, abort_flag, 8);
-      // this thread's share of the 256-k span: one 16-byte chunk (4 words = one scale group) and
-      // one scale per K block.  Span layout: [128-k half h2][row][64 B]; K block j = half j>>1,
-      // chunks 2*(j&1), 2*(j&1)+1 of the row; scales: row r holds groups 0..7, K block j uses 2j, 2j+1.
+    const uint32_t total = (uint32_t)nspans * (uint32_t)((p.tiles - tile0 + tstep - 1) / tstep);
+    int s = grp >> 1;                          // ring slot (the ring's depth is even: a group stays on slots of its parity)
+    uint32_t phase = 0, use = 0;
+    for (uint32_t sidx = (uint32_t)(grp >> 1); sidx < total; sidx += 2, ++use) {
+      wait_or_abort(&bar.r_full[s], phase, abort_flag, 8);
+      const unsigned char* rbase = raw_ring + (size_t)s * kRawBytes;
       uint4 pk[4];
-      uint32_t scb[4];
-      const unsigned char* rbase = raw_ring + (size_t)s * kRawBytes + r * 128;
-      const __half* srow = reinterpret_cast<const __half*>(sc_ring + (size_t)s * kScBytes + r * 16);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        pk[j] = *reinterpret_cast<const uint4*>(rbase + (((2 * j + half) ^ r8) << 4));   // 128-byte swizzle: chunk ^ (row % 8)
-        scb[j] = __half_as_ushort(srow[2 * j + half]);
-      }
+      for (int j = 0; j < 4; ++j) pk[j] = *reinterpret_cast<const uint4*>(rbase + off[j]);
+      const uint2 scw = *reinterpret_cast<const uint2*>(sc_ring + (size_t)s * kScBytes + r * 16 + half * 8);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        pin_loaded(pk[j]);
-        pin_loaded(scb[j]);
-      }
-      fence_proxy_async_smem();              // generic reads ordered before the TMA refill (async proxy)
+      for (int j = 0; j < 4; ++j) pin_loaded(pk[j]);
+      pin_loaded(scw.x);
+      pin_loaded(scw.y);
+      fence_proxy_async_smem();                // generic reads ordered before the TMA refill (async proxy)
       __syncwarp();
       if (lane == 0) mbar_arrive(&bar.r_empty[s]);
-      // one dequantised stage = WK K blocks: one wait, one proxy fence and one arrival per stage
 #pragma unroll
-      for (int j0 = 0; j0 < 4; j0 += WK, rw.next(p.SW)) {
-        if (rw.wrapped) wait_or_abort(&bar.w_empty[rw.s], rw.phase ^ 1, abort_flag, 10);
-        unsigned char* wst = w_ring + (size_t)rw.s * wstage + r * 128;     // 8-row atoms of 1024 B, rows 128 B apart
+      for (int j = 0; j < 2; ++j) {            // K block of the pair
+        const __half2 scp = u32_as_h2(j ? scw.y : scw.x);
+        const __half2 s_lo = __low2half2(scp), s_hi = __high2half2(scp);
+        const uint32_t words[8] = {pk[2 * j].x, pk[2 * j].y, pk[2 * j].z, pk[2 * j].w,
+                                   pk[2 * j + 1].x, pk[2 * j + 1].y, pk[2 * j + 1].z, pk[2 * j + 1].w};
+        uint32_t o[32];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          if (j < j0 || j >= j0 + WK) continue;
-          const __half sch = __ushort_as_half((unsigned short)scb[j]);
-          const __half2 s2 = __half2(sch, sch);
-          unsigned char* wrow = wst + (j - j0) * kWBytes;
-          const uint32_t wd[4] = {pk[j].x, pk[j].y, pk[j].z, pk[j].w};
+        for (int c = 0; c < 8; ++c) {
+          const uint4 q = q4_dequant_ordered<PAIRED>(words[c], c < 4 ? s_lo : s_hi, qc);
+          o[4 * c] = q.x; o[4 * c + 1] = q.y; o[4 * c + 2] = q.z; o[4 * c + 3] = q.w;
+        }
+        if (j == 0) {                          // the MMAs of this slot's previous pair have read it
+          if (use > 0) wait_or_abort(&bar.a_empty[grp], (use - 1) & 1, abort_flag, 10);
+          tc_fence_after_sync();
+        }
+        tmem_st_32x32b_x32(tslot + j * 32, o);
+      }
+      tmem_st_wait();
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bar.a_full[grp]);
+      s += 2;
+      if (s >= p.SR) { s -= p.SR; phase ^= 1; }
+    }
+  } else {
+    // ------------------------------------------------------------------ epilogue
+    pdl_wait();                                      // y may still be read by the previous kernel
+    const int ew = warp & 3;                         // TMEM lane quadrant this warp may read
+    const int set = warp >= 24 ? 1 : 0;              // two warps per quadrant share the columns
+    const int r = ew * 32 + lane;                    // weight row inside the tile
+    const int M4 = (p.M + 3) & ~3;                   // columns that are exchanged
+    const uint32_t inbox_mine = smem_u32(inbox) + (uint32_t)(krank * p.cw * BR + r * 4) * 4;   // row r of the block that this CTA fills, in every inbox
+    const uint32_t full_addr = smem_u32(&bar.inbox_full), free_addr = smem_u32(&bar.inbox_free);
+    const int own = max(0, min(p.cw, M4 - krank * p.cw));     // columns that this CTA adds up and stores
+    const uint32_t cw_inv = (65536u + (uint32_t)p.cw - 1) / (uint32_t)p.cw;      // column / cw for columns below 128
+    uint32_t it = 0;
+    for (int tile = tile0; tile < p.tiles; tile += tstep, ++it) {
+      const uint32_t buf = it & 1;
+      const int row = tile * BR + r;
+      // the owners have read what this CTA sent for the tile before
+      if (p.ksplit > 1 && it > 0) wait_or_abort_cluster(&bar.inbox_free, (it - 1) & 1, abort_flag, 12);
+      // (a phase of inbox_full ends with the bytes of all ranks; the next one cannot end before every warp here
+      // has told the peers that it is done with this one)
+      if (p.ksplit > 1 && own > 0 && warp == 4 && lane == 0) mbar_arrive_expect_tx(&bar.inbox_full, (uint32_t)(p.ksplit * BR * own * 4));
+      wait_or_abort(&bar.acc_full[buf], (it >> 1) & 1, abort_flag, 7);
+      tc_fence_after_sync();
+      const uint32_t taddr = tmem_base + ((uint32_t)(ew * 32) << 16) + buf * 128;
+      for (int c0 = 16 * set; c0 < p.M; c0 += 32) {
+        uint32_t v[16];
+        tmem_ld_32x32b_x16(taddr + c0, v);
+        tmem_ld_wait();
+        if (p.ksplit == 1) {
+          if (row < p.N) {
+            __half* dst_y = p.y + (int64_t)c0 * p.N + row;
+            if (c0 + 16 <= p.M) {
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const uint4 o = q4_dequant_ordered<PAIRED>(wd[c], s2, qc);
-            *reinterpret_cast<uint4*>(wrow + (((4 * half + c) ^ r8) << 4)) = o;
+              for (int q = 0; q < 16; ++q, dst_y += p.N) *dst_y = __float2half_rn(__uint_as_float(v[q]));
+            } else {
+#pragma unroll
+              for (int q = 0; q < 16; ++q, dst_y += p.N)
+                if (c0 + q < p.M) *dst_y = __float2half_rn(__uint_as_float(v[q]));
+            }
+          }
+        } else {
+#pragma unroll
+          for (int q = 0; q < 16; q += 4) {
+            if (c0 + q < M4) {
+              const uint32_t owner = ((uint32_t)(c0 + q) * cw_inv) >> 16;
+              const uint32_t lc = (uint32_t)(c0 + q) - owner * (uint32_t)p.cw;
+              st_async_v4(map_to_rank(inbox_mine + lc * (BR * 4), owner), map_to_rank(full_addr, owner), v[q], v[q + 1], v[q + 2], v[q + 3]);
+            }
           }
         }
-        fence_proxy_async_smem();          // generic-proxy stores -> visible to the tensor core's async proxy
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&bar.w_full[rw.s]);
       }
-    }
-  }
-
-  // ---------------------------------------------------------------------- TMEM -> this CTA's partial tile
-  if (warp >= 4 && warp < 8) {
-    const int ew = warp - 4;                       // TMEM lane quadrant this warp may read
-    // acc_full is committed after every MMA (and with it every read of the x ring) has completed,
-    // so the x ring may now be overwritten with the partial tile
-    wait_or_abort_relaxed(&bar.acc_full, 0, abort_flag, 7);
-    tc_fence_after_sync();
-    const int r = ew * 32 + lane;                  // weight row inside the tile = TMEM lane
-    const uint32_t taddr = tmem_base + ((uint32_t)(ew * 32) << 16);
-    for (int c0 = 0; c0 < p.NB; c0 += 32) {
-      uint32_t v[32];
-      tmem_ld_32x32b_x32(taddr + c0, v);
-      tmem_ld_wait();
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bar.acc_empty[buf]);
+      if (p.ksplit == 1) continue;
+      // ---- this CTA's columns: sum over the K slices in rank order
+      if (own > 0) wait_or_abort_cluster(&bar.inbox_full, it & 1, abort_flag, 11);
+      for (int l = 4 * set; l < own; l += 8) {
+        const int col = krank * p.cw + l;
+        const float* src = inbox + l * BR + r * 4;
+        float4 v[8];
 #pragma unroll
-      for (int q = 0; q < 32; ++q)
-        if (c0 + q < p.NB) part[(c0 + q) * BR + r] = num_kb > 0 ? __uint_as_float(v[q]) : 0.f;
-    }
-    tc_fence_before_sync();
-  }
-
-  // ---------------------------------------------------------------------- sum over the K slices
-  cluster.sync();                                    // every CTA's partial tile is complete and visible
-  pdl_wait();                                        // y may still be read by the previous kernel
-  {
-    // This CTA's batch columns are krank, krank + ksplit, ...  A work item is (column, four consecutive weight
-    // rows): one 16-byte load per rank, all of a thread's loads in flight together; a warp covers a column's 128
-    // rows.  The ranks are added in rank order whatever the unrolling: deterministic.
-    const int ncols = p.M > krank ? (p.M - krank + p.ksplit - 1) / p.ksplit : 0;
-    const bool vec_store = (p.N & 3) == 0;
-    auto item = [&](auto ks_tag, int c, int rg) {
-      constexpr int KS = decltype(ks_tag)::value;
-      float4 v[KS];
+        for (int q = 0; q < 8; ++q)
+          if (q < p.ksplit) v[q] = *reinterpret_cast<const float4*>(src + (size_t)q * p.cw * BR);
+        float4 sum = v[0];
 #pragma unroll
-      for (int q = 0; q < KS; ++q) v[q] = *reinterpret_cast<const float4*>(cluster.map_shared_rank(part, q) + c * BR + rg * 4);
-      float4 sum = v[0];
-#pragma unroll
-      for (int q = 1; q < KS; ++q) { sum.x += v[q].x; sum.y += v[q].y; sum.z += v[q].z; sum.w += v[q].w; }
-      const int row = row0 + rg * 4;
-      __half* dst = p.y + (int64_t)c * p.N + row;
-      if (vec_store && row + 4 <= p.N) {
-        uint2 o;
-        o.x = h2_as_u32(__floats2half2_rn(sum.x, sum.y));
-        o.y = h2_as_u32(__floats2half2_rn(sum.z, sum.w));
-        *reinterpret_cast<uint2*>(dst) = o;
-      } else {
-        if (row + 0 < p.N) dst[0] = __float2half_rn(sum.x);
-        if (row + 1 < p.N) dst[1] = __float2half_rn(sum.y);
-        if (row + 2 < p.N) dst[2] = __float2half_rn(sum.z);
-        if (row + 3 < p.N) dst[3] = __float2half_rn(sum.w);
-      }
-    };
-    for (int it = tid; it < ncols * 32; it += kNumThreads) {
-      const int c = krank + (it >> 5) * p.ksplit, rg = it & 31;
-      switch (p.ksplit) {
-        case 1: item(std::integral_constant<int, 1>{}, c, rg); break;
-        case 2: item(std::integral_constant<int, 2>{}, c, rg); break;
-        case 4: item(std::integral_constant<int, 4>{}, c, rg); break;
-        case 8: item(std::integral_constant<int, 8>{}, c, rg); break;
-        default: {                                   // a K with fewer 256-k units than the next power of two
-          float sum[4] = {0.f, 0.f, 0.f, 0.f};
-          for (int q = 0; q < p.ksplit; ++q) {
-            const float4 v = *reinterpret_cast<const float4*>(cluster.map_shared_rank(part, q) + c * BR + rg * 4);
-            sum[0] += v.x; sum[1] += v.y; sum[2] += v.z; sum[3] += v.w;
-          }
-          for (int i = 0; i < 4; ++i)
-            if (row0 + rg * 4 + i < p.N) p.y[(int64_t)c * p.N + row0 + rg * 4 + i] = __float2half_rn(sum[i]);
+        for (int q = 1; q < 8; ++q)
+          if (q < p.ksplit) { sum.x += v[q].x; sum.y += v[q].y; sum.z += v[q].z; sum.w += v[q].w; }
+        if (row < p.N) {
+          __half* dst_y = p.y + (int64_t)col * p.N + row;
+          dst_y[0] = __float2half_rn(sum.x);
+          if (col + 1 < p.M) dst_y[p.N] = __float2half_rn(sum.y);
+          if (col + 2 < p.M) dst_y[2 * (int64_t)p.N] = __float2half_rn(sum.z);
+          if (col + 3 < p.M) dst_y[3 * (int64_t)p.N] = __float2half_rn(sum.w);
         }
       }
+      // Not after the last tile: the arrival's release would wait for the stores to y.
+      __syncwarp();
+      if (tile + tstep < p.tiles && lane < p.ksplit && lane != krank) mbar_arrive_cluster(map_to_rank(free_addr, lane));
     }
   }
-  cluster.sync();                                    // nobody leaves while a peer still reads its tile
 
   // ---------------------------------------------------------------------- teardown
+  if (p.ksplit > 1) {
+    __syncwarp();
+    cluster.sync();                                  // nobody leaves while a peer still writes or arrives here
+  }
   if (*abort_flag) {
+    // loads may still be in flight into this CTA's shared memory: let them land before it is released
     const uint64_t t0 = globaltimer_ns();
     while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
   }
@@ -416,8 +428,42 @@ q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
   __syncthreads();
   if (warp == 1) {
     tc_fence_after_sync();
-    tmem_dealloc(tmem_base, p.tmem_cols);
+    tmem_dealloc(tmem_base, kTmemCols);
   }
+}
+
+constexpr size_t kSmemCap = 227 * 1024;
+// More than half of an SM: one such CTA per SM, whatever its rings would need.  (It takes all of tensor memory; two
+// of them on one SM, from clusters of two streams, could wait for each other's.)
+constexpr size_t kSmemFloor = 116 * 1024;
+
+// How many clusters of `ksplit` CTAs run at once (one CTA per SM; a cluster stays inside a GPC, so fewer than
+// SMs / ksplit for the larger sizes).  Asked once per device and size.
+int max_clusters(int ksplit, const void* kern) {
+  static std::atomic<int> cache[64][4];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return sm_count() / ksplit;
+  const int slot = ksplit == 1 ? 0 : ksplit == 2 ? 1 : ksplit == 4 ? 2 : 3;
+  int v = cache[dev][slot].load(std::memory_order_relaxed);
+  if (v > 0) return v;
+  v = sm_count() / ksplit;
+  if (ksplit > 1) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)ksplit, (unsigned)v);
+    cfg.blockDim = dim3(kNumThreads);
+    cfg.dynamicSmemBytes = kSmemCap;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)ksplit;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n > 0) v = n < v ? n : v;
+    else cudaGetLastError();
+  }
+  cache[dev][slot].store(v, std::memory_order_relaxed);
+  return v;
 }
 
 }  // namespace
@@ -428,14 +474,77 @@ int launch_gemm_ws(const __half* x, const uint32_t* wq, const __half* scales, __
   if (M < 1 || M > kMaxNB || K % 256 != 0 || K < 256 || (reinterpret_cast<uintptr_t>(scales) & 15u)) return B200_ENOTREADY;
   WsParams p;
   int rc;
-  p.NB = (int)((M + 15) / 16) * 16;
-  // K blocks per stage: a whole 256-k span for a narrow batch (x stages are small), half a span otherwise
-  p.WK = p.NB <= 32 ? 4 : 2;
-  if (options().gemm_ws_xk == 2 || options().gemm_ws_xk == 4) p.WK = (int)options().gemm_ws_xk;
+  const bool paired = current_layout() == kLayoutPaired;
+  auto kern = paired ? q4f16_gemm_ws_tcgen05_kernel<true> : q4f16_gemm_ws_tcgen05_kernel<false>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemCap);
+  if (e != cudaSuccess) return fail(B200_ELAUNCH, "gemm_ws: cudaFuncSetAttribute(%zu): %s", kSmemCap, cudaGetErrorString(e));
+  p.y = y;
+  p.M = (int)M; p.N = (int)N; p.K = (int)K;
+  p.tiles = (int)((N + BR - 1) / BR);
+  const int units = (int)(K / 256);
+  const int nb16 = (int)((M + 15) / 16) * 16;
+  // K slices: a model of the time in nanoseconds, fitted to measurements at N = 4096, 12288 and 22016, K = 4096 and
+  // 11008 and batches of 16, 64 and 128 (it picks the fastest or one within 4 %).  A CTA spends 0.53-0.65 us per
+  // 256-k span; draining a tile is cheap with one slice (stores to y, behind the next tile's MMAs) and costs the
+  // exchange of the partial tiles with several, which the next tile hides only as far as its own MMAs last; a larger
+  // cluster starts later.  M = 64, K = 4096, 1 / 2 / 4 / 8 slices: N = 4096 11.0 / 8.7 / 9.0 / 10.8 us, N = 12288 12.9 / 14.3 /
+  // 15.6 / 23.2, N = 22016 22.1 / 20.5 / 24.0 / 40.3; N = 4096 and K = 11008: 26.4 / 16.4 / 13.5 / 14.6.
+  int ksplit = 1;
+  if (options().gemm_ws_ksplit > 0) {
+    while (ksplit * 2 <= options().gemm_ws_ksplit && ksplit * 2 <= units) ksplit *= 2;
+  } else {
+    int64_t best = 0;
+    for (int c = 1; c <= 8 && c <= units; c *= 2) {
+      const int nc = max_clusters(c, reinterpret_cast<const void*>(kern));
+      const int64_t rounds = (p.tiles + nc - 1) / nc;
+      const int64_t tile = (int64_t)((units + c - 1) / c) * (520 + nb16);        // a tile's MMAs
+      const int64_t drain = c == 1 ? 300 + 12 * nb16 : 800 + 50 * nb16;          // ... and what the next tile must hide
+      const int64_t tail = c == 1 ? drain : 1000 + 35 * nb16;                    // the last tile's drain
+      const int64_t start = c == 1 ? 0 : c == 2 ? 500 : c == 4 ? 2800 : 3500;
+      const int64_t cost = start + tile + (rounds - 1) * (tile > drain ? tile : drain) + tail;
+      if (best == 0 || cost < best) { best = cost; ksplit = c; }
+    }
+  }
+  // an owner's columns are exchanged four at a time
+  if (ksplit == 8 || (ksplit > 1 && (nb16 / ksplit) % 4 != 0)) p.NB = (nb16 + 4 * ksplit - 1) / (4 * ksplit) * (4 * ksplit);
+  else p.NB = nb16;
+  p.ksplit = ksplit;
+  p.cw = p.NB / ksplit;
+  int clusters = max_clusters(ksplit, reinterpret_cast<const void*>(kern));
+  if (clusters > p.tiles) clusters = p.tiles;
+
+  // Shared memory: the inbox, four packed spans (72 KB in flight cover HBM's latency at one SM's share of its
+  // rate), then x: the whole slice if it fits (it is then loaded once for all tiles), else up to six stages; what
+  // is left goes to the packed ring.
+  const size_t inbox = ksplit > 1 ? (size_t)BR * p.NB * sizeof(float) : 0;
+  const size_t xstage = (size_t)2 * p.NB * 128;
+  const size_t span = kRawBytes + kScBytes;
+  const size_t fixed = 1024 + inbox + sizeof(Bars) + 256;
+  const int slice_stages = 2 * ((units + ksplit - 1) / ksplit);
+  int sr = 4;
+  int fit = (int)((kSmemCap - fixed - sr * span) / xstage);
+  if (fit < 3) { sr = 2; fit = (int)((kSmemCap - fixed - sr * span) / xstage); }
+  if (fit < 2) return B200_ENOTREADY;     // (never: 128 columns in several slices leave three stages)
+  p.x_resident = slice_stages <= fit && slice_stages <= kMaxXStages && options().gemm_ws_x_stages == 0;
+  p.SX = p.x_resident ? slice_stages : fit < 6 ? fit : 6;
+  if (options().gemm_ws_x_stages > 1 && options().gemm_ws_x_stages < p.SX) p.SX = (int)options().gemm_ws_x_stages;
+  sr = (int)((kSmemCap - fixed - p.SX * xstage) / span);
+  if (sr > kMaxRawStages) sr = kMaxRawStages;
+  if (options().gemm_ws_r_stages >= 2 && options().gemm_ws_r_stages < sr) sr = (int)options().gemm_ws_r_stages;
+  // An even depth: the groups of one span parity take every second span, so every slot of the ring then belongs to the
+  // same groups, which wait for its next load only after they have consumed the one before themselves (with an
+  // odd depth two parities would share a slot, each would meet it with the same phase parity every time, and its
+  // wait could pass on the load before last).
+  sr &= ~1;
+  if (sr < 2) return B200_ENOTREADY;
+  p.SR = sr;
+  size_t smem = fixed + p.SX * xstage + p.SR * span;
+  if (smem < kSmemFloor) smem = kSmemFloor;
+
   {
     const uint64_t d[3] = {BK, (uint64_t)M, (uint64_t)(K / BK)};
     const uint64_t s[2] = {(uint64_t)K * 2, BK * 2};
-    const uint32_t b[3] = {BK, (uint32_t)p.NB, (uint32_t)p.WK};
+    const uint32_t b[3] = {BK, (uint32_t)p.NB, 2};
     if ((rc = make_tmap(&p.tm_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, x, d, s, b, CU_TENSOR_MAP_SWIZZLE_128B))) return rc;
   }
   {
@@ -450,57 +559,8 @@ int launch_gemm_ws(const __half* x, const uint32_t* wq, const __half* scales, __
     const uint32_t b[2] = {8, BR};
     if ((rc = make_tmap(&p.tm_s, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, scales, d, s, b, CU_TENSOR_MAP_SWIZZLE_NONE))) return rc;
   }
-  p.y = y;
-  p.M = (int)M; p.N = (int)N; p.K = (int)K;
-  p.kb_total = (int)(K / BK);
-  p.tmem_cols = p.NB <= 32 ? 32 : (p.NB <= 64 ? 64 : 128);
-  const int row_tiles = (int)((N + BR - 1) / BR);
-  // K slices: enough CTAs to cover the SMs, at most 8 per cluster, at least one 256-k unit per slice
-  const int sms = sm_count();
-  int ksplit = 1;
-  const int units = p.kb_total / 4;
-  while (ksplit < 8 && row_tiles * ksplit * 2 <= sms + sms / 4 && ksplit * 2 <= units) ksplit *= 2;
-  if (options().gemm_ws_ksplit > 0) ksplit = (int)options().gemm_ws_ksplit;
-  if (ksplit > units) ksplit = units;
-  p.ksplit = ksplit;
-
-  // Ring depths.  Dequantised ring: its minimum.  At least one stage more than a span holds (P = 4 / WK
-  // stages): the two dequantiser groups share the ring's slots; a group that starts stage n has last waited for
-  // the consumption of stage n - P - 1 - SW, and its parity wait on w_empty for stage n - SW is only
-  // unambiguous if stage n - 2 SW is known to be consumed: n - P - 1 - SW >= n - 2 SW, i.e. SW >= P + 1 (a
-  // shallower ring lets a group run two phases ahead of a barrier, pass the wait at once and overwrite a stage
-  // that is still being read).  x ring: enough for the partial tile that reuses it (SX * WK >= 4) and for the L2
-  // latency.  Packed ring: the rest (even, see below); its depth is the number of 18 KB requests an SM keeps in
-  // flight to HBM.
-  const int sw_min = 4 / p.WK + 1;
-  p.SW = options().gemm_ws_w_stages > sw_min ? (int)options().gemm_ws_w_stages : sw_min;
-  p.SX = p.NB <= 64 ? 3 : 2;
-  if (options().gemm_ws_x_stages > 0) p.SX = (int)options().gemm_ws_x_stages;
-  if (p.SX * p.WK < 4) p.SX = 4 / p.WK;
-  const size_t xstage = (size_t)p.WK * p.NB * 128;
-  const size_t wstage = (size_t)p.WK * kWBytes;
-  const size_t others = 1024 + p.SX * xstage + p.SW * wstage + sizeof(Bars) + 256;
-  const size_t cap = 227 * 1024;
-  if (p.SX > kMaxStages || p.SW > kMaxStages || others + 2 * (size_t)(kRawBytes + kScBytes) > cap) return B200_ENOTREADY;
-  int sr = (int)((cap - others) / (kRawBytes + kScBytes));
-  if (sr > kMaxStages) sr = kMaxStages;
-  if (options().gemm_ws_r_stages >= 2 && options().gemm_ws_r_stages < sr) sr = (int)options().gemm_ws_r_stages;
-  // An even depth: the two dequantiser groups take alternate spans, so every slot of the ring then belongs to one
-  // group, which waits for a slot's next load only after it has consumed the previous one itself (with an odd
-  // depth the groups would share slots, and a load that completes out of order could let a group's parity wait
-  // pass one phase early).
-  sr &= ~1;
-  if (sr < 2) return B200_ENOTREADY;
-  p.SR = sr;
-  const size_t fixed = 1024 + p.SX * xstage + p.SR * (size_t)(kRawBytes + kScBytes) + sizeof(Bars) + 256;
-  const size_t smem = fixed + (size_t)p.SW * wstage;
-  const bool paired = current_layout() == kLayoutPaired;
-  auto kern = p.WK == 4 ? (paired ? q4f16_gemm_ws_tcgen05_kernel<4, true> : q4f16_gemm_ws_tcgen05_kernel<4, false>)
-                        : (paired ? q4f16_gemm_ws_tcgen05_kernel<2, true> : q4f16_gemm_ws_tcgen05_kernel<2, false>);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return fail(B200_ELAUNCH, "gemm_ws: cudaFuncSetAttribute(%zu): %s", smem, cudaGetErrorString(e));
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)ksplit, (unsigned)row_tiles);
+  cfg.gridDim = dim3((unsigned)ksplit, (unsigned)clusters);
   cfg.blockDim = dim3(kNumThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;

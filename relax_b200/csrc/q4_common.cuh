@@ -24,7 +24,7 @@ __device__ __forceinline__ uint32_t h2_as_u32(__half2 v) {
 // immediate); with the operands coming from the constant bank it is one LOP3, which halves the
 // integer-pipe work of the unpack (measured: 8.2 -> 4.1 logic instructions per packed word, and
 // the integer pipe was the busiest unit of the skinny matmul).
-static __constant__ uint32_t kQ4Bits[3] = {0x000F000Fu, 0x00F000F0u, 0x64006400u};
+static __constant__ uint32_t kQ4Bits[5] = {0x000F000Fu, 0x00F000F0u, 0x64006400u, 0x00F0000Fu, 0x54006400u};
 
 // (a & b) | c in one LOP3.
 __device__ __forceinline__ uint32_t lop3_and_or(uint32_t a, uint32_t b, uint32_t c) {
@@ -33,12 +33,13 @@ __device__ __forceinline__ uint32_t lop3_and_or(uint32_t a, uint32_t b, uint32_t
   return d;
 }
 
-// The three constants, fetched once per kernel (q4_consts()) and kept in registers: a kernel
+// The constants, fetched once per kernel (q4_consts()) and kept in registers: a kernel
 // whose loop contains a compiler memory barrier would otherwise re-read them every iteration.
 struct Q4Consts {
   uint32_t lo, hi, magic;   // nibble 0 / nibble 1 of each 16-bit half; (1024, 1024)
+  uint32_t mix, mix_magic;  // nibble 0 of the low half, nibble 1 of the high half; (1024, 64)
 };
-__device__ __forceinline__ Q4Consts q4_consts() { return Q4Consts{kQ4Bits[0], kQ4Bits[1], kQ4Bits[2]}; }
+__device__ __forceinline__ Q4Consts q4_consts() { return Q4Consts{kQ4Bits[0], kQ4Bits[1], kQ4Bits[2], kQ4Bits[3], kQ4Bits[4]}; }
 
 // One packed word (8 nibbles, k0 lowest) -> four half2 of exact (q-7):
 //   out[0] = (k0,k4)  out[1] = (k1,k5)  out[2] = (k2,k6)  out[3] = (k3,k7)
@@ -66,16 +67,19 @@ __device__ __forceinline__ void q4_dequant_pairs(uint32_t w, __half2 scale2, uin
   for (int i = 0; i < 4; ++i) out[i] = h2_as_u32(__hmul2(v[i], scale2));
 }
 
-// Dequantised word in natural order: out = (k0,k1) (k2,k3) (k4,k5) (k6,k7).
+// Dequantised word in natural order: out = (k0,k1) (k2,k3) (k4,k5) (k6,k7).  Byte i of the word holds the pair
+// (k 2i, k 2i+1): one byte permute copies it into both halves, one LOP3 keeps the low nibble of the low half
+// (mantissa of 1024: counts 1 per step) and the high nibble of the high half (bits 4-7 of the mantissa of 64: 1 per
+// step too), one HSUB2 removes the offsets exactly, one HMUL2 rounds.  8 integer and 8 half2 instructions per word.
 __device__ __forceinline__ uint4 q4_dequant_natural(uint32_t w, __half2 scale2, const Q4Consts& c) {
-  uint32_t p[4];
-  q4_dequant_pairs(w, scale2, p, c);
-  uint4 o;
-  o.x = __byte_perm(p[0], p[1], 0x5410);
-  o.y = __byte_perm(p[2], p[3], 0x5410);
-  o.z = __byte_perm(p[0], p[1], 0x7632);
-  o.w = __byte_perm(p[2], p[3], 0x7632);
-  return o;
+  const __half2 kSub = u32_as_h2(0x54706407u);         // (1031, 71)
+  uint32_t o[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t t = __byte_perm(w, 0u, 0x4040u + 0x0101u * i);
+    o[i] = h2_as_u32(__hmul2(__hsub2(u32_as_h2(lop3_and_or(t, c.mix, c.mix_magic)), kSub), scale2));
+  }
+  return make_uint4(o[0], o[1], o[2], o[3]);
 }
 
 // Weight layouts.  kLayoutReference: nibble j of a word is k % 8 = j (what the reference's encoder writes,

@@ -348,6 +348,29 @@ def test_gemm_ws_shapes(cuda_lib, m, n, k, ksplit):
     assert cuda_lib.b200_device_error_flags() == 0
 
 
+@pytest.mark.parametrize("m", [5, 128])
+def test_gemm_ws_more_tiles_than_clusters(cuda_lib, m):
+    # 151 row tiles (the last one 8 rows high): every cluster walks several of them, with both accumulators, the
+    # exchange of the partial tiles and, at 5 rows, x kept in shared memory from tile to tile
+    n, k = 150 * 128 + 8, 2048
+    x, wq, s = synth.make_case(m, n, k, seed=m)
+    sample = np.r_[0:130, 9000:9020, n - 140:n]          # the oracle on rows of the first, a middle and the last tiles
+    first = None
+    for ksplit in (0, 1, 2, 4, 8):
+        try:
+            relax_b200.set_option("gemm.ws_ksplit", ksplit)
+            outs = [run_matmul(x, wq, s, family="gemm_ws") for _ in range(2)]
+        finally:
+            relax_b200.set_option("gemm.ws_ksplit", 0)
+        assert_matmul_close(np.ascontiguousarray(outs[0][:, sample]), x, wq[sample], s[sample], f"gemm_ws M={m} ksplit={ksplit}")
+        assert_bits_equal(outs[1], outs[0], "the sum over the K slices has a fixed order")
+        if first is None:
+            first = outs[0].astype(np.float32)
+        # every other row against the first run: two fp16 roundings of nearly the same fp32 sum
+        assert np.abs(outs[0].astype(np.float32) - first).max() <= 2.0 ** -10 * np.abs(first).max() + 1e-3
+    assert cuda_lib.b200_device_error_flags() == 0
+
+
 def test_gemm_ws_one_hot_selects_weights_exactly(cuda_lib):
     # x row m is one-hot at k_m: y[m, n] = w[n, k_m] with no summation (the other K slices add exact
     # zeros), so the result must equal the reference's dequantised weight bit for bit
