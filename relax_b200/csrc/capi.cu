@@ -120,16 +120,18 @@ int matmul_impl(Family fam, const char* who, const void* x, const void* wq, cons
   auto wh = static_cast<const uint32_t*>(wq);
   auto sh = static_cast<const __half*>(scales);
   auto yh = static_cast<__half*>(y);
-  // 9..128 rows, and 5..8 where K is long: the weight-stationary kernel, whose weights stream once whatever the batch.
+  // 9 rows and more, and 5..8 where K is long: the weight-stationary kernel, whose weights stream once up to 192 rows.
   // Measured on B200, skinny / weight-stationary kernel in us at 4, 8 and 16 rows: N = K = 4096 6.0 / 6.1, 7.7 / 6.4,
   // 11.1 / 6.5; N = 22016 16.5 / 17.9, 17.9 / 18.1, 24.4 / 18.4; N = 4096, K = 11008 11.8 / 12.2, 18.9 / 12.3, 29.3 / 12.5;
   // N = 1280, K = 8192 6.6 / 5.9, 9.7 / 6.0, 17.0 / 6.1 (the skinny kernel stages all of x in every CTA, and its
   // arithmetic grows from 8 columns on).  At 5..8 rows and a shorter K the skinny kernel is the better one inside a
   // decode step, where two of its CTAs fit an SM and it starts beside the kernel before it (8 layers of hidden
-  // 2048 at 5 rows: 413 us with it, 440 without).  The prefill kernel's 256-token tiles would be waste up to 128 rows.
-  // (A variant of the skinny kernel asked for by option keeps its rows.)
-  if (fam == kGemmWs || (fam == kAuto && (M >= 9 || (M >= 5 && K >= 8192)) && M <= options().gemm_ws_max_m && (M > 16 || options().gemv_variant == 0))) {
-    rc = launch_gemm_ws(xh, wh, sh, yh, M, N, K, s);
+  // 2048 at 5 rows: 413 us with it, 440 without).  Above 128 rows it cuts the
+  // tokens into tiles to suit the shape; the prefill kernel with its 256-token tiles is left with the K that are not
+  // multiples of 256 (47.0 against 12.3 us at M = 129, N = K = 4096, 163 against 137 at M = 2048, N = 11008).  The
+  // option's largest value, 128, stands for no limit.  (A variant of the skinny kernel asked for by option keeps its rows.)
+  if (fam == kGemmWs || (fam == kAuto && (M >= 9 || (M >= 5 && K >= 8192)) && (M <= options().gemm_ws_max_m || options().gemm_ws_max_m == 128) && (M > 16 || options().gemv_variant == 0))) {
+    rc = fam == kGemmWs && M > 128 ? B200_ENOTREADY : launch_gemm_ws(xh, wh, sh, yh, M, N, K, s);
     if (rc != B200_ENOTREADY) return rc;
     if (fam == kGemmWs) return fail(B200_EINVAL, "%s: the weight-stationary kernel takes 1 <= M <= 128, K %% 256 == 0, 16-byte aligned scales", who);
   }

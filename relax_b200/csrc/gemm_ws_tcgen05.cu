@@ -1,15 +1,15 @@
-// Weight-stationary q4f16 matmul on the 5th-generation tensor cores for mid-sized batches
-// (M <= 128; the dispatcher gives it 9..128 rows, and 5..8 with a long K): y[M,N] = x[M,K] . decode(Wq,S)^T.
+// q4f16 matmul on the 5th-generation tensor cores (K a multiple of 256; the dispatcher gives it 9 rows and more, and
+// 5..8 with a long K): y[M,N] = x[M,K] . decode(Wq,S)^T.
 //
-// Decode at these batches is still bound by streaming the weights once, so the roles of a plain GEMM are swapped:
-// the MMA's M dimension is 128 WEIGHT rows (A operand), its N dimension is the batch (B operand = x, 16..128 columns).
+// Decode at batches up to 128 is still bound by streaming the weights once, so the roles of a plain GEMM are swapped:
+// the MMA's M dimension is 128 WEIGHT rows (A operand), its N dimension are tokens (B operand = x, 16..192 columns).
 //
 // The A operand lives in TENSOR MEMORY: a dequantiser thread turns the packed words of one row into registers and
 // stores them with tcgen05.st; the MMA reads them from there.  Shared memory then carries the packed words and x only
 // (no 16 KB of stores and 16 KB of operand reads per 64 k), no proxy fence stands between conversion and MMA, and
 // the room goes to the rings.
 //
-// Work: a tile is 128 weight rows over the whole K.  The CTAs of a cluster share tiles: CTA r takes the r-th slice of
+// Work: a tile is 128 weight rows by up to 192 tokens over the whole K (a prompt is cut into equal token tiles).  The CTAs of a cluster share tiles: CTA r takes the r-th slice of
 // K of every tile of the cluster's list (tile = cluster, cluster + clusters, ...), so the kernel starts once however
 // many tiles there are (a second wave of CTAs cost 7 us), and x of a slice stays in shared memory for all tiles where
 // it fits.  The accumulator is double-buffered: the next tile's MMAs run while the epilogue drains this one's.  The
@@ -32,7 +32,11 @@
 // word; the MMAs (45 clocks each or less) are hidden.  Before, with A in shared memory, the MMAs issued under a
 // branch on one lane and a grid of one tile per CTA: M = 64, N = 22016, K = 4096 46.1 -> 20.2 us; N = 12288
 // 23.3 -> 12.9; N = K = 4096 11.0 -> 9.0; N = 4096, K = 11008 18.9 -> 13.6; M = 128, N = 22016 49.5 -> 25.0; M = 16,
-// N = K = 4096 9.7 -> 6.5.
+// N = K = 4096 9.7 -> 6.5.  With many tokens the SMs' fetches of x from L2 (a tile's x serves 128 weight rows) are the
+// limit, about 14 TB/s over all SMs, and at the largest sizes the power cap.  Against the prefill kernel, whose
+// 256-token tiles leave SMs idle up to about 1000 tokens: K = 4096, N = 4096 at 129 tokens 47.0 -> 12.3 us, at 512
+// 47.6 -> 18.2; N = 3584, K = 8192 at 777 88.8 -> 38.0; N = 11008 at 2048 163 -> 137 (1350 TFLOP/s, where the library's
+// fp16 matmul under the same power cap reaches 1386).
 //
 // Launched with programmatic dependent launch: set-up and the weight loads run ahead of the previous
 // kernel's end; the loads of x and the stores of y wait for it.
@@ -59,20 +63,19 @@ using namespace ptx;
 
 constexpr int BR = 128;            // weight rows per tile (UMMA M)
 constexpr int BK = 64;             // k per K block (one 128-byte swizzled row of fp16)
-constexpr int kMaxNB = 128;        // batch columns (UMMA N), multiple of 16
-constexpr int kMaxXStages = 32;    // x stages (two K blocks each)
+constexpr int kMaxNB = 192;        // batch columns (UMMA N), multiple of 16
+constexpr int kMaxXStages = 32;    // x stages (SKB K blocks each)
 constexpr int kMaxRawStages = 8;
-constexpr int kASlots = 4;         // A ring: slots of two K blocks (64 TMEM columns), one per dequantiser group
+constexpr int kASlots = 4;         // A ring: slots of SKB K blocks (32 TMEM columns each), one per dequantiser group
 constexpr int kRawBytes = BR * 128;           // 16384: 128 rows x 32 words = 256 k, one 128-byte line per row
 constexpr int kScBytes = BR * 16;             // 2048:  128 rows x 8 scales  = 256 k
 constexpr int kDequantWarps = 16;
 constexpr int kNumThreads = 256 + kDequantWarps * 32 + 128;   // 896: warps 24-27 are a second set of epilogue warps
-constexpr uint32_t kTmemCols = 512;           // accumulators at 0 and 128, A ring at 256..511
-constexpr uint32_t kTmemA = 256;
+constexpr uint32_t kTmemCols = 512;           // two accumulators of 128 (SKB = 2) or 192 columns, then the A ring
 constexpr uint64_t kWaitNs = 4000000000ull;   // 4 s
 
 struct WsParams {
-  CUtensorMap tm_x;    // fp16   {64, M, K/64},    box {64, NB, 2},    SWIZZLE_128B: [K block][batch row][128 B]
+  CUtensorMap tm_x;    // fp16   {64, M, K/64},    box {64, NB, SKB},  SWIZZLE_128B: [K block][batch row][128 B]
   CUtensorMap tm_w;    // uint32 {K/8, N},         box {32, 128},      SWIZZLE_128B: [row][128 B] (whole lines: 64-byte pieces
                        //                                                    halve the rate the weights arrive at)
   CUtensorMap tm_s;    // fp16   {K/32, N},        box {8, 128}
@@ -82,7 +85,8 @@ struct WsParams {
   int SX, SR;          // ring depths: x stages, packed 256-k spans (weights + scales; even)
   int x_resident;      // the x ring holds a whole slice: loaded once, kept for every tile
   int ksplit;          // CTAs per cluster = K slices
-  int tiles;           // ceil(N / 128)
+  int mt;              // token tiles of NB rows of x: tile t is row tile t / mt, token tile t % mt
+  int tiles;           // ceil(N / 128) * mt
   int cw;              // batch columns per owner: NB / ksplit, a multiple of 4
 };
 
@@ -131,17 +135,19 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const void* tmap, in
       : "memory");
 }
 
-// Shared memory (1024-aligned base): x ring [SX][2][NB][128 B] | raw ring [SR][16 KB] | scale ring [SR][2 KB] |
+// Shared memory (1024-aligned base): x ring [SX][SKB][NB][128 B] | raw ring [SR][16 KB] | scale ring [SR][2 KB] |
 // inbox [ksplit source ranks][cw / 4][128 rows][4 columns] fp32 (ksplit > 1; a warp's 16-byte stores are then 512
 // contiguous bytes: with rows 80 bytes apart, so 16-byte pieces on the SM-to-SM network, the exchange of a tile of 64
 // columns took 3900 clocks instead of 1400) | barriers.
-// PAIRED: nibble order of the packed words (q4_common.cuh).
-template <bool PAIRED>
+// PAIRED: nibble order of the packed words (q4_common.cuh).  SKB: K blocks per x stage and A slot: 2 up to 128 batch
+// columns (fewer waits and arrivals), 1 above (tensor memory holds two accumulators of 192 columns and four slots of 32).
+template <bool PAIRED, int SKB>
 __global__ void __launch_bounds__(kNumThreads, 1)
 q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
   extern __shared__ unsigned char smem_unaligned[];
   unsigned char* base = smem_unaligned + ((1024u - (smem_u32(smem_unaligned) & 1023u)) & 1023u);
-  const int xstage = 2 * p.NB * 128;
+  const int xstage = SKB * p.NB * 128;
+  constexpr uint32_t kAccPitch = SKB == 2 ? 128 : 192, kTmemA = 2 * kAccPitch;
   unsigned char* x_ring = base;
   unsigned char* raw_ring = x_ring + (size_t)p.SX * xstage;
   unsigned char* sc_ring = raw_ring + (size_t)p.SR * kRawBytes;
@@ -160,7 +166,7 @@ q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
   const int ubase = units / p.ksplit, uextra = units % p.ksplit;
   const int span0 = krank * ubase + min(krank, uextra);
   const int nspans = ubase + (krank < uextra ? 1 : 0);
-  const int npairs = 2 * nspans;
+  const int nunits = 4 / SKB * nspans;                  // x stages = A slots of a tile
 
   if (tid == 0) {
     bar.abort_flag = 0;
@@ -174,13 +180,13 @@ q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
   if (tid == 64) {
     // The weights depend on nothing: the thread that will stream them sets up the packed ring's barriers itself
     // and fills the ring at once, ahead of the rest of the set-up (barriers, TMEM allocation, the cluster-wide sync).
-    for (int i = 0; i < p.SR; ++i) { mbar_init(&bar.r_full[i], 2); mbar_init(&bar.r_empty[i], kDequantWarps / 2); }
+    for (int i = 0; i < p.SR; ++i) { mbar_init(&bar.r_full[i], 2); mbar_init(&bar.r_empty[i], kDequantWarps / SKB); }
     mbar_fence_init();
     for (int i = 0; i < p.SR && i < nspans; ++i) {
       mbar_arrive_expect_tx(&bar.r_full[i], kRawBytes);
-      tma_load_2d(raw_ring + (size_t)i * kRawBytes, &p.tm_w, (span0 + i) * 32, tile0 * BR, &bar.r_full[i]);
+      tma_load_2d(raw_ring + (size_t)i * kRawBytes, &p.tm_w, (span0 + i) * 32, tile0 / p.mt * BR, &bar.r_full[i]);
       mbar_arrive_expect_tx(&bar.r_full[i], kScBytes);
-      tma_load_2d(sc_ring + (size_t)i * kScBytes, &p.tm_s, (span0 + i) * 8, tile0 * BR, &bar.r_full[i]);
+      tma_load_2d(sc_ring + (size_t)i * kScBytes, &p.tm_s, (span0 + i) * 8, tile0 / p.mt * BR, &bar.r_full[i]);
     }
   }
   if (warp == 1) {
@@ -196,17 +202,18 @@ q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
   pdl_launch_dependents();
 
   if (warp == 0) {
-    // ------------------------------------------------------------------ TMA producer: x (two K blocks per load)
+    // ------------------------------------------------------------------ TMA producer: x (SKB K blocks per load)
     if (lane == 0) {
       prefetch_tmap(&p.tm_x);
       pdl_wait();                                     // x may be the previous kernel's output
       Ring rx;
       for (int tile = tile0; tile < p.tiles; tile += tstep) {
-        for (int pr = 0; pr < npairs; ++pr, rx.next(p.SX)) {
+        const int tok0 = tile % p.mt * p.NB;
+        for (int u = 0; u < nunits; ++u, rx.next(p.SX)) {
           // (not a sleeping wait: a nanosleep lasts far longer than the time a stage takes)
           if (rx.wrapped) wait_or_abort(&bar.x_empty[rx.s], rx.phase ^ 1, abort_flag, 1);
           mbar_arrive_expect_tx(&bar.x_full[rx.s], xstage);
-          tma_load_3d(x_ring + (size_t)rx.s * xstage, &p.tm_x, 0, 0, span0 * 4 + 2 * pr, &bar.x_full[rx.s]);
+          tma_load_3d(x_ring + (size_t)rx.s * xstage, &p.tm_x, 0, tok0, span0 * 4 + SKB * u, &bar.x_full[rx.s]);
         }
         if (p.x_resident) break;                      // one trip: the stages stay
       }
@@ -217,16 +224,17 @@ q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
       const int first = min(p.SR, nspans);            // requested during set-up
       Ring rr;
       for (int tile = tile0; tile < p.tiles; tile += tstep) {
+        const int row0 = tile / p.mt * BR;
         for (int sp = 0; sp < nspans; ++sp, rr.next(p.SR)) {
           if (tile == tile0 && sp < first) continue;
           const int s = rr.s;
           if (rr.wrapped) wait_or_abort(&bar.r_empty[s], rr.phase ^ 1, abort_flag, 3);
           if (warp == 2) {
             mbar_arrive_expect_tx(&bar.r_full[s], kRawBytes);
-            tma_load_2d(raw_ring + (size_t)s * kRawBytes, &p.tm_w, (span0 + sp) * 32, tile * BR, &bar.r_full[s]);
+            tma_load_2d(raw_ring + (size_t)s * kRawBytes, &p.tm_w, (span0 + sp) * 32, row0, &bar.r_full[s]);
           } else {
             mbar_arrive_expect_tx(&bar.r_full[s], kScBytes);
-            tma_load_2d(sc_ring + (size_t)s * kScBytes, &p.tm_s, (span0 + sp) * 8, tile * BR, &bar.r_full[s]);
+            tma_load_2d(sc_ring + (size_t)s * kScBytes, &p.tm_s, (span0 + sp) * 8, row0, &bar.r_full[s]);
           }
         }
       }
@@ -234,7 +242,7 @@ q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
     // The whole warp walks the loop, converged: its values are warp-uniform and the tcgen05 wrappers elect the lane
-    // that issues (see there).  Straight-line code per pair of K blocks, one branch for both waits, cursors advanced
+    // that issues (see there).  Straight-line code per stage, one branch for both waits, cursors advanced
     // by selects, descriptors by 32-bit adds (every shared-memory address is below 256 KB, so nothing carries out of
     // the address field).
     const uint32_t idesc = umma_idesc_f16_f32(BR, p.NB);
@@ -247,9 +255,9 @@ q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
     for (int tile = tile0; tile < p.tiles; tile += tstep, ++it) {
       const uint32_t buf = it & 1;
       if (it >= 2) wait_or_abort(&bar.acc_empty[buf], ((it >> 1) - 1) & 1, abort_flag, 4);
-      const uint32_t td = tmem_base + buf * 128;
+      const uint32_t td = tmem_base + buf * kAccPitch;
       if (resident) xs = xphase = 0;
-      for (int pr = 0; pr < npairs; ++pr) {
+      for (int u = 0; u < nunits; ++u) {
         uint64_t* af = &bar.a_full[as];
         uint64_t* xf = &bar.x_full[xs];
         const bool ready = mbar_try_wait(af, aphase) & mbar_try_wait(xf, xphase);
@@ -258,15 +266,15 @@ q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
           wait_or_abort(xf, xphase, abort_flag, 5);
         }
         tc_fence_after_sync();
-        const uint32_t ta = tmem_base + kTmemA + as * 64;
+        const uint32_t ta = tmem_base + kTmemA + as * (32 * SKB);
         const uint64_t db = dconst | (uint64_t)(b0 + xs * b_step);
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
+        for (int j = 0; j < SKB; ++j) {
 #pragma unroll
           for (int k16 = 0; k16 < 4; ++k16) {
             // +16 k = +8 columns of A, +32 bytes inside the swizzled 128-byte row of x (+2 in 16-byte units)
             umma_f16_ts(td, ta + j * 32 + k16 * 8, db + (uint64_t)(j * b_kb + 2 * k16), idesc,
-                        (j | k16) == 0 ? (uint32_t)(pr != 0) : 1u);
+                        (j | k16) == 0 ? (uint32_t)(u != 0) : 1u);
           }
         }
         if (!resident) umma_commit(&bar.x_empty[xs]);
@@ -280,37 +288,41 @@ q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
     }
   } else if (warp >= 8 && warp < 24) {
     // ------------------------------------------------------------------ dequantisers
-    // Pair n of K blocks of the CTA's whole run goes to slot n % 4: group `grp` fills slot grp with the half grp % 2 of
-    // the spans whose running index has the parity grp / 2.
+    // Unit n (SKB K blocks) of the CTA's whole run goes to slot n % 4, which group n % 4 fills.  SKB = 2: group `grp`
+    // takes the half grp % 2 of the spans whose running index has the parity grp / 2; SKB = 1: K block grp of every span.
     const int grp = (warp - 8) >> 2;
-    const int half = grp & 1;
+    const int part = SKB == 2 ? grp & 1 : grp;
     const int r = (warp & 3) * 32 + lane;           // weight row inside the tile = TMEM lane (a warp reaches quadrant warp % 4)
     const int r8 = r & 7;
-    const uint32_t tslot = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + kTmemA + (uint32_t)grp * 64;
-    uint32_t off[4];                                // the four 16-byte chunks of the half span; 128-byte swizzle: chunk ^ (row % 8)
+    const uint32_t tslot = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + kTmemA + (uint32_t)grp * (32 * SKB);
+    uint32_t off[2 * SKB];                          // this part's 16-byte chunks; 128-byte swizzle: chunk ^ (row % 8)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) off[j] = (uint32_t)(r * 128 + (((4 * half + j) ^ r8) << 4));
+    for (int j = 0; j < 2 * SKB; ++j) off[j] = (uint32_t)(r * 128 + (((2 * SKB * part + j) ^ r8) << 4));
     const Q4Consts qc = q4_consts();
     const uint32_t total = (uint32_t)nspans * (uint32_t)((p.tiles - tile0 + tstep - 1) / tstep);
-    int s = grp >> 1;                          // ring slot (the ring's depth is even: a group stays on slots of its parity)
+    const uint32_t first = SKB == 2 ? (uint32_t)(grp >> 1) : 0;
+    int s = (int)first;                        // ring slot (the ring's depth is even: with SKB = 2 a group stays on slots of its parity)
     uint32_t phase = 0, use = 0;
-    for (uint32_t sidx = (uint32_t)(grp >> 1); sidx < total; sidx += 2, ++use) {
+    for (uint32_t sidx = first; sidx < total; sidx += SKB, ++use) {
       wait_or_abort(&bar.r_full[s], phase, abort_flag, 8);
       const unsigned char* rbase = raw_ring + (size_t)s * kRawBytes;
-      uint4 pk[4];
+      uint4 pk[2 * SKB];
+      uint32_t scw[SKB];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) pk[j] = *reinterpret_cast<const uint4*>(rbase + off[j]);
-      const uint2 scw = *reinterpret_cast<const uint2*>(sc_ring + (size_t)s * kScBytes + r * 16 + half * 8);
+      for (int j = 0; j < 2 * SKB; ++j) pk[j] = *reinterpret_cast<const uint4*>(rbase + off[j]);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) pin_loaded(pk[j]);
-      pin_loaded(scw.x);
-      pin_loaded(scw.y);
+      for (int j = 0; j < SKB; ++j)
+        scw[j] = *reinterpret_cast<const uint32_t*>(sc_ring + (size_t)s * kScBytes + r * 16 + (SKB * part + j) * 4);
+#pragma unroll
+      for (int j = 0; j < 2 * SKB; ++j) pin_loaded(pk[j]);
+#pragma unroll
+      for (int j = 0; j < SKB; ++j) pin_loaded(scw[j]);
       fence_proxy_async_smem();                // generic reads ordered before the TMA refill (async proxy)
       __syncwarp();
       if (lane == 0) mbar_arrive(&bar.r_empty[s]);
 #pragma unroll
-      for (int j = 0; j < 2; ++j) {            // K block of the pair
-        const __half2 scp = u32_as_h2(j ? scw.y : scw.x);
+      for (int j = 0; j < SKB; ++j) {          // K block of the unit
+        const __half2 scp = u32_as_h2(scw[j]);
         const __half2 s_lo = __low2half2(scp), s_hi = __high2half2(scp);
         const uint32_t words[8] = {pk[2 * j].x, pk[2 * j].y, pk[2 * j].z, pk[2 * j].w,
                                    pk[2 * j + 1].x, pk[2 * j + 1].y, pk[2 * j + 1].z, pk[2 * j + 1].w};
@@ -320,7 +332,7 @@ q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
           const uint4 q = q4_dequant_ordered<PAIRED>(words[c], c < 4 ? s_lo : s_hi, qc);
           o[4 * c] = q.x; o[4 * c + 1] = q.y; o[4 * c + 2] = q.z; o[4 * c + 3] = q.w;
         }
-        if (j == 0) {                          // the MMAs of this slot's previous pair have read it
+        if (j == 0) {                          // the MMAs of this slot's previous unit have read it
           if (use > 0) wait_or_abort(&bar.a_empty[grp], (use - 1) & 1, abort_flag, 10);
           tc_fence_after_sync();
         }
@@ -330,7 +342,7 @@ q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(&bar.a_full[grp]);
-      s += 2;
+      s += SKB;
       if (s >= p.SR) { s -= p.SR; phase ^= 1; }
     }
   } else {
@@ -339,15 +351,18 @@ q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
     const int ew = warp & 3;                         // TMEM lane quadrant this warp may read
     const int set = warp >= 24 ? 1 : 0;              // two warps per quadrant share the columns
     const int r = ew * 32 + lane;                    // weight row inside the tile
-    const int M4 = (p.M + 3) & ~3;                   // columns that are exchanged
     const uint32_t inbox_mine = smem_u32(inbox) + (uint32_t)(krank * p.cw * BR + r * 4) * 4;   // row r of the block that this CTA fills, in every inbox
     const uint32_t full_addr = smem_u32(&bar.inbox_full), free_addr = smem_u32(&bar.inbox_free);
-    const int own = max(0, min(p.cw, M4 - krank * p.cw));     // columns that this CTA adds up and stores
-    const uint32_t cw_inv = (65536u + (uint32_t)p.cw - 1) / (uint32_t)p.cw;      // column / cw for columns below 128
-    uint32_t it = 0;
+    const uint32_t cw_inv = (65536u + (uint32_t)p.cw - 1) / (uint32_t)p.cw;      // column / cw for columns below 256
+    uint32_t it = 0, inbox_phase = 0;
     for (int tile = tile0; tile < p.tiles; tile += tstep, ++it) {
       const uint32_t buf = it & 1;
-      const int row = tile * BR + r;
+      const int row = tile / p.mt * BR + r;
+      const int tok0 = tile % p.mt * p.NB;
+      const int ntok = min(p.NB, p.M - tok0);          // tokens of this tile
+      const int ntok4 = (ntok + 3) & ~3;               // columns that are exchanged
+      const int own = max(0, min(p.cw, ntok4 - krank * p.cw));     // columns that this CTA adds up and stores
+      __half* yt = p.y + (int64_t)tok0 * p.N + row;
       // the owners have read what this CTA sent for the tile before
       if (p.ksplit > 1 && it > 0) wait_or_abort_cluster(&bar.inbox_free, (it - 1) & 1, abort_flag, 12);
       // (a phase of inbox_full ends with the bytes of all ranks; the next one cannot end before every warp here
@@ -355,27 +370,27 @@ q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
       if (p.ksplit > 1 && own > 0 && warp == 4 && lane == 0) mbar_arrive_expect_tx(&bar.inbox_full, (uint32_t)(p.ksplit * BR * own * 4));
       wait_or_abort(&bar.acc_full[buf], (it >> 1) & 1, abort_flag, 7);
       tc_fence_after_sync();
-      const uint32_t taddr = tmem_base + ((uint32_t)(ew * 32) << 16) + buf * 128;
-      for (int c0 = 16 * set; c0 < p.M; c0 += 32) {
+      const uint32_t taddr = tmem_base + ((uint32_t)(ew * 32) << 16) + buf * kAccPitch;
+      for (int c0 = 16 * set; c0 < ntok; c0 += 32) {
         uint32_t v[16];
         tmem_ld_32x32b_x16(taddr + c0, v);
         tmem_ld_wait();
         if (p.ksplit == 1) {
           if (row < p.N) {
-            __half* dst_y = p.y + (int64_t)c0 * p.N + row;
-            if (c0 + 16 <= p.M) {
+            __half* dst_y = yt + (int64_t)c0 * p.N;
+            if (c0 + 16 <= ntok) {
 #pragma unroll
               for (int q = 0; q < 16; ++q, dst_y += p.N) *dst_y = __float2half_rn(__uint_as_float(v[q]));
             } else {
 #pragma unroll
               for (int q = 0; q < 16; ++q, dst_y += p.N)
-                if (c0 + q < p.M) *dst_y = __float2half_rn(__uint_as_float(v[q]));
+                if (c0 + q < ntok) *dst_y = __float2half_rn(__uint_as_float(v[q]));
             }
           }
         } else {
 #pragma unroll
           for (int q = 0; q < 16; q += 4) {
-            if (c0 + q < M4) {
+            if (c0 + q < ntok4) {
               const uint32_t owner = ((uint32_t)(c0 + q) * cw_inv) >> 16;
               const uint32_t lc = (uint32_t)(c0 + q) - owner * (uint32_t)p.cw;
               st_async_v4(map_to_rank(inbox_mine + lc * (BR * 4), owner), map_to_rank(full_addr, owner), v[q], v[q + 1], v[q + 2], v[q + 3]);
@@ -388,7 +403,8 @@ q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
       if (lane == 0) mbar_arrive(&bar.acc_empty[buf]);
       if (p.ksplit == 1) continue;
       // ---- this CTA's columns: sum over the K slices in rank order
-      if (own > 0) wait_or_abort_cluster(&bar.inbox_full, it & 1, abort_flag, 11);
+      if (own > 0) wait_or_abort_cluster(&bar.inbox_full, inbox_phase, abort_flag, 11);
+      inbox_phase ^= (uint32_t)(own > 0);            // (a CTA without columns in a tile's last tokens sits that phase out)
       for (int l = 4 * set; l < own; l += 8) {
         const int col = krank * p.cw + l;
         const float* src = inbox + l * BR + r * 4;
@@ -401,11 +417,11 @@ q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
         for (int q = 1; q < 8; ++q)
           if (q < p.ksplit) { sum.x += v[q].x; sum.y += v[q].y; sum.z += v[q].z; sum.w += v[q].w; }
         if (row < p.N) {
-          __half* dst_y = p.y + (int64_t)col * p.N + row;
+          __half* dst_y = yt + (int64_t)col * p.N;
           dst_y[0] = __float2half_rn(sum.x);
-          if (col + 1 < p.M) dst_y[p.N] = __float2half_rn(sum.y);
-          if (col + 2 < p.M) dst_y[2 * (int64_t)p.N] = __float2half_rn(sum.z);
-          if (col + 3 < p.M) dst_y[3 * (int64_t)p.N] = __float2half_rn(sum.w);
+          if (col + 1 < ntok) dst_y[p.N] = __float2half_rn(sum.y);
+          if (col + 2 < ntok) dst_y[2 * (int64_t)p.N] = __float2half_rn(sum.z);
+          if (col + 3 < ntok) dst_y[3 * (int64_t)p.N] = __float2half_rn(sum.w);
         }
       }
       // Not after the last tile: the arrival's release would wait for the stores to y.
@@ -432,6 +448,12 @@ q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
   }
 }
 
+using WsKernel = void (*)(const WsParams);
+WsKernel kernel_for(int nb, bool paired) {
+  return nb <= 128 ? (paired ? q4f16_gemm_ws_tcgen05_kernel<true, 2> : q4f16_gemm_ws_tcgen05_kernel<false, 2>)
+                   : (paired ? q4f16_gemm_ws_tcgen05_kernel<true, 1> : q4f16_gemm_ws_tcgen05_kernel<false, 1>);
+}
+
 constexpr size_t kSmemCap = 227 * 1024;
 // More than half of an SM: one such CTA per SM, whatever its rings would need.  (It takes all of tensor memory; two
 // of them on one SM, from clusters of two streams, could wait for each other's.)
@@ -447,7 +469,7 @@ int max_clusters(int ksplit, const void* kern) {
   int v = cache[dev][slot].load(std::memory_order_relaxed);
   if (v > 0) return v;
   v = sm_count() / ksplit;
-  if (ksplit > 1) {
+  if (ksplit > 1 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemCap) == cudaSuccess) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)ksplit, (unsigned)v);
     cfg.blockDim = dim3(kNumThreads);
@@ -471,45 +493,56 @@ int max_clusters(int ksplit, const void* kern) {
 // Returns B200_ENOTREADY when the shape is outside what this kernel takes.
 int launch_gemm_ws(const __half* x, const uint32_t* wq, const __half* scales, __half* y, int64_t M, int64_t N,
                    int64_t K, cudaStream_t stream) {
-  if (M < 1 || M > kMaxNB || K % 256 != 0 || K < 256 || (reinterpret_cast<uintptr_t>(scales) & 15u)) return B200_ENOTREADY;
+  if (M < 1 || K % 256 != 0 || K < 256 || (reinterpret_cast<uintptr_t>(scales) & 15u)) return B200_ENOTREADY;
   WsParams p;
   int rc;
   const bool paired = current_layout() == kLayoutPaired;
-  auto kern = paired ? q4f16_gemm_ws_tcgen05_kernel<true> : q4f16_gemm_ws_tcgen05_kernel<false>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemCap);
-  if (e != cudaSuccess) return fail(B200_ELAUNCH, "gemm_ws: cudaFuncSetAttribute(%zu): %s", kSmemCap, cudaGetErrorString(e));
   p.y = y;
   p.M = (int)M; p.N = (int)N; p.K = (int)K;
-  p.tiles = (int)((N + BR - 1) / BR);
   const int units = (int)(K / 256);
-  const int nb16 = (int)((M + 15) / 16) * 16;
-  // K slices: a model of the time in nanoseconds, fitted to measurements at N = 4096, 12288 and 22016, K = 4096 and
-  // 11008 and batches of 16, 64 and 128 (it picks the fastest or one within 4 %).  A CTA spends 0.53-0.65 us per
-  // 256-k span; draining a tile is cheap with one slice (stores to y, behind the next tile's MMAs) and costs the
-  // exchange of the partial tiles with several, which the next tile hides only as far as its own MMAs last; a larger
-  // cluster starts later.  M = 64, K = 4096, 1 / 2 / 4 / 8 slices: N = 4096 11.0 / 8.7 / 9.0 / 10.8 us, N = 12288 12.9 / 14.3 /
-  // 15.6 / 23.2, N = 22016 22.1 / 20.5 / 24.0 / 40.3; N = 4096 and K = 11008: 26.4 / 16.4 / 13.5 / 14.6.
-  int ksplit = 1;
-  if (options().gemm_ws_ksplit > 0) {
-    while (ksplit * 2 <= options().gemm_ws_ksplit && ksplit * 2 <= units) ksplit *= 2;
-  } else {
-    int64_t best = 0;
+  const int64_t row_tiles = (N + BR - 1) / BR;
+  if (row_tiles * ((M + 15) / 16) > 0x3fffffff) return B200_ENOTREADY;      // (tile numbers are 32-bit)
+  // Token tiles and K slices: a model of the time in nanoseconds, fitted to measurements at N = 4096, 12288 and 22016,
+  // K = 4096 and 11008 and batches of 16, 64 and 128, and at 129..2048 tokens.  A 256-k span takes a CTA 0.53-0.65 us (up
+  // to 128 columns) or 0.9-0.95 us; with many CTAs at work, what they fetch from L2 at about 14 TB/s if that is more.
+  // Draining a tile is cheap with one slice (stores to y, behind the next tile's MMAs) and costs the exchange of the
+  // partial tiles with several, which the next tile hides only as far as its own MMAs last; a larger cluster starts
+  // later.  M = 64, K = 4096, 1 / 2 / 4 / 8 slices: N = 4096 11.0 / 8.7 / 9.0 / 10.8 us, N = 12288 12.9 / 14.3 / 15.6 / 23.2,
+  // N = 22016 22.1 / 20.5 / 24.0 / 40.3; N = 4096 and K = 11008: 26.4 / 16.4 / 13.5 / 14.6.  M = 300, N = 12288, K = 4096 in 2 / 3 / 4
+  // token tiles: 31.7 / 29.5 / 34.8.
+  const int forced = (int)options().gemm_ws_ksplit;
+  int ksplit = 1, nb16 = 0;
+  int64_t best = 0;
+  const int64_t mt0 = (M + kMaxNB - 1) / kMaxNB;
+  for (int64_t mt = mt0; mt <= mt0 + mt0 / 2 + 3 && (mt == mt0 || mt * 16 <= M); ++mt) {
+    const int nb = (int)(((M + mt - 1) / mt + 15) / 16) * 16;
+    const int64_t tiles = row_tiles * ((M + nb - 1) / nb);
     for (int c = 1; c <= 8 && c <= units; c *= 2) {
-      const int nc = max_clusters(c, reinterpret_cast<const void*>(kern));
-      const int64_t rounds = (p.tiles + nc - 1) / nc;
-      const int64_t tile = (int64_t)((units + c - 1) / c) * (520 + nb16);        // a tile's MMAs
-      const int64_t drain = c == 1 ? 300 + 12 * nb16 : 800 + 50 * nb16;          // ... and what the next tile must hide
-      const int64_t tail = c == 1 ? drain : 1000 + 35 * nb16;                    // the last tile's drain
+      if (forced > 0 && !(c <= forced && (c * 2 > forced || c * 2 > units || c == 8))) continue;
+      const int nc = max_clusters(c, reinterpret_cast<const void*>(kernel_for(nb, paired)));
+      const int64_t rounds = (tiles + nc - 1) / nc;
+      const int64_t busy = tiles * c / rounds;                                   // CTAs at work, on average
+      const int64_t l2 = busy * (nb * 512 + kRawBytes + kScBytes) / 14000;
+      const int64_t span = nb <= 128 ? 520 + nb : 760 + nb;
+      const int64_t tile = (int64_t)((units + c - 1) / c) * (span > l2 ? span : l2);   // a tile's MMAs
+      const int64_t drain = c == 1 ? 300 + 12 * nb : 800 + 50 * nb;              // ... and what the next tile must hide
+      const int64_t tail = c == 1 ? drain : 1000 + 35 * nb;                      // the last tile's drain
       const int64_t start = c == 1 ? 0 : c == 2 ? 500 : c == 4 ? 2800 : 3500;
       const int64_t cost = start + tile + (rounds - 1) * (tile > drain ? tile : drain) + tail;
-      if (best == 0 || cost < best) { best = cost; ksplit = c; }
+      if (best == 0 || cost < best) { best = cost; ksplit = c; nb16 = nb; }
     }
   }
+  const int skb = nb16 <= 128 ? 2 : 1;
+  auto kern = kernel_for(nb16, paired);
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemCap);
+  if (e != cudaSuccess) return fail(B200_ELAUNCH, "gemm_ws: cudaFuncSetAttribute(%zu): %s", kSmemCap, cudaGetErrorString(e));
   // an owner's columns are exchanged four at a time
   if (ksplit == 8 || (ksplit > 1 && (nb16 / ksplit) % 4 != 0)) p.NB = (nb16 + 4 * ksplit - 1) / (4 * ksplit) * (4 * ksplit);
   else p.NB = nb16;
   p.ksplit = ksplit;
   p.cw = p.NB / ksplit;
+  p.mt = (int)((M + p.NB - 1) / p.NB);
+  p.tiles = (int)row_tiles * p.mt;
   int clusters = max_clusters(ksplit, reinterpret_cast<const void*>(kern));
   if (clusters > p.tiles) clusters = p.tiles;
 
@@ -517,15 +550,15 @@ int launch_gemm_ws(const __half* x, const uint32_t* wq, const __half* scales, __
   // rate), then x: the whole slice if it fits (it is then loaded once for all tiles), else up to six stages; what
   // is left goes to the packed ring.
   const size_t inbox = ksplit > 1 ? (size_t)BR * p.NB * sizeof(float) : 0;
-  const size_t xstage = (size_t)2 * p.NB * 128;
+  const size_t xstage = (size_t)skb * p.NB * 128;
   const size_t span = kRawBytes + kScBytes;
   const size_t fixed = 1024 + inbox + sizeof(Bars) + 256;
-  const int slice_stages = 2 * ((units + ksplit - 1) / ksplit);
+  const int slice_stages = 4 / skb * ((units + ksplit - 1) / ksplit);
   int sr = 4;
   int fit = (int)((kSmemCap - fixed - sr * span) / xstage);
   if (fit < 3) { sr = 2; fit = (int)((kSmemCap - fixed - sr * span) / xstage); }
-  if (fit < 2) return B200_ENOTREADY;     // (never: 128 columns in several slices leave three stages)
-  p.x_resident = slice_stages <= fit && slice_stages <= kMaxXStages && options().gemm_ws_x_stages == 0;
+  if (fit < 2) return B200_ENOTREADY;     // (never: 192 columns in several slices leave three stages)
+  p.x_resident = p.mt == 1 && slice_stages <= fit && slice_stages <= kMaxXStages && options().gemm_ws_x_stages == 0;
   p.SX = p.x_resident ? slice_stages : fit < 6 ? fit : 6;
   if (options().gemm_ws_x_stages > 1 && options().gemm_ws_x_stages < p.SX) p.SX = (int)options().gemm_ws_x_stages;
   sr = (int)((kSmemCap - fixed - p.SX * xstage) / span);
@@ -544,7 +577,7 @@ int launch_gemm_ws(const __half* x, const uint32_t* wq, const __half* scales, __
   {
     const uint64_t d[3] = {BK, (uint64_t)M, (uint64_t)(K / BK)};
     const uint64_t s[2] = {(uint64_t)K * 2, BK * 2};
-    const uint32_t b[3] = {BK, (uint32_t)p.NB, 2};
+    const uint32_t b[3] = {BK, (uint32_t)p.NB, (uint32_t)skb};
     if ((rc = make_tmap(&p.tm_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, x, d, s, b, CU_TENSOR_MAP_SWIZZLE_128B))) return rc;
   }
   {

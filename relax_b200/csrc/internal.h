@@ -32,7 +32,7 @@ struct Options {
   int64_t gemm_ws_w_stages = 0; // accepted and kept; the dequantised weights sit in a fixed ring in tensor memory
   int64_t gemm_ws_r_stages = 0; // 0 = auto: cap on the depth of its packed-weight ring (>= 2)
   int64_t gemm_ws_xk = 0;       // accepted and kept (2 or 4); a stage is two K blocks
-  int64_t gemm_ws_max_m = 128; // largest M the automatic dispatch gives to the weight-stationary kernel (0 = never)
+  int64_t gemm_ws_max_m = 128; // largest M the automatic dispatch gives to the weight-stationary kernel (0 = never, 128 = no limit)
 };
 Options& options();
 

@@ -398,9 +398,25 @@ def test_gemm_ws_rejects_what_it_cannot_take(cuda_lib):
 
 @pytest.mark.parametrize("m", [17, 48, 128, 129, 200])
 def test_auto_dispatch_mid_batches(cuda_lib, m):
-    # 16 < M <= 128 goes to the weight-stationary kernel, above that to the prefill kernel; both must agree with the oracle
+    # one and several token tiles of the weight-stationary kernel agree with the oracle
     x, wq, s = synth.make_case(m, 768, 1024, seed=m)
     assert_matmul_close(run_matmul(x, wq, s), x, wq, s, f"auto M={m}")
+    assert cuda_lib.b200_device_error_flags() == 0
+
+
+@pytest.mark.parametrize("ksplit", [0, 1, 8])
+@pytest.mark.parametrize("m,n,k", [(129, 300, 256), (200, 1280, 2048), (193, 129, 4096), (385, 20000, 256), (777, 520, 512)])
+def test_token_tiles(cuda_lib, m, n, k, ksplit):
+    # more than one token tile: the last one shorter than the others (in 8 slices some owners then have no columns),
+    # one or two K blocks per stage, more tiles than clusters
+    x, wq, s = synth.make_case(m, n, k, seed=m + n + k)
+    rows = np.arange(n) if n < 2000 else np.r_[0:130, n - 300:n]
+    try:
+        relax_b200.set_option("gemm.ws_ksplit", ksplit)
+        out = run_matmul(x, wq, s)
+    finally:
+        relax_b200.set_option("gemm.ws_ksplit", 0)
+    assert_matmul_close(np.ascontiguousarray(out[:, rows]), x, wq[rows], s[rows], f"M={m} N={n} K={k} ksplit={ksplit}")
     assert cuda_lib.b200_device_error_flags() == 0
 
 
