@@ -10,6 +10,8 @@
 //
 // All of them are HBM/latency bound and tiny next to the weight streams, except the attention,
 // which reads 2 * ctx * heads * 128 fp16 per sequence.
+#include <type_traits>
+
 #include "internal.h"
 #include "sm100_ptx.cuh"
 
@@ -28,67 +30,127 @@ __device__ __forceinline__ float warp_max(float v) {
   return v;
 }
 
+// Where a kernel lets its successor start (griddepcontrol.launch_dependents): the matmuls read nothing but weights
+// before their own wait, so a kernel in front of one triggers in its first instruction, and the matmul's set-up and
+// first weight loads run beside it.  The kernels in front of the attention, which may read old cache entries and the
+// position before its wait, trigger after their own wait: everything up to the launch before them is then complete.
+
 // y[b,:] = fp16( f32(x) * rsqrt(mean(f32(x)^2) + eps) * f32(w) ); optionally x += delta first (the
-// updated x is written back: it is the residual stream).  One CTA per row, H % 8 == 0.
+// updated x is written back: it is the residual stream).  One CTA per row, H % 8 == 0.  A thread's share of the row,
+// of delta and of w (up to kRmsWords words of 8 values: H <= 8192) is loaded in one go and stays in registers; a longer
+// row makes the trip for w after the statistics, through a copy of x in shared memory.
+constexpr int kRmsWords = 4;
 template <bool kAdd>
 __global__ void __launch_bounds__(256)
 rmsnorm_kernel(__half* __restrict__ x, const __half* __restrict__ delta, const __half* __restrict__ w,
                __half* __restrict__ y, int H, float eps) {
+  ptx::pdl_launch_dependents();
   ptx::pdl_wait();
-  extern __shared__ float xs[];                 // H floats
+  extern __shared__ float xs[];                 // H floats (H > 8192)
   __shared__ float red[8];
   const int b = blockIdx.x;
   __half* xr = x + (int64_t)b * H;
+  const bool one_go = H <= kRmsWords * 256 * 8;
   float ss = 0.f;
-  for (int i = threadIdx.x * 8; i < H; i += blockDim.x * 8) {
-    uint4 v = *reinterpret_cast<const uint4*>(xr + i);
-    __half2* h = reinterpret_cast<__half2*>(&v);
-    float f[8];
+  uint4 v[kRmsWords], wv[kRmsWords];
+  // the residual stream is stored in fp16: round the sum once, then normalise what was stored
+  auto add = [&](uint4& val, const uint4& dv) {
+    __half2* h = reinterpret_cast<__half2*>(&val);
+    const __half2* dh = reinterpret_cast<const __half2*>(&dv);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      float2 t = __half22float2(h[j]);
-      f[2 * j] = t.x;
-      f[2 * j + 1] = t.y;
+      const float2 f = __half22float2(h[j]), t = __half22float2(dh[j]);
+      h[j] = __floats2half2_rn(f.x + t.x, f.y + t.y);
     }
-    if (kAdd) {
-      uint4 dv = *reinterpret_cast<const uint4*>(delta + (int64_t)b * H + i);
-      __half2* dh = reinterpret_cast<__half2*>(&dv);
+  };
+  auto squares = [&](const uint4& val) {
+    const __half2* h = reinterpret_cast<const __half2*>(&val);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 f = __half22float2(h[j]);
+      ss += f.x * f.x;
+      ss += f.y * f.y;
+    }
+  };
+  if (one_go) {
+    uint4 dv[kRmsWords];
+#pragma unroll
+    for (int r = 0; r < kRmsWords; ++r) {
+      const int i = (threadIdx.x + r * 256) * 8;
+      v[r] = wv[r] = dv[r] = make_uint4(0, 0, 0, 0);
+      if (i < H) {
+        v[r] = *reinterpret_cast<const uint4*>(xr + i);
+        if (kAdd) dv[r] = *reinterpret_cast<const uint4*>(delta + (int64_t)b * H + i);
+        wv[r] = *reinterpret_cast<const uint4*>(w + i);
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < kRmsWords; ++r) {
+      const int i = (threadIdx.x + r * 256) * 8;
+      if (i >= H) continue;
+      if (kAdd) {
+        add(v[r], dv[r]);
+        *reinterpret_cast<uint4*>(xr + i) = v[r];
+      }
+      squares(v[r]);
+    }
+  } else {
+    for (int i = threadIdx.x * 8; i < H; i += 256 * 8) {
+      uint4 val = *reinterpret_cast<const uint4*>(xr + i);
+      if (kAdd) {
+        add(val, *reinterpret_cast<const uint4*>(delta + (int64_t)b * H + i));
+        *reinterpret_cast<uint4*>(xr + i) = val;
+      }
+      squares(val);
+      const __half2* h = reinterpret_cast<const __half2*>(&val);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        float2 t = __half22float2(dh[j]);
-        // the residual stream is stored in fp16: round the sum once, then normalise what was stored
-        __half2 r = __floats2half2_rn(f[2 * j] + t.x, f[2 * j + 1] + t.y);
-        h[j] = r;
-        float2 rf = __half22float2(r);
-        f[2 * j] = rf.x;
-        f[2 * j + 1] = rf.y;
+        const float2 f = __half22float2(h[j]);
+        xs[i + 2 * j] = f.x;
+        xs[i + 2 * j + 1] = f.y;
       }
-      *reinterpret_cast<uint4*>(xr + i) = v;
-    }
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      xs[i + j] = f[j];
-      ss += f[j] * f[j];
     }
   }
   ss = warp_sum(ss);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
   __syncthreads();
   float tot = 0.f;
-  for (int i = 0; i < (int)(blockDim.x >> 5); ++i) tot += red[i];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) tot += red[i];
   const float inv = rsqrtf(tot / (float)H + eps);
-  ptx::pdl_launch_dependents();
-  for (int i = threadIdx.x * 8; i < H; i += blockDim.x * 8) {
-    uint4 wv = *reinterpret_cast<const uint4*>(w + i);
-    const __half2* wh = reinterpret_cast<const __half2*>(&wv);
+  auto scaled = [&](const float (&f)[8], const uint4& wr) {
+    const __half2* wh = reinterpret_cast<const __half2*>(&wr);
     uint4 o;
     __half2* oh = reinterpret_cast<__half2*>(&o);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      float2 wf = __half22float2(wh[j]);
-      oh[j] = __floats2half2_rn(xs[i + 2 * j] * inv * wf.x, xs[i + 2 * j + 1] * inv * wf.y);
+      const float2 wf = __half22float2(wh[j]);
+      oh[j] = __floats2half2_rn(f[2 * j] * inv * wf.x, f[2 * j + 1] * inv * wf.y);
     }
-    *reinterpret_cast<uint4*>(y + (int64_t)b * H + i) = o;
+    return o;
+  };
+  if (one_go) {
+#pragma unroll
+    for (int r = 0; r < kRmsWords; ++r) {
+      const int i = (threadIdx.x + r * 256) * 8;
+      if (i >= H) continue;
+      const __half2* h = reinterpret_cast<const __half2*>(&v[r]);
+      float f[8];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 t = __half22float2(h[j]);
+        f[2 * j] = t.x;
+        f[2 * j + 1] = t.y;
+      }
+      *reinterpret_cast<uint4*>(y + (int64_t)b * H + i) = scaled(f, wv[r]);
+    }
+  } else {
+    for (int i = threadIdx.x * 8; i < H; i += 256 * 8) {
+      float f[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f[j] = xs[i + j];
+      *reinterpret_cast<uint4*>(y + (int64_t)b * H + i) = scaled(f, *reinterpret_cast<const uint4*>(w + i));
+    }
   }
 }
 
@@ -100,6 +162,7 @@ rope_kv_append_kernel(const __half* __restrict__ qkv, const float* __restrict__ 
                       const int* __restrict__ pos_ptr, __half* __restrict__ q_out, __half* __restrict__ k_cache,
                       __half* __restrict__ v_cache, int nh, int max_ctx) {
   ptx::pdl_wait();
+  ptx::pdl_launch_dependents();
   const int h = blockIdx.x, b = blockIdx.y, i = threadIdx.x;
   const int pos = pos_ptr[0];
   const float c = cos_t[(int64_t)pos * 64 + i], s = sin_t[(int64_t)pos * 64 + i];
@@ -117,7 +180,6 @@ rope_kv_append_kernel(const __half* __restrict__ qkv, const float* __restrict__ 
   k_cache[slot + i + 64] = __float2half_rn(k1 * c + k0 * s);
   v_cache[slot + i] = v[i];
   v_cache[slot + i + 64] = v[i + 64];
-  ptx::pdl_launch_dependents();
 }
 
 // Single-query attention, split over the context: CTA (split, head, batch) handles tokens
@@ -402,18 +464,20 @@ attn_decode_fused_kernel(const __half* __restrict__ qkv, const float* __restrict
 __global__ void __launch_bounds__(128)
 attn_decode_combine_kernel(const float* __restrict__ scratch, const int* __restrict__ pos_ptr, __half* __restrict__ out,
                            int nh, int nsplit) {
+  ptx::pdl_launch_dependents();
   ptx::pdl_wait();
   const int h = blockIdx.x, b = blockIdx.y, d = threadIdx.x;
   const int ctx = pos_ptr[0] + 1;
   const int used = (ctx + kAttnChunk - 1) / kAttnChunk;
   const float* p = scratch + ((int64_t)b * nh + h) * nsplit * 130;
-  // sixteen chunks per round, all 48 loads of a round issued together (the partials sit in L2), one
-  // online-softmax update per round
+  // R chunks per round, all 3 R loads of a round issued together (the partials sit in L2), one online-softmax update
+  // per round: sixteen, or eight where no more are in use (half of the loads would be repeats)
   float M = -INFINITY, L = 0.f, A = 0.f;
-  for (int s0 = 0; s0 < used; s0 += 16) {
-    float Ms[16], Ls[16], As[16];
+  auto round = [&](auto tag, int s0) {
+    constexpr int R = decltype(tag)::value;
+    float Ms[R], Ls[R], As[R];
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
+    for (int j = 0; j < R; ++j) {
       const int si = min(s0 + j, used - 1);
       Ms[j] = p[si * 130];
       Ls[j] = p[si * 130 + 1];
@@ -421,13 +485,13 @@ attn_decode_combine_kernel(const float* __restrict__ scratch, const int* __restr
     }
     float Mn = M;
 #pragma unroll
-    for (int j = 0; j < 16; ++j)
+    for (int j = 0; j < R; ++j)
       if (s0 + j < used) Mn = fmaxf(Mn, Ms[j]);
     const float corr = exp2f(M - Mn);            // first round: exp2f(-inf) = 0
     L *= corr;
     A *= corr;
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
+    for (int j = 0; j < R; ++j) {
       if (s0 + j < used) {
         const float f = exp2f(Ms[j] - Mn);
         L += Ls[j] * f;
@@ -435,14 +499,17 @@ attn_decode_combine_kernel(const float* __restrict__ scratch, const int* __restr
       }
     }
     M = Mn;
-  }
-  ptx::pdl_launch_dependents();
+  };
+  if (used <= 8) round(std::integral_constant<int, 8>{}, 0);
+  else
+    for (int s0 = 0; s0 < used; s0 += 16) round(std::integral_constant<int, 16>{}, s0);
   out[((int64_t)b * nh + h) * 128 + d] = __float2half_rn(A / L);
 }
 
 // out[b,i] = fp16( silu(f32(g)) * f32(u) ), gu row = [gate (I) | up (I)].  I % 8 == 0.
 __global__ void __launch_bounds__(256)
 silu_mul_kernel(const __half* __restrict__ gu, __half* __restrict__ out, int I, int64_t total8) {
+  ptx::pdl_launch_dependents();
   ptx::pdl_wait();
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= total8) return;
@@ -462,7 +529,6 @@ silu_mul_kernel(const __half* __restrict__ gu, __half* __restrict__ out, int I, 
     float c = g.y / (1.f + __expf(-g.y)) * u.y;
     oh[j] = __floats2half2_rn(a, c);
   }
-  ptx::pdl_launch_dependents();
   *reinterpret_cast<uint4*>(out + b * I + i) = o;
 }
 
@@ -521,9 +587,9 @@ int b200_rmsnorm(void* x, const void* delta, const void* w, void* y, int64_t B, 
   if (rc) return rc;
   auto s = static_cast<cudaStream_t>(stream);
   if (delta)
-    return launch("add_rmsnorm", rmsnorm_kernel<true>, dim3((unsigned)B), dim3(256), (size_t)H * 4, s, (__half*)x,
+    return launch("add_rmsnorm", rmsnorm_kernel<true>, dim3((unsigned)B), dim3(256), H > kRmsWords * 256 * 8 ? (size_t)H * 4 : 0, s, (__half*)x,
                   (const __half*)delta, (const __half*)w, (__half*)y, (int)H, eps);
-  return launch("rmsnorm", rmsnorm_kernel<false>, dim3((unsigned)B), dim3(256), (size_t)H * 4, s, (__half*)x,
+  return launch("rmsnorm", rmsnorm_kernel<false>, dim3((unsigned)B), dim3(256), H > kRmsWords * 256 * 8 ? (size_t)H * 4 : 0, s, (__half*)x,
                 (const __half*)nullptr, (const __half*)w, (__half*)y, (int)H, eps);
 }
 

@@ -514,7 +514,9 @@ int launch_gemm_ws(const __half* x, const uint32_t* wq, const __half* scales, __
   int ksplit = 1, nb16 = 0;
   int64_t best = 0;
   const int64_t mt0 = (M + kMaxNB - 1) / kMaxNB;
-  for (int64_t mt = mt0; mt <= mt0 + mt0 / 2 + 3 && (mt == mt0 || mt * 16 <= M); ++mt) {
+  // (up to 128 rows the weights stream once: one token tile)
+  const int64_t mt_max = M <= 128 ? 1 : mt0 + mt0 / 2 + 3;
+  for (int64_t mt = mt0; mt <= mt_max; ++mt) {
     const int nb = (int)(((M + mt - 1) / mt + 15) / 16) * 16;
     const int64_t tiles = row_tiles * ((M + nb - 1) / nb);
     for (int c = 1; c <= 8 && c <= units; c *= 2) {
