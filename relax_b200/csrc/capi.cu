@@ -186,15 +186,18 @@ using namespace b200;
 
 // Small host transfers as kernels.  A copy-engine transfer on either side of a 5 us matmul costs
 // more than the matmul (each switch between the copy engine and the SMs is a few microseconds), so
-// activations and results up to kHostKernelBytes travel by a one-CTA-per-16-KB kernel that reads or
-// writes the pinned host buffer through its device mapping; the result copy is launched as a
-// programmatic dependent of the matmul.  Pageable host memory and larger transfers use cudaMemcpyAsync.
+// activations and results up to kHostKernelBytes travel by a kernel that reads or writes the pinned host
+// buffer through its device mapping: 16 bytes per thread and one CTA per 4 KB, so that a read makes one round trip
+// over the bus however many bytes it moves.  The copy lets the matmul start beside it (the matmul reads only weights
+// before its own wait), and the result copy is launched as a programmatic dependent of the matmul.  Pageable host
+// memory and larger transfers use cudaMemcpyAsync.
 namespace b200 {
 namespace {
 constexpr size_t kHostKernelBytes = 256 * 1024;
 
 __global__ void __launch_bounds__(256) host_copy_kernel(const unsigned char* __restrict__ src, unsigned char* __restrict__ dst,
                                                         size_t bytes, int wait_for_primary) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (wait_for_primary) asm volatile("griddepcontrol.wait;" ::: "memory");
   const size_t n16 = bytes >> 4;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n16; i += (size_t)gridDim.x * blockDim.x)
@@ -218,7 +221,7 @@ void* mapped_host_pointer(const void* host) {
 // of the kernel before it in the stream (the copy waits for that kernel's completion itself).
 int host_copy(const void* src, void* dst, size_t bytes, bool dependent, cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)((bytes + 16383) / 16384));
+  cfg.gridDim = dim3((unsigned)((bytes + 4095) / 4096));
   cfg.blockDim = dim3(256);
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
