@@ -126,12 +126,20 @@ int matmul_impl(Family fam, const char* who, const void* x, const void* wq, cons
   // N = 1280, K = 8192 6.6 / 5.9, 9.7 / 6.0, 17.0 / 6.1 (the skinny kernel stages all of x in every CTA, and its
   // arithmetic grows from 8 columns on).  At 5..8 rows and a shorter K the skinny kernel is the better one inside a
   // decode step, where two of its CTAs fit an SM and it starts beside the kernel before it (8 layers of hidden
-  // 2048 at 5 rows: 413 us with it, 440 without).  Above 128 rows it cuts the
-  // tokens into tiles to suit the shape; the prefill kernel with its 256-token tiles is left with the K that are not
-  // multiples of 256 (47.0 against 12.3 us at M = 129, N = K = 4096, 163 against 137 at M = 2048, N = 11008).  The
-  // option's largest value, 128, stands for no limit.  (A variant of the skinny kernel asked for by option keeps its rows.)
-  if (fam == kGemmWs || (fam == kAuto && (M >= 9 || (M >= 5 && K >= 8192)) && (M <= options().gemm_ws_max_m || options().gemm_ws_max_m == 128) && (M > 16 || options().gemv_variant == 0))) {
-    rc = fam == kGemmWs && M > 128 ? B200_ENOTREADY : launch_gemm_ws(xh, wh, sh, yh, M, N, K, s);
+  // 2048 at 5 rows: 413 us with it, 440 without).  Above 128 rows it cuts the tokens into tiles to suit the shape; the
+  // prefill kernel with its 256-token tiles has no shape left where it is faster (47.0 against 12.3 us at M = 129,
+  // N = K = 4096, 163 against 137 at M = 2048, N = 11008) and serves its own entry point.
+  // Where K is not a multiple of 256 (or the scales are not 16-byte aligned) the other choice up to 16 rows is the
+  // register-streaming kernel, whose time grows with the rows: it keeps one row and small products, M * N * K < 50 M
+  // (streaming / weight-stationary in us: 4 x 4096 x 2080 5.1 / 5.3, 16 x 1024 x 1056 4.5 / 4.5, 2 x 8640 x 3200 11.0 /
+  // 11.0, 3 x 8640 x 3200 13.8 / 11.0, 8 x 4096 x 2080 7.0 / 5.5, 16 x 22016 x 4128 86 / 24; above 16 rows, against the
+  // prefill kernel, 32 x 8640 x 3200 43 / 11.5, 2048 x 11008 x 4128 188 / 159).
+  // The option's largest value, 128, stands for no limit.  (A variant of the skinny kernel asked for by option keeps its rows.)
+  const bool ragged = K % 256 != 0 || !aligned16(scales);
+  const bool ws_auto = M > 16 || (ragged ? M >= 2 && M * N * K >= 50000000 : M >= 9 || (M >= 5 && K >= 8192));
+  if (fam == kGemmWs || (fam == kAuto && ws_auto && (M <= options().gemm_ws_max_m || options().gemm_ws_max_m == 128) &&
+                         (M > 16 || options().gemv_variant == 0))) {
+    rc = fam == kGemmWs && (M > 128 || ragged) ? B200_ENOTREADY : launch_gemm_ws(xh, wh, sh, yh, M, N, K, s);
     if (rc != B200_ENOTREADY) return rc;
     if (fam == kGemmWs) return fail(B200_EINVAL, "%s: the weight-stationary kernel takes 1 <= M <= 128, K %% 256 == 0, 16-byte aligned scales", who);
   }

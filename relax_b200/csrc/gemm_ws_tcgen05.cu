@@ -1,5 +1,4 @@
-// q4f16 matmul on the 5th-generation tensor cores (K a multiple of 256; the dispatcher gives it 9 rows and more, and
-// 5..8 with a long K): y[M,N] = x[M,K] . decode(Wq,S)^T.
+// q4f16 matmul on the 5th-generation tensor cores (the dispatcher gives it 9 rows and more, and 5..8 with a long K): y[M,N] = x[M,K] . decode(Wq,S)^T.
 //
 // Decode at batches up to 128 is still bound by streaming the weights once, so the roles of a plain GEMM are swapped:
 // the MMA's M dimension is 128 WEIGHT rows (A operand), its N dimension are tokens (B operand = x, 16..192 columns).
@@ -79,6 +78,7 @@ struct WsParams {
   CUtensorMap tm_w;    // uint32 {K/8, N},         box {32, 128},      SWIZZLE_128B: [row][128 B] (whole lines: 64-byte pieces
                        //                                                    halve the rate the weights arrive at)
   CUtensorMap tm_s;    // fp16   {K/32, N},        box {8, 128}
+  const __half* scales;
   __half* y;
   int M, N, K;
   int NB;              // batch columns of the MMA: M rounded up to 16 (32 with 8 slices)
@@ -139,9 +139,12 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const void* tmap, in
 // inbox [ksplit source ranks][cw / 4][128 rows][4 columns] fp32 (ksplit > 1; a warp's 16-byte stores are then 512
 // contiguous bytes: with rows 80 bytes apart, so 16-byte pieces on the SM-to-SM network, the exchange of a tile of 64
 // columns took 3900 clocks instead of 1400) | barriers.
-// PAIRED: nibble order of the packed words (q4_common.cuh).  SKB: K blocks per x stage and A slot: 2 up to 128 batch
+// PAIRED: nibble order of the packed words (q4_common.cuh).  RAGGED: K is not a multiple of 256, or the scales are not
+// 16-byte aligned, so that the scales' rows cannot be a tensor map's: the dequantisers then read their scales from global
+// memory one trip ahead, and x comes one K block per load through a map that ends at K.  What lies past K is zero
+// on both sides (packed words, scales and x).  SKB: K blocks per x stage and A slot: 2 up to 128 batch
 // columns (fewer waits and arrivals), 1 above (tensor memory holds two accumulators of 192 columns and four slots of 32).
-template <bool PAIRED, int SKB>
+template <bool PAIRED, int SKB, bool RAGGED>
 __global__ void __launch_bounds__(kNumThreads, 1)
 q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
   extern __shared__ unsigned char smem_unaligned[];
@@ -162,7 +165,7 @@ q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
   const int krank = (int)cluster.block_rank();          // K slice of this CTA (gridDim.x == ksplit)
   const int tile0 = blockIdx.y, tstep = gridDim.y;
   // 256-k spans, the first slices one span longer (every slice has at least one)
-  const int units = p.K >> 8;
+  const int units = (p.K + 255) >> 8;
   const int ubase = units / p.ksplit, uextra = units % p.ksplit;
   const int span0 = krank * ubase + min(krank, uextra);
   const int nspans = ubase + (krank < uextra ? 1 : 0);
@@ -180,13 +183,15 @@ q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
   if (tid == 64) {
     // The weights depend on nothing: the thread that will stream them sets up the packed ring's barriers itself
     // and fills the ring at once, ahead of the rest of the set-up (barriers, TMEM allocation, the cluster-wide sync).
-    for (int i = 0; i < p.SR; ++i) { mbar_init(&bar.r_full[i], 2); mbar_init(&bar.r_empty[i], kDequantWarps / SKB); }
+    for (int i = 0; i < p.SR; ++i) { mbar_init(&bar.r_full[i], RAGGED ? 1 : 2); mbar_init(&bar.r_empty[i], kDequantWarps / SKB); }
     mbar_fence_init();
     for (int i = 0; i < p.SR && i < nspans; ++i) {
       mbar_arrive_expect_tx(&bar.r_full[i], kRawBytes);
       tma_load_2d(raw_ring + (size_t)i * kRawBytes, &p.tm_w, (span0 + i) * 32, tile0 / p.mt * BR, &bar.r_full[i]);
-      mbar_arrive_expect_tx(&bar.r_full[i], kScBytes);
-      tma_load_2d(sc_ring + (size_t)i * kScBytes, &p.tm_s, (span0 + i) * 8, tile0 / p.mt * BR, &bar.r_full[i]);
+      if (!RAGGED) {
+        mbar_arrive_expect_tx(&bar.r_full[i], kScBytes);
+        tma_load_2d(sc_ring + (size_t)i * kScBytes, &p.tm_s, (span0 + i) * 8, tile0 / p.mt * BR, &bar.r_full[i]);
+      }
     }
   }
   if (warp == 1) {
@@ -213,14 +218,20 @@ q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
           // (not a sleeping wait: a nanosleep lasts far longer than the time a stage takes)
           if (rx.wrapped) wait_or_abort(&bar.x_empty[rx.s], rx.phase ^ 1, abort_flag, 1);
           mbar_arrive_expect_tx(&bar.x_full[rx.s], xstage);
-          tma_load_3d(x_ring + (size_t)rx.s * xstage, &p.tm_x, 0, tok0, span0 * 4 + SKB * u, &bar.x_full[rx.s]);
+          if (RAGGED) {
+#pragma unroll
+            for (int j = 0; j < SKB; ++j)
+              tma_load_2d(x_ring + (size_t)rx.s * xstage + j * p.NB * 128, &p.tm_x, (span0 * 4 + SKB * u + j) * BK, tok0, &bar.x_full[rx.s]);
+          } else {
+            tma_load_3d(x_ring + (size_t)rx.s * xstage, &p.tm_x, 0, tok0, span0 * 4 + SKB * u, &bar.x_full[rx.s]);
+          }
         }
         if (p.x_resident) break;                      // one trip: the stages stay
       }
     }
   } else if (warp == 2 || warp == 3) {
     // ------------------------------------------------------------------ TMA producers: packed weights (warp 2), scales (warp 3), 256 k per load
-    if (lane == 0) {
+    if (lane == 0 && !(RAGGED && warp == 3)) {
       const int first = min(p.SR, nspans);            // requested during set-up
       Ring rr;
       for (int tile = tile0; tile < p.tiles; tile += tstep) {
@@ -303,6 +314,21 @@ q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
     const uint32_t first = SKB == 2 ? (uint32_t)(grp >> 1) : 0;
     int s = (int)first;                        // ring slot (the ring's depth is even: with SKB = 2 a group stays on slots of its parity)
     uint32_t phase = 0, use = 0;
+    const int groups = p.K >> 5;
+    auto global_scales = [&](uint32_t i, uint32_t (&out)[SKB]) {       // of the span with running index i
+      const int row = (tile0 + (int)(i / (uint32_t)nspans) * tstep) / p.mt * BR + r;
+      const int g0 = (span0 + (int)(i % (uint32_t)nspans)) * 8 + 2 * SKB * part;
+      const __half* src = p.scales + (int64_t)row * groups + g0;
+#pragma unroll
+      for (int j = 0; j < SKB; ++j) {
+        uint32_t lo = 0, hi = 0;
+        if (i < total && row < p.N && g0 + 2 * j < groups) lo = __half_as_ushort(__ldg(src + 2 * j));
+        if (i < total && row < p.N && g0 + 2 * j + 1 < groups) hi = __half_as_ushort(__ldg(src + 2 * j + 1));
+        out[j] = lo | (hi << 16);
+      }
+    };
+    uint32_t next_sc[SKB];
+    if (RAGGED) global_scales(first, next_sc);
     for (uint32_t sidx = first; sidx < total; sidx += SKB, ++use) {
       wait_or_abort(&bar.r_full[s], phase, abort_flag, 8);
       const unsigned char* rbase = raw_ring + (size_t)s * kRawBytes;
@@ -312,7 +338,8 @@ q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
       for (int j = 0; j < 2 * SKB; ++j) pk[j] = *reinterpret_cast<const uint4*>(rbase + off[j]);
 #pragma unroll
       for (int j = 0; j < SKB; ++j)
-        scw[j] = *reinterpret_cast<const uint32_t*>(sc_ring + (size_t)s * kScBytes + r * 16 + (SKB * part + j) * 4);
+        scw[j] = RAGGED ? next_sc[j] : *reinterpret_cast<const uint32_t*>(sc_ring + (size_t)s * kScBytes + r * 16 + (SKB * part + j) * 4);
+      if (RAGGED) global_scales(sidx + SKB, next_sc);
 #pragma unroll
       for (int j = 0; j < 2 * SKB; ++j) pin_loaded(pk[j]);
 #pragma unroll
@@ -449,10 +476,12 @@ q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
 }
 
 using WsKernel = void (*)(const WsParams);
-WsKernel kernel_for(int nb, bool paired) {
-  return nb <= 128 ? (paired ? q4f16_gemm_ws_tcgen05_kernel<true, 2> : q4f16_gemm_ws_tcgen05_kernel<false, 2>)
-                   : (paired ? q4f16_gemm_ws_tcgen05_kernel<true, 1> : q4f16_gemm_ws_tcgen05_kernel<false, 1>);
+template <bool RAGGED>
+WsKernel kernel_of(int nb, bool paired) {
+  return nb <= 128 ? (paired ? q4f16_gemm_ws_tcgen05_kernel<true, 2, RAGGED> : q4f16_gemm_ws_tcgen05_kernel<false, 2, RAGGED>)
+                   : (paired ? q4f16_gemm_ws_tcgen05_kernel<true, 1, RAGGED> : q4f16_gemm_ws_tcgen05_kernel<false, 1, RAGGED>);
 }
+WsKernel kernel_for(int nb, bool paired, bool ragged) { return ragged ? kernel_of<true>(nb, paired) : kernel_of<false>(nb, paired); }
 
 constexpr size_t kSmemCap = 227 * 1024;
 // More than half of an SM: one such CTA per SM, whatever its rings would need.  (It takes all of tensor memory; two
@@ -493,13 +522,15 @@ int max_clusters(int ksplit, const void* kern) {
 // Returns B200_ENOTREADY when the shape is outside what this kernel takes.
 int launch_gemm_ws(const __half* x, const uint32_t* wq, const __half* scales, __half* y, int64_t M, int64_t N,
                    int64_t K, cudaStream_t stream) {
-  if (M < 1 || K % 256 != 0 || K < 256 || (reinterpret_cast<uintptr_t>(scales) & 15u)) return B200_ENOTREADY;
+  if (M < 1 || K < 32 || K % 32 != 0) return B200_ENOTREADY;
+  const bool ragged = K % 256 != 0 || (reinterpret_cast<uintptr_t>(scales) & 15u) != 0;
   WsParams p;
   int rc;
   const bool paired = current_layout() == kLayoutPaired;
+  p.scales = scales;
   p.y = y;
   p.M = (int)M; p.N = (int)N; p.K = (int)K;
-  const int units = (int)(K / 256);
+  const int units = (int)((K + 255) / 256);
   const int64_t row_tiles = (N + BR - 1) / BR;
   if (row_tiles * ((M + 15) / 16) > 0x3fffffff) return B200_ENOTREADY;      // (tile numbers are 32-bit)
   // Token tiles and K slices: a model of the time in nanoseconds, fitted to measurements at N = 4096, 12288 and 22016,
@@ -521,7 +552,7 @@ int launch_gemm_ws(const __half* x, const uint32_t* wq, const __half* scales, __
     const int64_t tiles = row_tiles * ((M + nb - 1) / nb);
     for (int c = 1; c <= 8 && c <= units; c *= 2) {
       if (forced > 0 && !(c <= forced && (c * 2 > forced || c * 2 > units || c == 8))) continue;
-      const int nc = max_clusters(c, reinterpret_cast<const void*>(kernel_for(nb, paired)));
+      const int nc = max_clusters(c, reinterpret_cast<const void*>(kernel_for(nb, paired, ragged)));
       const int64_t rounds = (tiles + nc - 1) / nc;
       const int64_t busy = tiles * c / rounds;                                   // CTAs at work, on average
       const int64_t l2 = busy * (nb * 512 + kRawBytes + kScBytes) / 14000;
@@ -535,7 +566,7 @@ int launch_gemm_ws(const __half* x, const uint32_t* wq, const __half* scales, __
     }
   }
   const int skb = nb16 <= 128 ? 2 : 1;
-  auto kern = kernel_for(nb16, paired);
+  auto kern = kernel_for(nb16, paired, ragged);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemCap);
   if (e != cudaSuccess) return fail(B200_ELAUNCH, "gemm_ws: cudaFuncSetAttribute(%zu): %s", kSmemCap, cudaGetErrorString(e));
   // an owner's columns are exchanged four at a time
@@ -576,7 +607,12 @@ int launch_gemm_ws(const __half* x, const uint32_t* wq, const __half* scales, __
   size_t smem = fixed + p.SX * xstage + p.SR * span;
   if (smem < kSmemFloor) smem = kSmemFloor;
 
-  {
+  if (ragged) {
+    const uint64_t d[2] = {(uint64_t)K, (uint64_t)M};
+    const uint64_t s[1] = {(uint64_t)K * 2};
+    const uint32_t b[2] = {BK, (uint32_t)p.NB};
+    if ((rc = make_tmap(&p.tm_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, x, d, s, b, CU_TENSOR_MAP_SWIZZLE_128B))) return rc;
+  } else {
     const uint64_t d[3] = {BK, (uint64_t)M, (uint64_t)(K / BK)};
     const uint64_t s[2] = {(uint64_t)K * 2, BK * 2};
     const uint32_t b[3] = {BK, (uint32_t)p.NB, (uint32_t)skb};
@@ -588,7 +624,7 @@ int launch_gemm_ws(const __half* x, const uint32_t* wq, const __half* scales, __
     const uint32_t b[2] = {32, BR};
     if ((rc = make_tmap(&p.tm_w, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, wq, d, s, b, CU_TENSOR_MAP_SWIZZLE_128B))) return rc;
   }
-  {
+  if (!ragged) {
     const uint64_t d[2] = {(uint64_t)(K / 32), (uint64_t)N};
     const uint64_t s[1] = {(uint64_t)(K / 32) * 2};
     const uint32_t b[2] = {8, BR};

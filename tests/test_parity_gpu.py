@@ -420,6 +420,35 @@ def test_token_tiles(cuda_lib, m, n, k, ksplit):
     assert cuda_lib.b200_device_error_flags() == 0
 
 
+@pytest.mark.parametrize("layout", [None, "paired"])
+@pytest.mark.parametrize("m,n,k,ksplit", [(17, 300, 32, 0), (20, 129, 96, 0), (17, 600, 3200, 0), (17, 600, 3200, 8), (200, 300, 2080, 4),
+                                          (777, 130, 544, 0), (5, 4000, 2528, 0)])
+def test_k_not_a_multiple_of_256(cuda_lib, m, n, k, ksplit, layout):
+    # the last span ends inside K: the scales come from global memory, and the values behind a row of x (here NaN behind
+    # the last one) must not reach the sum
+    x, wq, s = synth.make_case(m, n, k, seed=m + n + k)
+    tx = torch.full((m + 1, k), float("nan"), dtype=torch.float16, device="cuda")
+    tx[:m] = torch.from_numpy(x).cuda()
+    twq, ts = dev(wq, s)
+    try:
+        relax_b200.set_option("gemm.ws_ksplit", ksplit)
+        out = ops.q4f16_matmul(tx[:m], ops.q4f16_repack(twq, layout) if layout else twq, ts, layout=layout).cpu().numpy()
+    finally:
+        relax_b200.set_option("gemm.ws_ksplit", 0)
+    assert_matmul_close(out, x, wq, s, f"M={m} N={n} K={k} ksplit={ksplit}")
+    assert cuda_lib.b200_device_error_flags() == 0
+
+
+def test_unaligned_scales_mid_batch(cuda_lib):
+    x, wq, s = synth.make_case(40, 300, 1024, seed=5)
+    tx, twq, ts = dev(x, wq, s)
+    buf = torch.zeros(ts.numel() + 1, dtype=torch.float16, device="cuda")
+    shifted = buf[1:].view_as(ts)
+    shifted.copy_(ts)
+    assert_matmul_close(ops.q4f16_matmul(tx, twq, shifted).cpu().numpy(), x, wq, s, "scales two bytes off")
+    assert cuda_lib.b200_device_error_flags() == 0
+
+
 @pytest.mark.parametrize("m,n,k", [(9, 512, 11008), (16, 1280, 8192), (12, 300, 16384)])
 def test_auto_dispatch_small_batch_long_k(cuda_lib, m, n, k):
     # 9..16 rows whose x block does not fit beside the skinny kernel's ring go to the weight-stationary kernel
