@@ -408,8 +408,8 @@ def run_decode(args, world, rank, dev, batches):
 # summarised under profiles/ (one capture per kernel change; not re-measured by this script).
 NCU_TRAFFIC_BYTES = {
     ("gemv", 1, 4096, 4096): (9476352, "profiles/gemv_pipe_kernel__decode_gemv_M1_N4096_K4096.md (ncu capture, not re-measured by this run)"),
-    ("gemv", 64, 4096, 4096): (10006272, "profiles/gemm_ws_tcgen05_kernel__mid_batch_M64_N4096_K4096.md (ncu capture, not re-measured by this run)"),
-    ("prefill", 2048, 11008, 4096): (42236416 + 2993664, "profiles/gemm_tcgen05_kernel__prefill_M2048_N11008_K4096.md (ncu capture, not re-measured by this run)"),
+    ("gemv", 64, 4096, 4096): (10000384, "profiles/gemm_ws_tcgen05_kernel__M64_and_prefill.md (ncu capture, not re-measured by this run)"),
+    ("prefill", 2048, 11008, 4096): (42176768 + 12126976, "profiles/gemm_ws_tcgen05_kernel__M64_and_prefill.md (ncu capture, not re-measured by this run)"),
 }
 
 
@@ -536,7 +536,7 @@ def measure_matmul(args, workload, world, rank, dev, steps, warmup, reps, with_c
         roofline = {"bound": "tensor", "achieved": achieved, "peak": peaks["tflops"], "unit": "TFLOP/s",
                     "frac": achieved / peaks["tflops"], "frac_of_sustained": achieved / peaks["tflops_sustained"],
                     "frac_of_nominal_2250": achieved / 2250.0, "traffic": traffic, "traffic_source": traffic_source,
-                    "peak_source": peaks["source"], "kernel": "q4f16_gemm_tcgen05_kernel", "us_per_launch": us_per_launch,
+                    "peak_source": peaks["source"], "kernel": "q4f16_gemm_ws_tcgen05_kernel", "us_per_launch": us_per_launch,
                     "us_x_sm_mhz": us_per_launch * sm_mhz if sm_mhz else None,
                     "algorithmic_flops_per_launch": flops}
     cpu = None
