@@ -177,7 +177,7 @@ q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
     for (int i = 0; i < kASlots; ++i) { mbar_init(&bar.a_full[i], 4); mbar_init(&bar.a_empty[i], 1); }
     for (int i = 0; i < 2; ++i) { mbar_init(&bar.acc_full[i], 1); mbar_init(&bar.acc_empty[i], 8); }
     mbar_init(&bar.inbox_full, 1);
-    mbar_init(&bar.inbox_free, p.ksplit > 1 ? 8 * (p.ksplit - 1) : 1);
+    mbar_init(&bar.inbox_free, 8 * p.ksplit);         // the epilogue warps of every CTA of the cluster, this one's too
     mbar_fence_init();
   }
   if (tid == 64) {
@@ -390,10 +390,12 @@ q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
       const int ntok4 = (ntok + 3) & ~3;               // columns that are exchanged
       const int own = max(0, min(p.cw, ntok4 - krank * p.cw));     // columns that this CTA adds up and stores
       __half* yt = p.y + (int64_t)tok0 * p.N + row;
-      // the owners have read what this CTA sent for the tile before
+      // The owners have read what this CTA sent for the tile before.  This CTA is an owner itself: the two warps of a
+      // quadrant send and sum different columns of the same rows, so without its own eight warps among the arrivals
+      // the faster of the two could overwrite what the slower one has yet to add up.
       if (p.ksplit > 1 && it > 0) wait_or_abort_cluster(&bar.inbox_free, (it - 1) & 1, abort_flag, 12);
       // (a phase of inbox_full ends with the bytes of all ranks; the next one cannot end before every warp here
-      // has told the peers that it is done with this one)
+      // has told all ranks that it is done with this one)
       if (p.ksplit > 1 && own > 0 && warp == 4 && lane == 0) mbar_arrive_expect_tx(&bar.inbox_full, (uint32_t)(p.ksplit * BR * own * 4));
       wait_or_abort(&bar.acc_full[buf], (it >> 1) & 1, abort_flag, 7);
       tc_fence_after_sync();
@@ -453,7 +455,7 @@ q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
       }
       // Not after the last tile: the arrival's release would wait for the stores to y.
       __syncwarp();
-      if (tile + tstep < p.tiles && lane < p.ksplit && lane != krank) mbar_arrive_cluster(map_to_rank(free_addr, lane));
+      if (tile + tstep < p.tiles && lane < p.ksplit) mbar_arrive_cluster(map_to_rank(free_addr, lane));
     }
   }
 

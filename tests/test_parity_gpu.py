@@ -420,6 +420,28 @@ def test_token_tiles(cuda_lib, m, n, k, ksplit):
     assert cuda_lib.b200_device_error_flags() == 0
 
 
+@pytest.mark.parametrize("ksplit", [2, 4, 8])
+@pytest.mark.parametrize("m", [64, 200])
+def test_partial_tile_exchange_repeats_bit_for_bit(cuda_lib, m, ksplit):
+    # one 256-k span per slice, so a tile's accumulator is ready soon after the one before; more tiles than clusters, so
+    # every inbox is refilled again and again; at 200 rows the last token tile is short (some owners have no columns)
+    n, k = 150 * 128 + 8, 256 * ksplit
+    x, wq, s = synth.make_case(m, n, k, seed=m + ksplit)
+    tx, twq, ts = dev(x, wq, s)
+    outs = torch.empty((60, m, n), dtype=torch.float16, device="cuda")
+    try:
+        relax_b200.set_option("gemm.ws_ksplit", ksplit)
+        for out in outs:
+            ops.q4f16_matmul(tx, twq, ts, out=out)
+    finally:
+        relax_b200.set_option("gemm.ws_ksplit", 0)
+    sample = np.r_[0:130, 9000:9020, n - 140:n]
+    assert_matmul_close(np.ascontiguousarray(outs[0].cpu().numpy()[:, sample]), x, wq[sample], s[sample], f"M={m} ksplit={ksplit}")
+    bits = outs.view(torch.int16)
+    assert [i for i in range(1, 60) if not torch.equal(bits[i], bits[0])] == []
+    assert cuda_lib.b200_device_error_flags() == 0
+
+
 @pytest.mark.parametrize("layout", [None, "paired"])
 @pytest.mark.parametrize("m,n,k,ksplit", [(17, 300, 32, 0), (20, 129, 96, 0), (17, 600, 3200, 0), (17, 600, 3200, 8), (200, 300, 2080, 4),
                                           (777, 130, 544, 0), (5, 4000, 2528, 0)])
