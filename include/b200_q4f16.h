@@ -308,6 +308,16 @@ B200_API int b200_decode_layer(const B200DecodeLayer* layer, void* cuda_stream);
 B200_API int b200_rmsnorm(void* x, const void* delta, const void* w, void* y, int64_t B, int64_t H, float eps,
                           void* cuda_stream);
 
+/* Early-release forms.  b200_rmsnorm, b200_silu_mul and the merge inside b200_attn_decode let the next programmatic
+ * dependent launch begin once everything in front of them is complete (griddepcontrol.wait, then
+ * griddepcontrol.launch_dependents).  The three *_early_release entry points compute the same and let it begin
+ * in their first instruction, so that the set-up and first weight loads of a matmul of this library behind them run
+ * beside them.  Use one only where the next launch reads nothing before its own wait that an earlier launch of the
+ * stream may still be writing: the q4f16 matmuls qualify (they read weights and scales early), and so do the glue
+ * kernels, which wait first; an attention with B200_ATTN_EARLY_KV_LOADS does not. */
+B200_API int b200_rmsnorm_early_release(void* x, const void* delta, const void* w, void* y, int64_t B, int64_t H, float eps,
+                                        void* cuda_stream);
+
 /* Rotary embedding of q and k (pairs i, i+64 of a 128-wide head; cos/sin fp32 [max_pos,64]), then k
  * and v are stored in the caches at position *pos.  qkv fp16 [B, 3*nh*128] = [q | k | v];
  * q_out fp16 [B, nh, 128]; caches fp16 [B, max_ctx, nh, 128]. */
@@ -330,8 +340,10 @@ B200_API int b200_rope_kv_append(const void* qkv, const void* cos_t, const void*
  *   (1) the launch directly in front of this call writes neither *pos nor a cache entry below *pos, and
  *       it is either not a programmatic-dependent launch or one that executes griddepcontrol.wait before
  *       griddepcontrol.launch_dependents (b200_rope_kv_append, b200_rmsnorm, b200_silu_mul,
- *       b200_embed_rows and b200_advance_pos of this library do; the q4f16 matmul entry points do NOT:
- *       they release their dependents first, so with one of them directly in front, leave the flag clear);
+ *       the ordinary attention entry points, b200_embed_rows and b200_advance_pos of this library do; the
+ *       q4f16 matmul entry points, b200_lm_head, b200_decode_layer, the sums over ranks and the
+ *       *_early_release forms do NOT: they release their dependents first, so with one of them directly in
+ *       front, leave the flag clear);
  *   (2) whatever last wrote *pos or those cache entries was launched before that launch.
  * The entry at *pos itself and q may be written by the launch directly in front (that is what
  * b200_rope_kv_append does; the decode engine of this repository calls it there and sets the flag). */
@@ -339,6 +351,10 @@ B200_API int b200_rope_kv_append(const void* qkv, const void* cos_t, const void*
 B200_API int64_t b200_attn_decode_scratch_bytes(int64_t B, int64_t nh, int64_t max_ctx);
 B200_API int b200_attn_decode(const void* q, const void* k_cache, const void* v_cache, const void* pos, void* out,
                               void* scratch, int64_t B, int64_t nh, int64_t max_ctx, uint32_t flags, void* cuda_stream);
+/* The same; the merge is an early-release form (see b200_rmsnorm_early_release). */
+B200_API int b200_attn_decode_early_release(const void* q, const void* k_cache, const void* v_cache, const void* pos, void* out,
+                                            void* scratch, int64_t B, int64_t nh, int64_t max_ctx, uint32_t flags,
+                                            void* cuda_stream);
 
 /* Rotary embedding of q and k, KV append at *pos, attention over positions 0..*pos and the merge of
  * the per-chunk partials in one launch (what b200_rope_kv_append + b200_attn_decode do in three).
@@ -384,6 +400,8 @@ B200_API int b200_advance_pos(void* pos, int64_t delta, void* cuda_stream);
 
 /* out[b,i] = silu(gu[b,i]) * gu[b,I+i]; gu fp16 [B,2I], out fp16 [B,I]; I % 8 == 0. */
 B200_API int b200_silu_mul(const void* gu, void* out, int64_t B, int64_t I, void* cuda_stream);
+/* The same in its early-release form (see b200_rmsnorm_early_release). */
+B200_API int b200_silu_mul_early_release(const void* gu, void* out, int64_t B, int64_t I, void* cuda_stream);
 
 /* ---- introspection used by tests and the benchmark --------------------------------------- */
 

@@ -116,14 +116,17 @@ PROTOTYPES = {
     "b200_decode_layer_scratch_bytes": (_i64, [_i64, _i64]),
     "b200_decode_layer": (_ci, [ctypes.POINTER(DecodeLayer), _vp]),
     "b200_rmsnorm": (_ci, [_vp, _vp, _vp, _vp, _i64, _i64, ctypes.c_float, _vp]),
+    "b200_rmsnorm_early_release": (_ci, [_vp, _vp, _vp, _vp, _i64, _i64, ctypes.c_float, _vp]),
     "b200_rope_kv_append": (_ci, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _vp]),
     "b200_attn_decode_scratch_bytes": (_i64, [_i64, _i64, _i64]),
     "b200_attn_decode": (_ci, [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, ctypes.c_uint32, _vp]),
+    "b200_attn_decode_early_release": (_ci, [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, ctypes.c_uint32, _vp]),
     "b200_attn_decode_fused_scratch_bytes": (_i64, [_i64, _i64, _i64]),
     "b200_attn_decode_fused": (_ci, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _vp]),
     "b200_attn_decode_rope": (_ci, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _vp]),
     "b200_attn_decode_static": (_ci, [_vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, ctypes.c_uint32, _vp]),
     "b200_silu_mul": (_ci, [_vp, _vp, _i64, _i64, _vp]),
+    "b200_silu_mul_early_release": (_ci, [_vp, _vp, _i64, _i64, _vp]),
     "b200_embed_rows": (_ci, [_vp, _vp, _vp, _i64, _i64, _i64, _vp]),
     "b200_advance_pos": (_ci, [_vp, _i64, _vp]),
     "b200_launch_count": (_i64, []),

@@ -30,22 +30,28 @@ __device__ __forceinline__ float warp_max(float v) {
   return v;
 }
 
-// Where a kernel lets its successor start (griddepcontrol.launch_dependents): the matmuls read nothing but weights
-// before their own wait, so a kernel in front of one triggers in its first instruction, and the matmul's set-up and
-// first weight loads run beside it.  The kernels in front of the attention, which may read old cache entries and the
-// position before its wait, trigger after their own wait: everything up to the launch before them is then complete.
+// Where a kernel lets its successor start (griddepcontrol.launch_dependents).  The entry points' ordinary forms do so
+// right after their own wait: everything up to the launch before them is then complete, which is what an attention
+// with early loads of old cache entries and of the position relies on when one of them is directly in front.  The
+// early-release forms (kEarly) do so in their first instruction, for a caller that knows that nothing is read
+// early behind them but weights: a matmul's set-up and first weight loads then run beside them.
+template <bool kEarly>
+__device__ __forceinline__ void wait_and_release() {
+  if (kEarly) ptx::pdl_launch_dependents();
+  ptx::pdl_wait();
+  if (!kEarly) ptx::pdl_launch_dependents();
+}
 
 // y[b,:] = fp16( f32(x) * rsqrt(mean(f32(x)^2) + eps) * f32(w) ); optionally x += delta first (the
 // updated x is written back: it is the residual stream).  One CTA per row, H % 8 == 0.  A thread's share of the row,
 // of delta and of w (up to kRmsWords words of 8 values: H <= 8192) is loaded in one go and stays in registers; a longer
 // row makes the trip for w after the statistics, through a copy of x in shared memory.
 constexpr int kRmsWords = 4;
-template <bool kAdd>
+template <bool kAdd, bool kEarly>
 __global__ void __launch_bounds__(256)
 rmsnorm_kernel(__half* __restrict__ x, const __half* __restrict__ delta, const __half* __restrict__ w,
                __half* __restrict__ y, int H, float eps) {
-  ptx::pdl_launch_dependents();
-  ptx::pdl_wait();
+  wait_and_release<kEarly>();
   extern __shared__ float xs[];                 // H floats (H > 8192)
   __shared__ float red[8];
   const int b = blockIdx.x;
@@ -461,11 +467,11 @@ attn_decode_fused_kernel(const __half* __restrict__ qkv, const float* __restrict
 }
 
 // Merges the nsplit partials of one (batch, head) and writes fp16 [B, nh*128].  grid (nh, B), 128 threads.
+template <bool kEarly>
 __global__ void __launch_bounds__(128)
 attn_decode_combine_kernel(const float* __restrict__ scratch, const int* __restrict__ pos_ptr, __half* __restrict__ out,
                            int nh, int nsplit) {
-  ptx::pdl_launch_dependents();
-  ptx::pdl_wait();
+  wait_and_release<kEarly>();
   const int h = blockIdx.x, b = blockIdx.y, d = threadIdx.x;
   const int ctx = pos_ptr[0] + 1;
   const int used = (ctx + kAttnChunk - 1) / kAttnChunk;
@@ -507,10 +513,10 @@ attn_decode_combine_kernel(const float* __restrict__ scratch, const int* __restr
 }
 
 // out[b,i] = fp16( silu(f32(g)) * f32(u) ), gu row = [gate (I) | up (I)].  I % 8 == 0.
+template <bool kEarly>
 __global__ void __launch_bounds__(256)
 silu_mul_kernel(const __half* __restrict__ gu, __half* __restrict__ out, int I, int64_t total8) {
-  ptx::pdl_launch_dependents();
-  ptx::pdl_wait();
+  wait_and_release<kEarly>();
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= total8) return;
   const int per_row = I / 8;
@@ -579,18 +585,26 @@ using namespace b200;
 
 extern "C" {
 
-int b200_rmsnorm(void* x, const void* delta, const void* w, void* y, int64_t B, int64_t H, float eps, void* stream) {
-  if (B < 0 || H <= 0 || H % 8 != 0 || H > 16384) return fail(B200_EINVAL, "rmsnorm: need 0 < H <= 16384, H %% 8 == 0");
+static int rmsnorm_impl(const char* who, void* x, const void* delta, const void* w, void* y, int64_t B, int64_t H, float eps,
+                        bool early, void* stream) {
+  if (B < 0 || H <= 0 || H % 8 != 0 || H > 16384) return fail(B200_EINVAL, "%s: need 0 < H <= 16384, H %% 8 == 0", who);
   if (B == 0) return B200_OK;
-  if (!x || !w || !y) return fail(B200_EINVAL, "rmsnorm: null pointer");
+  if (!x || !w || !y) return fail(B200_EINVAL, "%s: null pointer", who);
   int rc = ensure_device();
   if (rc) return rc;
-  auto s = static_cast<cudaStream_t>(stream);
-  if (delta)
-    return launch("add_rmsnorm", rmsnorm_kernel<true>, dim3((unsigned)B), dim3(256), H > kRmsWords * 256 * 8 ? (size_t)H * 4 : 0, s, (__half*)x,
-                  (const __half*)delta, (const __half*)w, (__half*)y, (int)H, eps);
-  return launch("rmsnorm", rmsnorm_kernel<false>, dim3((unsigned)B), dim3(256), H > kRmsWords * 256 * 8 ? (size_t)H * 4 : 0, s, (__half*)x,
-                (const __half*)nullptr, (const __half*)w, (__half*)y, (int)H, eps);
+  auto kern = delta ? (early ? rmsnorm_kernel<true, true> : rmsnorm_kernel<true, false>)
+                    : (early ? rmsnorm_kernel<false, true> : rmsnorm_kernel<false, false>);
+  return launch(delta ? "add_rmsnorm" : "rmsnorm", kern, dim3((unsigned)B), dim3(256),
+                H > kRmsWords * 256 * 8 ? (size_t)H * 4 : 0, static_cast<cudaStream_t>(stream), (__half*)x, (const __half*)delta,
+                (const __half*)w, (__half*)y, (int)H, eps);
+}
+
+int b200_rmsnorm(void* x, const void* delta, const void* w, void* y, int64_t B, int64_t H, float eps, void* stream) {
+  return rmsnorm_impl("rmsnorm", x, delta, w, y, B, H, eps, false, stream);
+}
+
+int b200_rmsnorm_early_release(void* x, const void* delta, const void* w, void* y, int64_t B, int64_t H, float eps, void* stream) {
+  return rmsnorm_impl("rmsnorm_early_release", x, delta, w, y, B, H, eps, true, stream);
 }
 
 int b200_rope_kv_append(const void* qkv, const void* cos_t, const void* sin_t, const void* pos, void* q_out,
@@ -644,12 +658,12 @@ int b200_attn_decode_rope(const void* qkv, const void* cos_t, const void* sin_t,
               (const float*)sin_t, (const int*)pos, (__half*)k_cache, (__half*)v_cache, (__half*)out, (float*)scratch, (int)nh,
               (int)max_ctx, nsplit, scale_log2e, 0);
   if (rc) return rc;
-  return launch("attn_decode_combine", attn_decode_combine_kernel, dim3((unsigned)nh, (unsigned)B), dim3(128), 0, s,
+  return launch("attn_decode_combine", attn_decode_combine_kernel<false>, dim3((unsigned)nh, (unsigned)B), dim3(128), 0, s,
                 (const float*)scratch, (const int*)pos, (__half*)out, (int)nh, nsplit);
 }
 
-int b200_attn_decode(const void* q, const void* k_cache, const void* v_cache, const void* pos, void* out, void* scratch,
-                     int64_t B, int64_t nh, int64_t max_ctx, uint32_t flags, void* stream) {
+static int attn_decode_impl(const void* q, const void* k_cache, const void* v_cache, const void* pos, void* out, void* scratch,
+                            int64_t B, int64_t nh, int64_t max_ctx, uint32_t flags, bool early, void* stream) {
   if (B <= 0 || nh <= 0 || max_ctx <= 0) return fail(B200_EINVAL, "attn_decode: bad sizes");
   if (B > 65535 || nh > 65535 || max_ctx > 0x3fffffffLL)
     return fail(B200_EINVAL, "attn_decode: batch and heads are limited to 65535 (grid dimensions), max_ctx to 2^30");
@@ -668,8 +682,18 @@ int b200_attn_decode(const void* q, const void* k_cache, const void* v_cache, co
               dim3(128), 0, s, (const __half*)q, (const __half*)k_cache, (const __half*)v_cache, (const int*)pos,
               (float*)scratch, (int)nh, (int)max_ctx, nsplit, scale_log2e, (int)(flags & B200_ATTN_EARLY_KV_LOADS));
   if (rc) return rc;
-  return launch("attn_decode_combine", attn_decode_combine_kernel, dim3((unsigned)nh, (unsigned)B), dim3(128), 0, s,
+  return launch("attn_decode_combine", early ? attn_decode_combine_kernel<true> : attn_decode_combine_kernel<false>, dim3((unsigned)nh, (unsigned)B), dim3(128), 0, s,
                 (const float*)scratch, (const int*)pos, (__half*)out, (int)nh, nsplit);
+}
+
+int b200_attn_decode(const void* q, const void* k_cache, const void* v_cache, const void* pos, void* out, void* scratch,
+                     int64_t B, int64_t nh, int64_t max_ctx, uint32_t flags, void* stream) {
+  return attn_decode_impl(q, k_cache, v_cache, pos, out, scratch, B, nh, max_ctx, flags, false, stream);
+}
+
+int b200_attn_decode_early_release(const void* q, const void* k_cache, const void* v_cache, const void* pos, void* out,
+                                   void* scratch, int64_t B, int64_t nh, int64_t max_ctx, uint32_t flags, void* stream) {
+  return attn_decode_impl(q, k_cache, v_cache, pos, out, scratch, B, nh, max_ctx, flags, true, stream);
 }
 
 int b200_embed_rows(const void* table, const void* ids, void* out, int64_t B, int64_t H, int64_t vocab, void* stream) {
@@ -726,15 +750,23 @@ int b200_attn_decode_static(const void* q, const void* k_cache, const void* v_ca
   return b200_attn_decode(q, k_cache, v_cache, pos, out, scratch_of_device[dev], B, nh, max_ctx, flags, stream);
 }
 
-int b200_silu_mul(const void* gu, void* out, int64_t B, int64_t I, void* stream) {
-  if (B < 0 || I <= 0 || I % 8 != 0) return fail(B200_EINVAL, "silu_mul: need I %% 8 == 0");
+static int silu_mul_impl(const char* who, const void* gu, void* out, int64_t B, int64_t I, bool early, void* stream) {
+  if (B < 0 || I <= 0 || I % 8 != 0) return fail(B200_EINVAL, "%s: need I %% 8 == 0", who);
   if (B == 0) return B200_OK;
-  if (!gu || !out) return fail(B200_EINVAL, "silu_mul: null pointer");
+  if (!gu || !out) return fail(B200_EINVAL, "%s: null pointer", who);
   int rc = ensure_device();
   if (rc) return rc;
   const int64_t total8 = B * (I / 8);
-  return launch("silu_mul", silu_mul_kernel, dim3((unsigned)((total8 + 255) / 256)), dim3(256), 0,
+  return launch("silu_mul", early ? silu_mul_kernel<true> : silu_mul_kernel<false>, dim3((unsigned)((total8 + 255) / 256)), dim3(256), 0,
                 static_cast<cudaStream_t>(stream), (const __half*)gu, (__half*)out, (int)I, total8);
+}
+
+int b200_silu_mul(const void* gu, void* out, int64_t B, int64_t I, void* stream) {
+  return silu_mul_impl("silu_mul", gu, out, B, I, false, stream);
+}
+
+int b200_silu_mul_early_release(const void* gu, void* out, int64_t B, int64_t I, void* stream) {
+  return silu_mul_impl("silu_mul_early_release", gu, out, B, I, true, stream);
 }
 
 }  // extern "C"

@@ -265,7 +265,10 @@ class DecodeEngine:
 
     def layer_step(self, i: int, delta, sp: int):
         """One layer; `delta` is the tensor still to be added to the residual stream (or None).
-        Returns the layer's MLP output (to be added by whoever consumes the stream next)."""
+        Returns the layer's MLP output (to be added by whoever consumes the stream next).
+
+        The early-release forms: behind every one of them is a matmul (or the output projection), which reads nothing
+        but weights before it has waited for the kernel in front."""
         cfg, L, B, w = self.cfg, self.L, self.batch, self.layers[i]
         H, hl, il = cfg.hidden, cfg.hidden // self.world, w["inter_local"]
         dptr = delta.data_ptr() if delta is not None else None
@@ -289,16 +292,17 @@ class DecodeEngine:
                                                   w["qkv"][0].data_ptr(), w["qkv"][1].data_ptr(), self.qkv.data_ptr(),
                                                   B, 3 * hl, H, sp))
         else:
-            self._check(L.b200_rmsnorm(self.x.data_ptr(), dptr, w["norm1"].data_ptr(), self.h.data_ptr(), B, H, cfg.eps, sp))
+            self._check(L.b200_rmsnorm_early_release(self.x.data_ptr(), dptr, w["norm1"].data_ptr(), self.h.data_ptr(), B, H,
+                                                     cfg.eps, sp))
             self._matmul(self.h, w["qkv"], self.qkv, 3 * hl, H, sp)
         if roped:
             # The position and the older cache entries were final before the matmul in front began (the position was
             # advanced two launches before this step's first kernel, each of which waits before it lets the next
             # one start; the matmul's epilogue writes only the new token's slot, which the attention reads after
             # its own wait)
-            self._check(L.b200_attn_decode(self.q.data_ptr(), self.kc[i].data_ptr(), self.vc[i].data_ptr(), self.pos.data_ptr(),
-                                           self.attn.data_ptr(), self.scratch.data_ptr(), B, self.nh_local, self.max_ctx,
-                                           _lib.ATTN_EARLY_KV_LOADS, sp))
+            self._check(L.b200_attn_decode_early_release(self.q.data_ptr(), self.kc[i].data_ptr(), self.vc[i].data_ptr(),
+                                                         self.pos.data_ptr(), self.attn.data_ptr(), self.scratch.data_ptr(), B,
+                                                         self.nh_local, self.max_ctx, _lib.ATTN_EARLY_KV_LOADS, sp))
         elif self.fused_attention == "rope":
             # rotary embedding + KV append + per-chunk attention in one launch, the merge in a second
             self._check(L.b200_attn_decode_rope(self.qkv.data_ptr(), self.cos.data_ptr(), self.sin.data_ptr(), self.pos.data_ptr(),
@@ -313,10 +317,11 @@ class DecodeEngine:
             self._check(L.b200_rope_kv_append(self.qkv.data_ptr(), self.cos.data_ptr(), self.sin.data_ptr(), self.pos.data_ptr(),
                                               self.q.data_ptr(), self.kc[i].data_ptr(), self.vc[i].data_ptr(), B, self.nh_local,
                                               self.max_ctx, sp))
-            self._check(L.b200_attn_decode(self.q.data_ptr(), self.kc[i].data_ptr(), self.vc[i].data_ptr(), self.pos.data_ptr(),
-                                           self.attn.data_ptr(), self.scratch.data_ptr(), B, self.nh_local, self.max_ctx,
-                                           _lib.ATTN_EARLY_KV_LOADS,   # rope_kv_append sits directly in front and waits first
-                                           sp))
+            self._check(L.b200_attn_decode_early_release(self.q.data_ptr(), self.kc[i].data_ptr(), self.vc[i].data_ptr(),
+                                                         self.pos.data_ptr(), self.attn.data_ptr(), self.scratch.data_ptr(), B,
+                                                         self.nh_local, self.max_ctx,
+                                                         _lib.ATTN_EARLY_KV_LOADS,   # rope_kv_append sits directly in front and waits first
+                                                         sp))
         if self.peer is not None and B <= self.PEER_FUSED_MAX_ROWS:
             d = self._reduce_desc(0, i, self.o)
             self._check(L.b200_q4f16_gemv_allreduce(self.attn.data_ptr(), w["o"][0].data_ptr(), w["o"][1].data_ptr(),
@@ -338,10 +343,10 @@ class DecodeEngine:
             self._check(L.b200_q4f16_gemv_swiglu(self.gu.data_ptr(), w["down"][0].data_ptr(), w["down"][1].data_ptr(),
                                                  self.down.data_ptr(), B, H, il, sp))
         else:
-            self._check(L.b200_rmsnorm(self.x.data_ptr(), self.o.data_ptr(), w["norm2"].data_ptr(), self.h.data_ptr(), B, H,
-                                       cfg.eps, sp))
+            self._check(L.b200_rmsnorm_early_release(self.x.data_ptr(), self.o.data_ptr(), w["norm2"].data_ptr(), self.h.data_ptr(),
+                                                     B, H, cfg.eps, sp))
             self._matmul(self.h, w["gu"], self.gu, 2 * il, H, sp)
-            self._check(L.b200_silu_mul(self.gu.data_ptr(), self.act.data_ptr(), B, il, sp))
+            self._check(L.b200_silu_mul_early_release(self.gu.data_ptr(), self.act.data_ptr(), B, il, sp))
             if self.peer is not None and B <= self.PEER_FUSED_MAX_ROWS:
                 d = self._reduce_desc(1, i, self.down)
                 self._check(L.b200_q4f16_gemv_allreduce(self.act.data_ptr(), w["down"][0].data_ptr(), w["down"][1].data_ptr(),
@@ -374,8 +379,8 @@ class DecodeEngine:
         else:
             for i in range(len(self.layers)):
                 delta = self.layer_step(i, delta, sp)
-        self._check(L.b200_rmsnorm(xlast.data_ptr(), delta.data_ptr() if delta is not None else None,
-                                   self.final_norm.data_ptr(), self.h.data_ptr(), B, cfg.hidden, cfg.eps, sp))
+        self._check(L.b200_rmsnorm_early_release(xlast.data_ptr(), delta.data_ptr() if delta is not None else None,
+                                                 self.final_norm.data_ptr(), self.h.data_ptr(), B, cfg.hidden, cfg.eps, sp))
         if self.lm_head is not None:
             own = B <= 16                       # the library's output projection takes up to 16 rows; above that a library GEMM
             if own:

@@ -239,6 +239,71 @@ def test_attention_after_a_matmul_after_a_position_writer(cuda_lib):
     assert L.b200_attn_decode(None, kc.data_ptr(), vc.data_ptr(), kc.data_ptr(), kc.data_ptr(), scratch.data_ptr(), 1, nh, max_ctx, 6, 0) == _lib.EINVAL
 
 
+@pytest.mark.parametrize("between", ["rmsnorm", "silu_mul", "attn_decode"])
+def test_early_loads_behind_the_glue_kernels(cuda_lib, between):
+    """advance_pos -> a glue kernel -> attention with B200_ATTN_EARLY_KV_LOADS, 200 times with no host synchronisation.
+    advance_pos releases its dependents before it stores the position, so the kernel between has to wait for it before
+    it releases the attention, which reads *pos before its own wait.  Equal, bit for bit, to the same sequence with a
+    synchronisation after every launch."""
+    L = cuda_lib
+    nh, max_ctx, H = 8, 512, 1024
+    iters, pos0 = 200, 100
+    g = torch.Generator(device="cuda")
+    g.manual_seed(6)
+    kc, vc = (torch.randn((1, max_ctx, nh, 128), device="cuda", generator=g).to(torch.float16) for _ in "kv")
+    x, gate_up, w = (torch.randn(k, device="cuda", generator=g).to(torch.float16) for k in (H, 2 * H, H))
+    q = torch.randn((1, nh * 128), device="cuda", generator=g).to(torch.float16)
+    scratch, scratch2 = (torch.empty(L.b200_attn_decode_scratch_bytes(1, nh, max_ctx) // 4, dtype=torch.float32, device="cuda") for _ in "12")
+
+    def run(serialised):
+        pos = torch.tensor([pos0], dtype=torch.int32, device="cuda")
+        side = torch.zeros(nh * 128, dtype=torch.float16, device="cuda")
+        outs = torch.zeros((iters, nh * 128), dtype=torch.float16, device="cuda")
+        torch.cuda.synchronize()
+        sp = torch.cuda.current_stream().cuda_stream
+        calls = {
+            "rmsnorm": lambda: L.b200_rmsnorm(x.data_ptr(), None, w.data_ptr(), side.data_ptr(), 1, H, 1e-5, sp),
+            "silu_mul": lambda: L.b200_silu_mul(gate_up.data_ptr(), side.data_ptr(), 1, H, sp),
+            "attn_decode": lambda: L.b200_attn_decode(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), pos.data_ptr(), side.data_ptr(),
+                                                      scratch2.data_ptr(), 1, nh, max_ctx, 0, sp),
+        }
+        for i in range(iters):
+            for call in (lambda: L.b200_advance_pos(pos.data_ptr(), 1, sp), calls[between],
+                         lambda: L.b200_attn_decode(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), pos.data_ptr(), outs[i].data_ptr(),
+                                                    scratch.data_ptr(), 1, nh, max_ctx, _lib.ATTN_EARLY_KV_LOADS, sp)):
+                assert call() == 0, _lib.last_error()
+                if serialised:
+                    torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        assert int(pos.item()) == pos0 + iters
+        return outs.cpu().numpy().view(np.uint16)
+
+    want, got = run(True), run(False)
+    assert not (want[0] == want[1]).all()            # another position, another result
+    bad = np.flatnonzero((got != want).any(axis=1))
+    assert bad.size == 0, f"iterations {bad[:8]} differ from the serialised run"
+
+
+@pytest.mark.parametrize("B,H", [(1, 4096), (3, 16), (2, 11008)])
+def test_early_release_forms_equal_the_ordinary_ones(cuda_lib, B, H):
+    L = cuda_lib
+    g = torch.Generator(device="cuda")
+    g.manual_seed(B + H)
+    x, d, gate_up, w = (torch.randn(s, device="cuda", generator=g).to(torch.float16) for s in ((B, H), (B, H), (B, 2 * H), (H,)))
+    outs = {}
+    for form in ("", "_early_release"):
+        xs, y, act = x.clone(), torch.empty_like(x), torch.empty_like(x)
+        assert getattr(L, "b200_rmsnorm" + form)(xs.data_ptr(), d.data_ptr(), w.data_ptr(), y.data_ptr(), B, H, 1e-5, 0) == 0
+        assert getattr(L, "b200_silu_mul" + form)(gate_up.data_ptr(), act.data_ptr(), B, H, 0) == 0
+        assert getattr(L, "b200_rmsnorm" + form)(None, None, w.data_ptr(), y.data_ptr(), B, H, 1e-5, 0) == _lib.EINVAL
+        assert "rmsnorm" + form + ":" in _lib.last_error()
+        assert getattr(L, "b200_silu_mul" + form)(gate_up.data_ptr(), None, B, H, 0) == _lib.EINVAL
+        torch.cuda.synchronize()
+        outs[form] = [t.cpu().numpy().view(np.uint16) for t in (xs, y, act)]
+    for a, b in zip(outs[""], outs["_early_release"]):
+        assert np.array_equal(a, b)
+
+
 # ------------------------------------------------------------------------------ bounded wait of the fused sum over ranks
 def test_peer_wait_runs_out_without_hanging(cuda_lib):
     """The row-parallel matmul with the fused sum over ranks, told that there are two ranks whose buffers both
