@@ -100,9 +100,14 @@ struct Bars {
   int abort_flag;
 };
 
+// The conversion, the MMAs and the refills of the rings wait for x, so for the kernels in front of this one, which may
+// legitimately run for longer than the limit (a sum over ranks waits up to gemv.peer_wait_ms for a late one).  A
+// limit that runs out is therefore started once more behind griddepcontrol.wait.
 __device__ __forceinline__ void wait_or_abort(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int code) {
   if (mbar_try_wait(bar, parity)) return;   // completed barrier: no read of the flag on the fast path
   if (*abort_flag) return;
+  if (mbar_wait_ns(bar, parity, kWaitNs)) return;
+  pdl_wait();
   if (!mbar_wait_ns(bar, parity, kWaitNs)) {
     *abort_flag = 1;
     atomicExch(&g_gemm_ws_error, code);

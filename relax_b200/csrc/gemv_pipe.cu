@@ -73,7 +73,7 @@ using namespace skinny;
 constexpr int kRows = 16;                // rows per stage / row tile
 constexpr int kMaxStages = 8;
 constexpr uint64_t kConsumerWaitNs = 2000000000ull;     // 2 s: a stage copy takes microseconds
-constexpr uint64_t kProducerWaitNs = 30000000000ull;    // 30 s: may span the previous kernel's whole run
+constexpr uint64_t kProducerWaitNs = 30000000000ull;    // 30 s: may span the previous kernels' whole run
 
 enum { kPrologueNone = 0, kPrologueRmsNorm = 1, kPrologueSwiGLU = 2 };
 
@@ -254,9 +254,16 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
           const int row0 = tile * kRows;
           for (int k0 = k_lo; k0 < k_hi; k0 += KC, s = (s + 1 == p.nstages ? 0 : s + 1), round += (s == 0)) {
             if (round > 0) {
-              // Legitimately as long as the previous kernel in the stream runs (the consumers
-              // that free the stages sit in griddepcontrol.wait until then): bound it by time.
-              if (*(volatile int*)&s_abort || !mbar_wait_ns_relaxed(&empty[s], (round - 1) & 1, kProducerWaitNs)) {
+              // Legitimately as long as the previous kernels in the stream run (the consumers
+              // that free the stages sit in griddepcontrol.wait until then): bounded by time, and
+              // the limit starts once more behind griddepcontrol.wait (a sum over ranks in front
+              // may wait for a late one for longer than that).
+              bool ok = !*(volatile int*)&s_abort && mbar_wait_ns_relaxed(&empty[s], (round - 1) & 1, kProducerWaitNs);
+              if (!ok && !*(volatile int*)&s_abort) {
+                pdl_wait();
+                ok = mbar_wait_ns_relaxed(&empty[s], (round - 1) & 1, kProducerWaitNs);
+              }
+              if (!ok) {
                 atomicExch(&g_gemv_pipe_error, 1);
                 *(volatile int*)&s_abort = 1;
                 return;   // copies already issued land in stages the consumers still own

@@ -345,6 +345,52 @@ def test_peer_wait_runs_out_without_hanging(cuda_lib):
     assert L.b200_device_error_flags() == 0
 
 
+def test_a_late_rank_is_waited_for_in_front_of_the_tensor_core_matmul(cuda_lib):
+    """A sum over ranks whose second rank publishes 4.5 s late (its flag is written by a copy on another stream; nothing
+    runs out), a norm that releases first and the weight-stationary matmul behind it, which is resident all that
+    time: its own limit of 4 s counts from the end of the kernels in front, so no error is raised and the results equal
+    those of the same launches one by one."""
+    import time
+
+    L = cuda_lib
+    M, N, K = 16, 1024, 2048
+    x, wq, s = synth.make_case(M, N, K, seed=45)
+    twq, ts = dev(wq), dev(s)
+    parts = [dev(x), torch.ones((M, K), dtype=torch.float16, device="cuda")]
+    w = torch.ones(K, dtype=torch.float16, device="cuda")
+    one = torch.ones(1, dtype=torch.int32).pin_memory()
+    side = torch.cuda.Stream()
+    outs = []
+    for late in (False, True):
+        flags = torch.zeros(16, dtype=torch.int32, device="cuda")
+        epoch, done = (torch.zeros(1, dtype=torch.int32, device="cuda") for _ in "12")
+        total, h = (torch.zeros((M, K), dtype=torch.float16, device="cuda") for _ in "12")
+        y = torch.zeros((M, N), dtype=torch.float16, device="cuda")
+        d = _lib.PeerReduce()
+        d.world, d.rank = 2, 0
+        d.peer_y[0], d.peer_y[1] = parts[0].data_ptr(), parts[1].data_ptr()
+        d.peer_flags[0], d.peer_flags[1] = flags.data_ptr(), flags.data_ptr() + 32
+        d.flag_base, d.epoch, d.done_counter, d.out = 0, epoch.data_ptr(), done.data_ptr(), total.data_ptr()
+        if not late:
+            flags[1] = 1
+        torch.cuda.synchronize()
+        try:
+            _lib.set_option("gemv.peer_wait_ms", 8000)
+            assert L.b200_allreduce_peer(M * K, ctypes.byref(d), 0) == 0, _lib.last_error()
+        finally:
+            _lib.set_option("gemv.peer_wait_ms", 2000)
+        assert L.b200_rmsnorm_early_release(total.data_ptr(), None, w.data_ptr(), h.data_ptr(), M, K, 1e-5, 0) == 0
+        assert L.b200_q4f16_gemm_ws(h.data_ptr(), twq.data_ptr(), ts.data_ptr(), y.data_ptr(), M, N, K, 0) == 0, _lib.last_error()
+        if late:
+            time.sleep(4.5)
+            with torch.cuda.stream(side):
+                flags[1:2].copy_(one, non_blocking=True)
+        torch.cuda.synchronize()
+        assert L.b200_device_error_flags() == 0
+        outs.append(y.cpu().numpy().view(np.uint16))
+    assert outs[0].any() and np.array_equal(outs[0], outs[1])
+
+
 # ------------------------------------------------------------------------------ the layer kernel's own contracts
 def _small_layer_engine(layers=2, max_ctx=16):
     cfg = decoder.DecoderConfig(hidden=512, heads=4, inter=768, layers=layers, vocab=100)
