@@ -134,11 +134,11 @@ int matmul_impl(Family fam, const char* who, const void* x, const void* wq, cons
   // (streaming / weight-stationary in us: 4 x 4096 x 2080 5.1 / 5.3, 16 x 1024 x 1056 4.5 / 4.5, 2 x 8640 x 3200 11.0 /
   // 11.0, 3 x 8640 x 3200 13.8 / 11.0, 8 x 4096 x 2080 7.0 / 5.5, 16 x 22016 x 4128 86 / 24; above 16 rows, against the
   // prefill kernel, 32 x 8640 x 3200 43 / 11.5, 2048 x 11008 x 4128 188 / 159).
-  // The option's largest value, 128, stands for no limit.  (A variant of the skinny kernel asked for by option keeps its rows.)
+  // (Above a gemm.ws_max_m that was lowered the skinny and prefill kernels take over, and a variant of the skinny kernel
+  // asked for by option keeps its rows.)
   const bool ragged = K % 256 != 0 || !aligned16(scales);
   const bool ws_auto = M > 16 || (ragged ? M >= 2 && M * N * K >= 50000000 : M >= 9 || (M >= 5 && K >= 8192));
-  if (fam == kGemmWs || (fam == kAuto && ws_auto && (M <= options().gemm_ws_max_m || options().gemm_ws_max_m == 128) &&
-                         (M > 16 || options().gemv_variant == 0))) {
+  if (fam == kGemmWs || (fam == kAuto && ws_auto && M <= options().gemm_ws_max_m && (M > 16 || options().gemv_variant == 0))) {
     rc = fam == kGemmWs && (M > 128 || ragged) ? B200_ENOTREADY : launch_gemm_ws(xh, wh, sh, yh, M, N, K, s);
     if (rc != B200_ENOTREADY) return rc;
     if (fam == kGemmWs) return fail(B200_EINVAL, "%s: the weight-stationary kernel takes 1 <= M <= 128, K %% 256 == 0, 16-byte aligned scales", who);
@@ -282,10 +282,10 @@ int b200_set_option(const char* name, int64_t v) {
   else if (!strcmp(name, "layer.max_ctas")) { if (v < 0 || v > 1024) return fail(B200_EINVAL, "layer.max_ctas in 0..1024"); o.layer_max_ctas = v; }
   else if (!strcmp(name, "gemm.ws_ksplit")) { if (v < 0 || v > 8 || (v & (v - 1))) return fail(B200_EINVAL, "gemm.ws_ksplit is 0, 1, 2, 4 or 8"); o.gemm_ws_ksplit = v; }
   else if (!strcmp(name, "gemm.ws_x_stages")) { if (v < 0 || v > 8) return fail(B200_EINVAL, "gemm.ws_x_stages in 0..8"); o.gemm_ws_x_stages = v; }
-  else if (!strcmp(name, "gemm.ws_w_stages")) { if (v < 0 || v > 8) return fail(B200_EINVAL, "gemm.ws_w_stages in 0..8"); o.gemm_ws_w_stages = v; }
+  else if (!strcmp(name, "gemm.ws_w_stages")) { if (v != 0) return fail(B200_EINVAL, "gemm.ws_w_stages is 0: the dequantised weights sit in a fixed ring in tensor memory"); }
   else if (!strcmp(name, "gemm.ws_r_stages")) { if (v < 0 || v == 1 || v > 8) return fail(B200_EINVAL, "gemm.ws_r_stages is 0 or in 2..8"); o.gemm_ws_r_stages = v; }
-  else if (!strcmp(name, "gemm.ws_xk")) { if (v != 0 && v != 2 && v != 4) return fail(B200_EINVAL, "gemm.ws_xk is 0, 2 or 4"); o.gemm_ws_xk = v; }
-  else if (!strcmp(name, "gemm.ws_max_m")) { if (v < 0 || v > 128) return fail(B200_EINVAL, "gemm.ws_max_m in 0..128"); o.gemm_ws_max_m = v; }
+  else if (!strcmp(name, "gemm.ws_xk")) { if (v != 0) return fail(B200_EINVAL, "gemm.ws_xk is 0: the K blocks per stage follow from the token tile"); }
+  else if (!strcmp(name, "gemm.ws_max_m")) { if (v < 0 || v > kWsNoLimit) return fail(B200_EINVAL, "gemm.ws_max_m in 0..%lld (no limit)", (long long)kWsNoLimit); o.gemm_ws_max_m = v; }
   else if (!strcmp(name, "weights.layout")) { if (v != B200_LAYOUT_REFERENCE && v != B200_LAYOUT_PAIRED) return fail(B200_EINVAL, "weights.layout is 0 (reference) or 1 (paired)"); o.weights_layout = v; }
   else if (!strcmp(name, "gemm.max_ctas")) { if (v < 0 || v > 1024) return fail(B200_EINVAL, "gemm.max_ctas in 0..1024"); o.gemm_max_ctas = v; }
   else return fail(B200_EINVAL, "set_option: unknown option '%s'", name);
@@ -309,8 +309,7 @@ int64_t b200_get_option(const char* name) {
   if (!strcmp(name, "gemm.ws_ksplit")) return o.gemm_ws_ksplit;
   if (!strcmp(name, "gemm.ws_max_m")) return o.gemm_ws_max_m;
   if (!strcmp(name, "gemm.ws_x_stages")) return o.gemm_ws_x_stages;
-  if (!strcmp(name, "gemm.ws_w_stages")) return o.gemm_ws_w_stages;
-  if (!strcmp(name, "gemm.ws_xk")) return o.gemm_ws_xk;
+  if (!strcmp(name, "gemm.ws_w_stages") || !strcmp(name, "gemm.ws_xk")) return 0;
   if (!strcmp(name, "gemm.ws_r_stages")) return o.gemm_ws_r_stages;
   if (!strcmp(name, "weights.layout")) return o.weights_layout;
   return -1;

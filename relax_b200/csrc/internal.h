@@ -13,6 +13,8 @@ int fail(int code, const char* fmt, ...);
 void count_launch(int n = 1);
 
 // Tuning knobs (b200_set_option).  Plain ints; read at launch time.
+constexpr int64_t kWsNoLimit = 0x7fffffff;   // more rows than any call takes
+
 struct Options {
   int64_t gemv_variant = 0;   // 0 = auto, 1 = register-streaming kernel, 2 = bulk-copy pipelined kernel
   int64_t gemv_warps = 0;     // 0 = auto
@@ -29,10 +31,8 @@ struct Options {
   int64_t gemm_ws_ksplit = 0; // 0 = auto: K slices (= cluster size) of the weight-stationary kernel
   int64_t weights_layout = 0; // B200_LAYOUT_*: the nibble order every matmul entry point assumes unless the call names one
   int64_t gemm_ws_x_stages = 0; // 0 = auto: cap on the depth of the weight-stationary kernel's x ring (>= 2; x is then never kept)
-  int64_t gemm_ws_w_stages = 0; // accepted and kept; the dequantised weights sit in a fixed ring in tensor memory
   int64_t gemm_ws_r_stages = 0; // 0 = auto: cap on the depth of its packed-weight ring (>= 2)
-  int64_t gemm_ws_xk = 0;       // accepted and kept (2 or 4); a stage is two K blocks
-  int64_t gemm_ws_max_m = 128; // largest M the automatic dispatch gives to the weight-stationary kernel (0 = never, 128 = no limit)
+  int64_t gemm_ws_max_m = kWsNoLimit; // largest M the automatic dispatch gives to the weight-stationary kernel (0 = never)
 };
 Options& options();
 

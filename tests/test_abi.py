@@ -219,3 +219,17 @@ def test_argument_checks_of_the_newer_entry_points_need_no_gpu():
     assert L.b200_q4f16_gemv_rmsnorm_rope(*(args[:7] + [None] + args[8:]), 2, 256, None) == _lib.EINVAL
     if no_gpu:
         assert L.b200_q4f16_gemv_rmsnorm_rope(*args, 2, 256, None) == _lib.ENODEVICE
+
+
+def test_options_of_the_weight_stationary_kernel():
+    L = _lib.lib()
+    # what the weight-stationary kernel cannot honour is refused, its default is not
+    for name in (b"gemm.ws_w_stages", b"gemm.ws_xk"):
+        assert L.b200_set_option(name, 2) == _lib.EINVAL and name.decode() in _lib.last_error()
+        assert L.b200_set_option(name, 0) == 0 and L.b200_get_option(name) == 0
+    # a limit of 128 rows is a value like any other, the default is above every M
+    unlimited = L.b200_get_option(b"gemm.ws_max_m")
+    assert unlimited >= 0x7fffffff // 64
+    for v in (0, 127, 128, 129, unlimited):
+        assert L.b200_set_option(b"gemm.ws_max_m", v) == 0 and L.b200_get_option(b"gemm.ws_max_m") == v
+    assert L.b200_set_option(b"gemm.ws_max_m", -1) == _lib.EINVAL and L.b200_get_option(b"gemm.ws_max_m") == unlimited

@@ -471,6 +471,24 @@ def test_unaligned_scales_mid_batch(cuda_lib):
     assert cuda_lib.b200_device_error_flags() == 0
 
 
+@pytest.mark.parametrize("limit,m,k,family", [(128, 129, 1024, "gemm"), (128, 128, 1024, "gemm_ws"), (0, 40, 1024, "gemm"),
+                                              (0, 16, 1024, "gemv"), (15, 16, 1056, "gemv"), (0, 20, 1056, "gemm")])
+def test_a_lowered_row_limit_takes_the_other_kernels(cuda_lib, limit, m, k, family):
+    # bit for bit what the named kernel's own entry point gives (16 x 4000 x 1056 is above the small products that
+    # the skinny kernel keeps anyway)
+    n = 4000
+    x, wq, s = synth.make_case(m, n, k, seed=m + k)
+    saved = relax_b200.get_option("gemm.ws_max_m")
+    try:
+        relax_b200.set_option("gemm.ws_max_m", limit)
+        out = run_matmul(x, wq, s)
+    finally:
+        relax_b200.set_option("gemm.ws_max_m", saved)
+    assert_matmul_close(out, x, wq, s, f"limit {limit} M={m} K={k}")
+    assert_bits_equal(out, run_matmul(x, wq, s, family=family), f"limit {limit} M={m} K={k}")
+    assert cuda_lib.b200_device_error_flags() == 0
+
+
 @pytest.mark.parametrize("m,n,k", [(9, 512, 11008), (16, 1280, 8192), (12, 300, 16384)])
 def test_auto_dispatch_small_batch_long_k(cuda_lib, m, n, k):
     # 9..16 rows whose x block does not fit beside the skinny kernel's ring go to the weight-stationary kernel
