@@ -50,6 +50,7 @@
 #include "q4_common.cuh"
 #include "sm100_ptx.cuh"
 #include "tmap.h"
+#include "ws_plan.h"
 
 namespace b200 {
 
@@ -62,13 +63,13 @@ using namespace ptx;
 
 constexpr int BR = 128;            // weight rows per tile (UMMA M)
 constexpr int BK = 64;             // k per K block (one 128-byte swizzled row of fp16)
-constexpr int kMaxNB = 192;        // batch columns (UMMA N), multiple of 16
 constexpr int kMaxXStages = 32;    // x stages (SKB K blocks each)
 constexpr int kMaxRawStages = 8;
 constexpr int kASlots = 4;         // A ring: slots of SKB K blocks (32 TMEM columns each), one per dequantiser group
 constexpr int kRawBytes = BR * 128;           // 16384: 128 rows x 32 words = 256 k, one 128-byte line per row
 constexpr int kScBytes = BR * 16;             // 2048:  128 rows x 8 scales  = 256 k
 constexpr int kDequantWarps = 16;
+static_assert(kRawBytes + kScBytes == kWsSpanBytes, "the plan counts these bytes");
 constexpr int kNumThreads = 256 + kDequantWarps * 32 + 128;   // 896: warps 24-27 are a second set of epilogue warps
 constexpr uint32_t kTmemCols = 512;           // two accumulators of 128 (SKB = 2) or 192 columns, then the A ring
 constexpr uint64_t kWaitNs = 4000000000ull;   // 4 s
@@ -540,38 +541,10 @@ int launch_gemm_ws(const __half* x, const uint32_t* wq, const __half* scales, __
   const int units = (int)((K + 255) / 256);
   const int64_t row_tiles = (N + BR - 1) / BR;
   if (row_tiles * ((M + 15) / 16) > 0x3fffffff) return B200_ENOTREADY;      // (tile numbers are 32-bit)
-  // Token tiles and K slices: a model of the time in nanoseconds, fitted to measurements at N = 4096, 12288 and 22016,
-  // K = 4096 and 11008 and batches of 16, 64 and 128, and at 129..2048 tokens.  A 256-k span takes a CTA 0.53-0.65 us (up
-  // to 128 columns) or 0.9-0.95 us; with many CTAs at work, what they fetch from L2 at about 14 TB/s if that is more.
-  // Draining a tile is cheap with one slice (stores to y, behind the next tile's MMAs) and costs the exchange of the
-  // partial tiles with several, which the next tile hides only as far as its own MMAs last; a larger cluster starts
-  // later.  M = 64, K = 4096, 1 / 2 / 4 / 8 slices: N = 4096 11.0 / 8.7 / 9.0 / 10.8 us, N = 12288 12.9 / 14.3 / 15.6 / 23.2,
-  // N = 22016 22.1 / 20.5 / 24.0 / 40.3; N = 4096 and K = 11008: 26.4 / 16.4 / 13.5 / 14.6.  M = 300, N = 12288, K = 4096 in 2 / 3 / 4
-  // token tiles: 31.7 / 29.5 / 34.8.
-  const int forced = (int)options().gemm_ws_ksplit;
-  int ksplit = 1, nb16 = 0;
-  int64_t best = 0;
-  const int64_t mt0 = (M + kMaxNB - 1) / kMaxNB;
-  // (up to 128 rows the weights stream once: one token tile)
-  const int64_t mt_max = M <= 128 ? 1 : mt0 + mt0 / 2 + 3;
-  for (int64_t mt = mt0; mt <= mt_max; ++mt) {
-    const int nb = (int)(((M + mt - 1) / mt + 15) / 16) * 16;
-    const int64_t tiles = row_tiles * ((M + nb - 1) / nb);
-    for (int c = 1; c <= 8 && c <= units; c *= 2) {
-      if (forced > 0 && !(c <= forced && (c * 2 > forced || c * 2 > units || c == 8))) continue;
-      const int nc = max_clusters(c, reinterpret_cast<const void*>(kernel_for(nb, paired, ragged)));
-      const int64_t rounds = (tiles + nc - 1) / nc;
-      const int64_t busy = tiles * c / rounds;                                   // CTAs at work, on average
-      const int64_t l2 = busy * (nb * 512 + kRawBytes + kScBytes) / 14000;
-      const int64_t span = nb <= 128 ? 520 + nb : 760 + nb;
-      const int64_t tile = (int64_t)((units + c - 1) / c) * (span > l2 ? span : l2);   // a tile's MMAs
-      const int64_t drain = c == 1 ? 300 + 12 * nb : 800 + 50 * nb;              // ... and what the next tile must hide
-      const int64_t tail = c == 1 ? drain : 1000 + 35 * nb;                      // the last tile's drain
-      const int64_t start = c == 1 ? 0 : c == 2 ? 500 : c == 4 ? 2800 : 3500;
-      const int64_t cost = start + tile + (rounds - 1) * (tile > drain ? tile : drain) + tail;
-      if (best == 0 || cost < best) { best = cost; ksplit = c; nb16 = nb; }
-    }
-  }
+  int clusters_of[4];
+  for (int i = 0; i < 4; ++i) clusters_of[i] = max_clusters(1 << i, reinterpret_cast<const void*>(kernel_for(16, paired, ragged)));
+  const WsSplit split = choose_ws_split(M, row_tiles, units, (int)options().gemm_ws_ksplit, clusters_of);
+  const int ksplit = split.ksplit, nb16 = split.nb;
   const int skb = nb16 <= 128 ? 2 : 1;
   auto kern = kernel_for(nb16, paired, ragged);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemCap);
@@ -583,7 +556,7 @@ int launch_gemm_ws(const __half* x, const uint32_t* wq, const __half* scales, __
   p.cw = p.NB / ksplit;
   p.mt = (int)((M + p.NB - 1) / p.NB);
   p.tiles = (int)row_tiles * p.mt;
-  int clusters = max_clusters(ksplit, reinterpret_cast<const void*>(kern));
+  int clusters = clusters_of[ksplit == 1 ? 0 : ksplit == 2 ? 1 : ksplit == 4 ? 2 : 3];
   if (clusters > p.tiles) clusters = p.tiles;
 
   // Shared memory: the inbox, four packed spans (72 KB in flight cover HBM's latency at one SM's share of its

@@ -1,0 +1,56 @@
+// Token tiles and K slices of the weight-stationary matmul (host arithmetic only).
+#pragma once
+#include <cstdint>
+
+namespace b200 {
+
+constexpr int kWsMaxNB = 192;                  // batch columns of a token tile (UMMA N), multiple of 16
+constexpr int kWsSpanBytes = 128 * 128 + 128 * 16;   // packed words and scales of 256 k of a row tile
+
+struct WsSplit {
+  int nb;       // rows of x per token tile, a multiple of 16
+  int ksplit;   // K slices = CTAs per cluster
+  int tried;    // combinations looked at
+};
+
+// A model of the time in nanoseconds, fitted to measurements at N = 4096, 12288 and 22016,
+// K = 4096 and 11008 and batches of 16, 64 and 128, and at 129..2048 tokens.  A 256-k span takes a CTA 0.53-0.65 us (up
+// to 128 columns) or 0.9-0.95 us; with many CTAs at work, what they fetch from L2 at about 14 TB/s if that is more.
+// Draining a tile is cheap with one slice (stores to y, behind the next tile's MMAs) and costs the exchange of the
+// partial tiles with several, which the next tile hides only as far as its own MMAs last; a larger cluster starts
+// later.  M = 64, K = 4096, 1 / 2 / 4 / 8 slices: N = 4096 11.0 / 8.7 / 9.0 / 10.8 us, N = 12288 12.9 / 14.3 / 15.6 / 23.2,
+// N = 22016 22.1 / 20.5 / 24.0 / 40.3; N = 4096 and K = 11008: 26.4 / 16.4 / 13.5 / 14.6.  M = 300, N = 12288, K = 4096 in 2 / 3 / 4
+// token tiles: 31.7 / 29.5 / 34.8.
+// M rows of x, row_tiles tiles of 128 weight rows, units spans of 256 k; forced: the largest power of two of slices up to
+// it (0 = by the model); clusters[i]: clusters of 2^i CTAs that run at once.  Every width of a token tile is looked at
+// once, so at most 12 x 4 combinations whatever M is.
+inline WsSplit choose_ws_split(int64_t M, int64_t row_tiles, int units, int forced, const int (&clusters)[4]) {
+  WsSplit best = {0, 1, 0};
+  int64_t best_cost = 0;
+  const int64_t mt0 = (M + kWsMaxNB - 1) / kWsMaxNB;
+  // (up to 128 rows the weights stream once: one token tile)
+  const int64_t mt_max = M <= 128 ? 1 : mt0 + mt0 / 2 + 3;
+  for (int nb = M < kWsMaxNB ? (int)((M + 15) / 16) * 16 : kWsMaxNB; nb >= 16; nb -= 16) {
+    const int64_t mt = (M + nb - 1) / nb;
+    if (mt > mt_max) break;
+    if (((M + mt - 1) / mt + 15) / 16 * 16 != nb) continue;      // as many token tiles of fewer columns do it
+    const int64_t tiles = row_tiles * mt;
+    for (int i = 0, c = 1; i < 4 && c <= units; ++i, c *= 2) {
+      if (forced > 0 && !(c <= forced && (c * 2 > forced || c * 2 > units || c == 8))) continue;
+      const int64_t rounds = (tiles + clusters[i] - 1) / clusters[i];
+      const int64_t busy = tiles * c / rounds;                                   // CTAs at work, on average
+      const int64_t l2 = busy * (nb * 512 + kWsSpanBytes) / 14000;
+      const int64_t span = nb <= 128 ? 520 + nb : 760 + nb;
+      const int64_t tile = (int64_t)((units + c - 1) / c) * (span > l2 ? span : l2);   // a tile's MMAs
+      const int64_t drain = c == 1 ? 300 + 12 * nb : 800 + 50 * nb;              // ... and what the next tile must hide
+      const int64_t tail = c == 1 ? drain : 1000 + 35 * nb;                      // the last tile's drain
+      const int64_t start = c == 1 ? 0 : c == 2 ? 500 : c == 4 ? 2800 : 3500;
+      const int64_t cost = start + tile + (rounds - 1) * (tile > drain ? tile : drain) + tail;
+      ++best.tried;
+      if (best_cost == 0 || cost < best_cost) { best_cost = cost; best.ksplit = c; best.nb = nb; }
+    }
+  }
+  return best;
+}
+
+}  // namespace b200

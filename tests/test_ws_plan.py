@@ -1,0 +1,67 @@
+"""CPU test of the weight-stationary matmul's choice of token tiles and K slices: the same as a search over every number
+of token tiles, in a number of steps that does not grow with the rows."""
+import os
+import random
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+MAIN = r"""
+#include <cstdio>
+#include "ws_plan.h"
+int main() {
+  long long m, rt; int u, f, c[4];
+  while (std::scanf("%lld %lld %d %d %d %d %d %d", &m, &rt, &u, &f, c, c + 1, c + 2, c + 3) == 8) {
+    const b200::WsSplit s = b200::choose_ws_split(m, rt, u, f, c);
+    std::printf("%d %d %d\n", s.nb, s.ksplit, s.tried);
+  }
+}
+"""
+
+
+def exhaustive(m, row_tiles, units, forced, clusters):
+    """Every number of token tiles in turn, times 1, 2, 4 and 8 slices; the first of equal costs."""
+    best = None
+    mt0 = -(-m // 192)
+    for mt in range(mt0, (1 if m <= 128 else mt0 + mt0 // 2 + 3) + 1):
+        nb = -(-(-(-m // mt)) // 16) * 16
+        tiles = row_tiles * -(-m // nb)
+        for i, c in enumerate((1, 2, 4, 8)):
+            if c > units or (forced and not (c <= forced and (c * 2 > forced or c * 2 > units or c == 8))):
+                continue
+            rounds = -(-tiles // clusters[i])
+            span = max(520 + nb if nb <= 128 else 760 + nb, tiles * c // rounds * (nb * 512 + 18432) // 14000)
+            tile = -(-units // c) * span
+            drain = 300 + 12 * nb if c == 1 else 800 + 50 * nb
+            cost = (0, 500, 2800, 3500)[i] + tile + (rounds - 1) * max(tile, drain) + (drain if c == 1 else 1000 + 35 * nb)
+            if best is None or cost < best[0]:
+                best = (cost, nb, c)
+    return best[1:]
+
+
+@pytest.fixture(scope="module")
+def program(tmp_path_factory):
+    d = tmp_path_factory.mktemp("ws_plan")
+    (d / "main.cc").write_text(MAIN)
+    exe = str(d / "plan")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-Wall", "-Werror", "-I", os.path.join(ROOT, "relax_b200", "csrc"), str(d / "main.cc"),
+                    "-o", exe], check=True)
+    return lambda cases: [tuple(map(int, line.split())) for line in subprocess.run(
+        [exe], input="\n".join(" ".join(map(str, (m, rt, u, f, *c))) for m, rt, u, f, c in cases), capture_output=True, text=True,
+        check=True).stdout.splitlines()]
+
+
+def test_choice_equals_the_exhaustive_search(program):
+    rng = random.Random(7)
+    cases = [(m, rt, 16, 0, (148, 74, 36, 16)) for m in list(range(1, 700)) + [2047, 2048, 5000, 100000] for rt in (1, 32, 172)]
+    cases += [(int(2 ** rng.uniform(0, 15)), rng.randint(1, 300), rng.randint(1, 64), rng.choice((0, 0, 1, 2, 4, 8)),
+               rng.choice(((148, 74, 36, 16), (132, 66, 33, 16), (8, 4, 2, 1)))) for _ in range(3000)]
+    for case, got in zip(cases, program(cases)):
+        assert got[:2] == exhaustive(*case), case
+
+
+def test_the_search_does_not_grow_with_the_rows(program):
+    for m in (2048, 65536, 1_000_000, 0x7fffffff // 64):
+        (nb, ksplit, tried), = program([(m, 86, 16, 0, (148, 74, 36, 16))])
+        assert tried <= 48 and nb in range(16, 193, 16) and ksplit in (1, 2, 4, 8)
