@@ -195,13 +195,17 @@ using namespace b200;
 // Small host transfers as kernels.  A copy-engine transfer on either side of a 5 us matmul costs
 // more than the matmul (each switch between the copy engine and the SMs is a few microseconds), so
 // activations and results up to kHostKernelBytes travel by a kernel that reads or writes the pinned host
-// buffer through its device mapping: 16 bytes per thread and one CTA per 4 KB, so that a read makes one round trip
-// over the bus however many bytes it moves.  The copy lets the matmul start beside it (the matmul reads only weights
+// buffer through its device mapping: 16 bytes per thread and one CTA per 4 KB, up to kHostCopyCtas of them, so that a
+// read of up to 32 KB makes one round trip over the bus; more requests at a time than that slow the larger copies down.
+// Measured, a call among others in us with one CTA per 16 KB / one per 4 KB / the same up to eight: 1 x 4096 x 4096
+// 14.0 / 12.4 / 12.3, 3 x 8640 x 3200 22.6 / 20.3 / 20.4, 4 x 12288 x 4096 21.0 / 23.8 / 21.8, 6 x 4096 x 8192 20.6 / 22.4 / 20.5,
+// 16 x 4096 x 4096 24.7 / 22.1 / 20.6, 16 x 8192 x 8192 34.9 / 32.0 / 30.8; waited for, 8 x 4096 x 11008 33.6 / 34.9 / 30.6.  The copy lets the matmul start beside it (the matmul reads only weights
 // before its own wait), and the result copy is launched as a programmatic dependent of the matmul.  Pageable host
 // memory and larger transfers use cudaMemcpyAsync.
 namespace b200 {
 namespace {
 constexpr size_t kHostKernelBytes = 256 * 1024;
+constexpr size_t kHostCopyCtas = 8;
 
 __global__ void __launch_bounds__(256) host_copy_kernel(const unsigned char* __restrict__ src, unsigned char* __restrict__ dst,
                                                         size_t bytes, int wait_for_primary) {
@@ -229,7 +233,8 @@ void* mapped_host_pointer(const void* host) {
 // of the kernel before it in the stream (the copy waits for that kernel's completion itself).
 int host_copy(const void* src, void* dst, size_t bytes, bool dependent, cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)((bytes + 4095) / 4096));
+  const size_t ctas = (bytes + 4095) / 4096;
+  cfg.gridDim = dim3((unsigned)(ctas < kHostCopyCtas ? ctas : kHostCopyCtas));
   cfg.blockDim = dim3(256);
   cfg.stream = s;
   cudaLaunchAttribute attr[1];

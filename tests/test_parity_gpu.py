@@ -220,6 +220,23 @@ def test_host_buffer_entry_point(cuda_lib, m, n, k, pinned):
     assert np.array_equal(xd.cpu().numpy().view(np.uint16), x.view(np.uint16))
 
 
+@pytest.mark.parametrize("m,n,k", [(4, 4096, 4096), (1, 2047, 16384), (5, 3277, 4064), (8, 16383, 256)])
+def test_host_transfers_around_one_trip_per_thread(cuda_lib, m, n, k):
+    # 32 KB are one trip of the copy kernel's threads: exactly that, a little more and (8 x 16383 results) eight trips,
+    # the last of them incomplete
+    x, wq, s = synth.make_case(m, n, k, seed=m + n)
+    _, twq, ts = dev(x, wq, s)
+    xh, yh = torch.from_numpy(x).pin_memory(), torch.zeros((m, n), dtype=torch.float16).pin_memory()
+    xd, yd = (torch.zeros(shape, dtype=torch.float16, device="cuda") for shape in ((m, k), (m, n)))
+    rc = cuda_lib.b200_q4f16_matmul_host(xh.data_ptr(), xd.data_ptr(), twq.data_ptr(), ts.data_ptr(), yd.data_ptr(), yh.data_ptr(),
+                                         m, n, k, torch.cuda.current_stream().cuda_stream)
+    assert rc == 0, _lib.last_error()
+    torch.cuda.synchronize()
+    assert np.array_equal(xd.cpu().numpy().view(np.uint16), x.view(np.uint16))
+    assert_bits_equal(yh.numpy(), yd.cpu().numpy(), "result on the host")
+    assert_matmul_close(yh.numpy(), x, wq, s, "host buffers")
+
+
 def test_launch_counter(cuda_lib):
     x, wq, s = synth.make_case(1, 64, 128)
     tx, twq, ts = dev(x, wq, s)
