@@ -18,9 +18,11 @@ struct WsSplit {
 // to 128 columns) or 0.9-0.95 us; with many CTAs at work, what they fetch from L2 at about 14 TB/s if that is more.
 // Draining a tile is cheap with one slice (stores to y, behind the next tile's MMAs) and costs the exchange of the
 // partial tiles with several, which the next tile hides only as far as its own MMAs last; a larger cluster starts
-// later.  M = 64, K = 4096, 1 / 2 / 4 / 8 slices: N = 4096 11.0 / 8.7 / 9.0 / 10.8 us, N = 12288 12.9 / 14.3 / 15.6 / 23.2,
+// later, unless (one token tile, four or eight CTAs) the clusters at work leave room for as many again: the set-up of a
+// launch then runs beside the launch before it; in part for more than four clusters of eight.  M = 64, K = 4096, 1 / 2 / 4 / 8 slices: N = 4096 11.0 / 8.7 / 9.0 / 10.8 us, N = 12288 12.9 / 14.3 / 15.6 / 23.2,
 // N = 22016 22.1 / 20.5 / 24.0 / 40.3; N = 4096 and K = 11008: 26.4 / 16.4 / 13.5 / 14.6.  M = 300, N = 12288, K = 4096 in 2 / 3 / 4
-// token tiles: 31.7 / 29.5 / 34.8.
+// token tiles: 31.7 / 29.5 / 34.8.  Few row tiles, M = 64, K = 2048, N = 512: 6.7 / 6.3 / 5.1 / 4.9, N = 1024: 6.7 / 6.3 / 5.2 / 5.8,
+// N = 2048: 6.8 / 6.5 / 5.1 / 7.3; N = 1024, K = 8192: 20.0 / 13.0 / 8.4 / 7.6.
 // M rows of x, row_tiles tiles of 128 weight rows, units spans of 256 k; forced: the largest power of two of slices up to
 // it (0 = by the model); clusters[i]: clusters of 2^i CTAs that run at once.  Every width of a token tile is looked at
 // once, so at most 12 x 4 combinations whatever M is.
@@ -43,8 +45,9 @@ inline WsSplit choose_ws_split(int64_t M, int64_t row_tiles, int units, int forc
       const int64_t span = nb <= 128 ? 520 + nb : 760 + nb;
       const int64_t tile = (int64_t)((units + c - 1) / c) * (span > l2 ? span : l2);   // a tile's MMAs
       const int64_t drain = c == 1 ? 300 + 12 * nb : 800 + 50 * nb;              // ... and what the next tile must hide
-      const int64_t tail = c == 1 ? drain : 1000 + 35 * nb;                      // the last tile's drain
-      const int64_t start = c == 1 ? 0 : c == 2 ? 500 : c == 4 ? 2800 : 3500;
+      const bool room = M <= 128 && c >= 4 && 2 * tiles <= clusters[i] + (c == 8 ? 2 : 0);
+      const int64_t tail = c == 1 ? drain : room ? 900 + 38 * nb : 1000 + 35 * nb;   // the last tile's drain
+      const int64_t start = room ? (c == 8 && tiles > 4 ? 1600 - 8 * nb : 0) : c == 1 ? 0 : c == 2 ? 500 : c == 4 ? 2800 : 3500;
       const int64_t cost = start + tile + (rounds - 1) * (tile > drain ? tile : drain) + tail;
       ++best.tried;
       if (best_cost == 0 || cost < best_cost) { best_cost = cost; best.ksplit = c; best.nb = nb; }

@@ -34,7 +34,10 @@ def exhaustive(m, row_tiles, units, forced, clusters):
             span = max(520 + nb if nb <= 128 else 760 + nb, tiles * c // rounds * (nb * 512 + 18432) // 14000)
             tile = -(-units // c) * span
             drain = 300 + 12 * nb if c == 1 else 800 + 50 * nb
-            cost = (0, 500, 2800, 3500)[i] + tile + (rounds - 1) * max(tile, drain) + (drain if c == 1 else 1000 + 35 * nb)
+            room = m <= 128 and c >= 4 and 2 * tiles <= clusters[i] + (2 if c == 8 else 0)
+            start = (1600 - 8 * nb if c == 8 and tiles > 4 else 0) if room else (0, 500, 2800, 3500)[i]
+            tail = drain if c == 1 else 900 + 38 * nb if room else 1000 + 35 * nb
+            cost = start + tile + (rounds - 1) * max(tile, drain) + tail
             if best is None or cost < best[0]:
                 best = (cost, nb, c)
     return best[1:]
