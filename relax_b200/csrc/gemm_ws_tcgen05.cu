@@ -527,7 +527,7 @@ int max_clusters(int ksplit, const void* kern) {
 
 }  // namespace
 
-// Returns B200_ENOTREADY when the shape is outside what this kernel takes.
+// Returns B200_ENOTREADY when the shape is outside what this kernel takes, or one for the prefill kernel.
 int launch_gemm_ws(const __half* x, const uint32_t* wq, const __half* scales, __half* y, int64_t M, int64_t N,
                    int64_t K, cudaStream_t stream) {
   if (M < 1 || K < 32 || K % 32 != 0) return B200_ENOTREADY;
@@ -544,6 +544,7 @@ int launch_gemm_ws(const __half* x, const uint32_t* wq, const __half* scales, __
   int clusters_of[4];
   for (int i = 0; i < 4; ++i) clusters_of[i] = max_clusters(1 << i, reinterpret_cast<const void*>(kernel_for(16, paired, ragged)));
   const WsSplit split = choose_ws_split(M, row_tiles, units, (int)options().gemm_ws_ksplit, clusters_of);
+  if (options().gemm_ws_ksplit == 0 && prefill_kernel_is_ahead(M, N, K, split, row_tiles, clusters_of[0])) return B200_ENOTREADY;
   const int ksplit = split.ksplit, nb16 = split.nb;
   const int skb = nb16 <= 128 ? 2 : 1;
   auto kern = kernel_for(nb16, paired, ragged);

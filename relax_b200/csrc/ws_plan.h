@@ -56,4 +56,17 @@ inline WsSplit choose_ws_split(int64_t M, int64_t row_tiles, int units, int forc
   return best;
 }
 
+// Whether the prefill kernel's 256 x 256 tiles suit a prompt better.  One wave of them takes a long K as long as three rounds of
+// wide token tiles here, so where these leave more of their last round empty than its wave leaves of the SMs, it is
+// ahead: this kernel / the prefill kernel in us, M x N x K 2048 x 4096 x 8192 104.0 / 103.8, 2048 x 4096 x 11008 142 / 134,
+// 4096 x 2048 x 8192 114 / 111, 4096 x 2048 x 11008 154 / 140, 8192 x 1024 x 8192 126 / 113; with equal shares or a shorter K it is
+// not: 1024 x 8192 x 8192 104 / 105, 2048 x 4096 x 4096 53 / 56, 4096 x 2048 x 4096 54 / 57.
+inline bool prefill_kernel_is_ahead(int64_t M, int64_t N, int64_t K, const WsSplit& split, int64_t row_tiles, int sms) {
+  if (K < 8192 || split.nb < 160 || split.ksplit != 1) return false;
+  const int64_t wave = ((M + 255) / 256) * ((N + 255) / 256);
+  const int64_t tiles = row_tiles * ((M + split.nb - 1) / split.nb);
+  const int64_t rounds = (tiles + sms - 1) / sms;
+  return wave <= sms && rounds >= 3 && 100 * wave * rounds > 100 * tiles + 3 * rounds * sms;
+}
+
 }  // namespace b200

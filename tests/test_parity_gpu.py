@@ -488,6 +488,16 @@ def test_unaligned_scales_mid_batch(cuda_lib):
     assert cuda_lib.b200_device_error_flags() == 0
 
 
+def test_a_long_prompt_that_fills_one_wave_takes_the_prefill_kernel(cuda_lib):
+    m, n, k = 2048, 4000, 8192
+    x, wq, s = synth.make_case(m, n, k, seed=12)
+    out = run_matmul(x, wq, s)
+    sample = np.r_[0:20, 2040:2060, n - 20:n]
+    assert_matmul_close(np.ascontiguousarray(out[:, sample]), x, wq[sample], s[sample], "2048 tokens")
+    assert_bits_equal(out, run_matmul(x, wq, s, family="gemm"), "the prefill kernel's own entry point")
+    assert cuda_lib.b200_device_error_flags() == 0
+
+
 @pytest.mark.parametrize("limit,m,k,family", [(128, 129, 1024, "gemm"), (128, 128, 1024, "gemm_ws"), (0, 40, 1024, "gemm"),
                                               (0, 16, 1024, "gemv"), (15, 16, 1056, "gemv"), (0, 20, 1056, "gemm")])
 def test_a_lowered_row_limit_takes_the_other_kernels(cuda_lib, limit, m, k, family):

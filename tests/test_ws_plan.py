@@ -14,7 +14,7 @@ int main() {
   long long m, rt; int u, f, c[4];
   while (std::scanf("%lld %lld %d %d %d %d %d %d", &m, &rt, &u, &f, c, c + 1, c + 2, c + 3) == 8) {
     const b200::WsSplit s = b200::choose_ws_split(m, rt, u, f, c);
-    std::printf("%d %d %d\n", s.nb, s.ksplit, s.tried);
+    std::printf("%d %d %d %d\n", s.nb, s.ksplit, s.tried, (int)b200::prefill_kernel_is_ahead(m, 128 * rt, 256LL * u, s, rt, c[0]));
   }
 }
 """
@@ -66,5 +66,14 @@ def test_choice_equals_the_exhaustive_search(program):
 
 def test_the_search_does_not_grow_with_the_rows(program):
     for m in (2048, 65536, 1_000_000, 0x7fffffff // 64):
-        (nb, ksplit, tried), = program([(m, 86, 16, 0, (148, 74, 36, 16))])
+        (nb, ksplit, tried, _), = program([(m, 86, 16, 0, (148, 74, 36, 16))])
         assert tried <= 48 and nb in range(16, 193, 16) and ksplit in (1, 2, 4, 8)
+
+
+def test_long_prompts_that_one_wave_of_the_prefill_kernel_holds(program):
+    # as measured: ahead on the left, not on the right
+    for ahead, shapes in ((1, [(2048, 4096, 11008), (4096, 2048, 8192), (2048, 4096, 8192), (8192, 1024, 11008)]),
+                          (0, [(1024, 8192, 8192), (2048, 4096, 4096), (4096, 2048, 4096), (777, 3584, 8192), (2048, 11008, 8192),
+                               (512, 8192, 8192), (128, 8192, 8192), (4096, 4096, 8192)])):
+        got = program([(m, n // 128, k // 256, 0, (148, 74, 36, 16)) for m, n, k in shapes])
+        assert [g[3] for g in got] == [ahead] * len(shapes), list(zip(shapes, got))
