@@ -131,14 +131,16 @@ int matmul_impl(Family fam, const char* who, const void* x, const void* wq, cons
   // ws_plan.h: the launcher says B200_ENOTREADY) and loses the rest (47.0 against 12.3 us at M = 129, N = K = 4096, 163 against
   // 137 at M = 2048, N = 11008).
   // Where K is not a multiple of 256 (or the scales are not 16-byte aligned) the other choice up to 16 rows is the
-  // register-streaming kernel, whose time grows with the rows: it keeps one row and small products, M * N * K < 50 M
-  // (streaming / weight-stationary in us: 4 x 4096 x 2080 5.1 / 5.3, 16 x 1024 x 1056 4.5 / 4.5, 2 x 8640 x 3200 11.0 /
-  // 11.0, 3 x 8640 x 3200 13.8 / 11.0, 8 x 4096 x 2080 7.0 / 5.5, 16 x 22016 x 4128 86 / 24; above 16 rows, against the
-  // prefill kernel, 32 x 8640 x 3200 43 / 11.5, 2048 x 11008 x 4128 188 / 159).
+  // register-streaming kernel, whose time grows with the rows: it keeps one row and small products, M * N * K < 50 M, at two
+  // rows < 100 M where K < 5000 (streaming / weight-stationary in us: 4 x 4096 x 2080 5.1 / 5.3, 16 x 1024 x 1056 4.5 / 4.5;
+  // 2 x 8192 x 3200 9.4 / 10.7, 2 x 11008 x 4128 13.3 / 16.2, with weights from HBM 15.3 / 15.6, 2 x 22016 x 2080 13.7 / 15.1, but
+  // 2 x 8192 x 5152 21.6 / 19.0 and 2 x 16384 x 3200 16.1 / 13.7; 3 x 8640 x 3200 13.8 / 11.0, 8 x 4096 x 2080 7.0 / 5.5,
+  // 16 x 22016 x 4128 86 / 24; above 16 rows, against the prefill kernel, 32 x 8640 x 3200 43 / 11.5, 2048 x 11008 x 4128 188 / 159).
   // (Above a gemm.ws_max_m that was lowered the skinny and prefill kernels take over, and a variant of the skinny kernel
   // asked for by option keeps its rows.)
   const bool ragged = K % 256 != 0 || !aligned16(scales);
-  const bool ws_auto = M > 16 || (ragged ? M >= 2 && M * N * K >= 50000000 : M >= 9 || (M >= 5 && K >= 8192));
+  const int64_t streamed = M == 2 && K < 5000 ? 100000000 : 50000000;
+  const bool ws_auto = M > 16 || (ragged ? M >= 2 && M * N * K >= streamed : M >= 9 || (M >= 5 && K >= 8192));
   if (fam == kGemmWs || (fam == kAuto && ws_auto && M <= options().gemm_ws_max_m && (M > 16 || options().gemv_variant == 0))) {
     rc = fam == kGemmWs && (M > 128 || ragged) ? B200_ENOTREADY : launch_gemm_ws(xh, wh, sh, yh, M, N, K, s);
     if (rc != B200_ENOTREADY) return rc;
