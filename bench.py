@@ -406,10 +406,11 @@ def run_decode(args, world, rank, dev, batches):
 
 # dram__bytes_read.sum + dram__bytes_write.sum per launch of the dominant kernel, from the ncu captures
 # summarised under profiles/ (one capture per kernel change; not re-measured by this script).
+NCU_SOURCE = ": dram__bytes_read.sum + dram__bytes_write.sum of one launch under ncu, captured beforehand and not re-measured by this run"
 NCU_TRAFFIC_BYTES = {
-    ("gemv", 1, 4096, 4096): (9476352, "profiles/gemv_pipe_kernel__decode_gemv_M1_N4096_K4096.md (ncu capture, not re-measured by this run)"),
-    ("gemv", 64, 4096, 4096): (10000384, "profiles/gemm_ws_tcgen05_kernel__M64_and_prefill.md (ncu capture, not re-measured by this run)"),
-    ("prefill", 2048, 11008, 4096): (42176768 + 12126976, "profiles/gemm_ws_tcgen05_kernel__M64_and_prefill.md (ncu capture, not re-measured by this run)"),
+    ("gemv", 1, 4096, 4096): (9476352, "q4f16_gemv_pipe_kernel" + NCU_SOURCE),
+    ("gemv", 64, 4096, 4096): (10003456, "q4f16_gemm_ws_tcgen05_kernel" + NCU_SOURCE),
+    ("prefill", 2048, 11008, 4096): (42205440 + 12076544, "q4f16_gemm_ws_tcgen05_kernel" + NCU_SOURCE),
 }
 
 

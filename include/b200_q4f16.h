@@ -107,8 +107,8 @@ B200_API int b200_q4f16_gemm(const void* x, const void* wq, const void* scales, 
 /* Weight-stationary tensor-core kernel for mid-sized batches (1 <= M <= 128, K % 256 == 0, scales
  * 16-byte aligned): 128 weight rows are the MMA's M, the batch its N, K is split over a thread-block
  * cluster whose partial tiles are added through distributed shared memory.  b200_q4f16_matmul picks
- * it for M >= 9 (in token tiles above 192 rows), for M >= 5 where K >= 8192, and from 2 rows on where
- * K % 256 != 0 and the product is large. */
+ * it for M >= 9 (above 128 rows in token tiles of up to 192), for M >= 5 where K >= 8192, and from 2 rows
+ * on where K % 256 != 0 and the product is large. */
 B200_API int b200_q4f16_gemm_ws(const void* x, const void* wq, const void* scales, void* y, int64_t M, int64_t N,
                                 int64_t K, void* cuda_stream);
 

@@ -120,7 +120,7 @@ int matmul_impl(Family fam, const char* who, const void* x, const void* wq, cons
   auto wh = static_cast<const uint32_t*>(wq);
   auto sh = static_cast<const __half*>(scales);
   auto yh = static_cast<__half*>(y);
-  // 9 rows and more, and 5..8 where K is long: the weight-stationary kernel, whose weights stream once up to 192 rows.
+  // 9 rows and more, and 5..8 where K is long: the weight-stationary kernel, whose weights stream once up to 128 rows.
   // Measured on B200, skinny / weight-stationary kernel in us at 4, 8 and 16 rows: N = K = 4096 6.0 / 6.1, 7.7 / 6.4,
   // 11.1 / 6.5; N = 22016 16.5 / 17.9, 17.9 / 18.1, 24.4 / 18.4; N = 4096, K = 11008 11.8 / 12.2, 18.9 / 12.3, 29.3 / 12.5;
   // N = 1280, K = 8192 6.6 / 5.9, 9.7 / 6.0, 17.0 / 6.1 (the skinny kernel stages all of x in every CTA, and its
@@ -202,9 +202,9 @@ using namespace b200;
 // read of up to 32 KB makes one round trip over the bus; more requests at a time than that slow the larger copies down.
 // Measured, a call among others in us with one CTA per 16 KB / one per 4 KB / the same up to eight: 1 x 4096 x 4096
 // 14.0 / 12.4 / 12.3, 3 x 8640 x 3200 22.6 / 20.3 / 20.4, 4 x 12288 x 4096 21.0 / 23.8 / 21.8, 6 x 4096 x 8192 20.6 / 22.4 / 20.5,
-// 16 x 4096 x 4096 24.7 / 22.1 / 20.6, 16 x 8192 x 8192 34.9 / 32.0 / 30.8; waited for, 8 x 4096 x 11008 33.6 / 34.9 / 30.6.  The copy lets the matmul start beside it (the matmul reads only weights
-// before its own wait), and the result copy is launched as a programmatic dependent of the matmul.  Pageable host
-// memory and larger transfers use cudaMemcpyAsync.
+// 16 x 4096 x 4096 24.7 / 22.1 / 20.6, 16 x 8192 x 8192 34.9 / 32.0 / 30.8; waited for, 8 x 4096 x 11008 33.6 / 34.9 / 30.6.
+// The copy lets the matmul start beside it (the matmul reads only weights before its own wait), and the result copy is
+// launched as a programmatic dependent of the matmul.  Pageable host memory and larger transfers use cudaMemcpyAsync.
 namespace b200 {
 namespace {
 constexpr size_t kHostKernelBytes = 256 * 1024;

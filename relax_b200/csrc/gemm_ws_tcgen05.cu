@@ -1,4 +1,5 @@
-// q4f16 matmul on the 5th-generation tensor cores (the dispatcher gives it 9 rows and more, and 5..8 with a long K): y[M,N] = x[M,K] . decode(Wq,S)^T.
+// q4f16 matmul on the 5th-generation tensor cores (the dispatcher gives it 9 rows and more, and fewer with a long or a
+// ragged K): y[M,N] = x[M,K] . decode(Wq,S)^T.
 //
 // Decode at batches up to 128 is still bound by streaming the weights once, so the roles of a plain GEMM are swapped:
 // the MMA's M dimension is 128 WEIGHT rows (A operand), its N dimension are tokens (B operand = x, 16..192 columns).
@@ -8,10 +9,10 @@
 // (no 16 KB of stores and 16 KB of operand reads per 64 k), no proxy fence stands between conversion and MMA, and
 // the room goes to the rings.
 //
-// Work: a tile is 128 weight rows by up to 192 tokens over the whole K (a prompt is cut into equal token tiles).  The CTAs of a cluster share tiles: CTA r takes the r-th slice of
-// K of every tile of the cluster's list (tile = cluster, cluster + clusters, ...), so the kernel starts once however
-// many tiles there are (a second wave of CTAs cost 7 us), and x of a slice stays in shared memory for all tiles where
-// it fits.  The accumulator is double-buffered: the next tile's MMAs run while the epilogue drains this one's.  The
+// Work: a tile is 128 weight rows by up to 192 tokens over the whole K (above 128 rows x is cut into equal token
+// tiles).  The CTAs of a cluster share tiles: CTA r takes the r-th slice of K of every tile of the cluster's list (tile =
+// cluster, cluster + clusters, ...), so the kernel starts once however many tiles there are (a second wave of CTAs
+// cost 7 us), and x of a slice stays in shared memory for all tiles where it fits.  The accumulator is double-buffered: the next tile's MMAs run while the epilogue drains this one's.  The
 // partial tiles are exchanged by 16-byte stores into the owners' shared memory (owner o of a tile: batch columns
 // [o * cw, (o + 1) * cw)) and added up there in rank order: deterministic, no atomics, no scratch in global memory.
 //
@@ -27,8 +28,7 @@
 //               slice, straight to y); two warps per TMEM quadrant share the columns
 //
 // What bounds it (measured at a batch of 64): 0.56 us per 256-k span and CTA, of which 0.37-0.39 us is the delivery of
-// the span's 18 KB (a copy of the kernel without the conversion) and the rest the conversion's 16 instructions per packed
-// word; the MMAs (45 clocks each or less) are hidden.  Before, with A in shared memory, the MMAs issued under a
+// the span's 18 KB (a copy of the kernel without the conversion) and the rest the conversion; the MMAs (45 clocks each or less) are hidden.  Before, with A in shared memory, the MMAs issued under a
 // branch on one lane and a grid of one tile per CTA: M = 64, N = 22016, K = 4096 46.1 -> 20.2 us; N = 12288
 // 23.3 -> 12.9; N = K = 4096 11.0 -> 9.0; N = 4096, K = 11008 18.9 -> 13.6; M = 128, N = 22016 49.5 -> 25.0; M = 16,
 // N = K = 4096 9.7 -> 6.5.  With many tokens the SMs' fetches of x from L2 (a tile's x serves 128 weight rows) are the

@@ -201,7 +201,7 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
   static_assert(kStageBytes % 1024 == 0, "stage alignment");
   extern __shared__ unsigned char smem_unaligned[];
   // Round the base up to 1024 bytes by OFFSETTING the shared array (not by casting through an
-  // integer): the compiler then still knows these are shared-memory addresses and emits LDS/STS.
+  // integer): the pointer stays one into shared memory.
   unsigned char* ring = smem_unaligned + ((1024u - (smem_u32(smem_unaligned) & 1023u)) & 1023u);
   uint64_t* full = reinterpret_cast<uint64_t*>(ring + (size_t)p.nstages * kStageBytes);
   uint64_t* empty = full + kMaxStages;

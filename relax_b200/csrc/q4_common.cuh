@@ -19,11 +19,8 @@ __device__ __forceinline__ uint32_t h2_as_u32(__half2 v) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
-// Masks and the magic number live in constant memory on purpose.  Written as literals, ptxas
-// encodes (w & mask) | magic as TWO instructions (an instruction has room for one 32-bit
-// immediate); with the operands coming from the constant bank it is one LOP3, which halves the
-// integer-pipe work of the unpack (measured: 8.2 -> 4.1 logic instructions per packed word, and
-// the integer pipe was the busiest unit of the skinny matmul).
+// Masks and the magic number live in constant memory and reach (w & mask) | magic as three register operands of
+// the one lop3.b32 below; the integer pipe was the busiest unit of the skinny matmul (ncu).
 static __constant__ uint32_t kQ4Bits[5] = {0x000F000Fu, 0x00F000F0u, 0x64006400u, 0x00F0000Fu, 0x54006400u};
 
 // (a & b) | c in one LOP3.
