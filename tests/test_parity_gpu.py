@@ -437,6 +437,27 @@ def test_token_tiles(cuda_lib, m, n, k, ksplit):
     assert cuda_lib.b200_device_error_flags() == 0
 
 
+@pytest.mark.parametrize("m,n,k,ksplit", [(20, 3000, 2048, 1), (20, 3000, 2048, 4), (100, 1300, 1056, 2), (190, 20000, 1024, 0)])
+def test_shallow_rings_do_not_change_the_result(cuda_lib, m, n, k, ksplit):
+    # the caps on the x ring and on the packed ring (rounded down to an even depth) change when a load is issued, not what
+    # is added up: bit for bit the default's result
+    x, wq, s = synth.make_case(m, n, k, seed=m + n)
+    tx, twq, ts = dev(x, wq, s)
+    try:
+        relax_b200.set_option("gemm.ws_ksplit", ksplit)
+        want = ops.q4f16_matmul(tx, twq, ts).cpu().numpy()
+        for x_stages, r_stages in ((2, 2), (3, 0), (0, 2), (8, 3), (1, 5)):
+            relax_b200.set_option("gemm.ws_x_stages", x_stages)
+            relax_b200.set_option("gemm.ws_r_stages", r_stages)
+            assert_bits_equal(ops.q4f16_matmul(tx, twq, ts).cpu().numpy(), want, f"x_stages {x_stages} r_stages {r_stages}")
+    finally:
+        for name in ("gemm.ws_ksplit", "gemm.ws_x_stages", "gemm.ws_r_stages"):
+            relax_b200.set_option(name, 0)
+    rows = np.arange(300)
+    assert_matmul_close(np.ascontiguousarray(want[:, rows]), x, wq[rows], s[rows], f"M={m} ksplit={ksplit}")
+    assert cuda_lib.b200_device_error_flags() == 0
+
+
 @pytest.mark.parametrize("ksplit", [2, 4, 8])
 @pytest.mark.parametrize("m", [64, 200])
 def test_partial_tile_exchange_repeats_bit_for_bit(cuda_lib, m, ksplit):
