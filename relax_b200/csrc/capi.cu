@@ -128,8 +128,8 @@ int matmul_impl(Family fam, const char* who, const void* x, const void* wq, cons
   // decode step, where two of its CTAs fit an SM and it starts beside the kernel before it (8 layers of hidden
   // 2048 at 5 rows: 413 us with it, 440 without).  Above 128 rows it cuts the tokens into tiles to suit the shape; the
   // prefill kernel with its 256-token tiles keeps the long prompts that one wave of them holds (prefill_kernel_is_ahead in
-  // ws_plan.h: the launcher says B200_ENOTREADY) and loses the rest (47.0 against 12.3 us at M = 129, N = K = 4096, 163 against
-  // 137 at M = 2048, N = 11008).
+  // ws_plan.h: the launcher says B200_ENOTREADY) and loses the rest (44 against 11.8 us at M = 129, N = K = 4096, 164 against
+  // 134-140 at M = 2048, N = 11008).
   // Where K is not a multiple of 256 (or the scales are not 16-byte aligned) the other choice up to 16 rows is the
   // register-streaming kernel, whose time grows with the rows: it keeps one row and small products, M * N * K < 50 M, at two
   // rows < 100 M where K < 5000 (streaming / weight-stationary in us: 4 x 4096 x 2080 5.1 / 5.3, 16 x 1024 x 1056 4.5 / 4.5;

@@ -28,14 +28,14 @@
 //               slice, straight to y); two warps per TMEM quadrant share the columns
 //
 // What bounds it (measured at a batch of 64): 0.56 us per 256-k span and CTA, of which 0.37-0.39 us is the delivery of
-// the span's 18 KB (a copy of the kernel without the conversion) and the rest the conversion; the MMAs (45 clocks each or less) are hidden.  Before, with A in shared memory, the MMAs issued under a
-// branch on one lane and a grid of one tile per CTA: M = 64, N = 22016, K = 4096 46.1 -> 20.2 us; N = 12288
-// 23.3 -> 12.9; N = K = 4096 11.0 -> 9.0; N = 4096, K = 11008 18.9 -> 13.6; M = 128, N = 22016 49.5 -> 25.0; M = 16,
-// N = K = 4096 9.7 -> 6.5.  With many tokens the SMs' fetches of x from L2 (a tile's x serves 128 weight rows) are the
-// limit, about 14 TB/s over all SMs, and at the largest sizes the power cap.  Against the prefill kernel, whose
-// 256-token tiles leave SMs idle up to about 1000 tokens: K = 4096, N = 4096 at 129 tokens 47.0 -> 12.3 us, at 512
-// 47.6 -> 18.2; N = 3584, K = 8192 at 777 88.8 -> 38.0; N = 11008 at 2048 163 -> 137 (1350 TFLOP/s, where the library's
-// fp16 matmul under the same power cap reaches 1386).
+// the span's 18 KB (a copy of the kernel without the conversion) and the rest the conversion; the MMAs (45 clocks
+// each or less) are hidden.  Before, with A in shared memory, the MMAs issued under a branch on one lane and a grid of
+// one tile per CTA, us in a chain over more weights than the L2 holds: M = 64, N = 22016, K = 4096 46.1 -> 20.0; N = 12288
+// 23.3 -> 13.0; N = K = 4096 11.0 -> 9.2; N = 4096, K = 11008 18.9 -> 13.8; M = 128, N = 22016 49.5 -> 24.8; M = 16, N = K = 4096
+// 9.7 -> 6.9.  With many tokens the SMs' fetches of x from L2 (a tile's x serves 128 weight rows) are the limit, about
+// 14 TB/s over all SMs, and at the largest sizes the power cap.  Against the prefill kernel, whose 256-token tiles leave
+// SMs idle up to about 1000 tokens: K = 4096, N = 4096 at 129 tokens 44 -> 11.8 us, at 512 45 -> 15.8; N = 3584, K = 8192 at
+// 777 84 -> 37; N = 11008 at 2048 164 -> 134-140 (1320-1380 TFLOP/s; 1249-1265 over 0.2 s).
 //
 // Launched with programmatic dependent launch: set-up and the weight loads run ahead of the previous
 // kernel's end; the loads of x and the stores of y wait for it.
