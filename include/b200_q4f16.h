@@ -202,6 +202,13 @@ B200_API int32_t b200_q4f16_dequantize_packed(void* args, int* type_codes, int n
 B200_API int b200_q4f16_gemv_rmsnorm(const void* x, const void* delta, const void* norm_w, void* x_out, float eps,
                                      const void* wq, const void* scales, void* y, int64_t M, int64_t N, int64_t K,
                                      void* cuda_stream);
+/* gemv_gate_up: act fp16 [M, I] = silu(h . Wg^T) * (h . Wu^T), W [2I, K] = gate rows | up rows, h = x, or gemv_rmsnorm's
+ * normalised activation where norm_w is given (delta and x_out only then).  The product is formed in the matmul's
+ * epilogue from its fp16-rounded results: the values of gemv_rmsnorm (or the plain skinny matmul) followed by b200_silu_mul,
+ * without the [M, 2I] buffer.  I % 8 == 0. */
+B200_API int b200_q4f16_gemv_gate_up(const void* x, const void* delta, const void* norm_w, void* x_out, float eps,
+                                     const void* wq, const void* scales, void* act, int64_t M, int64_t I, int64_t K,
+                                     void* cuda_stream);
 /* gemv_rmsnorm for the qkv projection of ONE decode row, with b200_rope_kv_append in its epilogue: the matmul's
  * rows are [q heads | k heads | v heads] (heads of 128); q is rotated (rotate-half pairing d <-> d+64, tables fp32
  * [max_pos, 64], position *pos) into q_out fp16 [heads*128], the rotated key and the value of the new token go

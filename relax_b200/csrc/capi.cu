@@ -468,6 +468,29 @@ int b200_q4f16_gemv_rmsnorm_rope(const void* x, const void* delta, const void* n
                                        static_cast<__half*>(v_cache), heads, K, static_cast<cudaStream_t>(stream));
 }
 
+int b200_q4f16_gemv_gate_up(const void* x, const void* delta, const void* norm_w, void* x_out, float eps, const void* wq,
+                            const void* scales, void* act, int64_t M, int64_t I, int64_t K, void* stream) {
+  const char* who = "q4f16_gemv_gate_up";
+  if (I < 8 || I % 8 != 0 || I > 0x3fffffffLL / 32) return fail(B200_EINVAL, "%s: needs I a positive multiple of 8, got %lld", who, (long long)I);
+  int rc = check_matmul(who, x, wq, scales, act, M, 2 * I, K);
+  if (rc) return rc;
+  if (M < 1 || M > 16) return fail(B200_EINVAL, "%s: takes 1 <= M <= 16, got %lld", who, (long long)M);
+  if (K < 256 || K % 256 != 0) return fail(B200_EINVAL, "%s: needs K a positive multiple of 256", who);
+  if (!aligned16(scales)) return fail(B200_EINVAL, "%s: scales must be 16-byte aligned", who);
+  if (!norm_w && (delta || x_out)) return fail(B200_EINVAL, "%s: delta and x_out go with a norm weight", who);
+  if (!aligned16(norm_w)) return fail(B200_EINVAL, "%s: norm weight must be 16-byte aligned", who);
+  if ((delta && !aligned16(delta)) || (x_out && !aligned16(x_out))) return fail(B200_EINVAL, "%s: delta / x_out must be 16-byte aligned", who);
+  if (x_out == x) return fail(B200_EINVAL, "%s: x_out must not alias x (other CTAs still read x)", who);
+  rc = ensure_device();
+  if (rc) return rc;
+  rc = launch_gemv_pipe_gate_up(static_cast<const __half*>(x), static_cast<const __half*>(delta), static_cast<const __half*>(norm_w),
+                                static_cast<__half*>(x_out), eps, static_cast<const uint32_t*>(wq),
+                                static_cast<const __half*>(scales), static_cast<__half*>(act), M, I, K,
+                                static_cast<cudaStream_t>(stream));
+  if (rc == B200_ENOTREADY) return fail(B200_EINVAL, "%s: shape outside the fused kernel's domain", who);
+  return rc;
+}
+
 int b200_q4f16_gemv_swiglu(const void* gu, const void* wq, const void* scales, void* y, int64_t M, int64_t N, int64_t K,
                            void* stream) {
   const char* who = "q4f16_gemv_swiglu";

@@ -182,7 +182,10 @@ __device__ __forceinline__ void fast_stage_fn(float (&acc)[2][MT][4], const uint
 //   accs:  tiles_per_cta * kOut * 4 (only when K is cut into several blocks)
 //
 // Warps: CW consumers, then one TMA warp (two issuing lanes), then one epilogue warp.
-template <int NC, int CW, int CH, int PRO, bool FAST>
+//
+// GU: W's rows are [gate: N / 2 | up: N / 2]; a tile takes eight of each and the epilogue stores silu(gate) * up, [M, N / 2].  A
+// form of its own: as a run-time flag it cost the plain batch-1 matmul 2.9 % (182.5 -> 187.8 us for 40 of N = K = 4096).
+template <int NC, int CW, int CH, int PRO, bool FAST, bool GU>
 __global__ void __launch_bounds__((CW + 2) * 32, FAST ? 2 : 1)
 q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
   constexpr int MT = (NC + 7) / 8;
@@ -276,6 +279,10 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
               mbar_arrive_expect_tx(&full[s], is_w ? kWBytes : kSBytes);
               tma_load_5d_hint(is_w ? st : st + kWBytes, is_w ? &p.tm_w : &p.tm_s, 0, (tile & 7) * 8, 0, tile >> 3, k0 >> 8,
                                &full[s], policy);
+            } else if (GU) {
+              // tile = 8 gate rows and the 8 up rows that they are multiplied with
+              mbar_arrive_expect_tx(&full[s], is_w ? kWBytes : kSBytes);
+              tma_load_4d_hint(is_w ? st : st + kWBytes, is_w ? &p.tm_w : &p.tm_s, 0, tile * 8, 0, k0 >> 8, &full[s], policy);
             } else if (is_w) {
               mbar_arrive_expect_tx(&full[s], kWBytes);
               tma_load_3d_hint(st, &p.tm_w, 0, row0, k0 >> 8, &full[s], policy);
@@ -316,6 +323,7 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
           }
         }
         const float* rbuf = red + rb * (CW * kOut);
+        float gate[2];                             // GU, exact form: row g's values until row g + 8's are known
 #pragma unroll
         for (int q = 0; q < (kOut + 31) / 32; ++q) {
           const int e = q * 32 + lane;
@@ -341,6 +349,28 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
               else if (u < 2 * nh) p.rope.k_cache[((int64_t)rope_pos * nh + (u - nh)) * 128 + d] = __float2half_rn(rot);
               else p.rope.v_cache[((int64_t)rope_pos * nh + (u - 2 * nh)) * 128 + d] = __float2half_rn(vr);
             }
+          } else if (GU && kb == nkb - 1) {
+            // rows 0..7 of the tile are gate rows, 8..15 the up rows of the same outputs; SwiGLU works on the fp16-rounded
+            // matmul results, as the separate kernel does
+            const float vr = __half2float(__float2half_rn(sum));
+            int col;
+            float g, u;
+            bool mine;
+            if (FAST) {
+              u = __shfl_xor_sync(0xffffffffu, vr, 16);
+              g = vr;
+              col = 0;
+              mine = (lane & 17) == 0;
+            } else {
+              const int i = q & 3;
+              if (i < 2) gate[i & 1] = vr;
+              g = gate[i & 1];
+              u = vr;
+              col = (q >> 2) * 8 + 2 * (lane & 3) + (i & 1);
+              mine = i >= 2 && col < p.M;
+            }
+            const int out = tile * 8 + (FAST ? lane >> 1 : lane >> 2);
+            if (mine) p.y[(int64_t)col * (p.N >> 1) + out] = __float2half_rn(g / (1.f + __expf(-g)) * u);
           } else if (kb == nkb - 1) {
             int row, col;
             if (FAST) {
@@ -880,7 +910,7 @@ struct Prologue {
   RopeOut rope;          // rotary embedding + KV append in the epilogue (qkv matmul of a batch-1 step)
 };
 
-template <int NC, int CW, int CH, int PRO, bool FAST>
+template <int NC, int CW, int CH, int PRO, bool FAST, bool GU>
 int launch_pipe(const __half* x, const uint32_t* wq, const __half* scales, __half* y, int M, int N, int K,
                 cudaStream_t stream, const Prologue& pro, const PeerReduce& red) {
   constexpr int MT = (NC + 7) / 8;
@@ -891,7 +921,20 @@ int launch_pipe(const __half* x, const uint32_t* wq, const __half* scales, __hal
   using XL = XLayout<NC>;
   PipeParams p;
   p.rope = pro.rope;
-  if (pro.rope.on) {
+  if (GU) {
+    // rows as {row: N/2 | half: 2}, tile = 8 rows x 2 halves
+    const uint64_t wd[4] = {32, (uint64_t)(N / 2), 2, (uint64_t)(K / 256)};
+    const uint64_t ws[3] = {(uint64_t)K / 2, (uint64_t)K / 2 * (N / 2), 128};
+    const uint32_t wb[4] = {32, 8, 2, CH};
+    int rc = make_tmap(&p.tm_w, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, wq, wd, ws, wb, CU_TENSOR_MAP_SWIZZLE_128B);
+    if (rc) return rc;
+    const uint64_t rp = (uint64_t)(K / 32) * 2;    // bytes per row of scales
+    const uint64_t sd[4] = {8, (uint64_t)(N / 2), 2, (uint64_t)(K / 256)};
+    const uint64_t ss[3] = {rp, rp * (N / 2), 16};
+    const uint32_t sb[4] = {8, 8, 2, CH};
+    rc = make_tmap(&p.tm_s, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, scales, sd, ss, sb, CU_TENSOR_MAP_SWIZZLE_NONE);
+    if (rc) return rc;
+  } else if (pro.rope.on) {
     // the fast form's epilogue layout, one K block, whole 128-row units
     if (!FAST || NC != 1 || M != 1 || N % 128 != 0 || N != 3 * pro.rope.nh * 128) return B200_ENOTREADY;
     // rows as {dim in half: 64 | half: 2 | unit: N/128}, tile = 8 dims x 2 halves of one unit
@@ -928,7 +971,7 @@ int launch_pipe(const __half* x, const uint32_t* wq, const __half* scales, __hal
   const int stages_per_tile = kpad / KC;
   const size_t kMaxSmem = 227 * 1024;
   const int sms = sm_count();
-  auto kern = q4f16_gemv_pipe_kernel<NC, CW, CH, PRO, FAST>;
+  auto kern = q4f16_gemv_pipe_kernel<NC, CW, CH, PRO, FAST, GU>;
   // Ask for the largest shared-memory carve-out: the default picks the smallest that fits ONE CTA,
   // which would keep further CTAs (or the next dependent launch) off the SM.
   cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
@@ -1037,7 +1080,7 @@ int launch_pipe(const __half* x, const uint32_t* wq, const __half* scales, __hal
   return B200_OK;
 }
 
-template <int CW, int CH, int PRO>
+template <int CW, int CH, int PRO, bool GU>
 int launch_pipe_m(const __half* x, const uint32_t* wq, const __half* scales, __half* y, int m, int n, int k,
                   cudaStream_t stream, const Prologue& pro, const PeerReduce& red) {
   if (m == 1) {
@@ -1048,28 +1091,29 @@ int launch_pipe_m(const __half* x, const uint32_t* wq, const __half* scales, __h
     // 2816, 4.88 / 4.58 at 4096, 7.26 / 6.80 at 8192, 9.16 / 8.72 at 11008 (and 14.3 / 12.9 at N = 22016, K = 4096).
     // gemv.exact = 2 forces the fast form for every K (tests).
     const bool fast = options().gemv_exact == 2 || (options().gemv_exact == 0 && k >= 2560);
-    if (fast) return launch_pipe<1, CW, CH, PRO, true>(x, wq, scales, y, m, n, k, stream, pro, red);
-    return launch_pipe<1, CW, CH, PRO, false>(x, wq, scales, y, m, n, k, stream, pro, red);
+    if (fast) return launch_pipe<1, CW, CH, PRO, true, GU>(x, wq, scales, y, m, n, k, stream, pro, red);
+    return launch_pipe<1, CW, CH, PRO, false, GU>(x, wq, scales, y, m, n, k, stream, pro, red);
   }
-  if (m == 2) return launch_pipe<2, CW, CH, PRO, false>(x, wq, scales, y, m, n, k, stream, pro, red);
-  if (m <= 4) return launch_pipe<4, CW, CH, PRO, false>(x, wq, scales, y, m, n, k, stream, pro, red);
-  if (m <= 8) return launch_pipe<8, CW, CH, PRO, false>(x, wq, scales, y, m, n, k, stream, pro, red);
-  return launch_pipe<16, CW, CH, PRO, false>(x, wq, scales, y, m, n, k, stream, pro, red);
+  if (m == 2) return launch_pipe<2, CW, CH, PRO, false, GU>(x, wq, scales, y, m, n, k, stream, pro, red);
+  if (m <= 4) return launch_pipe<4, CW, CH, PRO, false, GU>(x, wq, scales, y, m, n, k, stream, pro, red);
+  if (m <= 8) return launch_pipe<8, CW, CH, PRO, false, GU>(x, wq, scales, y, m, n, k, stream, pro, red);
+  return launch_pipe<16, CW, CH, PRO, false, GU>(x, wq, scales, y, m, n, k, stream, pro, red);
 }
 
-template <int PRO>
+template <int PRO, bool GU = false>
 int dispatch_form(const __half* x, const uint32_t* wq, const __half* scales, __half* y, int m, int n, int k,
                   cudaStream_t stream, const Prologue& pro, const PeerReduce& red) {
-  return launch_pipe_m<8, 16, PRO>(x, wq, scales, y, m, n, k, stream, pro, red);
+  return launch_pipe_m<8, 16, PRO, GU>(x, wq, scales, y, m, n, k, stream, pro, red);
 }
 
+template <bool GU = false>
 int dispatch_pipe(const __half* x, const uint32_t* wq, const __half* scales, __half* y, int64_t M, int64_t N, int64_t K,
                   cudaStream_t stream, const Prologue& pro, const PeerReduce& red) {
   if (K % 256 != 0 || (reinterpret_cast<uintptr_t>(scales) & 15u)) return B200_ENOTREADY;
   int m = (int)M, n = (int)N, k = (int)K;
-  if (pro.kind == kPrologueRmsNorm) return dispatch_form<kPrologueRmsNorm>(x, wq, scales, y, m, n, k, stream, pro, red);
-  if (pro.kind == kPrologueSwiGLU) return dispatch_form<kPrologueSwiGLU>(x, wq, scales, y, m, n, k, stream, pro, red);
-  return dispatch_form<kPrologueNone>(x, wq, scales, y, m, n, k, stream, pro, red);
+  if (pro.kind == kPrologueRmsNorm) return dispatch_form<kPrologueRmsNorm, GU>(x, wq, scales, y, m, n, k, stream, pro, red);
+  if (!GU && pro.kind == kPrologueSwiGLU) return dispatch_form<kPrologueSwiGLU>(x, wq, scales, y, m, n, k, stream, pro, red);
+  return dispatch_form<kPrologueNone, GU>(x, wq, scales, y, m, n, k, stream, pro, red);
 }
 
 // The sum over tensor-parallel ranks as a kernel of its own, for partial results that another kernel produced
@@ -1200,6 +1244,19 @@ int launch_gemv_pipe_rmsnorm_rope(const __half* x, const __half* delta, const __
   pro.rope.q_out = q_out; pro.rope.k_cache = k_cache; pro.rope.v_cache = v_cache;
   pro.rope.nh = (int)nh; pro.rope.on = 1;
   return dispatch_pipe(x, wq, scales, q_out /* unused */, 1, 3 * nh * 128, K, stream, pro, PeerReduce{});
+}
+
+// act = silu(h . Wg^T) * (h . Wu^T) for W = [Wg: I rows | Wu: I rows], h = x, or rmsnorm(fp16(x + delta)) * norm_w where a norm
+// weight is given.  The product is formed once per output in the epilogue; as a prologue of the next matmul every CTA
+// forms all of it again.
+int launch_gemv_pipe_gate_up(const __half* x, const __half* delta, const __half* norm_w, __half* x_out, float eps,
+                             const uint32_t* wq, const __half* scales, __half* act, int64_t M, int64_t I, int64_t K,
+                             cudaStream_t stream) {
+  Prologue pro;
+  if (norm_w) {
+    pro.kind = kPrologueRmsNorm; pro.delta = delta; pro.norm_w = norm_w; pro.x_out = x_out; pro.eps = eps;
+  }
+  return dispatch_pipe<true>(x, wq, scales, act, M, 2 * I, K, stream, pro, PeerReduce{});
 }
 
 // y = (silu(gu[:, :K]) * gu[:, K:]) . decode(W)^T

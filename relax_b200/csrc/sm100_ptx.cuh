@@ -161,6 +161,14 @@ __device__ __forceinline__ void tma_load_3d_hint(void* smem_dst, const void* tma
       "l"(tmap), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "l"(policy)
       : "memory");
 }
+__device__ __forceinline__ void tma_load_4d_hint(void* smem_dst, const void* tmap, int32_t c0, int32_t c1, int32_t c2,
+                                                 int32_t c3, uint64_t* bar, uint64_t policy) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4, %5, %6}], [%2], %7;" ::"r"(
+          smem_u32(smem_dst)),
+      "l"(tmap), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "l"(policy)
+      : "memory");
+}
 __device__ __forceinline__ void tma_load_5d_hint(void* smem_dst, const void* tmap, int32_t c0, int32_t c1, int32_t c2,
                                                  int32_t c3, int32_t c4, uint64_t* bar, uint64_t policy) {
   asm volatile(

@@ -93,6 +93,10 @@ def to_device(layer: dict, device):
     return out
 
 
+def _aligned(layers) -> bool:
+    return all(l["gu"][1].data_ptr() % 16 == 0 for l in layers)
+
+
 class DecodeEngine:
     """Buffers and kernel sequence of one decode step for `batch` sequences.
 
@@ -120,12 +124,13 @@ class DecodeEngine:
         f16 = dict(dtype=torch.float16, device=self.device)
         hl = H // world
         il_max = max(l["inter_local"] for l in layers) if layers else cfg.inter
-        # fused: RMSNorm (+ residual add) and SwiGLU run inside the staging of the next skinny matmul
-        # (7 kernels per layer instead of 11); needs batch <= 16, the skinny kernel's range.  By default only at
+        # fused: RMSNorm (+ residual add) runs inside the staging of the next skinny matmul; needs batch <= 16, the skinny kernel's range.  By default only at
         # batch 1: every CTA of a fused kernel recomputes the statistics of all the batch's rows, and from two rows on
         # the separate kernels are faster (measured per layer at context 2000: 80 against 88 us at batch 2, 124 against
         # 176 at batch 8, 174 against 291 at batch 16).
         self.fused = (B == 1) if fused is None else (bool(fused) and B <= 16)
+        # up to 8 rows (the skinny kernel's) SwiGLU runs in the epilogue of the gate|up matmul, one launch less per layer
+        self.gate_up_epilogue = B <= (8 if H < 8192 else 4) and H % 256 == 0 and _aligned(layers)
         # False: rotary/append, attention, merge as three launches; True: one launch; "rope": rotary/append
         # inside the attention launch, merge as a second launch
         self.fused_attention = "rope" if fused_attention == "rope" else bool(fused_attention)
@@ -331,31 +336,31 @@ class DecodeEngine:
         else:
             self._matmul(self.attn, w["o"], self.o, H, hl, sp)
             self._allreduce(self.o)
-        if self.fused:
-            self._check(L.b200_q4f16_gemv_rmsnorm(self.x2.data_ptr(), self.o.data_ptr(), w["norm2"].data_ptr(), self.x.data_ptr(),
-                                                  cfg.eps, w["gu"][0].data_ptr(), w["gu"][1].data_ptr(), self.gu.data_ptr(),
-                                                  B, 2 * il, H, sp))
-            if self.peer is not None:
-                d = self._reduce_desc(1, i, self.down)
-                self._check(L.b200_q4f16_gemv_allreduce(self.gu.data_ptr(), w["down"][0].data_ptr(), w["down"][1].data_ptr(),
-                                                        self.peer["y"][1][self.rank], B, H, il, 1, ctypes.byref(d), sp))
-                return self.down
-            self._check(L.b200_q4f16_gemv_swiglu(self.gu.data_ptr(), w["down"][0].data_ptr(), w["down"][1].data_ptr(),
-                                                 self.down.data_ptr(), B, H, il, sp))
+        if self.fused or self.gate_up_epilogue:
+            # gate, up and SwiGLU in one launch
+            if self.fused:
+                self._check(L.b200_q4f16_gemv_gate_up(self.x2.data_ptr(), self.o.data_ptr(), w["norm2"].data_ptr(), self.x.data_ptr(),
+                                                      cfg.eps, w["gu"][0].data_ptr(), w["gu"][1].data_ptr(), self.act.data_ptr(),
+                                                      B, il, H, sp))
+            else:
+                self._check(L.b200_rmsnorm_early_release(self.x.data_ptr(), self.o.data_ptr(), w["norm2"].data_ptr(),
+                                                         self.h.data_ptr(), B, H, cfg.eps, sp))
+                self._check(L.b200_q4f16_gemv_gate_up(self.h.data_ptr(), None, None, None, 0.0, w["gu"][0].data_ptr(),
+                                                      w["gu"][1].data_ptr(), self.act.data_ptr(), B, il, H, sp))
         else:
             self._check(L.b200_rmsnorm_early_release(self.x.data_ptr(), self.o.data_ptr(), w["norm2"].data_ptr(), self.h.data_ptr(),
                                                      B, H, cfg.eps, sp))
             self._matmul(self.h, w["gu"], self.gu, 2 * il, H, sp)
             self._check(L.b200_silu_mul_early_release(self.gu.data_ptr(), self.act.data_ptr(), B, il, sp))
-            if self.peer is not None and B <= self.PEER_FUSED_MAX_ROWS:
-                d = self._reduce_desc(1, i, self.down)
-                self._check(L.b200_q4f16_gemv_allreduce(self.act.data_ptr(), w["down"][0].data_ptr(), w["down"][1].data_ptr(),
-                                                        self.peer["y"][1][self.rank], B, H, il, 0, ctypes.byref(d), sp))
-                return self.down
-            if self.peer is not None:
-                self._matmul_then_peer_sum(1, i, self.act, w["down"], self.down, H, il, sp)
-                return self.down
-            self._matmul(self.act, w["down"], self.down, H, il, sp)
+        if self.peer is not None and B <= self.PEER_FUSED_MAX_ROWS:
+            d = self._reduce_desc(1, i, self.down)
+            self._check(L.b200_q4f16_gemv_allreduce(self.act.data_ptr(), w["down"][0].data_ptr(), w["down"][1].data_ptr(),
+                                                    self.peer["y"][1][self.rank], B, H, il, 0, ctypes.byref(d), sp))
+            return self.down
+        if self.peer is not None:
+            self._matmul_then_peer_sum(1, i, self.act, w["down"], self.down, H, il, sp)
+            return self.down
+        self._matmul(self.act, w["down"], self.down, H, il, sp)
         self._allreduce(self.down)
         return self.down
 
@@ -399,12 +404,12 @@ class DecodeEngine:
         self._check(L.b200_advance_pos(self.epoch.data_ptr(), 1, sp))
 
     def kernels_per_step(self) -> int:
-        """Kernels of this library launched by one step (embed + 5 or 11 per layer + final norm + output projection
+        """Kernels of this library launched by one step (embed + 6 to 11 per layer + final norm + output projection
         for up to 16 rows + advance)."""
         head = 1 if self.lm_head is not None and self.batch <= 16 else 0
         if self.layer_kernel:
             return 1 + len(self.layers) + 1 + head + 2
-        per_layer = (5 if self.fused else 9) + (1 if self.fused_attention == "rope" else (0 if self.fused_attention else 2))
+        per_layer = (5 if self.fused else 8 if self.gate_up_epilogue else 9) + (1 if self.fused_attention == "rope" else (0 if self.fused_attention else 2))
         if self.rope_epilogue:
             per_layer -= 1
         return 1 + len(self.layers) * per_layer + 1 + head + 2

@@ -379,3 +379,33 @@ def test_qkv_matmul_with_rotary_epilogue_equals_the_two_kernels(cuda_lib, nh, K,
         assert rc == _lib.ENOTREADY
     finally:
         _lib.set_option("gemv.exact", 0)
+
+
+@pytest.mark.parametrize("M,I,K,norm", [(1, 8, 256, False), (1, 1376, 4096, True), (1, 2744, 2560, True), (2, 24, 512, True), (3, 2400, 2048, False),
+                                        (5, 5632, 2048, False), (8, 136, 4096, True), (16, 200, 1024, False)])
+def test_gate_up_matmul_with_swiglu_epilogue_equals_the_two_kernels(cuda_lib, M, I, K, norm):
+    """b200_q4f16_gemv_gate_up against the skinny matmul followed by b200_silu_mul: the product is formed from the same
+    fp16-rounded results, so the outputs agree bit for bit (one tile, odd tile counts, every column count, a short K)."""
+    rng = np.random.default_rng(M + I + K)
+    x, wq, s = synth.make_case(M, 2 * I, K, seed=M + I)
+    x = (x.astype(np.float32) * 0.1).astype(F16)
+    tx, twq, ts, td, tn = (dev(a) for a in (x, wq, s, (0.1 * rng.standard_normal((M, K))).astype(F16), (1 + 0.1 * rng.standard_normal(K)).astype(F16)))
+    gu = torch.empty((M, 2 * I), dtype=torch.float16, device="cuda")
+    two, one = (torch.full((M + 1, I), 7.0, dtype=torch.float16, device="cuda") for _ in range(2))
+    xo = torch.zeros((2, M, K), dtype=torch.float16, device="cuda")
+    if norm:
+        assert cuda_lib.b200_q4f16_gemv_rmsnorm(tx.data_ptr(), td.data_ptr(), tn.data_ptr(), xo[0].data_ptr(), 1e-5, twq.data_ptr(), ts.data_ptr(),
+                                                gu.data_ptr(), M, 2 * I, K, 0) == 0, _lib.last_error()
+    else:
+        assert cuda_lib.b200_q4f16_gemv(tx.data_ptr(), twq.data_ptr(), ts.data_ptr(), gu.data_ptr(), M, 2 * I, K, 0) == 0, _lib.last_error()
+    assert cuda_lib.b200_silu_mul(gu.data_ptr(), two.data_ptr(), M, I, 0) == 0, _lib.last_error()
+    args = (td.data_ptr(), tn.data_ptr(), xo[1].data_ptr()) if norm else (None, None, None)
+    assert cuda_lib.b200_q4f16_gemv_gate_up(tx.data_ptr(), *args, 1e-5, twq.data_ptr(), ts.data_ptr(), one.data_ptr(), M, I, K, 0) == 0, _lib.last_error()
+    torch.cuda.synchronize()
+    assert torch.equal(one.view(torch.int16), two.view(torch.int16)) and torch.equal(xo[0], xo[1])
+    assert cuda_lib.b200_device_error_flags() == 0
+    # what the entry point refuses
+    p = tx.data_ptr()
+    assert cuda_lib.b200_q4f16_gemv_gate_up(p, None, None, None, 0.0, twq.data_ptr(), ts.data_ptr(), one.data_ptr(), M, I - 4, K, 0) == _lib.EINVAL
+    assert cuda_lib.b200_q4f16_gemv_gate_up(p, p, None, None, 0.0, twq.data_ptr(), ts.data_ptr(), one.data_ptr(), M, I, K, 0) == _lib.EINVAL
+    assert cuda_lib.b200_q4f16_gemv_gate_up(p, None, None, None, 0.0, twq.data_ptr(), ts.data_ptr(), one.data_ptr(), M, I, K - 128, 0) == _lib.EINVAL
