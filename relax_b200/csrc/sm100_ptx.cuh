@@ -137,6 +137,11 @@ __device__ __forceinline__ void bulk_g2s_hint(void* smem_dst, const void* gmem_s
       : "memory");
 }
 
+// Asks for `bytes` (a multiple of 16, 16-byte aligned address) in L2; nothing is read into the SM.
+__device__ __forceinline__ void prefetch_l2(const void* gmem, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(gmem), "r"(bytes) : "memory");
+}
+
 // ---- tiled TMA (tensor map) ---------------------------------------------------------------------
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const void* tmap, int32_t c0, int32_t c1, uint64_t* bar) {
   asm volatile(
