@@ -113,10 +113,8 @@ struct PipeParams {
   PeerReduce red;
 };
 
-// The arithmetic of the fast form over the first NU of a warp's U chunks of one stage (see the comment at its call
-// site in the kernel).  NU < U: the other chunks lie past K (zero-filled) and are skipped, so a short K costs what it
-// holds and not a whole stage.
-template <int NU, int U, int MT, int kXUnit, int kCUnit>
+// The arithmetic of the fast form over a warp's U chunks of one stage (see the comment at its call site in the kernel).
+template <int U, int MT, int kXUnit, int kCUnit>
 __device__ __forceinline__ void fast_stage_fn(float (&acc)[2][MT][4], const uint4 (&w)[U][2][2], const uint2 (&sc)[U][2],
                                             const uint4* xb, int x_mul, const float4* cu, const Q4Consts& qc,
                                             uint32_t magic_hi) {
@@ -126,7 +124,7 @@ __device__ __forceinline__ void fast_stage_fn(float (&acc)[2][MT][4], const uint
     uint32_t a[U][2][8];      // raw (offset) nibble pairs: [0..3] first MMA (rows g, g+8: even k, odd k), [4..7] second
     uint4 b[U][2];
 #pragma unroll
-    for (int u = 0; u < NU; ++u)
+    for (int u = 0; u < U; ++u)
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const uint32_t w0 = wd == 0 ? w[u][0][h].x : wd == 1 ? w[u][0][h].y : wd == 2 ? w[u][0][h].z : w[u][0][h].w;
@@ -143,7 +141,7 @@ __device__ __forceinline__ void fast_stage_fn(float (&acc)[2][MT][4], const uint
         a[u][h][7] = lop3_and_or(w1s, qc.hi, magic_hi);
       }
 #pragma unroll
-    for (int u = 0; u < NU; ++u)
+    for (int u = 0; u < U; ++u)
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         if (wd == 0) {
@@ -154,13 +152,13 @@ __device__ __forceinline__ void fast_stage_fn(float (&acc)[2][MT][4], const uint
         }
       }
 #pragma unroll
-    for (int u = 0; u < NU; ++u)
+    for (int u = 0; u < U; ++u)
 #pragma unroll
       for (int h = 0; h < 2; ++h)
         mma_16x8x16(d[u][h], a[u][h][4], a[u][h][5], a[u][h][6], a[u][h][7], b[u][h].z, b[u][h].w);
   }
 #pragma unroll
-  for (int u = 0; u < NU; ++u) {
+  for (int u = 0; u < U; ++u) {
     // scales of groups 4t'+0..3: (s0, s1) (s2, s3); even groups belong to set 0, odd ones to set 1
     const float2 g01 = __half22float2(u32_as_h2(sc[u][0].x)), g23 = __half22float2(u32_as_h2(sc[u][0].y));
     const float2 h01 = __half22float2(u32_as_h2(sc[u][1].x)), h23 = __half22float2(u32_as_h2(sc[u][1].y));
@@ -506,11 +504,9 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
   // minus the offset sums.  Afterwards d[u][h][0], [1] are row g's sums over groups 4t+h and 4t+2+h, [2], [3] row
   // g+8's.  The MMAs are issued round-robin over the 2U accumulators (an MMA that follows the one it depends on
   // waits out the tensor pipe's whole latency; with the accumulators interleaved nothing waits).
-  auto fast_stage = [&](int nu, const uint4 (&w)[U][2][2], const uint2 (&sc)[U][2], const uint4* xu, const float4* cu) {
-    static_assert(!FAST || U == 2, "the dispatch below lists the chunk counts of U = 2");
-    const uint4* xb = x_own ? xu : &s_zero;
-    if (nu >= 2) fast_stage_fn<(U < 2 ? U : 2), U, MT, kXUnit, kCUnit>(acc, w, sc, xb, x_mul, cu, qc, magic_hi);
-    else if (nu == 1) fast_stage_fn<1, U, MT, kXUnit, kCUnit>(acc, w, sc, xb, x_mul, cu, qc, magic_hi);
+  auto fast_stage = [&](const uint4 (&w)[U][2][2], const uint2 (&sc)[U][2], const uint4* xu, const float4* cu) {
+    static_assert(!FAST || U == 1, "a warp's chunk of a stage lies before or past the end of K as a whole");
+    fast_stage_fn<U, MT, kXUnit, kCUnit>(acc, w, sc, x_own ? xu : &s_zero, x_mul, cu, qc, magic_hi);
   };
   // Fast form: this warp's share of stage `s` into registers; the stage goes back to the producer at once.
   auto fast_load = [&](int s, uint32_t round, uint4 (&w)[U][2][2], uint2 (&sc)[U][2]) {
@@ -788,9 +784,8 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
         if (FAST) {
           // (the first stage of the launch is in registers already)
           if (!(kb == 0 && tile == (int)blockIdx.x && k0 == k_lo)) fast_load(s, round, fw, fsc);
-          // this warp's chunks of the stage are warp and warp + CW; those past K are skipped
-          const int nch = (min(k_hi, k0 + KC) - k0 + 255) >> 8;
-          fast_stage((warp < nch) + (warp + CW < nch), fw, fsc, xk, ck);
+          // this warp's chunk of the stage, unless it lies past K
+          if (k0 + warp * 256 < k_hi) fast_stage(fw, fsc, xk, ck);
         } else {
         // On a timeout the kernel keeps going without waiting (results are garbage, the error
         // flag says so) so that every warp still reaches the named barriers and the CTA ends.
@@ -997,11 +992,10 @@ int launch_pipe(const __half* x, const uint32_t* wq, const __half* scales, __hal
   int kblk = kpad, grid = 0, stages = (int)options().gemv_stages;
   bool placed = false;
   if (FAST) {
-    // Two CTAs per SM, one stage each (registers are the second buffer, as in the exact form): measured fastest
-    // for every shape of the 7B decode step.  Deeper rings (up to a CTA's whole share of W resident, one CTA per
-    // SM so that the next launch's CTAs prefetch beside this launch's) were measured too: no faster for
-    // N = K = 4096 and 10-20 % slower for the large matmuls.  Options gemv.ctas_per_sm and gemv.stages
-    // still select them.
+    // Two CTAs per SM with two stages each (launch_pipe_m; registers are a third buffer, as in the exact form): measured
+    // fastest for every shape of the 7B decode step.  One CTA per SM with a CTA's whole share of W resident, so that the next
+    // launch's CTAs prefetch beside this launch's, was measured too: no faster for N = K = 4096 and 10-20 % slower for the
+    // large matmuls.  Options gemv.ctas_per_sm and gemv.stages still select them.
     int per_sm = (int)options().gemv_ctas_per_sm;
     if (per_sm <= 0) per_sm = 2;
     if (per_sm > 2) per_sm = 2;
@@ -1010,8 +1004,9 @@ int launch_pipe(const __half* x, const uint32_t* wq, const __half* scales, __hal
     p.tiles_per_cta = (p.ntiles + grid - 1) / grid;
     // (an explicit stage count may use up to half an SM, so that two CTAs still fit)
     const size_t budget = stages > 0 ? (228 * 1024 - 2 * 1024) / 2 : 76 * 1024;
-    int want = stages > 0 ? stages : p.tiles_per_cta * stages_per_tile;
+    int want = stages > 0 ? stages : 2;
     if (want > kMaxStages) want = kMaxStages;
+    if (want > p.tiles_per_cta * stages_per_tile) want = p.tiles_per_cta * stages_per_tile;
     for (int st = want; st >= 1 && !placed; --st) {
       need = fixed_bytes(st) + block_bytes(kpad);
       if (need <= budget || (st == 1 && need <= kMaxSmem)) {
@@ -1104,7 +1099,11 @@ int launch_pipe_m(const __half* x, const uint32_t* wq, const __half* scales, __h
     // 2816, 4.88 / 4.58 at 4096, 7.26 / 6.80 at 8192, 9.16 / 8.72 at 11008 (and 14.3 / 12.9 at N = 22016, K = 4096).
     // gemv.exact = 2 forces the fast form for every K (tests).
     const bool fast = options().gemv_exact == 2 || (options().gemv_exact == 0 && k >= 2560);
-    if (fast) return launch_pipe<1, CW, CH, PRO, true, GU>(x, wq, scales, y, m, n, k, stream, pro, red);
+    // Two stages of 2048 k a CTA: against one of 4096 k the ring refills in halves and a warp's share of a stage takes half
+    // the registers (no spills in the RMSNorm form); three or more stages are slower again (bytes in flight beyond what
+    // HBM needs): N = 22016 one of 4096 / 2, 3, 4 of 2048: 12.07 / 11.68, 12.23, 13.00 us; N = 12288 8.26 / 8.03, 8.45, 9.01;
+    // N = 4096, K = 11008 8.46 / 8.18, 8.39, 8.39; N = K = 8192 9.97 / 9.63, 10.01, 10.81; N = K = 4096 4.72 / 4.70.
+    if (fast) return launch_pipe<1, CW, CW, PRO, true, GU>(x, wq, scales, y, m, n, k, stream, pro, red);
     return launch_pipe<1, CW, CH, PRO, false, GU>(x, wq, scales, y, m, n, k, stream, pro, red);
   }
   if (m == 2) return launch_pipe<2, CW, CH, PRO, false, GU>(x, wq, scales, y, m, n, k, stream, pro, red);
