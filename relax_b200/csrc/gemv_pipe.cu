@@ -909,6 +909,9 @@ tail:
   }
 }
 
+// More shared memory than two CTAs of one SM can have.
+constexpr size_t kExclusiveSmem = 114 * 1024;
+
 struct Prologue {
   int kind = kPrologueNone;
   const __half* delta = nullptr;
@@ -988,6 +991,7 @@ int launch_pipe(const __half* x, const uint32_t* wq, const __half* scales, __hal
            (size_t)(stages + 1) * CW * kOut * sizeof(float);
   };
   auto block_bytes = [&](int k) { return XL::bytes(k) + (FAST ? (size_t)(k / 256) * 32 * sizeof(float) : 0); };
+  static thread_local size_t attr_need = 0;        // the kernel's shared-memory limit as last set (per thread, per kernel variant)
   size_t need = 0;
   int kblk = kpad, grid = 0, stages = (int)options().gemv_stages;
   bool placed = false;
@@ -1018,7 +1022,8 @@ int launch_pipe(const __half* x, const uint32_t* wq, const __half* scales, __hal
     // Registers are the second buffer (a stage is handed back as soon as it has been copied out) and
     // two CTAs share an SM, so one stage per CTA measured fastest for one row and for 9..16 rows; with 2..8 rows a
     // second stage measured 0-12 % faster (M = 2: 11.7 -> 10.2 us at N = 4096, K = 11008; 16.7 -> 15.6 at N = 22016).
-    if (stages <= 0) stages = (M >= 2 && M <= 8) ? 2 : 1;
+    // (Half-length stages, see half_stages: four of them beside the eight columns' larger x, where one CTA fills an SM.)
+    if (stages <= 0) stages = (M >= 2 && M <= 8) ? (CH < 16 && NC == 8 ? 4 : 2) : 1;
     if (stages > kMaxStages) stages = kMaxStages;
     int max_per_sm = (int)options().gemv_ctas_per_sm;
     if (max_per_sm <= 0) max_per_sm = 2;
@@ -1034,6 +1039,7 @@ int launch_pipe(const __half* x, const uint32_t* wq, const __half* scales, __hal
       if (cached_need != need) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need);
         if (e != cudaSuccess) return fail(B200_ELAUNCH, "gemv: cudaFuncSetAttribute(%zu): %s", need, cudaGetErrorString(e));
+        attr_need = need;
         int q = 1;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&q, kern, kThreads, need) != cudaSuccess || q < 1) q = 1;
         cached_need = need;
@@ -1059,8 +1065,14 @@ int launch_pipe(const __half* x, const uint32_t* wq, const __half* scales, __hal
     kblk = (int)((kMaxSmem - fixed - carries) / block_bytes(KC)) * KC;
     need = fixed + carries + block_bytes(kblk);
   }
+  // No more tiles than SMs: one CTA per SM.  Where two fit, the CTAs of launch after launch come to lie in pairs on some SMs
+  // while others stay empty: in pairs / alone, us, M = 1 N = 1024, K = 8192 5.5 / 4.5, N = 2048, K = 8192 6.0 / 5.3, N = 2048, K = 1024
+  // 3.0 / 2.8, M = 4 N = 2048, K = 4096 5.7 / 4.5.  (Not the fast form up to K = 4096 on more than half of the SMs: the next
+  // launch's first copies, which need a place beside this one, are worth as much there: 3.84 / 3.89 at N = 2048, K = 4096; at
+  // N = 1024 3.46 / 3.23.  Not the longer stages of 2..8 rows, which mostly fill an SM by themselves.)
+  const bool alone = p.ntiles <= sms && (FAST ? K > 4096 || 2 * p.ntiles <= sms : NC == 1 || CH < 16);
+  if (alone && need < kExclusiveSmem) need = kExclusiveSmem;
   {
-    static thread_local size_t attr_need = 0;      // (per thread, per kernel variant)
     if (attr_need != need) {
       cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need);
       if (e != cudaSuccess) return fail(B200_ELAUNCH, "gemv: cudaFuncSetAttribute(%zu): %s", need, cudaGetErrorString(e));
@@ -1088,6 +1100,20 @@ int launch_pipe(const __half* x, const uint32_t* wq, const __half* scales, __hal
   return B200_OK;
 }
 
+// Stages of 2048 k instead of 4096 for 2..8 rows.  They waste less of a K that ends in the first half of a 4096-k stage;
+// and they take 18 registers less, so that a second CTA fits the SM, which is worth it where there are tiles for two and
+// both copies of x fit too (up to four columns; with eight the arithmetic fills the SM either way).  4096-k / 2048-k stages
+// in us: M = 2 N = 12288, K = 1024 6.3 / 4.9, K = 4096 10.0 / 9.3; M = 4 N = 12288, K = 2048 8.1 / 6.6, K = 4096 10.9 / 10.3, but (one
+// CTA either way) K = 8192 18.1 / 19.6, (160 tiles) N = 2560, K = 4096 5.5 / 5.8 and (32 tiles) N = 512, K = 4096 4.24 / 4.35; M = 8
+// N = 4096, K = 2048 5.7 / 5.0, K = 5632 10.4 / 9.9, but N = 12288, K = 3072 10.9 / 11.1.
+template <int NC>
+bool half_stages(int n, int k) {
+  const int tail = k % 4096;
+  if (tail > 0 && tail <= 2048) return true;
+  constexpr size_t kFixed = 2 * 8 * kRows * (128 + 16) + 3 * 8 * 128 * sizeof(float) + 2048;   // ring, partial sums, barriers
+  return NC <= 4 && n > sm_count() * kRows * 3 / 2 && kFixed + XLayout<NC>::bytes((k + 2047) / 2048 * 2048) <= kExclusiveSmem - 1024;
+}
+
 template <int CW, int CH, int PRO, bool GU>
 int launch_pipe_m(const __half* x, const uint32_t* wq, const __half* scales, __half* y, int m, int n, int k,
                   cudaStream_t stream, const Prologue& pro, const PeerReduce& red) {
@@ -1106,9 +1132,15 @@ int launch_pipe_m(const __half* x, const uint32_t* wq, const __half* scales, __h
     if (fast) return launch_pipe<1, CW, CW, PRO, true, GU>(x, wq, scales, y, m, n, k, stream, pro, red);
     return launch_pipe<1, CW, CH, PRO, false, GU>(x, wq, scales, y, m, n, k, stream, pro, red);
   }
-  if (m == 2) return launch_pipe<2, CW, CH, PRO, false, GU>(x, wq, scales, y, m, n, k, stream, pro, red);
-  if (m <= 4) return launch_pipe<4, CW, CH, PRO, false, GU>(x, wq, scales, y, m, n, k, stream, pro, red);
-  if (m <= 8) return launch_pipe<8, CW, CH, PRO, false, GU>(x, wq, scales, y, m, n, k, stream, pro, red);
+  if (m == 2)
+    return half_stages<2>(n, k) ? launch_pipe<2, CW, CW, PRO, false, GU>(x, wq, scales, y, m, n, k, stream, pro, red)
+                             : launch_pipe<2, CW, CH, PRO, false, GU>(x, wq, scales, y, m, n, k, stream, pro, red);
+  if (m <= 4)
+    return half_stages<4>(n, k) ? launch_pipe<4, CW, CW, PRO, false, GU>(x, wq, scales, y, m, n, k, stream, pro, red)
+                             : launch_pipe<4, CW, CH, PRO, false, GU>(x, wq, scales, y, m, n, k, stream, pro, red);
+  if (m <= 8)
+    return half_stages<8>(n, k) ? launch_pipe<8, CW, CW, PRO, false, GU>(x, wq, scales, y, m, n, k, stream, pro, red)
+                             : launch_pipe<8, CW, CH, PRO, false, GU>(x, wq, scales, y, m, n, k, stream, pro, red);
   return launch_pipe<16, CW, CH, PRO, false, GU>(x, wq, scales, y, m, n, k, stream, pro, red);
 }
 
