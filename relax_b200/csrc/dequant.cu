@@ -18,11 +18,12 @@ __global__ void __launch_bounds__(kDeqThreads)
 q4f16_dequantize_kernel(const uint32_t* __restrict__ wq, const __half* __restrict__ scales,
                         uint4* __restrict__ w, int64_t n_words) {
   // Programmatic dependent launch: this grid's blocks are set up while the launch in front drains and everything is
-  // read and written behind the wait.  Back to back, us: N = 11008, K = 4096 22.0 -> 19.7 (5.9 TB/s), N = K = 4096 9.7 -> 7.4,
-  // 28672 x 8192 93.0 -> 91.1.  (A persistent grid of eight blocks per SM with the next words
+  // read and written behind the wait.  Back to back, us: N = 11008, K = 4096 22.0 -> 19.7 (5.9 TB/s), N = K = 4096 9.6 -> 7.1,
+  // 28672 x 8192 92.9 -> 91.1.  (A persistent grid of eight blocks per SM with the next words
   // prefetched: 21.8 at N = 11008, 112 at 28672; with streaming stores 21.2.)
+  // The next launch begins when the last block has left: what it reads before its own wait (a matmul its scales) may be
+  // what this kernel writes.  Letting it begin behind this wait instead measured the same, 19.7, 7.2 and 91.1.
   ptx::pdl_wait();
-  ptx::pdl_launch_dependents();
   // a group of 32 k is 4 consecutive words, and rows hold a whole number of groups, so scale index = word index / 4
   const Q4Consts qc = q4_consts();
   int64_t base = (int64_t)blockIdx.x * (kDeqThreads * kDeqUnroll) + threadIdx.x;

@@ -46,6 +46,39 @@ def test_dequantize_all_scale_bit_patterns(cuda_lib):
     assert_bits_equal(out, oracle.c_dequantize(wq, s), "all scales x all nibbles")
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 4096, 4096), (1, 2048, 2080), (3, 4096, 2048), (40, 2048, 1024), (40, 2048, 2080)])
+def test_dequantize_between_dependent_launches(cuda_lib, m, n, k):
+    """A dequantiser between two matmuls: its scales are what the launch in front writes, its output is the scales of the
+    matmul behind it, which every matmul kernel reads before its own wait.  Two inputs take turns through the same
+    buffers without a wait, so whatever is read too early is the other input's."""
+    rows = n * (k // 32) // 32
+    x, wq, _ = synth.make_case(m, n, k, seed=n + k + m)
+    x0, wq0, s0 = synth.make_case(2, rows, 512, seed=k)
+    _, wq1, _ = synth.make_case(1, rows, 32, seed=m)
+    tx, twq, tx0, twq0, ts0, twq1 = dev((0.1 * x.astype(np.float32)).astype(np.float16), wq, (0.01 * x0.astype(np.float32)).astype(np.float16), wq0, s0, wq1)
+    s1 = torch.empty((rows, 1), dtype=torch.float16, device="cuda")
+    s2 = torch.empty((n, k // 32), dtype=torch.float16, device="cuda")
+    sp = torch.cuda.current_stream().cuda_stream
+
+    def chain(i, y, wait):
+        assert cuda_lib.b200_q4f16_matmul(tx0[i].data_ptr(), twq0.data_ptr(), ts0.data_ptr(), s1.data_ptr(), 1, rows, 512, sp) == 0, _lib.last_error()
+        wait()
+        assert cuda_lib.b200_q4f16_dequantize(twq1.data_ptr(), s1.data_ptr(), s2.data_ptr(), rows, 32, sp) == 0, _lib.last_error()
+        wait()
+        assert cuda_lib.b200_q4f16_matmul(tx.data_ptr(), twq.data_ptr(), s2.data_ptr(), y.data_ptr(), m, n, k, sp) == 0, _lib.last_error()
+        wait()
+
+    ref, out = (torch.full((c, m, n), float("nan"), dtype=torch.float16, device="cuda") for c in (2, 12))
+    for i in range(2):
+        chain(i, ref[i], torch.cuda.synchronize)
+    assert not torch.equal(ref[0], ref[1])
+    for j in range(12):
+        chain(j % 2, out[j], lambda: None)
+    torch.cuda.synchronize()
+    for j in range(12):
+        assert_bits_equal(out[j].cpu().numpy(), ref[j % 2].cpu().numpy(), f"pass {j}")
+
+
 def test_dequantize_empty(cuda_lib):
     twq = torch.zeros((0, 16), dtype=torch.uint32, device="cuda")
     ts = torch.zeros((0, 4), dtype=torch.float16, device="cuda")
