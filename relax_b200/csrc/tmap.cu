@@ -37,8 +37,16 @@ int make_tmap(CUtensorMap* out, CUtensorMapDataType dtype, int rank, const void*
     e[i] = 1;
     if (i + 1 < rank) s[i] = strides_bytes[i];
   }
-  CUresult r = g_encode(out, dtype, (cuuint32_t)rank, const_cast<void*>(base), d, s, b, e, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                        swizzle, promo, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  auto encode = [&] {
+    return g_encode(out, dtype, (cuuint32_t)rank, const_cast<void*>(base), d, s, b, e, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, promo,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  CUresult r = encode();
+  if (r == CUDA_ERROR_INVALID_CONTEXT) {
+    // a thread whose first CUDA call this is: unlike a runtime call, the encoder does not bind the device's context to it
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess) r = encode();
+  }
   if (r != CUDA_SUCCESS)
     return fail(B200_EINVAL, "cuTensorMapEncodeTiled failed (CUresult %d): rank=%d dims=[%llu,%llu,%llu] box=[%u,%u,%u]",
                 (int)r, rank, (unsigned long long)d[0], (unsigned long long)(rank > 1 ? d[1] : 0),

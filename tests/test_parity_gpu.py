@@ -1,5 +1,6 @@
 """GPU parity tests: the CUDA kernels, called through the C ABI, against the CPU oracle."""
 import ctypes
+import threading
 
 import numpy as np
 import pytest
@@ -165,6 +166,28 @@ def test_gemv_stage_lengths(cuda_lib, m, n, k):
     torch.cuda.synchronize()
     assert_matmul_close(out.cpu().numpy(), x, wq, s, f"{m}x{n}x{k}")
     assert cuda_lib.b200_device_error_flags() == 0
+
+
+@pytest.mark.parametrize("m,n,k,family", [(1, 512, 4096, "auto"), (40, 512, 1024, "auto"), (3, 512, 1056, "auto"), (300, 256, 512, "gemm")])
+def test_first_cuda_call_of_a_thread(cuda_lib, m, n, k, family):
+    """A matmul as the first CUDA call of a thread, to which no context is bound yet (tensor maps are encoded in one)."""
+    x, wq, s = synth.make_case(m, n, k, seed=m)
+    operands = dev(x, wq, s)
+    out = torch.empty((m, n), dtype=torch.float16, device="cuda")
+    raised = []
+
+    def launch():
+        try:
+            ops.q4f16_matmul(*operands, out=out, family=family)
+        except Exception as e:                       # (an exception in a thread would otherwise only be printed)
+            raised.append(e)
+
+    t = threading.Thread(target=launch)
+    t.start()
+    t.join()
+    assert not raised
+    torch.cuda.synchronize()
+    assert_matmul_close(out.cpu().numpy(), x, wq, s, family)
 
 
 @pytest.mark.parametrize("stages", [2, 3, 8, 16])
