@@ -53,6 +53,18 @@ int ensure_device() {
   return B200_OK;
 }
 
+int raise_smem_limit(SmemLimit& limit, const void* kern, size_t bytes, const char* who) {
+  int dev = -1;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess)
+    limit.raise(dev, bytes, [&](size_t n) {
+      e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)n);
+      return e == cudaSuccess ? 0 : 1;
+    });
+  if (e != cudaSuccess) return fail(B200_ELAUNCH, "%s: cudaFuncSetAttribute(%zu): %s", who, bytes, cudaGetErrorString(e));
+  return B200_OK;
+}
+
 int sm_count() {
   static int n[64] = {0};
   int dev = 0;

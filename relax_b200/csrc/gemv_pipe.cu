@@ -991,24 +991,8 @@ int launch_pipe(const __half* x, const uint32_t* wq, const __half* scales, __hal
            (size_t)(stages + 1) * CW * kOut * sizeof(float);
   };
   auto block_bytes = [&](int k) { return XL::bytes(k) + (FAST ? (size_t)(k / 256) * 32 * sizeof(float) : 0); };
-  // The kernel's dynamic shared-memory limit (per kernel variant) is a property of the kernel, which all threads share, and
-  // only ever raised: first to a size that nearly every launch keeps below, so that no thread lowers it under another's launch.
-  constexpr size_t kUsualLimit = 220 * 1024;
-  static thread_local size_t limit = 0;
-  auto raise_limit = [&](size_t bytes) -> int {
-    if (bytes <= limit) return B200_OK;
-    const size_t want = bytes > kUsualLimit ? kMaxSmem : kUsualLimit;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)want);
-    bool exact = false;
-    if (e != cudaSuccess && want > bytes) {          // (static shared memory counts against the 227 KB too)
-      cudaGetLastError();
-      exact = true;
-      e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    }
-    if (e != cudaSuccess) return fail(B200_ELAUNCH, "gemv: cudaFuncSetAttribute(%zu): %s", bytes, cudaGetErrorString(e));
-    limit = exact ? bytes : want;
-    return B200_OK;
-  };
+  static SmemLimit limit;                            // (one per kernel variant, for all threads)
+  const void* const func = reinterpret_cast<const void*>(kern);
   size_t need = 0;
   int kblk = kpad, grid = 0, stages = (int)options().gemv_stages;
   bool placed = false;
@@ -1050,11 +1034,11 @@ int launch_pipe(const __half* x, const uint32_t* wq, const __half* scales, __hal
       need = fixed_bytes(stages) + block_bytes(kpad);
       if (need > kMaxSmem) continue;
       // resident CTAs per SM as the hardware will place them (registers and threads count too);
-      // the answer for the last shared-memory size is remembered (per thread, per kernel variant)
+      // the answer for the last shared-memory size is remembered (per thread, per kernel variant; the same on every sm_100a)
       static thread_local size_t cached_need = 0;
       static thread_local int cached_per_sm = 0;
       if (cached_need != need) {
-        if (int rc = raise_limit(need)) return rc;
+        if (int rc = raise_smem_limit(limit, func, need, "gemv")) return rc;
         int q = 1;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&q, kern, kThreads, need) != cudaSuccess || q < 1) q = 1;
         cached_need = need;
@@ -1087,7 +1071,7 @@ int launch_pipe(const __half* x, const uint32_t* wq, const __half* scales, __hal
   // N = 1024 3.46 / 3.23.  Not the longer stages of 2..8 rows, which mostly fill an SM by themselves.)
   const bool alone = p.ntiles <= sms && (FAST ? K > 4096 || 2 * p.ntiles <= sms : NC == 1 || CH < 16);
   if (alone && need < kExclusiveSmem) need = kExclusiveSmem;
-  if (int rc = raise_limit(need)) return rc;
+  if (int rc = raise_smem_limit(limit, func, need, "gemv")) return rc;
   p.nstages = stages;
   p.kblk = kblk;
   if (pro.rope.on && kblk < kpad) return B200_ENOTREADY;   // (K cut into blocks: the rotary epilogue takes one)

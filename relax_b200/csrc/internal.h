@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include "../../include/b200_q4f16.h"
+#include "smem_limit.h"
 
 namespace b200 {
 
@@ -89,6 +90,9 @@ int gemv_pipe_error_read_and_clear();
 int gemm_error_read_and_clear();
 int gemm_ws_error_read_and_clear();
 int layer_error_read_and_clear();
+
+// Lets `kern` be launched with `bytes` of dynamic shared memory on the current device (`limit`: that kernel's own).
+int raise_smem_limit(SmemLimit& limit, const void* kern, size_t bytes, const char* who);
 
 // Device capability check, cached per device; 0 when the current device is sm_100.
 int ensure_device();

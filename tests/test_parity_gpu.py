@@ -190,6 +190,27 @@ def test_first_cuda_call_of_a_thread(cuda_lib, m, n, k, family):
     assert_matmul_close(out.cpu().numpy(), x, wq, s, family)
 
 
+def test_gemv_shared_memory_limit_across_threads(cuda_lib):
+    """One kernel variant (4 rows, 4096-k stages): a launch that fills the SM's shared memory, then a smaller one from
+    another thread, which must not take the larger one's limit away."""
+    big, small = synth.make_case(4, 64, 18944, seed=1), synth.make_case(4, 64, 4096, seed=2)
+    operands = {"big": dev(*big), "small": dev(*small)}
+    out = {}
+
+    def launch(name):
+        out.setdefault(name, []).append(ops.q4f16_matmul(*operands[name]).cpu().numpy())
+
+    launch("big")
+    t = threading.Thread(target=launch, args=("small",))
+    t.start()
+    t.join()
+    launch("big")
+    assert_matmul_close(out["small"][0], *small, "small")
+    assert len(out["big"]) == 2
+    for y in out["big"]:
+        assert_matmul_close(y, *big, "big")
+
+
 @pytest.mark.parametrize("stages", [2, 3, 8, 16])
 def test_gemv_pipeline_depths(cuda_lib, stages, gemv_form):
     x, wq, s = synth.make_case(3, 5000, 4096, seed=stages)
