@@ -986,13 +986,9 @@ int b200_decode_layer(const B200DecodeLayer* a, void* stream) {
   p.nstages = stages;
 
   auto kern = q4f16_decode_layer_kernel;
-  static thread_local size_t attr_smem = 0;
-  if (attr_smem != smem) {
-    cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return fail(B200_ELAUNCH, "%s: cudaFuncSetAttribute(%zu): %s", who, smem, cudaGetErrorString(e));
-    attr_smem = smem;
-  }
+  cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+  static SmemLimit limit;
+  if ((rc = raise_smem_limit(limit, reinterpret_cast<const void*>(kern), smem, who))) return rc;
   int grid = sm_count();
   if (options().layer_max_ctas > 0 && grid > options().layer_max_ctas) grid = (int)options().layer_max_ctas;
   cudaLaunchConfig_t cfg = {};

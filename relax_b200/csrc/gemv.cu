@@ -240,8 +240,8 @@ int launch_stream(const __half* x, const uint32_t* wq, const __half* scales, __h
   if (red > smem) smem = red;
   auto kern = q4f16_gemv_stream_kernel<NC, RT>;
   if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return fail(B200_ELAUNCH, "gemv: cudaFuncSetAttribute(%zu): %s", smem, cudaGetErrorString(e));
+    static SmemLimit limit;                          // (one per kernel variant, for all threads)
+    if (int rc = raise_smem_limit(limit, reinterpret_cast<const void*>(kern), smem, "gemv")) return rc;
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)((N + TILE_N - 1) / TILE_N));

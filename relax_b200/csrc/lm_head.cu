@@ -196,16 +196,10 @@ int launch_lm_head(const __half* x, const __half* w, __half* logits, int* tokens
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = options().gemv_pdl ? 1 : 0;
-  cudaError_t e;
-  if (ncb == 1) {
-    e = cudaFuncSetAttribute(f16_lm_head_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess)
-      e = cudaLaunchKernelEx(&cfg, f16_lm_head_kernel<1>, x, w, logits, tokens, scratch, (int)B, (int)V, (int)H, (int)token_offset);
-  } else {
-    e = cudaFuncSetAttribute(f16_lm_head_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess)
-      e = cudaLaunchKernelEx(&cfg, f16_lm_head_kernel<2>, x, w, logits, tokens, scratch, (int)B, (int)V, (int)H, (int)token_offset);
-  }
+  auto kern = ncb == 1 ? f16_lm_head_kernel<1> : f16_lm_head_kernel<2>;
+  static SmemLimit limits[2];
+  if (int rc = raise_smem_limit(limits[ncb - 1], reinterpret_cast<const void*>(kern), smem, "lm_head")) return rc;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, x, w, logits, tokens, scratch, (int)B, (int)V, (int)H, (int)token_offset);
   if (e != cudaSuccess) return fail(B200_ELAUNCH, "lm_head launch: %s", cudaGetErrorString(e));
   count_launch();
   return B200_OK;

@@ -1,4 +1,6 @@
 """GPU parity of the decode-step glue kernels and of whole decoder layers against the numpy oracle."""
+import threading
+
 import numpy as np
 import pytest
 import torch
@@ -319,6 +321,65 @@ def test_lm_head_matches_oracle(cuda_lib, B, V, H):
     torch.cuda.synchronize()
     assert (buf[:B * V].view(B, V).cpu().numpy().view(np.uint16) == logits.view(np.uint16)).all()
     assert (toks[:B].cpu().numpy() == want - 1000).all()
+
+
+def test_lm_head_and_streaming_matmul_from_two_threads(cuda_lib):
+    """Launches of one kernel that ask for more and for less than 64 KB of shared memory, from two threads at a time: the smaller
+    ones' limit must not come under the larger ones."""
+    sizes = {"large": (4096, 16), "small": (512, 1)}                  # hidden size of the output projection, rows of the matmul's W
+    bad = []
+
+    def launches(name):
+        H, N = sizes[name]
+        st = torch.cuda.Stream()
+        with torch.cuda.stream(st):
+            h, w = torch.randn((8, H), device="cuda").half(), torch.randn((64, H), device="cuda").half()
+            logits = torch.empty((8, 64), dtype=torch.float16, device="cuda")
+            K = 8192 if name == "large" else 3616                    # (+ 32: the streaming kernel, 64 and 60 KB of x)
+            x, wq, s = synth.make_case(8, N, K + 32, seed=1)
+            tx, twq, ts = dev(x), torch.from_numpy(wq).cuda(), dev(s)
+            y = torch.empty((8, N), dtype=torch.float16, device="cuda")
+            for _ in range(400):
+                rcs = (cuda_lib.b200_lm_head(h.data_ptr(), w.data_ptr(), logits.data_ptr(), None, None, 8, 64, H, 0, st.cuda_stream),
+                       cuda_lib.b200_q4f16_gemv(tx.data_ptr(), twq.data_ptr(), ts.data_ptr(), y.data_ptr(), 8, N, K + 32, st.cuda_stream))
+                if any(rcs):
+                    bad.append((name, rcs, _lib.last_error()))
+                    break
+            st.synchronize()
+
+    threads = [threading.Thread(target=launches, args=(n,)) for n in sizes]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
+
+
+def test_layer_kernel_shared_memory_limit_across_threads(cuda_lib):
+    """The one-kernel-per-layer step with a deep weight ring, with a shallow one from another thread, and with the deep one
+    again: each launch's shared memory stays allowed."""
+    cfg = SMALL
+    layers = [decoder.to_device(tp.shard_layer(decoder.synth_layer_numpy(cfg, 3 + i), 0, 1, cfg.hidden, cfg.inter), "cuda") for i in range(cfg.layers)]
+    eng = decoder.DecodeEngine(cfg, layers, dev(np.ones((cfg.vocab, cfg.hidden), F16)), dev(np.ones(cfg.hidden, F16)), None, 1, 16, "cuda",
+                               layer_kernel=True)
+    bad = []
+
+    def step(stages):
+        _lib.set_option("layer.stages", stages)
+        try:
+            eng.step()
+        except _lib.B200Error as e:
+            bad.append((stages, e))
+        finally:
+            _lib.set_option("layer.stages", 0)
+
+    step(5)
+    t = threading.Thread(target=step, args=(3,))
+    t.start()
+    t.join()
+    step(5)
+    torch.cuda.synchronize()
+    assert not bad and int(eng.pos.item()) == 3 and cuda_lib.b200_device_error_flags() == 0
 
 
 def test_lm_head_argument_checks(cuda_lib):
