@@ -1007,8 +1007,10 @@ int launch_pipe(const __half* x, const uint32_t* wq, const __half* scales, __hal
     grid = sms * per_sm;
     if (grid > p.ntiles) grid = p.ntiles;
     p.tiles_per_cta = (p.ntiles + grid - 1) / grid;
-    // (an explicit stage count may use up to half an SM, so that two CTAs still fit)
-    const size_t budget = stages > 0 ? (228 * 1024 - 2 * 1024) / 2 : 76 * 1024;
+    // Up to half an SM, so that two CTAs fit: two stages beside x up to K = 26624.  With 76 KB, which hold them up to K = 12288
+    // only, a longer K fell to one stage: one / two stages in us, N = 5120, K = 12544 16.6 / 12.0, K = 13824 17.0 / 12.4, N = 4096,
+    // K = 17920 13.1 / 11.4, K = 26624 18.5 / 15.7, N = 22016, K = 12800 40.2 / 32.2.
+    const size_t budget = (228 * 1024 - 2 * 1024) / 2;
     int want = stages > 0 ? stages : 2;
     if (want > kMaxStages) want = kMaxStages;
     if (want > p.tiles_per_cta * stages_per_tile) want = p.tiles_per_cta * stages_per_tile;

@@ -168,6 +168,14 @@ def test_gemv_stage_lengths(cuda_lib, m, n, k):
     assert cuda_lib.b200_device_error_flags() == 0
 
 
+@pytest.mark.parametrize("n,k", [(5000, 12288), (5000, 12544), (300, 14336), (300, 26624), (300, 26880), (100, 32768)])
+def test_gemv_one_row_long_k(cuda_lib, n, k, gemv_form):
+    """One row where two stages fit beside x in half an SM (up to K = 26624), and beyond."""
+    x, wq, s = synth.make_case(1, n, k, seed=n + k)
+    assert_matmul_close(run_matmul(x, wq, s), x, wq, s, f"N={n} K={k}")
+    assert cuda_lib.b200_device_error_flags() == 0
+
+
 @pytest.mark.parametrize("m,n,k,family", [(1, 512, 4096, "auto"), (40, 512, 1024, "auto"), (3, 512, 1056, "auto"), (300, 256, 512, "gemm")])
 def test_first_cuda_call_of_a_thread(cuda_lib, m, n, k, family):
     """A matmul as the first CUDA call of a thread, to which no context is bound yet (tensor maps are encoded in one)."""
