@@ -911,6 +911,7 @@ tail:
 
 // More shared memory than two CTAs of one SM can have.
 constexpr size_t kExclusiveSmem = 114 * 1024;
+constexpr size_t kMaxSmem = 227 * 1024;          // of one CTA
 
 struct Prologue {
   int kind = kPrologueNone;
@@ -980,7 +981,6 @@ int launch_pipe(const __half* x, const uint32_t* wq, const __half* scales, __hal
   p.ntiles = (N + kRows - 1) / kRows;
   const int kpad = ((K + KC - 1) / KC) * KC;
   const int stages_per_tile = kpad / KC;
-  const size_t kMaxSmem = 227 * 1024;
   const int sms = sm_count();
   auto kern = q4f16_gemv_pipe_kernel<NC, CW, CH, PRO, FAST, GU>;
   // Ask for the largest shared-memory carve-out: the default picks the smallest that fits ONE CTA,
@@ -1096,17 +1096,28 @@ int launch_pipe(const __half* x, const uint32_t* wq, const __half* scales, __hal
 }
 
 // Stages of 2048 k instead of 4096 for 2..8 rows.  They waste less of a K that ends in the first half of a 4096-k stage;
-// and they take 18 registers less, so that a second CTA fits the SM, which is worth it where there are tiles for two and
-// both copies of x fit too (up to four columns; with eight the arithmetic fills the SM either way).  4096-k / 2048-k stages
-// in us: M = 2 N = 12288, K = 1024 6.3 / 4.9, K = 4096 10.0 / 9.3; M = 4 N = 12288, K = 2048 8.1 / 6.6, K = 4096 10.9 / 10.3, but (one
-// CTA either way) K = 8192 18.1 / 19.6, (160 tiles) N = 2560, K = 4096 5.5 / 5.8 and (32 tiles) N = 512, K = 4096 4.24 / 4.35; M = 8
-// N = 4096, K = 2048 5.7 / 5.0, K = 5632 10.4 / 9.9, but N = 12288, K = 3072 10.9 / 11.1.
+// and they leave room for a second CTA on the SM, which is worth it where there are tiles for two and both copies of x fit too
+// (up to four columns; with eight the arithmetic fills the SM either way).  4096-k / 2048-k stages in us:
+//   K ends in a first half   M = 2 N = 12288, K = 1024 6.3 / 4.9; M = 4 N = 12288, K = 2048 8.1 / 6.6, K = 6144 15.4 / 14.0; M = 8 N = 4096,
+//                            K = 2048 5.7 / 5.0, K = 9216 17.2 / 14.3
+//   ... one CTA either way   M = 4: the shorter ones where two long ones do not fit beside x (N = 5120, K = 13824 20.7 / 18.6) and
+//                            up to two tiles an SM (N = 4736, K = 9216 11.3 / 10.9; N = 4752 12.6 / 13.3, N = 12288 21.3 / 22.8), not
+//                            for long K, of which a stage is little (M = 2 K = 17920 N = 4096 15.1 / 15.6, N = 12288 34.6 / 38.3)
+//   ... no two fit beside x  the longer ones, and K cut into blocks (M = 4 N = 4096, K = 21504 25.0 / 29.6, N = 8192, K = 26624 45 / 64;
+//                            M = 8 N = 5120, K = 13824 26.9 / 34.5)
+//   two CTAs of the shorter  M = 2 N = 12288, K = 4096 10.0 / 9.3, K = 14336 28.1 / 26.7; M = 4 N = 12288, K = 4096 10.9 / 10.3, but 160 tiles
+//                            (N = 2560) 5.5 / 5.8 and 32 tiles 4.24 / 4.35; M = 8 N = 12288, K = 3072 10.9 / 11.1
 template <int NC>
 bool half_stages(int n, int k) {
+  constexpr size_t kRing = 8 * kRows * (128 + 16);                            // a short stage
+  constexpr size_t kRest = 3 * 8 * 128 * sizeof(float) + 2048;                // partial sums, barriers, alignment
+  const size_t x_short = XLayout<NC>::bytes((k + 2047) / 2048 * 2048), x_long = XLayout<NC>::bytes((k + 4095) / 4096 * 4096);
+  const bool pair = 2 * kRing + kRest + x_short <= kExclusiveSmem - 1024;
   const int tail = k % 4096;
-  if (tail > 0 && tail <= 2048) return true;
-  constexpr size_t kFixed = 2 * 8 * kRows * (128 + 16) + 3 * 8 * 128 * sizeof(float) + 2048;   // ring, partial sums, barriers
-  return NC <= 4 && n > sm_count() * kRows * 3 / 2 && kFixed + XLayout<NC>::bytes((k + 2047) / 2048 * 2048) <= kExclusiveSmem - 1024;
+  if (tail == 0 || tail > 2048) return NC <= 4 && pair && n > sm_count() * kRows * 3 / 2;
+  if (2 * kRing + kRest + x_short > kMaxSmem) return false;
+  const bool two_long = 4 * kRing + kRest + x_long <= kMaxSmem;
+  return NC >= 8 || pair || !two_long || (k <= 12288 && n <= 2 * sm_count() * kRows);
 }
 
 template <int CW, int CH, int PRO, bool GU>

@@ -168,6 +168,15 @@ def test_gemv_stage_lengths(cuda_lib, m, n, k):
     assert cuda_lib.b200_device_error_flags() == 0
 
 
+@pytest.mark.parametrize("m,n,k", [(2, 4736, 9216), (2, 300, 17920), (3, 4752, 10240), (4, 4736, 8448), (4, 300, 13824), (4, 300, 18432),
+                                   (4, 300, 21504), (3, 300, 26624), (8, 300, 10240), (5, 300, 13824), (8, 300, 18432)])
+def test_gemv_stage_lengths_of_a_long_k(cuda_lib, m, n, k):
+    """K ends in the first half of a long stage: two short stages fit beside x for two CTAs, for one, or K is cut into blocks."""
+    x, wq, s = synth.make_case(m, n, k, seed=m + n + k)
+    assert_matmul_close(run_matmul(x, wq, s, family="gemv"), x, wq, s, f"{m}x{n}x{k}")
+    assert cuda_lib.b200_device_error_flags() == 0
+
+
 @pytest.mark.parametrize("n,k", [(5000, 12288), (5000, 12544), (300, 14336), (300, 26624), (300, 26880), (100, 32768)])
 def test_gemv_one_row_long_k(cuda_lib, n, k, gemv_form):
     """One row where two stages fit beside x in half an SM (up to K = 26624), and beyond."""
