@@ -205,7 +205,12 @@ B200_API int b200_q4f16_gemv_rmsnorm(const void* x, const void* delta, const voi
 /* gemv_gate_up: act fp16 [M, I] = silu(h . Wg^T) * (h . Wu^T), W [2I, K] = gate rows | up rows, h = x, or gemv_rmsnorm's
  * normalised activation where norm_w is given (delta and x_out only then).  The product is formed in the matmul's
  * epilogue from its fp16-rounded results: the values of gemv_rmsnorm (or the plain skinny matmul) followed by b200_silu_mul,
- * without the [M, 2I] buffer.  I % 8 == 0. */
+ * without the [M, 2I] buffer.  I % 8 == 0.  Returns B200_ENOTREADY, with nothing launched, where W has so many rows and K is so long
+ * that the kernel cannot hold its partial sums: call the separate entry points then.
+ * gemv_gate_up_applies: 1 where, under the present options, b200_q4f16_matmul would take these weights (M rows, [2I, K])
+ * through the kernel that gemv_gate_up extends; 0 where it would take another one, or the shape or alignment of the
+ * scales is not gemv_gate_up's. */
+B200_API int b200_q4f16_gemv_gate_up_applies(const void* scales, int64_t M, int64_t I, int64_t K);
 B200_API int b200_q4f16_gemv_gate_up(const void* x, const void* delta, const void* norm_w, void* x_out, float eps,
                                      const void* wq, const void* scales, void* act, int64_t M, int64_t I, int64_t K,
                                      void* cuda_stream);

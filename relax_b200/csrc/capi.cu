@@ -116,6 +116,31 @@ int zero_output(void* y, int64_t M, int64_t N, cudaStream_t s) {
 
 enum Family { kAuto, kGemv, kGemm, kGemmWs };
 
+// Whether the automatic choice asks the weight-stationary kernel first.
+// 9 rows and more, and 5..8 where K is long: the weight-stationary kernel, whose weights stream once up to 128 rows.
+// Measured on B200, skinny / weight-stationary kernel in us at 4, 8 and 16 rows: N = K = 4096 6.0 / 6.1, 7.7 / 6.4,
+// 11.1 / 6.5; N = 22016 16.5 / 17.9, 17.9 / 18.1, 24.4 / 18.4; N = 4096, K = 11008 11.8 / 12.2, 18.9 / 12.3, 29.3 / 12.5;
+// N = 1280, K = 8192 6.6 / 5.9, 9.7 / 6.0, 17.0 / 6.1 (the skinny kernel stages all of x in every CTA, and its
+// arithmetic grows from 8 columns on).  At 5..8 rows and a shorter K the skinny kernel is the better one inside a
+// decode step, where two of its CTAs fit an SM and it starts beside the kernel before it (8 layers of hidden
+// 2048 at 5 rows: 413 us with it, 440 without).  Above 128 rows it cuts the tokens into tiles to suit the shape; the
+// prefill kernel with its 256-token tiles keeps the long prompts that one wave of them holds (prefill_kernel_is_ahead in
+// ws_plan.h: the launcher says B200_ENOTREADY) and loses the rest (44 against 11.8 us at M = 129, N = K = 4096, 164 against
+// 134-140 at M = 2048, N = 11008).
+// Where K is not a multiple of 256 (or the scales are not 16-byte aligned) the other choice up to 16 rows is the
+// register-streaming kernel, whose time grows with the rows: it keeps one row and small products, M * N * K < 50 M, at two
+// rows < 100 M where K < 5000 (streaming / weight-stationary in us: 4 x 4096 x 2080 5.1 / 5.3, 16 x 1024 x 1056 4.5 / 4.5;
+// 2 x 8192 x 3200 9.4 / 10.7, 2 x 11008 x 4128 13.3 / 16.2, with weights from HBM 15.3 / 15.6, 2 x 22016 x 2080 13.7 / 15.1, but
+// 2 x 8192 x 5152 21.6 / 19.0 and 2 x 16384 x 3200 16.1 / 13.7; 3 x 8640 x 3200 13.8 / 11.0, 8 x 4096 x 2080 7.0 / 5.5,
+// 16 x 22016 x 4128 86 / 24; above 16 rows, against the prefill kernel, 32 x 8640 x 3200 43 / 11.5, 2048 x 11008 x 4128 188 / 159).
+// (Above a gemm.ws_max_m that was lowered the skinny and prefill kernels take over, and a variant of the skinny kernel
+// asked for by option keeps its rows.)
+bool weight_stationary_first(int64_t M, int64_t N, int64_t K, bool ragged) {
+  const int64_t streamed = M == 2 && K < 5000 ? 100000000 : 50000000;
+  const bool ahead = M > 16 || (ragged ? M >= 2 && M * N * K >= streamed : M >= 9 || (M >= 5 && K >= 8192));
+  return ahead && M <= options().gemm_ws_max_m && (M > 16 || options().gemv_variant == 0);
+}
+
 int matmul_impl(Family fam, const char* who, const void* x, const void* wq, const void* scales, void* y, int64_t M,
                 int64_t N, int64_t K, void* stream) {
   int rc = check_matmul(who, x, wq, scales, y, M, N, K);
@@ -132,28 +157,8 @@ int matmul_impl(Family fam, const char* who, const void* x, const void* wq, cons
   auto wh = static_cast<const uint32_t*>(wq);
   auto sh = static_cast<const __half*>(scales);
   auto yh = static_cast<__half*>(y);
-  // 9 rows and more, and 5..8 where K is long: the weight-stationary kernel, whose weights stream once up to 128 rows.
-  // Measured on B200, skinny / weight-stationary kernel in us at 4, 8 and 16 rows: N = K = 4096 6.0 / 6.1, 7.7 / 6.4,
-  // 11.1 / 6.5; N = 22016 16.5 / 17.9, 17.9 / 18.1, 24.4 / 18.4; N = 4096, K = 11008 11.8 / 12.2, 18.9 / 12.3, 29.3 / 12.5;
-  // N = 1280, K = 8192 6.6 / 5.9, 9.7 / 6.0, 17.0 / 6.1 (the skinny kernel stages all of x in every CTA, and its
-  // arithmetic grows from 8 columns on).  At 5..8 rows and a shorter K the skinny kernel is the better one inside a
-  // decode step, where two of its CTAs fit an SM and it starts beside the kernel before it (8 layers of hidden
-  // 2048 at 5 rows: 413 us with it, 440 without).  Above 128 rows it cuts the tokens into tiles to suit the shape; the
-  // prefill kernel with its 256-token tiles keeps the long prompts that one wave of them holds (prefill_kernel_is_ahead in
-  // ws_plan.h: the launcher says B200_ENOTREADY) and loses the rest (44 against 11.8 us at M = 129, N = K = 4096, 164 against
-  // 134-140 at M = 2048, N = 11008).
-  // Where K is not a multiple of 256 (or the scales are not 16-byte aligned) the other choice up to 16 rows is the
-  // register-streaming kernel, whose time grows with the rows: it keeps one row and small products, M * N * K < 50 M, at two
-  // rows < 100 M where K < 5000 (streaming / weight-stationary in us: 4 x 4096 x 2080 5.1 / 5.3, 16 x 1024 x 1056 4.5 / 4.5;
-  // 2 x 8192 x 3200 9.4 / 10.7, 2 x 11008 x 4128 13.3 / 16.2, with weights from HBM 15.3 / 15.6, 2 x 22016 x 2080 13.7 / 15.1, but
-  // 2 x 8192 x 5152 21.6 / 19.0 and 2 x 16384 x 3200 16.1 / 13.7; 3 x 8640 x 3200 13.8 / 11.0, 8 x 4096 x 2080 7.0 / 5.5,
-  // 16 x 22016 x 4128 86 / 24; above 16 rows, against the prefill kernel, 32 x 8640 x 3200 43 / 11.5, 2048 x 11008 x 4128 188 / 159).
-  // (Above a gemm.ws_max_m that was lowered the skinny and prefill kernels take over, and a variant of the skinny kernel
-  // asked for by option keeps its rows.)
   const bool ragged = K % 256 != 0 || !aligned16(scales);
-  const int64_t streamed = M == 2 && K < 5000 ? 100000000 : 50000000;
-  const bool ws_auto = M > 16 || (ragged ? M >= 2 && M * N * K >= streamed : M >= 9 || (M >= 5 && K >= 8192));
-  if (fam == kGemmWs || (fam == kAuto && ws_auto && M <= options().gemm_ws_max_m && (M > 16 || options().gemv_variant == 0))) {
+  if (fam == kGemmWs || (fam == kAuto && weight_stationary_first(M, N, K, ragged))) {
     rc = fam == kGemmWs && (M > 128 || ragged) ? B200_ENOTREADY : launch_gemm_ws(xh, wh, sh, yh, M, N, K, s);
     if (rc != B200_ENOTREADY) return rc;
     if (fam == kGemmWs) return fail(B200_EINVAL, "%s: the weight-stationary kernel takes 1 <= M <= 128, K %% 256 == 0, 16-byte aligned scales", who);
@@ -480,6 +485,11 @@ int b200_q4f16_gemv_rmsnorm_rope(const void* x, const void* delta, const void* n
                                        static_cast<__half*>(v_cache), heads, K, static_cast<cudaStream_t>(stream));
 }
 
+int b200_q4f16_gemv_gate_up_applies(const void* scales, int64_t M, int64_t I, int64_t K) {
+  if (M < 1 || M > 16 || I < 8 || I % 8 != 0 || I > 0x3fffffffLL / 32 || K < 256 || K % 256 != 0 || !scales || !aligned16(scales)) return 0;
+  return options().gemv_variant != 1 && !weight_stationary_first(M, 2 * I, K, false);
+}
+
 int b200_q4f16_gemv_gate_up(const void* x, const void* delta, const void* norm_w, void* x_out, float eps, const void* wq,
                             const void* scales, void* act, int64_t M, int64_t I, int64_t K, void* stream) {
   const char* who = "q4f16_gemv_gate_up";
@@ -499,7 +509,7 @@ int b200_q4f16_gemv_gate_up(const void* x, const void* delta, const void* norm_w
                                 static_cast<__half*>(x_out), eps, static_cast<const uint32_t*>(wq),
                                 static_cast<const __half*>(scales), static_cast<__half*>(act), M, I, K,
                                 static_cast<cudaStream_t>(stream));
-  if (rc == B200_ENOTREADY) return fail(B200_EINVAL, "%s: shape outside the fused kernel's domain", who);
+  if (rc == B200_ENOTREADY) return fail(rc, "%s: shape outside the fused kernel's domain", who);
   return rc;
 }
 

@@ -93,10 +93,6 @@ def to_device(layer: dict, device):
     return out
 
 
-def _aligned(layers) -> bool:
-    return all(l["gu"][1].data_ptr() % 16 == 0 for l in layers)
-
-
 class DecodeEngine:
     """Buffers and kernel sequence of one decode step for `batch` sequences.
 
@@ -129,8 +125,6 @@ class DecodeEngine:
         # the separate kernels are faster (measured per layer at context 2000: 80 against 88 us at batch 2, 124 against
         # 176 at batch 8, 174 against 291 at batch 16).
         self.fused = (B == 1) if fused is None else (bool(fused) and B <= 16)
-        # up to 8 rows (the skinny kernel's) SwiGLU runs in the epilogue of the gate|up matmul, one launch less per layer
-        self.gate_up_epilogue = B <= (8 if H < 8192 else 4) and H % 256 == 0 and _aligned(layers)
         # False: rotary/append, attention, merge as three launches; True: one launch; "rope": rotary/append
         # inside the attention launch, merge as a second launch
         self.fused_attention = "rope" if fused_attention == "rope" else bool(fused_attention)
@@ -264,6 +258,11 @@ class DecodeEngine:
                                              self.batch, n, k, sp))
         self._check(self.L.b200_allreduce_peer(self.batch * n, ctypes.byref(d), sp))
 
+    def _gate_up_in_one(self, w) -> bool:
+        """Whether SwiGLU runs in the epilogue of the gate|up matmul: with fused prologues, else where the library would
+        take that matmul through the kernel that has the epilogue (asked anew each time: options may change)."""
+        return self.fused or bool(self.L.b200_q4f16_gemv_gate_up_applies(w["gu"][1].data_ptr(), self.batch, w["inter_local"], self.cfg.hidden))
+
     def _allreduce(self, t):
         if self.world > 1:
             torch.distributed.all_reduce(t, group=self.group)
@@ -336,22 +335,21 @@ class DecodeEngine:
         else:
             self._matmul(self.attn, w["o"], self.o, H, hl, sp)
             self._allreduce(self.o)
-        if self.fused or self.gate_up_epilogue:
-            # gate, up and SwiGLU in one launch
-            if self.fused:
-                self._check(L.b200_q4f16_gemv_gate_up(self.x2.data_ptr(), self.o.data_ptr(), w["norm2"].data_ptr(), self.x.data_ptr(),
-                                                      cfg.eps, w["gu"][0].data_ptr(), w["gu"][1].data_ptr(), self.act.data_ptr(),
-                                                      B, il, H, sp))
-            else:
-                self._check(L.b200_rmsnorm_early_release(self.x.data_ptr(), self.o.data_ptr(), w["norm2"].data_ptr(),
-                                                         self.h.data_ptr(), B, H, cfg.eps, sp))
-                self._check(L.b200_q4f16_gemv_gate_up(self.h.data_ptr(), None, None, None, 0.0, w["gu"][0].data_ptr(),
-                                                      w["gu"][1].data_ptr(), self.act.data_ptr(), B, il, H, sp))
+        if self.fused:
+            self._check(L.b200_q4f16_gemv_gate_up(self.x2.data_ptr(), self.o.data_ptr(), w["norm2"].data_ptr(), self.x.data_ptr(),
+                                                  cfg.eps, w["gu"][0].data_ptr(), w["gu"][1].data_ptr(), self.act.data_ptr(),
+                                                  B, il, H, sp))
         else:
             self._check(L.b200_rmsnorm_early_release(self.x.data_ptr(), self.o.data_ptr(), w["norm2"].data_ptr(), self.h.data_ptr(),
                                                      B, H, cfg.eps, sp))
-            self._matmul(self.h, w["gu"], self.gu, 2 * il, H, sp)
-            self._check(L.b200_silu_mul_early_release(self.gu.data_ptr(), self.act.data_ptr(), B, il, sp))
+            rc = _lib.ENOTREADY
+            if self._gate_up_in_one(w):
+                rc = L.b200_q4f16_gemv_gate_up(self.h.data_ptr(), None, None, None, 0.0, w["gu"][0].data_ptr(),
+                                               w["gu"][1].data_ptr(), self.act.data_ptr(), B, il, H, sp)
+            if rc == _lib.ENOTREADY:
+                self._matmul(self.h, w["gu"], self.gu, 2 * il, H, sp)
+                rc = L.b200_silu_mul_early_release(self.gu.data_ptr(), self.act.data_ptr(), B, il, sp)
+            self._check(rc)
         if self.peer is not None and B <= self.PEER_FUSED_MAX_ROWS:
             d = self._reduce_desc(1, i, self.down)
             self._check(L.b200_q4f16_gemv_allreduce(self.act.data_ptr(), w["down"][0].data_ptr(), w["down"][1].data_ptr(),
@@ -409,7 +407,7 @@ class DecodeEngine:
         head = 1 if self.lm_head is not None and self.batch <= 16 else 0
         if self.layer_kernel:
             return 1 + len(self.layers) + 1 + head + 2
-        per_layer = (5 if self.fused else 8 if self.gate_up_epilogue else 9) + (1 if self.fused_attention == "rope" else (0 if self.fused_attention else 2))
+        per_layer = (5 if self.fused else 8 if self.layers and self._gate_up_in_one(self.layers[0]) else 9) + (1 if self.fused_attention == "rope" else (0 if self.fused_attention else 2))
         if self.rope_epilogue:
             per_layer -= 1
         return 1 + len(self.layers) * per_layer + 1 + head + 2

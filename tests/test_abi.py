@@ -233,3 +233,27 @@ def test_options_of_the_weight_stationary_kernel():
     for v in (0, 127, 128, 129, unlimited):
         assert L.b200_set_option(b"gemm.ws_max_m", v) == 0 and L.b200_get_option(b"gemm.ws_max_m") == v
     assert L.b200_set_option(b"gemm.ws_max_m", -1) == _lib.EINVAL and L.b200_get_option(b"gemm.ws_max_m") == unlimited
+
+
+def test_gate_up_applies_where_the_automatic_matmul_takes_its_kernel():
+    L = _lib.lib()
+    scales = 1 << 20                                       # an address: only its alignment is looked at
+
+    def applies(m, i, k, at=scales):
+        return L.b200_q4f16_gemv_gate_up_applies(at, m, i, k)
+
+    assert all(applies(m, 5632, 2048) for m in (1, 2, 5, 8)) and not any(applies(m, 5632, 2048) for m in (0, 9, 16, 17))
+    assert applies(4, 5632, 8192) and not applies(5, 5632, 8192)
+    assert not applies(4, 5632, 2080) and not applies(4, 5636, 2048) and not applies(4, 0, 2048) and not applies(4, 8, 0)
+    assert not applies(4, 5632, 2048, at=scales + 8) and not applies(4, 5632, 2048, at=None)
+    try:
+        _lib.set_option("gemv.variant", 1)                 # the register-streaming kernel has no such epilogue
+        assert not applies(5, 5632, 2048)
+        _lib.set_option("gemv.variant", 2)                 # rows that the weight-stationary kernel would have had
+        assert applies(5, 5632, 8192) and applies(16, 5632, 2048)
+        _lib.set_option("gemv.variant", 0)
+        _lib.set_option("gemm.ws_max_m", 8)
+        assert applies(9, 5632, 2048) and not applies(8, 5632, 8192)
+    finally:
+        _lib.set_option("gemv.variant", 0)
+        _lib.set_option("gemm.ws_max_m", 0x7fffffff)

@@ -257,6 +257,42 @@ def test_decoder_steps_match_oracle(cuda_lib, B, fused):
     assert cuda_lib.b200_device_error_flags() == 0
 
 
+def test_decoder_follows_the_matmul_options(cuda_lib):
+    """At 2..8 rows gate|up goes where b200_q4f16_matmul would take it: with SwiGLU in the epilogue, or as the kernel that an option
+    asks for and a SwiGLU launch behind it; scales that come to lie off 16 bytes after the engine was built take that way too."""
+    cfg, B = SMALL, 5
+    rng = np.random.default_rng(17)
+    layers = [decoder.to_device(tp.shard_layer(decoder.synth_layer_numpy(cfg, 40 + i), 0, 1, cfg.hidden, cfg.inter), "cuda") for i in range(cfg.layers)]
+    eng = decoder.DecodeEngine(cfg, layers, dev((0.5 * rng.standard_normal((cfg.vocab, cfg.hidden))).astype(F16)), dev(np.ones(cfg.hidden, F16)),
+                               dev((0.05 * rng.standard_normal((cfg.vocab, cfg.hidden))).astype(F16)), B, 16, "cuda")
+
+    def step():
+        eng.set_position(0)
+        eng.tokens.copy_(torch.arange(B, dtype=torch.int32))
+        before = cuda_lib.b200_launch_count()
+        eng.step()
+        torch.cuda.synchronize()
+        return cuda_lib.b200_launch_count() - before, eng.logits.float().cpu().numpy()
+
+    count, ref = step()
+    scale = np.abs(ref).max()
+    try:
+        _lib.set_option("gemv.variant", 1)
+        count1, out1 = step()
+    finally:
+        _lib.set_option("gemv.variant", 0)
+    assert count1 == count + cfg.layers
+    close(out1, ref, 1e-2, 1e-2 * scale, "streaming kernel")
+    for w in layers:
+        off = torch.empty(w["gu"][1].numel() + 1, dtype=torch.float16, device="cuda")[1:].view(w["gu"][1].shape)
+        off.copy_(w["gu"][1])
+        w["gu"] = (w["gu"][0], off)
+    count2, out2 = step()
+    assert count2 == count + cfg.layers
+    close(out2, ref, 1e-2, 1e-2 * scale, "scales off 16 bytes")
+    assert cuda_lib.b200_device_error_flags() == 0
+
+
 def test_decoder_graph_replay_matches_eager(cuda_lib):
     cfg = SMALL
     rng = np.random.default_rng(5)
