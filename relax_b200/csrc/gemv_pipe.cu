@@ -113,9 +113,8 @@ struct PipeParams {
   PeerReduce red;
 };
 
-// The arithmetic of the fast form over the first NU of a warp's U chunks of one stage (see the comment at its call site in
-// the kernel).  NU < U: the others lie past K (zero-filled) and are skipped.
-template <int NU, int U, int MT, int kXUnit, int kCUnit>
+// The arithmetic of the fast form over a warp's U chunks of one stage (see the comment at its call site in the kernel).
+template <int U, int MT, int kXUnit, int kCUnit>
 __device__ __forceinline__ void fast_stage_fn(float (&acc)[2][MT][4], const uint4 (&w)[U][2][2], const uint2 (&sc)[U][2],
                                             const uint4* xb, int x_mul, const float4* cu, const Q4Consts& qc,
                                             uint32_t magic_hi) {
@@ -125,7 +124,7 @@ __device__ __forceinline__ void fast_stage_fn(float (&acc)[2][MT][4], const uint
     uint32_t a[U][2][8];      // raw (offset) nibble pairs: [0..3] first MMA (rows g, g+8: even k, odd k), [4..7] second
     uint4 b[U][2];
 #pragma unroll
-    for (int u = 0; u < NU; ++u)
+    for (int u = 0; u < U; ++u)
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const uint32_t w0 = wd == 0 ? w[u][0][h].x : wd == 1 ? w[u][0][h].y : wd == 2 ? w[u][0][h].z : w[u][0][h].w;
@@ -142,7 +141,7 @@ __device__ __forceinline__ void fast_stage_fn(float (&acc)[2][MT][4], const uint
         a[u][h][7] = lop3_and_or(w1s, qc.hi, magic_hi);
       }
 #pragma unroll
-    for (int u = 0; u < NU; ++u)
+    for (int u = 0; u < U; ++u)
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         if (wd == 0) {
@@ -153,13 +152,13 @@ __device__ __forceinline__ void fast_stage_fn(float (&acc)[2][MT][4], const uint
         }
       }
 #pragma unroll
-    for (int u = 0; u < NU; ++u)
+    for (int u = 0; u < U; ++u)
 #pragma unroll
       for (int h = 0; h < 2; ++h)
         mma_16x8x16(d[u][h], a[u][h][4], a[u][h][5], a[u][h][6], a[u][h][7], b[u][h].z, b[u][h].w);
   }
 #pragma unroll
-  for (int u = 0; u < NU; ++u) {
+  for (int u = 0; u < U; ++u) {
     // scales of groups 4t'+0..3: (s0, s1) (s2, s3); even groups belong to set 0, odd ones to set 1
     const float2 g01 = __half22float2(u32_as_h2(sc[u][0].x)), g23 = __half22float2(u32_as_h2(sc[u][0].y));
     const float2 h01 = __half22float2(u32_as_h2(sc[u][1].x)), h23 = __half22float2(u32_as_h2(sc[u][1].y));
@@ -503,14 +502,11 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
   // Fast form, the U chunks of one stage together.  Set h = 0 / 1 is the lane's 16-byte unit 2t / 2t+1 (an even /
   // odd group); its four words for rows g and g+8 give eight MMAs into one accumulator d[u][h] that starts at
   // minus the offset sums.  Afterwards d[u][h][0], [1] are row g's sums over groups 4t+h and 4t+2+h, [2], [3] row
-  // g+8's.  The MMAs are issued round-robin over the 2U accumulators, so that one does not follow the one it depends on
-  // (which would wait out the tensor pipe's whole latency; with U = 1, two accumulators, half of it is left).
-  // `left`: how much of K there is from this warp's first chunk on.
-  auto fast_stage = [&](int left, const uint4 (&w)[U][2][2], const uint2 (&sc)[U][2], const uint4* xu, const float4* cu) {
-    static_assert(!FAST || U <= 2, "one or two chunks a warp and stage");
-    const uint4* xb = x_own ? xu : &s_zero;
-    if (U == 2 && left > CW * 256) fast_stage_fn<U, U, MT, kXUnit, kCUnit>(acc, w, sc, xb, x_mul, cu, qc, magic_hi);
-    else if (left > 0) fast_stage_fn<1, U, MT, kXUnit, kCUnit>(acc, w, sc, xb, x_mul, cu, qc, magic_hi);
+  // g+8's.  The MMAs are issued round-robin over the 2U accumulators (an MMA that follows the one it depends on
+  // waits out the tensor pipe's whole latency; with the accumulators interleaved nothing waits).
+  auto fast_stage = [&](const uint4 (&w)[U][2][2], const uint2 (&sc)[U][2], const uint4* xu, const float4* cu) {
+    static_assert(!FAST || U == 1, "a warp's chunk of a stage lies before or past the end of K as a whole");
+    fast_stage_fn<U, MT, kXUnit, kCUnit>(acc, w, sc, x_own ? xu : &s_zero, x_mul, cu, qc, magic_hi);
   };
   // Fast form: this warp's share of stage `s` into registers; the stage goes back to the producer at once.
   auto fast_load = [&](int s, uint32_t round, uint4 (&w)[U][2][2], uint2 (&sc)[U][2]) {
@@ -788,7 +784,8 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
         if (FAST) {
           // (the first stage of the launch is in registers already)
           if (!(kb == 0 && tile == (int)blockIdx.x && k0 == k_lo)) fast_load(s, round, fw, fsc);
-          fast_stage(k_hi - (k0 + warp * 256), fw, fsc, xk, ck);
+          // this warp's chunk of the stage, unless it lies past K
+          if (k0 + warp * 256 < k_hi) fast_stage(fw, fsc, xk, ck);
         } else {
         // On a timeout the kernel keeps going without waiting (results are garbage, the error
         // flag says so) so that every warp still reaches the named barriers and the CTA ends.
@@ -1000,7 +997,7 @@ int launch_pipe(const __half* x, const uint32_t* wq, const __half* scales, __hal
   int kblk = kpad, grid = 0, stages = (int)options().gemv_stages;
   bool placed = false;
   if (FAST) {
-    // Two CTAs per SM with two stages each (one of the longer ones: launch_pipe_m; registers are a further buffer): measured
+    // Two CTAs per SM with two stages each (launch_pipe_m; registers are a third buffer, as in the exact form): measured
     // fastest for every shape of the 7B decode step.  One CTA per SM with a CTA's whole share of W resident, so that the next
     // launch's CTAs prefetch beside this launch's, was measured too: no faster for N = K = 4096 and 10-20 % slower for the
     // large matmuls.  Options gemv.ctas_per_sm and gemv.stages still select them.
@@ -1138,15 +1135,6 @@ int launch_pipe_m(const __half* x, const uint32_t* wq, const __half* scales, __h
     // the registers (no spills in the RMSNorm form); three or more stages are slower again (bytes in flight beyond what
     // HBM needs): N = 22016 one of 4096 / 2, 3, 4 of 2048: 12.07 / 11.68, 12.23, 13.00 us; N = 12288 8.26 / 8.03, 8.45, 9.01;
     // N = 4096, K = 11008 8.46 / 8.18, 8.39, 8.39; N = K = 8192 9.97 / 9.63, 10.01, 10.81; N = K = 4096 4.72 / 4.70.
-    // One stage of 4096 k where a CTA has one tile of that length: nothing is refilled, and all of a warp's share of W is in
-    // registers when the wait for x returns.  Short / long at K = 4096: N = 1024 3.21 / 3.16, N = 1536 3.82 / 3.74, N = 2048
-    // 3.89 / 3.86, N = 4096 4.77 / 4.75, N = 4736 4.98 / 4.88, and 40 of N = K = 4096 183.5 / 182.3; at K = 3840 within 1 % either way, at
-    // K = 3072 4.24 / 4.31.  Not between one and one and a half tiles an SM (N = 2368 3.71 / 3.87, N = 2752 3.96 / 4.02), nor
-    // in the forms with RMSNorm (5.91 / 6.02) or SwiGLU.
-    const int tiles = (n + kRows - 1) / kRows, sms = sm_count();
-    constexpr bool kPlain = PRO == kPrologueNone && !GU;
-    if (fast && kPlain && k > 3584 && k <= 4096 && tiles <= 2 * sms && (tiles < sms || 2 * tiles > 3 * sms))
-      return launch_pipe<1, CW, kPlain ? CH : CW, PRO, true, GU>(x, wq, scales, y, m, n, k, stream, pro, red);
     if (fast) return launch_pipe<1, CW, CW, PRO, true, GU>(x, wq, scales, y, m, n, k, stream, pro, red);
     return launch_pipe<1, CW, CH, PRO, false, GU>(x, wq, scales, y, m, n, k, stream, pro, red);
   }

@@ -177,21 +177,6 @@ def test_gemv_stage_lengths_of_a_long_k(cuda_lib, m, n, k):
     assert cuda_lib.b200_device_error_flags() == 0
 
 
-@pytest.mark.parametrize("n,k", [(2352, 4096), (2368, 4096), (3552, 3840), (3568, 3840), (4736, 4096), (4752, 4096), (4096, 3584), (4090, 3840), (16, 4096)])
-def test_gemv_one_row_one_tile_a_cta(cuda_lib, n, k, gemv_form):
-    """Either side of the lines within which a CTA's one tile comes as one 4096-k stage (rows of W, K), K that leaves chunks of
-    that stage empty, a ragged last tile; three launches back to back, each into an output of its own."""
-    x, wq, s = synth.make_case(1, n, k, seed=n + k)
-    tx, twq, ts = dev(x, wq, s)
-    out = torch.full((3, 1, n), float("nan"), dtype=torch.float16, device="cuda")
-    for i in range(3):
-        ops.q4f16_matmul(tx, twq, ts, out=out[i])
-    torch.cuda.synchronize()
-    for y in out.cpu().numpy():
-        assert_matmul_close(y, x, wq, s, f"N={n} K={k}")
-    assert cuda_lib.b200_device_error_flags() == 0
-
-
 @pytest.mark.parametrize("n,k", [(5000, 12288), (5000, 12544), (300, 14336), (300, 26624), (300, 26880), (100, 32768)])
 def test_gemv_one_row_long_k(cuda_lib, n, k, gemv_form):
     """One row where two stages fit beside x in half an SM (up to K = 26624), and beyond."""
