@@ -502,8 +502,9 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
   // Fast form, the U chunks of one stage together.  Set h = 0 / 1 is the lane's 16-byte unit 2t / 2t+1 (an even /
   // odd group); its four words for rows g and g+8 give eight MMAs into one accumulator d[u][h] that starts at
   // minus the offset sums.  Afterwards d[u][h][0], [1] are row g's sums over groups 4t+h and 4t+2+h, [2], [3] row
-  // g+8's.  The MMAs are issued round-robin over the 2U accumulators (an MMA that follows the one it depends on
-  // waits out the tensor pipe's whole latency; with the accumulators interleaved nothing waits).
+  // g+8's.  The MMAs are issued round-robin over the 2U accumulators, so that one does not directly follow the one it
+  // depends on.  (With U = 1 there are two; four, each over half of the words, measured 0-3 % slower: the other
+  // warps fill the gaps.)
   auto fast_stage = [&](const uint4 (&w)[U][2][2], const uint2 (&sc)[U][2], const uint4* xu, const float4* cu) {
     static_assert(!FAST || U == 1, "a warp's chunk of a stage lies before or past the end of K as a whole");
     fast_stage_fn<U, MT, kXUnit, kCUnit>(acc, w, sc, x_own ? xu : &s_zero, x_mul, cu, qc, magic_hi);
@@ -1134,7 +1135,11 @@ int launch_pipe_m(const __half* x, const uint32_t* wq, const __half* scales, __h
     // Two stages of 2048 k a CTA: against one of 4096 k the ring refills in halves and a warp's share of a stage takes half
     // the registers (no spills in the RMSNorm form); three or more stages are slower again (bytes in flight beyond what
     // HBM needs): N = 22016 one of 4096 / 2, 3, 4 of 2048: 12.07 / 11.68, 12.23, 13.00 us; N = 12288 8.26 / 8.03, 8.45, 9.01;
-    // N = 4096, K = 11008 8.46 / 8.18, 8.39, 8.39; N = K = 8192 9.97 / 9.63, 10.01, 10.81; N = K = 4096 4.72 / 4.70.
+    // N = 4096, K = 11008 8.46 / 8.18, 8.39, 8.39; N = K = 8192 9.97 / 9.63, 10.01, 10.81.
+    // Where a CTA has one tile of up to 4096 k nothing is refilled, and one long stage, all of it in registers when the wait for x
+    // returns, is 0-2 % faster back to back (N = 2048, K = 4096 3.84 / 3.79, N = 4736 4.97 / 4.88, 40 of N = K = 4096 183.3 / 182.4).
+    // But it is a kernel of its own, and inside a decode step, where other kernels run in between, the o projection took
+    // 0.3 us longer with it (a step of the 7B shape 1646 / 1656): one form for every K.
     if (fast) return launch_pipe<1, CW, CW, PRO, true, GU>(x, wq, scales, y, m, n, k, stream, pro, red);
     return launch_pipe<1, CW, CH, PRO, false, GU>(x, wq, scales, y, m, n, k, stream, pro, red);
   }
