@@ -402,15 +402,19 @@ class DecodeEngine:
         self._check(L.b200_advance_pos(self.epoch.data_ptr(), 1, sp))
 
     def kernels_per_step(self) -> int:
-        """Kernels of this library launched by one step (embed + 6 to 11 per layer + final norm + output projection
-        for up to 16 rows + advance)."""
+        """Kernels of this library launched by one step: embed, 5 to 12 per layer, final norm, output projection for up to
+        16 rows, two counters."""
         head = 1 if self.lm_head is not None and self.batch <= 16 else 0
         if self.layer_kernel:
             return 1 + len(self.layers) + 1 + head + 2
-        per_layer = (5 if self.fused else 8 if self.layers and self._gate_up_in_one(self.layers[0]) else 9) + (1 if self.fused_attention == "rope" else (0 if self.fused_attention else 2))
-        if self.rope_epilogue:
-            per_layer -= 1
-        return 1 + len(self.layers) * per_layer + 1 + head + 2
+        # rotary + append (unless the qkv matmul does it), attention, merge; or the forms that put two or all of them in one
+        attention = 2 if self.fused_attention == "rope" or self.rope_epilogue else 1 if self.fused_attention else 3
+        peer_sums = 2 if self.peer is not None and self.batch > self.PEER_FUSED_MAX_ROWS else 0
+        per_layer = 0
+        for w in self.layers:
+            mlp = 2 if self.fused else 3 if self._gate_up_in_one(w) else 4        # (norm,) gate|up (, SwiGLU), down
+            per_layer += (1 if self.fused else 2) + attention + 1 + mlp + peer_sums
+        return 1 + per_layer + 1 + head + 2
 
     def capture(self, stream):
         """Captures one step into a CUDA graph on `stream` (after one eager warm-up step, which

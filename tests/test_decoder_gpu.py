@@ -293,6 +293,21 @@ def test_decoder_follows_the_matmul_options(cuda_lib):
     assert cuda_lib.b200_device_error_flags() == 0
 
 
+@pytest.mark.parametrize("B,kw", [(1, {}), (1, dict(rope_epilogue=False)), (1, dict(fused_attention=True)), (1, dict(fused_attention="rope")),
+                                  (1, dict(fused=False)), (1, dict(layer_kernel=True)), (3, dict(fused=True)), (5, {}), (5, dict(fused_attention=True)),
+                                  (16, {}), (16, dict(fused=True)), (20, {})])
+def test_kernels_per_step_is_what_a_step_launches(cuda_lib, B, kw):
+    cfg = decoder.DecoderConfig(hidden=2560, heads=20, inter=768, layers=2, vocab=300)        # (K = 2560: the rotary epilogue's form)
+    layers = [decoder.to_device(tp.shard_layer(decoder.synth_layer_numpy(cfg, 60 + i), 0, 1, cfg.hidden, cfg.inter), "cuda") for i in range(cfg.layers)]
+    eng = decoder.DecodeEngine(cfg, layers, dev(np.ones((cfg.vocab, cfg.hidden), F16)), dev(np.ones(cfg.hidden, F16)),
+                               dev(np.ones((cfg.vocab, cfg.hidden), F16)), B, 16, "cuda", **kw)
+    before = cuda_lib.b200_launch_count()
+    eng.step()
+    torch.cuda.synchronize()
+    assert cuda_lib.b200_launch_count() - before == eng.kernels_per_step()
+    assert cuda_lib.b200_device_error_flags() == 0
+
+
 def test_decoder_graph_replay_matches_eager(cuda_lib):
     cfg = SMALL
     rng = np.random.default_rng(5)
