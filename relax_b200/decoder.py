@@ -120,8 +120,8 @@ class DecodeEngine:
         f16 = dict(dtype=torch.float16, device=self.device)
         hl = H // world
         il_max = max(l["inter_local"] for l in layers) if layers else cfg.inter
-        # fused: RMSNorm (+ residual add) runs inside the staging of the next skinny matmul; needs batch <= 16, the skinny kernel's range.  By default only at
-        # batch 1: every CTA of a fused kernel recomputes the statistics of all the batch's rows, and from two rows on
+        # fused: RMSNorm (+ residual add) runs inside the staging of the next skinny matmul; needs batch <= 16, the skinny
+        # kernel's range.  By default only at batch 1: every CTA of a fused kernel recomputes the statistics of all the batch's rows, and from two rows on
         # the separate kernels are faster (measured per layer at context 2000: 80 against 88 us at batch 2, 124 against
         # 176 at batch 8, 174 against 291 at batch 16).
         self.fused = (B == 1) if fused is None else (bool(fused) and B <= 16)
@@ -135,7 +135,7 @@ class DecodeEngine:
         self.q = torch.zeros((B, self.nh_local, 128), **f16)
         self.attn = torch.zeros((B, hl), **f16)
         self.o = torch.zeros((B, H), **f16)
-        self.gu = torch.zeros((B, 2 * il_max), **f16)
+        self.gu = None if self.fused else torch.zeros((B, 2 * il_max), **f16)       # (where SwiGLU is a launch of its own)
         self.act = torch.zeros((B, il_max), **f16)
         self.down = torch.zeros((B, H), **f16)
         self.kc = [torch.zeros((B, max_ctx, self.nh_local, 128), **f16) for _ in layers]
@@ -152,10 +152,10 @@ class DecodeEngine:
         self.lm_scratch = torch.zeros((max(int(self.L.b200_lm_head_scratch_bytes()), 16) // 4,), dtype=torch.float32, device=self.device)
         self.graph = None
         self.launches_per_step = 0
-        # batch 1: one persistent kernel per layer (b200_decode_layer) instead of seven launches.  Off by default:
-        # measured on B200 at the 7B shape it is as fast as the seven launches on one GPU (1.94 against 1.90 ms per
-        # token) and slower on two (2.07 against 1.89), because every stage boundary inside it costs what a
-        # dependent launch costs, and its attention stage has only eight warps per SM with loads in flight
+        # batch 1: one persistent kernel per layer (b200_decode_layer) instead of six launches.  Off by default:
+        # measured on B200 at the 7B shape it is slower (2.00 against 1.64 ms per token), because every stage boundary
+        # inside it costs what a dependent launch costs, and its attention stage has only eight warps per SM with loads in
+        # flight
         self.layer_kernel = False if layer_kernel is None else bool(layer_kernel)
         # batch 1, fused prologues, three-launch attention: rotary embedding + KV append run in the epilogue of the
         # qkv matmul (b200_q4f16_gemv_rmsnorm_rope), one launch less per layer
