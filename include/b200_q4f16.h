@@ -218,7 +218,8 @@ B200_API int b200_q4f16_gemv_gate_up(const void* x, const void* delta, const voi
  * rows are [q heads | k heads | v heads] (heads of 128); q is rotated (rotate-half pairing d <-> d+64, tables fp32
  * [max_pos, 64], position *pos) into q_out fp16 [heads*128], the rotated key and the value of the new token go
  * into k_cache / v_cache fp16 [max_ctx, heads, 128] at slot *pos; there is no qkv buffer.  Same arithmetic as the
- * two separate kernels (the rotation works on the fp16-rounded matmul results).  The caches' entries below *pos are
+ * two separate kernels (the rotation works on the fp16-rounded matmul results; which of its two products is fused into
+ * the sum is the compiler's choice in either, so a few values in ten thousand differ by one fp16 step).  The caches' entries below *pos are
  * asked for in L2 on the way out (a hint), for the attention that reads them next.  Returns B200_ENOTREADY, with
  * nothing launched, when this launch would not use the skinny kernel's fast form (option gemv.exact = 1, or K below
  * 2560): call the two separate entry points then. */

@@ -169,7 +169,7 @@ def oracle_steps(cfg, layers, embed, final_norm, lm_head, tokens, steps, max_ctx
 
 # M = 1 with K <= 4096 takes the one-pass form of the RMSNorm prologue (row kept in registers)
 @pytest.mark.parametrize("M,N,K", [(1, 512, 1024), (1, 4096, 4096), (1, 272, 2304), (1, 128, 8192), (3, 300, 4096), (16, 64, 256),
-                                   (8, 4096, 2816)])
+                                   (8, 4096, 2816), (2, 512, 1024), (8, 300, 5120), (5, 300, 13824), (1, 300, 13824)])
 def test_gemv_with_fused_neighbours(cuda_lib, M, N, K, gemv_form):
     from relax_b200 import synth
     from util import assert_matmul_close, skinny_form_is_unrounded, unrounded_slack
@@ -521,3 +521,76 @@ def test_gate_up_matmul_with_swiglu_epilogue_equals_the_two_kernels(cuda_lib, M,
     assert cuda_lib.b200_q4f16_gemv_gate_up(p, None, None, None, 0.0, twq.data_ptr(), ts.data_ptr(), one.data_ptr(), M, I - 4, K, 0) == _lib.EINVAL
     assert cuda_lib.b200_q4f16_gemv_gate_up(p, p, None, None, 0.0, twq.data_ptr(), ts.data_ptr(), one.data_ptr(), M, I, K, 0) == _lib.EINVAL
     assert cuda_lib.b200_q4f16_gemv_gate_up(p, None, None, None, 0.0, twq.data_ptr(), ts.data_ptr(), one.data_ptr(), M, I, K - 128, 0) == _lib.EINVAL
+
+
+@pytest.mark.parametrize("M,I,K,norm,exact,layout", [(1, 1376, 4096, True, 1, 0), (1, 200, 1024, True, 2, 0), (1, 200, 1024, False, 2, 1), (1, 1376, 4096, True, 0, 1),
+                                                     (1, 136, 13824, True, 0, 0), (4, 200, 2048, True, 0, 1), (9, 72, 5120, True, 0, 0), (16, 2400, 5120, False, 0, 0),
+                                                     (8, 200, 13824, False, 0, 1), (5, 72, 13824, True, 0, 0), (3, 72, 26624, False, 0, 0)])
+def test_gate_up_matmul_forms_and_k_blocks(cuda_lib, M, I, K, norm, exact, layout):
+    """b200_q4f16_gemv_gate_up against the two kernels, bit for bit: each arithmetic form of one row, both nibble orders, and an
+    x that does not fit shared memory, so that K is cut into blocks and partial sums are carried."""
+    rng = np.random.default_rng(M + I + K)
+    x, wq, s = synth.make_case(M, 2 * I, K, seed=M + I)
+    tx, twq, ts, td, tn = (dev(a) for a in ((0.1 * x.astype(np.float32)).astype(F16), wq, s, (0.1 * rng.standard_normal((M, K))).astype(F16),
+                                            (1 + 0.1 * rng.standard_normal(K)).astype(F16)))
+    gu = torch.empty((M, 2 * I), dtype=torch.float16, device="cuda")
+    two, one = (torch.full((M, I), float("nan"), dtype=torch.float16, device="cuda") for _ in range(2))
+    xo = torch.zeros((2, M, K), dtype=torch.float16, device="cuda")
+    args = (td.data_ptr(), tn.data_ptr(), xo[1].data_ptr()) if norm else (None, None, None)
+    try:
+        _lib.set_option("gemv.exact", exact)
+        _lib.set_option("weights.layout", layout)
+        if norm:
+            assert cuda_lib.b200_q4f16_gemv_rmsnorm(tx.data_ptr(), td.data_ptr(), tn.data_ptr(), xo[0].data_ptr(), 1e-5, twq.data_ptr(), ts.data_ptr(),
+                                                    gu.data_ptr(), M, 2 * I, K, 0) == 0, _lib.last_error()
+        else:
+            assert cuda_lib.b200_q4f16_gemv(tx.data_ptr(), twq.data_ptr(), ts.data_ptr(), gu.data_ptr(), M, 2 * I, K, 0) == 0, _lib.last_error()
+        assert cuda_lib.b200_silu_mul(gu.data_ptr(), two.data_ptr(), M, I, 0) == 0, _lib.last_error()
+        assert cuda_lib.b200_q4f16_gemv_gate_up(tx.data_ptr(), *args, 1e-5, twq.data_ptr(), ts.data_ptr(), one.data_ptr(), M, I, K, 0) == 0, _lib.last_error()
+        torch.cuda.synchronize()
+    finally:
+        _lib.set_option("gemv.exact", 0)
+        _lib.set_option("weights.layout", 0)
+    assert torch.equal(one.view(torch.int16), two.view(torch.int16)) and torch.equal(xo[0], xo[1])
+    assert bool(torch.isfinite(gu).all()) and float(one.float().abs().max()) > 0
+    assert cuda_lib.b200_device_error_flags() == 0
+
+
+@pytest.mark.parametrize("nh,K,max_ctx,pos,offset", [(4, 2560, 8, 0, 0), (4, 2560, 8, 7, 0), (4, 2560, 8, 7, 1), (32, 4096, 4300, 4095, 0), (32, 4096, 4300, 4299, 0),
+                                                     (32, 4096, 4300, 4200, 4)])
+def test_qkv_matmul_with_older_cache_entries(cuda_lib, nh, K, max_ctx, pos, offset):
+    """b200_q4f16_gemv_rmsnorm_rope asks for the caches' older entries in L2: none of them (position 0), more than it asks for
+    (32 MB of each cache), and caches that do not start on 16 bytes (`offset` values in).  Outputs are those of the two
+    kernels, up to the rounding of the rotation, and the caches' other entries stay."""
+    N = 3 * nh * 128
+    x, wq, s = synth.make_case(1, N, K, seed=nh + pos)
+    tx, twq, ts, tn = (dev(a) for a in (x, wq, s, np.ones(K, F16)))
+    cos, sin = decoder.rope_tables(max_ctx, 128, 10000.0, "cuda")
+    tpos = torch.tensor([pos], dtype=torch.int32, device="cuda")
+    n = max_ctx * nh * 128
+    fill = torch.randn(n, device="cuda", generator=torch.Generator("cuda").manual_seed(pos)).half()
+    kc, vc = (torch.empty((2, n + 8), dtype=torch.float16, device="cuda")[:, offset:offset + n] for _ in range(2))     # rows start 16 bytes on
+    kc.copy_(fill.expand(2, n))
+    vc.copy_(fill.expand(2, n))
+    q = torch.zeros((2, nh * 128), dtype=torch.float16, device="cuda")
+    qkv = torch.zeros((1, N), dtype=torch.float16, device="cuda")
+    assert cuda_lib.b200_q4f16_gemv_rmsnorm(tx.data_ptr(), None, tn.data_ptr(), None, 1e-5, twq.data_ptr(), ts.data_ptr(), qkv.data_ptr(), 1, N, K,
+                                            0) == 0, _lib.last_error()
+    assert cuda_lib.b200_rope_kv_append(qkv.data_ptr(), cos.data_ptr(), sin.data_ptr(), tpos.data_ptr(), q[0].data_ptr(), kc[0].data_ptr(),
+                                        vc[0].data_ptr(), 1, nh, max_ctx, 0) == 0, _lib.last_error()
+    assert cuda_lib.b200_q4f16_gemv_rmsnorm_rope(tx.data_ptr(), None, tn.data_ptr(), None, 1e-5, twq.data_ptr(), ts.data_ptr(), cos.data_ptr(),
+                                                 sin.data_ptr(), tpos.data_ptr(), q[1].data_ptr(), kc[1].data_ptr(), vc[1].data_ptr(), nh, K,
+                                                 0) == 0, _lib.last_error()
+    torch.cuda.synchronize()
+    # a rotated value is a * c - b * s in fp32 with one of the products fused, whichever the compiler takes: the other one's
+    # rounding, 2^-24 of it, may move the fp16 result to its neighbour (2^-10 of it at most)
+    new = slice(pos * nh * 128, (pos + 1) * nh * 128)
+    for one, two in ((q[1], q[0]), (kc[1, new], kc[0, new])):
+        two = two.float()
+        assert bool(((one.float() - two).abs() <= 2.0 ** -10 * two.abs() + 2.0 ** -23 * qkv.abs().max()).all())
+        assert int((one.float() != two).sum()) <= 8
+    assert torch.equal(vc[0], vc[1]) and not torch.equal(kc[1, new], fill[new])
+    for cache in (kc, vc):
+        for part in (slice(0, new.start), slice(new.stop, n)):
+            assert torch.equal(cache[1, part], fill[part])
+    assert cuda_lib.b200_device_error_flags() == 0

@@ -154,17 +154,19 @@ def test_gemv_both_kernels(cuda_lib, variant, m, n, k, gemv_form):
 
 
 @pytest.mark.parametrize("m,n,k", [(1, 1184, 4096), (1, 1200, 4096), (1, 2368, 8192), (1, 2384, 8192), (2, 3552, 4096), (2, 3568, 4096),
-                                   (3, 2368, 1024), (3, 2384, 2304), (4, 3600, 7168), (4, 3600, 7424), (5, 100, 4352), (8, 48, 2048), (7, 48, 2304)])
+                                   (3, 2368, 1024), (3, 2384, 2304), (4, 3552, 4096), (4, 3568, 4096), (4, 3600, 4096), (4, 3600, 6400),
+                                   (2, 3600, 14336), (2, 3600, 14848), (4, 3600, 7168), (4, 3600, 7424), (5, 100, 4352), (8, 48, 2048), (7, 48, 2304)])
 def test_gemv_stage_lengths(cuda_lib, m, n, k):
-    """Either side of the lines between the stage lengths (columns, rows of W, where K ends in a stage) and of the rule
-    that keeps a CTA alone on its SM, three launches back to back into the same output."""
+    """Either side of the lines between the stage lengths (columns, rows of W, where K ends in a stage, room for two CTAs' x) and of
+    the rule that keeps a CTA alone on its SM; three launches back to back, each into an output of its own."""
     x, wq, s = synth.make_case(m, n, k, seed=m * 7 + n + k)
     tx, twq, ts = dev(x, wq, s)
-    out = torch.empty((m, n), dtype=torch.float16, device="cuda")
-    for _ in range(3):
-        ops.q4f16_matmul(tx, twq, ts, out=out)
+    out = torch.full((3, m, n), float("nan"), dtype=torch.float16, device="cuda")
+    for i in range(3):
+        ops.q4f16_matmul(tx, twq, ts, out=out[i])
     torch.cuda.synchronize()
-    assert_matmul_close(out.cpu().numpy(), x, wq, s, f"{m}x{n}x{k}")
+    for y in out.cpu().numpy():
+        assert_matmul_close(y, x, wq, s, f"{m}x{n}x{k}")
     assert cuda_lib.b200_device_error_flags() == 0
 
 
