@@ -408,7 +408,7 @@ def run_decode(args, world, rank, dev, batches):
 # summarised under profiles/ (one capture per kernel change; not re-measured by this script).
 NCU_SOURCE = ": dram__bytes_read.sum + dram__bytes_write.sum of one launch under ncu, captured beforehand and not re-measured by this run"
 NCU_TRAFFIC_BYTES = {
-    ("gemv", 1, 4096, 4096): (9476352, "q4f16_gemv_pipe_kernel" + NCU_SOURCE),
+    ("gemv", 1, 4096, 4096): (9476608, "q4f16_gemv_pipe_kernel" + NCU_SOURCE),
     ("gemv", 64, 4096, 4096): (10003456, "q4f16_gemm_ws_tcgen05_kernel" + NCU_SOURCE),
     ("prefill", 2048, 11008, 4096): (42205440 + 12076544, "q4f16_gemm_ws_tcgen05_kernel" + NCU_SOURCE),
 }

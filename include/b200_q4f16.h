@@ -197,7 +197,8 @@ B200_API int32_t b200_q4f16_dequantize_packed(void* args, int* type_codes, int n
  *
  * gemv_rmsnorm:  r = fp16(x + delta)  (delta may be NULL);  if x_out != NULL, x_out = r (the updated
  *                residual stream; must not alias x);  y = (r * rsqrt(mean(r^2) + eps) * norm_w) . W^T
- * gemv_swiglu:   gu fp16 [M, 2K] = gate | up;  y = (silu(gate) * up) . W^T
+ * gemv_swiglu:   gu fp16 [M, 2K] = gate | up;  y = (silu(gate) * up) . W^T.  For callers that hold gate | up already: every CTA
+ *                forms the product again, which gemv_gate_up below does once per output (DecodeEngine uses that one)
  * Statistics and products in fp32, one fp16 rounding of the activation, as the stand-alone kernels. */
 B200_API int b200_q4f16_gemv_rmsnorm(const void* x, const void* delta, const void* norm_w, void* x_out, float eps,
                                      const void* wq, const void* scales, void* y, int64_t M, int64_t N, int64_t K,

@@ -1126,10 +1126,10 @@ int launch_pipe_m(const __half* x, const uint32_t* wq, const __half* scales, __h
                   cudaStream_t stream, const Prologue& pro, const PeerReduce& red) {
   if (m == 1) {
     // batch 1: the fast form unless the caller asks for the reference's rounding of every weight (gemv.exact = 1)
-    // or, by default (gemv.exact = 0), K is short.  The fast form's staging of x also builds the offset sums and the
-    // block-diagonal operand, about 0.15 us more per launch, which it wins back from K of about 2500 on: measured at
-    // N = 4096, exact / fast = 2.96 / 3.12 us at K = 512, 3.38 / 3.51 at 1536, 3.62 / 3.69 at 2048, 4.16 / 4.13 at
-    // 2816, 4.88 / 4.58 at 4096, 7.26 / 6.80 at 8192, 9.16 / 8.72 at 11008 (and 14.3 / 12.9 at N = 22016, K = 4096).
+    // or, by default (gemv.exact = 0), K is short.  The line was drawn when the fast form had stages of 4096 k, which a short
+    // K fills poorly: exact / fast at N = 4096 2.96 / 3.17 us at K = 512, 3.70 / 3.79 at 2048, 4.09 / 4.09 at 2560, 4.42 / 4.33 at
+    // 3072.  With stages of 2048 k the fast form is ahead below it as well (2.94 / 2.79 at 512, 3.69 / 3.51 at 2048, 4.09 / 4.06 at
+    // 2560, 4.43 / 4.23 at 3072; N = 12288 6.06 / 4.76 at 1024); it stays where it is because results below it would change.
     // gemv.exact = 2 forces the fast form for every K (tests).
     const bool fast = options().gemv_exact == 2 || (options().gemv_exact == 0 && k >= 2560);
     // Two stages of 2048 k a CTA: against one of 4096 k the ring refills in halves and a warp's share of a stage takes half

@@ -36,7 +36,7 @@ def gemv_form(request, cuda_lib):
     fp32 group sums) and the exact one (every weight rounded to fp16 first, option gemv.exact)."""
     from relax_b200 import _lib
 
-    # 2 forces the fast form for every K (the default, 0, picks the exact form where K fills its stages poorly)
+    # 2 forces the fast form for every K (the default, 0, picks the exact form below K = 2560)
     _lib.set_option("gemv.exact", 1 if request.param == "exact" else 2)
     yield request.param
     _lib.set_option("gemv.exact", 0)
