@@ -341,9 +341,8 @@ B200_API int b200_rope_kv_append(const void* qkv, const void* cos_t, const void*
                                  void* cuda_stream);
 
 /* out fp16 [B, nh*128] = softmax(q.K^T / sqrt(128)) . V over positions 0..*pos.  `scratch` is
- * caller-owned device memory of b200_attn_decode_scratch_bytes(B, nh, max_ctx) bytes holding the
- * per-chunk partial results (two launches: partials over 128-token chunks, then the merge).
- * B, nh <= 65535.
+ * caller-owned device memory of b200_attn_decode_scratch_bytes(B, nh, max_ctx) bytes; the present kernel (one launch) stores
+ * nothing there, but the pointer is still required.  q and the caches must be 8-byte aligned (16 is faster).  B, nh <= 65535.
  *
  * flags = 0: every input is read after the kernel has synchronised with the launch in front of it in
  * the stream; any sequence of launches is safe.
@@ -363,27 +362,33 @@ B200_API int b200_rope_kv_append(const void* qkv, const void* cos_t, const void*
  * The entry at *pos itself and q may be written by the launch directly in front (that is what
  * b200_rope_kv_append does; the decode engine of this repository calls it there and sets the flag). */
 #define B200_ATTN_EARLY_KV_LOADS 1u
+#define B200_ATTN_EARLY_RELEASE 2u      /* b200_attn_decode_step only */
 B200_API int64_t b200_attn_decode_scratch_bytes(int64_t B, int64_t nh, int64_t max_ctx);
 B200_API int b200_attn_decode(const void* q, const void* k_cache, const void* v_cache, const void* pos, void* out,
                               void* scratch, int64_t B, int64_t nh, int64_t max_ctx, uint32_t flags, void* cuda_stream);
-/* The same; the merge is an early-release form (see b200_rmsnorm_early_release). */
+/* The same as an early-release form (see b200_rmsnorm_early_release). */
 B200_API int b200_attn_decode_early_release(const void* q, const void* k_cache, const void* v_cache, const void* pos, void* out,
                                             void* scratch, int64_t B, int64_t nh, int64_t max_ctx, uint32_t flags,
                                             void* cuda_stream);
 
-/* Rotary embedding of q and k, KV append at *pos, attention over positions 0..*pos and the merge of
- * the per-chunk partials in one launch (what b200_rope_kv_append + b200_attn_decode do in three).
- * qkv fp16 [B, 3*nh*128] = [q | k | v] of the new token; out fp16 [B, nh*128].  `scratch`:
- * b200_attn_decode_fused_scratch_bytes(B, nh, max_ctx) bytes of caller-owned device memory whose last
- * B*nh int32 (the arrival counters) must be ZERO before the first call; the kernel leaves them zero. */
+/* Rotary embedding of q and k, KV append at *pos and attention over positions 0..*pos in one launch (what
+ * b200_rope_kv_append + b200_attn_decode do in two; the new token's k and v are not read back from the caches).
+ * qkv fp16 [B, 3*nh*128] = [q | k | v] of the new token; out fp16 [B, nh*128]; cos/sin fp32 [max_pos,64], 16-byte aligned.
+ * flags: B200_ATTN_EARLY_KV_LOADS: *pos, the row of the tables that it selects and the cache entries BELOW *pos are read before
+ * the kernel has synchronised with the launch in front.  Set it where all of them were complete before that launch could begin:
+ * rules (1) and (2) above, or any chain of launches in front of it of which one waits for its predecessor before it lets its
+ * dependents start and whatever wrote them was launched before that one (every kernel of this library waits for its
+ * predecessor before it ends).  B200_ATTN_EARLY_RELEASE: an early-release form (see b200_rmsnorm_early_release). */
+B200_API int b200_attn_decode_step(const void* qkv, const void* cos_t, const void* sin_t, const void* pos, void* k_cache,
+                                   void* v_cache, void* out, int64_t B, int64_t nh, int64_t max_ctx, uint32_t flags,
+                                   void* cuda_stream);
+
+/* The same with flags = 0.  `scratch`: b200_attn_decode_fused_scratch_bytes (b200_attn_decode_scratch_bytes for _rope) bytes of
+ * caller-owned device memory; the present kernel stores nothing there, but the pointer is still required. */
 B200_API int64_t b200_attn_decode_fused_scratch_bytes(int64_t B, int64_t nh, int64_t max_ctx);
 B200_API int b200_attn_decode_fused(const void* qkv, const void* cos_t, const void* sin_t, const void* pos, void* k_cache,
                                     void* v_cache, void* out, void* scratch, int64_t B, int64_t nh, int64_t max_ctx,
                                     void* cuda_stream);
-
-/* The same in two launches: rotary embedding, KV append and the per-chunk attention in the first, the
- * merge of the partials in the second (no arrival counters).  Arguments as b200_attn_decode_fused;
- * `scratch` needs b200_attn_decode_scratch_bytes(B, nh, max_ctx) bytes and no initialisation. */
 B200_API int b200_attn_decode_rope(const void* qkv, const void* cos_t, const void* sin_t, const void* pos, void* k_cache,
                                    void* v_cache, void* out, void* scratch, int64_t B, int64_t nh, int64_t max_ctx,
                                    void* cuda_stream);
@@ -392,15 +397,9 @@ B200_API int b200_attn_decode_rope(const void* qkv, const void* cos_t, const voi
  * reference.)  Some hosts of this library are not allowed to allocate device memory at the point
  * where they call it: a runtime whose memory planner has already fixed every buffer of the step,
  * or a plugin running under a host that forbids cudaMalloc on its threads.  This entry point
- * allocates nothing, neither here nor in anything it calls: the partial results of the two-pass
- * attention go to a 4.26 MB array that is part of the library image on every GPU that loads it.
+ * allocates nothing, neither here nor in anything it calls, and holds no state between calls.
  *   - Limit: B * nh * ceil(max_ctx / 128) <= 8192 (e.g. 16 sequences x 32 heads x 2048 tokens);
  *     larger problems are refused with B200_EINVAL and a message, nothing is launched.
- *   - The first call on each device looks up the array's device address (make that device current;
- *     do this first call outside any stream capture).
- *   - All calls on a device share the one array: two calls that overlap on the GPU (different
- *     streams) overwrite each other's partial results.  Calls ordered on one stream are safe; every
- *     slot that is read has been written by the same call, so nothing needs clearing in between.
  *   - `flags` as for b200_attn_decode (0 is always safe). */
 B200_API int b200_attn_decode_static(const void* q, const void* k_cache, const void* v_cache, const void* pos, void* out,
                                      int64_t B, int64_t nh, int64_t max_ctx, uint32_t flags, void* cuda_stream);

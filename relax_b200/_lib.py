@@ -13,6 +13,7 @@ LIB_PATH = os.environ.get("B200_Q4F16_LIB") or os.path.join(_HERE, "libb200_q4f1
 
 OK, EINVAL, ENODEVICE, ELAUNCH, EDEVICE, ENOTREADY = 0, -1, -2, -3, -4, -5
 ATTN_EARLY_KV_LOADS = 1   # B200_ATTN_EARLY_KV_LOADS
+ATTN_EARLY_RELEASE = 2    # B200_ATTN_EARLY_RELEASE
 FAMILY_AUTO, FAMILY_GEMV, FAMILY_GEMM = 0, 1, 2
 LAYOUT_REFERENCE, LAYOUT_PAIRED = 0, 1
 
@@ -126,6 +127,7 @@ PROTOTYPES = {
     "b200_attn_decode_fused_scratch_bytes": (_i64, [_i64, _i64, _i64]),
     "b200_attn_decode_fused": (_ci, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _vp]),
     "b200_attn_decode_rope": (_ci, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _vp]),
+    "b200_attn_decode_step": (_ci, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, ctypes.c_uint32, _vp]),
     "b200_attn_decode_static": (_ci, [_vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, ctypes.c_uint32, _vp]),
     "b200_silu_mul": (_ci, [_vp, _vp, _i64, _i64, _vp]),
     "b200_silu_mul_early_release": (_ci, [_vp, _vp, _i64, _i64, _vp]),

@@ -125,8 +125,8 @@ class DecodeEngine:
         # the separate kernels are faster (measured per layer at context 2000: 80 against 88 us at batch 2, 124 against
         # 176 at batch 8, 174 against 291 at batch 16).
         self.fused = (B == 1) if fused is None else (bool(fused) and B <= 16)
-        # False: rotary/append, attention, merge as three launches; True: one launch; "rope": rotary/append
-        # inside the attention launch, merge as a second launch
+        # rotary embedding, KV append and attention are one launch; True and "rope" take the entry points whose loads all wait for
+        # the qkv matmul, False the one whose first loads of older cache entries run beside it
         self.fused_attention = "rope" if fused_attention == "rope" else bool(fused_attention)
         self.x = torch.zeros((B, H), **f16)            # residual stream
         self.x2 = torch.zeros((B, H), **f16)           # its second buffer (fused path ping-pongs)
@@ -140,8 +140,7 @@ class DecodeEngine:
         self.down = torch.zeros((B, H), **f16)
         self.kc = [torch.zeros((B, max_ctx, self.nh_local, 128), **f16) for _ in layers]
         self.vc = [torch.zeros((B, max_ctx, self.nh_local, 128), **f16) for _ in layers]
-        nbytes = int(self.L.b200_attn_decode_fused_scratch_bytes(B, self.nh_local, max_ctx))
-        self.scratch = torch.zeros((max(nbytes, 4) // 4,), dtype=torch.float32, device=self.device)   # counters start at 0
+        self.scratch = torch.zeros((4,), dtype=torch.float32, device=self.device)     # (the attention entry points ask for one)
         self.pos = torch.zeros((1,), dtype=torch.int32, device=self.device)
         self.tokens = torch.zeros((B,), dtype=torch.int32, device=self.device)
         self.cos, self.sin = rope_tables(max_ctx, 128, cfg.theta, self.device)
@@ -157,8 +156,8 @@ class DecodeEngine:
         # inside it costs what a dependent launch costs, and its attention stage has only eight warps per SM with loads in
         # flight
         self.layer_kernel = False if layer_kernel is None else bool(layer_kernel)
-        # batch 1, fused prologues, three-launch attention: rotary embedding + KV append run in the epilogue of the
-        # qkv matmul (b200_q4f16_gemv_rmsnorm_rope), one launch less per layer
+        # batch 1, fused prologues: rotary embedding + KV append run in the epilogue of the qkv matmul
+        # (b200_q4f16_gemv_rmsnorm_rope)
         self.rope_epilogue = bool(rope_epilogue) and self.fused and B == 1 and not self.fused_attention and not self.layer_kernel
         if self.layer_kernel and B != 1:
             raise ValueError("the one-kernel-per-layer path is the batch-1 path")
@@ -308,24 +307,19 @@ class DecodeEngine:
                                                          self.pos.data_ptr(), self.attn.data_ptr(), self.scratch.data_ptr(), B,
                                                          self.nh_local, self.max_ctx, _lib.ATTN_EARLY_KV_LOADS, sp))
         elif self.fused_attention == "rope":
-            # rotary embedding + KV append + per-chunk attention in one launch, the merge in a second
             self._check(L.b200_attn_decode_rope(self.qkv.data_ptr(), self.cos.data_ptr(), self.sin.data_ptr(), self.pos.data_ptr(),
                                                 self.kc[i].data_ptr(), self.vc[i].data_ptr(), self.attn.data_ptr(),
                                                 self.scratch.data_ptr(), B, self.nh_local, self.max_ctx, sp))
         elif self.fused_attention:
-            # rotary embedding + KV append + attention + merge in one launch
             self._check(L.b200_attn_decode_fused(self.qkv.data_ptr(), self.cos.data_ptr(), self.sin.data_ptr(), self.pos.data_ptr(),
                                                  self.kc[i].data_ptr(), self.vc[i].data_ptr(), self.attn.data_ptr(),
                                                  self.scratch.data_ptr(), B, self.nh_local, self.max_ctx, sp))
         else:
-            self._check(L.b200_rope_kv_append(self.qkv.data_ptr(), self.cos.data_ptr(), self.sin.data_ptr(), self.pos.data_ptr(),
-                                              self.q.data_ptr(), self.kc[i].data_ptr(), self.vc[i].data_ptr(), B, self.nh_local,
-                                              self.max_ctx, sp))
-            self._check(L.b200_attn_decode_early_release(self.q.data_ptr(), self.kc[i].data_ptr(), self.vc[i].data_ptr(),
-                                                         self.pos.data_ptr(), self.attn.data_ptr(), self.scratch.data_ptr(), B,
-                                                         self.nh_local, self.max_ctx,
-                                                         _lib.ATTN_EARLY_KV_LOADS,   # rope_kv_append sits directly in front and waits first
-                                                         sp))
+            # rotary embedding + KV append + attention in one launch.  Early loads as above: no kernel of a step begins before
+            # embed_rows has waited for all of the step before
+            self._check(L.b200_attn_decode_step(self.qkv.data_ptr(), self.cos.data_ptr(), self.sin.data_ptr(), self.pos.data_ptr(),
+                                                self.kc[i].data_ptr(), self.vc[i].data_ptr(), self.attn.data_ptr(), B, self.nh_local,
+                                                self.max_ctx, _lib.ATTN_EARLY_KV_LOADS | _lib.ATTN_EARLY_RELEASE, sp))
         if self.peer is not None and B <= self.PEER_FUSED_MAX_ROWS:
             d = self._reduce_desc(0, i, self.o)
             self._check(L.b200_q4f16_gemv_allreduce(self.attn.data_ptr(), w["o"][0].data_ptr(), w["o"][1].data_ptr(),
@@ -402,18 +396,16 @@ class DecodeEngine:
         self._check(L.b200_advance_pos(self.epoch.data_ptr(), 1, sp))
 
     def kernels_per_step(self) -> int:
-        """Kernels of this library launched by one step: embed, 5 to 12 per layer, final norm, output projection for up to
+        """Kernels of this library launched by one step: embed, 5 to 10 per layer, final norm, output projection for up to
         16 rows, two counters."""
         head = 1 if self.lm_head is not None and self.batch <= 16 else 0
         if self.layer_kernel:
             return 1 + len(self.layers) + 1 + head + 2
-        # rotary + append (unless the qkv matmul does it), attention, merge; or the forms that put two or all of them in one
-        attention = 2 if self.fused_attention == "rope" or self.rope_epilogue else 1 if self.fused_attention else 3
         peer_sums = 2 if self.peer is not None and self.batch > self.PEER_FUSED_MAX_ROWS else 0
         per_layer = 0
         for w in self.layers:
             mlp = 2 if self.fused else 3 if self._gate_up_in_one(w) else 4        # (norm,) gate|up (, SwiGLU), down
-            per_layer += (1 if self.fused else 2) + attention + 1 + mlp + peer_sums
+            per_layer += (1 if self.fused else 2) + 2 + mlp + peer_sums           # (norm,) qkv, attention, o
         return 1 + per_layer + 1 + head + 2
 
     def capture(self, stream):
