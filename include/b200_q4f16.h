@@ -156,6 +156,11 @@ B200_API int b200_q4f16_matmul_dl_family(const B200DLTensor* x, const B200DLTens
 B200_API int64_t b200_lm_head_scratch_bytes(void);
 B200_API int b200_lm_head(const void* h, const void* w, void* logits, int32_t* tokens, void* scratch, int64_t B,
                           int64_t V, int64_t H, int64_t token_offset, void* stream);
+/* The same for B <= 8 rows of a residual stream x with its statistics (b200_q4f16_gemv_add): h = rmsnorm(x) * norm_w is formed on
+ * the way in, and stored to h_out if that is not NULL.  H % 64 == 0. */
+B200_API int b200_lm_head_norm(const void* x, const void* stats, const void* norm_w, float eps, void* h_out, const void* w,
+                               void* logits, int32_t* tokens, void* scratch, int64_t B, int64_t V, int64_t H, int64_t token_offset,
+                               void* cuda_stream);
 
 /* ---- offline weight repack --------------------------------------------------------------
  * The reference binds weights into the executable as constants when it builds
@@ -230,6 +235,26 @@ B200_API int b200_q4f16_gemv_rmsnorm_rope(const void* x, const void* delta, cons
                                           int64_t K, void* cuda_stream);
 B200_API int b200_q4f16_gemv_swiglu(const void* gu, const void* wq, const void* scales, void* y, int64_t M, int64_t N,
                                     int64_t K, void* cuda_stream);
+
+/* ---- the residual stream with its statistics (up to eight rows) -----------------------------------
+ * b200_q4f16_gemv_add: y += x . W^T (y is the residual stream, fp16 [M,N], N % 16 == 0; the product is rounded to fp16, then the
+ * sum, as the matmul and the residual add in b200_rmsnorm do), and stats, fp32 [M][N / 16], receives the sums of squares of the new
+ * values over each 16 columns.  swiglu != 0: x is gate|up [M,2K] as in b200_q4f16_gemv_swiglu.  The forms below read x as the residual stream of K values with such statistics ([M][K / 16],
+ * 16-byte aligned) and normalise it on its way in, as b200_rmsnorm does: no launch for the norm, no pass over the row.  norm_w is
+ * read before the kernel has synchronised with the launch in front, as weights and scales are.  K % 256 == 0, scales 16-byte aligned.
+ * B200_ENOTREADY, and nothing launched: a shape that the skinny kernel does not take in one piece (a long K), for _norm_rope
+ * also one that would not use the fast form; b200_rmsnorm and the plain matmul take those.
+ * b200_q4f16_gemv_add_applies: 1 where the automatic dispatch would not give the matmul to the weight-stationary kernel. */
+B200_API int b200_q4f16_gemv_add_applies(const void* scales, int64_t M, int64_t N, int64_t K);
+B200_API int b200_q4f16_gemv_add(const void* x, const void* wq, const void* scales, void* y, void* stats, int64_t M, int64_t N,
+                                 int64_t K, int32_t swiglu, void* cuda_stream);
+B200_API int b200_q4f16_gemv_norm(const void* x, const void* stats, const void* norm_w, float eps, const void* wq,
+                                  const void* scales, void* y, int64_t M, int64_t N, int64_t K, void* cuda_stream);
+B200_API int b200_q4f16_gemv_norm_gate_up(const void* x, const void* stats, const void* norm_w, float eps, const void* wq,
+                                          const void* scales, void* act, int64_t M, int64_t I, int64_t K, void* cuda_stream);
+B200_API int b200_q4f16_gemv_norm_rope(const void* x, const void* stats, const void* norm_w, float eps, const void* wq,
+                                       const void* scales, const void* cos_t, const void* sin_t, const void* pos, void* q_out,
+                                       void* k_cache, void* v_cache, int64_t heads, int64_t K, void* cuda_stream);
 
 /* ---- row-parallel skinny matmul with the sum over tensor-parallel ranks fused in ------------------
  * The reference has no sharding or collective; this is the row-parallel half of the tensor-parallel
@@ -408,6 +433,9 @@ B200_API int b200_attn_decode_static(const void* q, const void* k_cache, const v
  * to the table).  H % 8 == 0.  (reference: relax.take, python/tvm/relax/transform/legalize_ops.py:168) */
 B200_API int b200_embed_rows(const void* table, const void* ids, void* out, int64_t B, int64_t H, int64_t vocab,
                              void* cuda_stream);
+/* The same, and the statistics of the rows as b200_q4f16_gemv_add leaves them: stats fp32 [B][H / 16], H % 16 == 0. */
+B200_API int b200_embed_rows_stats(const void* table, const void* ids, void* out, void* stats, int64_t B, int64_t H, int64_t vocab,
+                                   void* cuda_stream);
 
 /* *pos += delta on the device (pos: one int32). */
 B200_API int b200_advance_pos(void* pos, int64_t delta, void* cuda_stream);

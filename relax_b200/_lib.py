@@ -104,6 +104,7 @@ PROTOTYPES = {
     "b200_allreduce_peer": (_ci, [_i64, ctypes.POINTER(PeerReduce), _vp]),
     "b200_lm_head_scratch_bytes": (_i64, []),
     "b200_lm_head": (_ci, [_vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _vp]),
+    "b200_lm_head_norm": (_ci, [_vp, _vp, _vp, ctypes.c_float, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _vp]),
     "b200_q4f16_repack": (_ci, [_vp, _vp, _i64, _i64, ctypes.c_int32, _vp]),
     "b200_q4f16_unpack": (_ci, [_vp, _vp, _i64, _i64, ctypes.c_int32, _vp]),
     "b200_q4f16_matmul_layout": (_ci, [_vp, _vp, _vp, _vp, _i64, _i64, _i64, ctypes.c_int32, _vp]),
@@ -114,6 +115,11 @@ PROTOTYPES = {
     "b200_q4f16_gemv_rmsnorm_rope": (_ci, [_vp, _vp, _vp, _vp, ctypes.c_float, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _vp]),
     "b200_q4f16_gemv_gate_up": (_ci, [_vp, _vp, _vp, _vp, ctypes.c_float, _vp, _vp, _vp, _i64, _i64, _i64, _vp]),
     "b200_q4f16_gemv_gate_up_applies": (_ci, [_vp, _i64, _i64, _i64]),
+    "b200_q4f16_gemv_add_applies": (_ci, [_vp, _i64, _i64, _i64]),
+    "b200_q4f16_gemv_add": (_ci, [_vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, ctypes.c_int32, _vp]),
+    "b200_q4f16_gemv_norm": (_ci, [_vp, _vp, _vp, ctypes.c_float, _vp, _vp, _vp, _i64, _i64, _i64, _vp]),
+    "b200_q4f16_gemv_norm_gate_up": (_ci, [_vp, _vp, _vp, ctypes.c_float, _vp, _vp, _vp, _i64, _i64, _i64, _vp]),
+    "b200_q4f16_gemv_norm_rope": (_ci, [_vp, _vp, _vp, ctypes.c_float, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _vp]),
     "b200_q4f16_gemv_swiglu": (_ci, [_vp, _vp, _vp, _vp, _i64, _i64, _i64, _vp]),
     "b200_q4f16_gemv_allreduce": (_ci, [_vp, _vp, _vp, _vp, _i64, _i64, _i64, ctypes.c_int32, ctypes.POINTER(PeerReduce), _vp]),
     "b200_decode_layer_scratch_bytes": (_i64, [_i64, _i64]),
@@ -131,6 +137,7 @@ PROTOTYPES = {
     "b200_attn_decode_static": (_ci, [_vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, ctypes.c_uint32, _vp]),
     "b200_silu_mul": (_ci, [_vp, _vp, _i64, _i64, _vp]),
     "b200_silu_mul_early_release": (_ci, [_vp, _vp, _i64, _i64, _vp]),
+    "b200_embed_rows_stats": (_ci, [_vp, _vp, _vp, _vp, _i64, _i64, _i64, _vp]),
     "b200_embed_rows": (_ci, [_vp, _vp, _vp, _i64, _i64, _i64, _vp]),
     "b200_advance_pos": (_ci, [_vp, _i64, _vp]),
     "b200_launch_count": (_i64, []),

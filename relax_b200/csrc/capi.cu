@@ -382,8 +382,8 @@ int64_t b200_lm_head_scratch_bytes(void) {
   return lm_head_scratch_bytes();
 }
 
-int b200_lm_head(const void* h, const void* w, void* logits, int32_t* tokens, void* scratch, int64_t B, int64_t V,
-                 int64_t H, int64_t token_offset, void* stream) {
+static int lm_head_impl(const void* h, const void* stats, const void* norm_w, float eps, void* h_out, const void* w, void* logits,
+                        int32_t* tokens, void* scratch, int64_t B, int64_t V, int64_t H, int64_t token_offset, void* stream) {
   if (B < 1 || B > 16) return fail(B200_EINVAL, "lm_head: takes 1 <= B <= 16 rows, got %lld", (long long)B);
   if (V < 1 || V > 0x7fffff00LL || H < 32 || H % 32 != 0)
     return fail(B200_EINVAL, "lm_head: need 1 <= V < 2^31, H >= 32 and H %% 32 == 0 (V=%lld H=%lld)", (long long)V, (long long)H);
@@ -395,10 +395,26 @@ int b200_lm_head(const void* h, const void* w, void* logits, int32_t* tokens, vo
   if (token_offset < 0 || token_offset + V > 0x7fffffffLL) return fail(B200_EINVAL, "lm_head: token_offset + V overflows int32");
   int rc = ensure_device();
   if (rc) return rc;
-  rc = launch_lm_head(static_cast<const __half*>(h), static_cast<const __half*>(w), static_cast<__half*>(logits), tokens,
+  rc = launch_lm_head(static_cast<const __half*>(h), static_cast<const float*>(stats), static_cast<const __half*>(norm_w), eps,
+                      static_cast<__half*>(h_out), static_cast<const __half*>(w), static_cast<__half*>(logits), tokens,
                       static_cast<float*>(scratch), B, V, H, token_offset, static_cast<cudaStream_t>(stream));
   if (rc == B200_ENOTREADY) return fail(B200_EINVAL, "lm_head: %lld rows of H=%lld do not fit in shared memory", (long long)B, (long long)H);
   return rc;
+}
+
+int b200_lm_head(const void* h, const void* w, void* logits, int32_t* tokens, void* scratch, int64_t B, int64_t V,
+                 int64_t H, int64_t token_offset, void* stream) {
+  return lm_head_impl(h, nullptr, nullptr, 0.f, nullptr, w, logits, tokens, scratch, B, V, H, token_offset, stream);
+}
+
+int b200_lm_head_norm(const void* x, const void* stats, const void* norm_w, float eps, void* h_out, const void* w, void* logits,
+                      int32_t* tokens, void* scratch, int64_t B, int64_t V, int64_t H, int64_t token_offset, void* stream) {
+  if (B > 8) return fail(B200_EINVAL, "lm_head_norm: takes 1 <= B <= 8 rows, got %lld", (long long)B);
+  if (H % 64 != 0) return fail(B200_EINVAL, "lm_head_norm: needs H %% 64 == 0");
+  if (!stats || !norm_w || !aligned16(stats) || !aligned16(norm_w))
+    return fail(B200_EINVAL, "lm_head_norm: statistics and norm weight must be non-null and 16-byte aligned");
+  if (h_out == x || !aligned16(h_out)) return fail(B200_EINVAL, "lm_head_norm: h_out must be 16-byte aligned and not x");
+  return lm_head_impl(x, stats, norm_w, eps, h_out, w, logits, tokens, scratch, B, V, H, token_offset, stream);
 }
 
 int b200_q4f16_repack(const void* wq, void* packed_out, int64_t N, int64_t K, int32_t layout, void* stream) {
@@ -478,7 +494,7 @@ int b200_q4f16_gemv_rmsnorm_rope(const void* x, const void* delta, const void* n
   // B200_ENOTREADY (no message): the launch would not use the fast form; the caller runs b200_q4f16_gemv_rmsnorm and
   // b200_rope_kv_append instead
   return launch_gemv_pipe_rmsnorm_rope(static_cast<const __half*>(x), static_cast<const __half*>(delta),
-                                       static_cast<const __half*>(norm_w), static_cast<__half*>(x_out), eps,
+                                       static_cast<const __half*>(norm_w), static_cast<__half*>(x_out), eps, nullptr,
                                        static_cast<const uint32_t*>(wq), static_cast<const __half*>(scales),
                                        static_cast<const float*>(cos_t), static_cast<const float*>(sin_t),
                                        static_cast<const int*>(pos), static_cast<__half*>(q_out), static_cast<__half*>(k_cache),
@@ -506,11 +522,92 @@ int b200_q4f16_gemv_gate_up(const void* x, const void* delta, const void* norm_w
   rc = ensure_device();
   if (rc) return rc;
   rc = launch_gemv_pipe_gate_up(static_cast<const __half*>(x), static_cast<const __half*>(delta), static_cast<const __half*>(norm_w),
-                                static_cast<__half*>(x_out), eps, static_cast<const uint32_t*>(wq),
+                                static_cast<__half*>(x_out), eps, nullptr, static_cast<const uint32_t*>(wq),
                                 static_cast<const __half*>(scales), static_cast<__half*>(act), M, I, K,
                                 static_cast<cudaStream_t>(stream));
   if (rc == B200_ENOTREADY) return fail(rc, "%s: shape outside the fused kernel's domain", who);
   return rc;
+}
+
+// ---- the residual stream with its statistics -------------------------------------------------------------------
+// Common to the forms that normalise x by statistics left behind: up to eight rows.
+static int check_norm_stats(const char* who, const void* stats, const void* norm_w, const void* scales, int64_t M, int64_t K) {
+  if (M < 1 || M > 8) return fail(B200_EINVAL, "%s: takes 1 <= M <= 8, got %lld", who, (long long)M);
+  if (K < 256 || K % 256 != 0) return fail(B200_EINVAL, "%s: needs K a positive multiple of 256", who);
+  if (!aligned16(scales)) return fail(B200_EINVAL, "%s: scales must be 16-byte aligned", who);
+  if (!norm_w || !aligned16(norm_w)) return fail(B200_EINVAL, "%s: norm weight must be non-null and 16-byte aligned", who);
+  if (!stats || !aligned16(stats)) return fail(B200_EINVAL, "%s: statistics must be non-null and 16-byte aligned", who);
+  return ensure_device();
+}
+
+int b200_q4f16_gemv_add_applies(const void* scales, int64_t M, int64_t N, int64_t K) {
+  if (M < 1 || M > 8 || N < 16 || N % 16 != 0 || N > 0x7fffffffLL / 32 || K < 256 || K % 256 != 0 || !scales || !aligned16(scales)) return 0;
+  return !weight_stationary_first(M, N, K, false);
+}
+
+int b200_q4f16_gemv_add(const void* x, const void* wq, const void* scales, void* y, void* stats, int64_t M, int64_t N, int64_t K,
+                        int32_t swiglu, void* stream) {
+  const char* who = "q4f16_gemv_add";
+  int rc = check_matmul(who, x, wq, scales, y, M, N, K);
+  if (rc) return rc;
+  if (M < 1 || M > 8) return fail(B200_EINVAL, "%s: takes 1 <= M <= 8, got %lld", who, (long long)M);
+  if (N < 16 || N % 16 != 0 || K < 256 || K % 256 != 0)
+    return fail(B200_EINVAL, "%s: needs N a positive multiple of 16 and K a positive multiple of 256", who);
+  if (!aligned16(scales)) return fail(B200_EINVAL, "%s: scales must be 16-byte aligned", who);
+  if (!stats || (reinterpret_cast<uintptr_t>(stats) & 3u)) return fail(B200_EINVAL, "%s: statistics must be non-null and 4-byte aligned", who);
+  if (x == y) return fail(B200_EINVAL, "%s: y must not alias x (other CTAs still read x)", who);
+  if ((rc = ensure_device())) return rc;
+  rc = launch_gemv_pipe_add(static_cast<const __half*>(x), static_cast<const uint32_t*>(wq), static_cast<const __half*>(scales),
+                            static_cast<__half*>(y), static_cast<float*>(stats), M, N, K, swiglu, static_cast<cudaStream_t>(stream));
+  if (rc == B200_ENOTREADY) return fail(rc, "%s: shape outside the fused kernel's domain", who);
+  return rc;
+}
+
+int b200_q4f16_gemv_norm(const void* x, const void* stats, const void* norm_w, float eps, const void* wq, const void* scales, void* y,
+                         int64_t M, int64_t N, int64_t K, void* stream) {
+  const char* who = "q4f16_gemv_norm";
+  int rc = check_matmul(who, x, wq, scales, y, M, N, K);
+  if (rc) return rc;
+  if (N < 1) return fail(B200_EINVAL, "%s: needs N >= 1", who);
+  if ((rc = check_norm_stats(who, stats, norm_w, scales, M, K))) return rc;
+  rc = launch_gemv_pipe_norm(static_cast<const __half*>(x), static_cast<const float*>(stats), static_cast<const __half*>(norm_w), eps,
+                             static_cast<const uint32_t*>(wq), static_cast<const __half*>(scales), static_cast<__half*>(y), M, N, K,
+                             static_cast<cudaStream_t>(stream));
+  if (rc == B200_ENOTREADY) return fail(rc, "%s: shape outside the fused kernel's domain", who);
+  return rc;
+}
+
+int b200_q4f16_gemv_norm_gate_up(const void* x, const void* stats, const void* norm_w, float eps, const void* wq, const void* scales,
+                                 void* act, int64_t M, int64_t I, int64_t K, void* stream) {
+  const char* who = "q4f16_gemv_norm_gate_up";
+  if (I < 8 || I % 8 != 0 || I > 0x3fffffffLL / 32) return fail(B200_EINVAL, "%s: needs I a positive multiple of 8, got %lld", who, (long long)I);
+  int rc = check_matmul(who, x, wq, scales, act, M, 2 * I, K);
+  if (rc) return rc;
+  if ((rc = check_norm_stats(who, stats, norm_w, scales, M, K))) return rc;
+  rc = launch_gemv_pipe_gate_up(static_cast<const __half*>(x), nullptr, static_cast<const __half*>(norm_w), nullptr, eps,
+                                static_cast<const float*>(stats), static_cast<const uint32_t*>(wq), static_cast<const __half*>(scales),
+                                static_cast<__half*>(act), M, I, K, static_cast<cudaStream_t>(stream));
+  if (rc == B200_ENOTREADY) return fail(rc, "%s: shape outside the fused kernel's domain", who);
+  return rc;
+}
+
+int b200_q4f16_gemv_norm_rope(const void* x, const void* stats, const void* norm_w, float eps, const void* wq, const void* scales,
+                              const void* cos_t, const void* sin_t, const void* pos, void* q_out, void* k_cache, void* v_cache,
+                              int64_t heads, int64_t K, void* stream) {
+  const char* who = "q4f16_gemv_norm_rope";
+  if (heads < 1 || heads > 4096) return fail(B200_EINVAL, "%s: heads %lld out of range", who, (long long)heads);
+  int rc = check_matmul(who, x, wq, scales, q_out, 1, 3 * heads * 128, K);
+  if (rc) return rc;
+  if (!cos_t || !sin_t || !pos || !k_cache || !v_cache) return fail(B200_EINVAL, "%s: null table, position or cache pointer", who);
+  if ((rc = check_norm_stats(who, stats, norm_w, scales, 1, K))) return rc;
+  // B200_ENOTREADY (no message): the launch would not use the fast form; the caller runs b200_q4f16_gemv_norm and
+  // b200_attn_decode_step instead
+  return launch_gemv_pipe_rmsnorm_rope(static_cast<const __half*>(x), nullptr, static_cast<const __half*>(norm_w), nullptr, eps,
+                                       static_cast<const float*>(stats), static_cast<const uint32_t*>(wq),
+                                       static_cast<const __half*>(scales), static_cast<const float*>(cos_t),
+                                       static_cast<const float*>(sin_t), static_cast<const int*>(pos), static_cast<__half*>(q_out),
+                                       static_cast<__half*>(k_cache), static_cast<__half*>(v_cache), heads, K,
+                                       static_cast<cudaStream_t>(stream));
 }
 
 int b200_q4f16_gemv_swiglu(const void* gu, const void* wq, const void* scales, void* y, int64_t M, int64_t N, int64_t K,

@@ -205,10 +205,12 @@ silu_mul_kernel(const __half* __restrict__ gu, __half* __restrict__ out, int I, 
   *reinterpret_cast<uint4*>(out + b * I + i) = o;
 }
 
-// out[b,:] = table[ids[b],:] (fp16 rows of H, H % 8 == 0).  grid (B), 128 threads.
+// out[b,:] = table[ids[b],:] (fp16 rows of H, H % 8 == 0).  grid (B), 128 threads.  kStats: the row's sum of squares goes to
+// stats[b][0] and zeros to the other H / 16 - 1 places of its partial sums.
+template <bool kStats>
 __global__ void __launch_bounds__(128)
-embed_rows_kernel(const __half* __restrict__ table, const int* __restrict__ ids, __half* __restrict__ out, int H,
-                  int vocab) {
+embed_rows_kernel(const __half* __restrict__ table, const int* __restrict__ ids, __half* __restrict__ out, float* __restrict__ stats,
+                  int H, int vocab) {
   ptx::pdl_wait();
   const int b = blockIdx.x;
   int id = ids[b];
@@ -216,7 +218,27 @@ embed_rows_kernel(const __half* __restrict__ table, const int* __restrict__ ids,
   const uint4* src = reinterpret_cast<const uint4*>(table + (int64_t)id * H);
   uint4* dst = reinterpret_cast<uint4*>(out + (int64_t)b * H);
   ptx::pdl_launch_dependents();
-  for (int i = threadIdx.x; i < H / 8; i += blockDim.x) dst[i] = src[i];
+  float ss = 0.f;
+  for (int i = threadIdx.x; i < H / 8; i += blockDim.x) {
+    const uint4 v = src[i];
+    dst[i] = v;
+    if (kStats) {
+      const __half2* h = reinterpret_cast<const __half2*>(&v);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 f = __half22float2(h[j]);
+        ss += f.x * f.x + f.y * f.y;
+      }
+    }
+  }
+  if (kStats) {
+    __shared__ float red[4];
+    ss = warp_sum(ss);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+    __syncthreads();
+    for (int i = threadIdx.x; i < H / 16; i += blockDim.x)
+      stats[(int64_t)b * (H / 16) + i] = i == 0 ? (red[0] + red[1]) + (red[2] + red[3]) : 0.f;
+  }
 }
 
 // *pos += delta (one thread): advances the decode position on the device so that a captured
@@ -285,14 +307,25 @@ int b200_rope_kv_append(const void* qkv, const void* cos_t, const void* sin_t, c
                 (const int*)pos, (__half*)q_out, (__half*)k_cache, (__half*)v_cache, (int)nh, (int)max_ctx);
 }
 
-int b200_embed_rows(const void* table, const void* ids, void* out, int64_t B, int64_t H, int64_t vocab, void* stream) {
-  if (B < 0 || H <= 0 || H % 8 != 0 || vocab <= 0) return fail(B200_EINVAL, "embed_rows: need H %% 8 == 0, vocab > 0");
+static int embed_rows_impl(const char* who, const void* table, const void* ids, void* out, void* stats, int64_t B, int64_t H,
+                           int64_t vocab, void* stream) {
+  if (B < 0 || H <= 0 || H % 8 != 0 || vocab <= 0) return fail(B200_EINVAL, "%s: need H %% 8 == 0, vocab > 0", who);
   if (B == 0) return B200_OK;
-  if (!table || !ids || !out) return fail(B200_EINVAL, "embed_rows: null pointer");
+  if (!table || !ids || !out) return fail(B200_EINVAL, "%s: null pointer", who);
   int rc = ensure_device();
   if (rc) return rc;
-  return launch("embed_rows", embed_rows_kernel, dim3((unsigned)B), dim3(128), 0, static_cast<cudaStream_t>(stream),
-                (const __half*)table, (const int*)ids, (__half*)out, (int)H, (int)vocab);
+  return launch("embed_rows", stats ? embed_rows_kernel<true> : embed_rows_kernel<false>, dim3((unsigned)B), dim3(128), 0,
+                static_cast<cudaStream_t>(stream), (const __half*)table, (const int*)ids, (__half*)out, (float*)stats, (int)H, (int)vocab);
+}
+
+int b200_embed_rows(const void* table, const void* ids, void* out, int64_t B, int64_t H, int64_t vocab, void* stream) {
+  return embed_rows_impl("embed_rows", table, ids, out, nullptr, B, H, vocab, stream);
+}
+
+int b200_embed_rows_stats(const void* table, const void* ids, void* out, void* stats, int64_t B, int64_t H, int64_t vocab, void* stream) {
+  if (!stats) return fail(B200_EINVAL, "embed_rows_stats: null pointer");
+  if (H % 16 != 0) return fail(B200_EINVAL, "embed_rows_stats: need H %% 16 == 0");
+  return embed_rows_impl("embed_rows_stats", table, ids, out, stats, B, H, vocab, stream);
 }
 
 int b200_advance_pos(void* pos, int64_t delta, void* stream) {

@@ -75,7 +75,14 @@ constexpr int kMaxStages = 8;
 constexpr uint64_t kConsumerWaitNs = 2000000000ull;     // 2 s: a stage copy takes microseconds
 constexpr uint64_t kProducerWaitNs = 30000000000ull;    // 30 s: may span the previous kernels' whole run
 
-enum { kPrologueNone = 0, kPrologueRmsNorm = 1, kPrologueSwiGLU = 2 };
+// What happens to x on its way into shared memory.  kPrologueNormStats: RMSNorm whose statistics the kernel that produced x has
+// left behind (kEpilogueAdd): no pass over the row, no residual add.
+enum { kPrologueNone = 0, kPrologueRmsNorm = 1, kPrologueSwiGLU = 2, kPrologueNormStats = 3 };
+// What happens to a finished tile.  kEpilogueGateUp: W's rows are [gate: N / 2 | up: N / 2]; a tile takes eight of each and
+// silu(gate) * up is stored, [M, N / 2].  kEpilogueAdd: y += the product (y is the residual stream), and the sum of squares of the
+// new values goes to stats_out[row of x][tile] for the norm that comes next.  Forms of their own: as a run-time flag the first
+// cost the plain batch-1 matmul 2.9 % (182.5 -> 187.8 us for 40 of N = K = 4096).
+enum { kEpilogueStore = 0, kEpilogueGateUp = 1, kEpilogueAdd = 2 };
 
 // Rotary embedding + KV append in the epilogue of the qkv matmul (batch 1, fast form).  The weight rows are then
 // fetched through a 5-D tensor map whose 16-row tile is dims d0..d0+7 of one 128-wide head AND their rotate-half
@@ -108,6 +115,8 @@ struct PipeParams {
   const __half* norm_w;      // RmsNorm: weight [K]
   __half* x_out;             // RmsNorm: fp16(x + delta) is written here by CTA 0 (or null)
   float eps;
+  const float* stats_in;     // NormStats: [M][K / 16] partial sums of squares of x's rows
+  float* stats_out;          // kEpilogueAdd: [M][ntiles]
   int paired;                // nibble order of the packed words: 0 reference, 1 paired (q4_common.cuh)
   RopeOut rope;
   PeerReduce red;
@@ -182,14 +191,13 @@ __device__ __forceinline__ void fast_stage_fn(float (&acc)[2][MT][4], const uint
 //   accs:  tiles_per_cta * kOut * 4 (only when K is cut into several blocks)
 //
 // Warps: CW consumers, then one TMA warp (two issuing lanes), then one epilogue warp.
-//
-// GU: W's rows are [gate: N / 2 | up: N / 2]; a tile takes eight of each and the epilogue stores silu(gate) * up, [M, N / 2].  A
-// form of its own: as a run-time flag it cost the plain batch-1 matmul 2.9 % (182.5 -> 187.8 us for 40 of N = K = 4096).
-template <int NC, int CW, int CH, int PRO, bool FAST, bool GU>
+template <int NC, int CW, int CH, int PRO, bool FAST, int EPI>
 __global__ void __launch_bounds__((CW + 2) * 32, FAST ? 2 : 1)
 q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
   constexpr int MT = (NC + 7) / 8;
+  constexpr bool GU = EPI == kEpilogueGateUp, ADD = EPI == kEpilogueAdd;
   static_assert(!FAST || NC == 1, "the fast form is the batch-1 kernel");
+  static_assert(MT == 1 || (!ADD && PRO != kPrologueNormStats), "up to eight rows");
   // outputs per row tile as one consumer warp leaves them: the exact form stores whole MMA fragments,
   // the fast form one value per row (padded to two)
   constexpr int NCP = 2;
@@ -327,6 +335,17 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
           rope_c = p.rope.cos_t[(int64_t)rope_pos * 64 + i];
           rope_s = p.rope.sin_t[(int64_t)rope_pos * 64 + i];
         }
+        // ADD: what the sums are added to, fetched before the wait for them
+        constexpr int kQ = (kOut + 31) / 32;
+        __half old[ADD ? kQ : 1];
+        if (ADD) {
+#pragma unroll
+          for (int q = 0; q < kQ; ++q) {
+            const int row = tile * kRows + (FAST ? lane / NCP : (lane >> 2) + 8 * ((q & 3) >> 1));
+            const int col = FAST ? lane % NCP : 2 * (lane & 3) + (q & 1);
+            old[q] = row < p.N && col < p.M ? p.y[(int64_t)col * p.N + row] : __ushort_as_half(0);
+          }
+        }
         if (!mbar_try_wait(&red_full[rb], rround & 1)) {
           if (!*(volatile int*)&s_abort && !mbar_wait_ns_relaxed(&red_full[rb], rround & 1, kProducerWaitNs)) {
             atomicExch(&g_gemv_pipe_error, 4);
@@ -334,6 +353,7 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
           }
         }
         const float* rbuf = red + rb * (CW * kOut);
+        float sq[2] = {0.f, 0.f};                  // ADD: squares of this lane's new values (exact form: of its two columns)
         float gate[2];                             // GU, exact form: row g's values until row g + 8's are known
 #pragma unroll
         for (int q = 0; q < (kOut + 31) / 32; ++q) {
@@ -392,7 +412,31 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
               row = tile * kRows + (lane >> 2) + 8 * (i >> 1);
               col = mt * 8 + 2 * (lane & 3) + (i & 1);
             }
-            if (row < p.N && col < p.M) p.y[(int64_t)col * p.N + row] = __float2half_rn(sum);
+            if (ADD) {
+              // one rounding of the product, one of the sum, as the separate kernels have it
+              const __half v = __float2half_rn(__half2float(old[q]) + __half2float(__float2half_rn(sum)));
+              if (row < p.N && col < p.M) {
+                p.y[(int64_t)col * p.N + row] = v;
+                const float f = __half2float(v);
+                sq[FAST ? 0 : q & 1] += f * f;
+              }
+            } else if (row < p.N && col < p.M) {
+              p.y[(int64_t)col * p.N + row] = __float2half_rn(sum);
+            }
+          }
+        }
+        if (ADD && kb == nkb - 1) {
+          if (FAST) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) sq[0] += __shfl_xor_sync(0xffffffffu, sq[0], o);
+            if (lane == 0) p.stats_out[tile] = sq[0];
+          } else {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {                  // column 2 (lane % 4) + i: over the lanes that share it
+#pragma unroll
+              for (int o = 16; o > 2; o >>= 1) sq[i] += __shfl_xor_sync(0xffffffffu, sq[i], o);
+              if (lane < 4 && 2 * lane + i < p.M) p.stats_out[(int64_t)(2 * lane + i) * p.ntiles + tile] = sq[i];
+            }
           }
         }
         __syncwarp();
@@ -571,6 +615,17 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
   uint4 fw[U][2][2];
   uint2 fsc[U][2];
   if (FAST) fast_load(0, 0, fw, fsc);
+  // NormStats: the items (words of eight values) that a thread stages at a time; the norm weights of the first ones are
+  // here when the wait returns
+  constexpr int kNormItems = NC >= 8 ? 4 : 2;
+  uint4 nw[kNormItems];
+  if (PRO == kPrologueNormStats) {
+#pragma unroll
+    for (int r = 0; r < kNormItems; ++r) {
+      const int k = (tid + r * kConsumers) / NC * 8;
+      nw[r] = k < p.K ? *reinterpret_cast<const uint4*>(p.norm_w + k) : make_uint4(0, 0, 0, 0);
+    }
+  }
   pdl_wait();                                    // x may be the previous kernel's output
   // ---- RMSNorm prologue: r = fp16(x + delta), inv[m] = rsqrt(mean(r^2) + eps) for every row ------
   // Every CTA computes the statistics itself (K values per row: nothing next to its share of W);
@@ -660,6 +715,54 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
     bar_sync(1, kConsumers);
   }
 
+  // ---- RMSNorm with the statistics of the kernel that wrote x (one K block: checked by the launcher) ----------------
+  // The first loads of x and the partial sums travel together; warp m adds up row m's.
+  if (PRO == kPrologueNormStats) {
+    const int items = (p.kblk >> 3) * NC;        // a multiple of kConsumers
+    const int parts = p.K >> 4;
+    uint4 a[kNormItems];
+    auto load = [&](int i0) {
+#pragma unroll
+      for (int r = 0; r < kNormItems; ++r) {
+        const int i = i0 + r * kConsumers, j = i / NC, m = i - j * NC;
+        a[r] = m < p.M && j * 8 < p.K ? *reinterpret_cast<const uint4*>(p.x + (int64_t)m * p.K + j * 8) : make_uint4(0, 0, 0, 0);
+      }
+    };
+    load(tid);
+    if (warp < p.M) {
+      float tot = 0.f;
+      for (int i = lane * 4; i < parts; i += 128) {
+        const float4 v = *reinterpret_cast<const float4*>(p.stats_in + (int64_t)warp * parts + i);
+        tot += (v.x + v.y) + (v.z + v.w);
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
+      if (lane == 0) s_inv[warp] = rsqrtf(tot / (float)p.K + p.eps);
+    }
+    bar_sync(1, kConsumers);
+    for (int i0 = tid; i0 < items; i0 += kNormItems * kConsumers) {
+      if (i0 != tid) {
+        load(i0);
+#pragma unroll
+        for (int r = 0; r < kNormItems; ++r) {
+          const int k = (i0 + r * kConsumers) / NC * 8;
+          nw[r] = k < p.K ? *reinterpret_cast<const uint4*>(p.norm_w + k) : make_uint4(0, 0, 0, 0);
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < kNormItems; ++r) {
+        const int i = i0 + r * kConsumers, j = i / NC, m = i - j * NC;
+        if (i >= items) continue;                  // (whole warps)
+        float psum = stage_word(j, m, scale_f16x8(a[r], m < p.M ? s_inv[m] : 0.f, nw[r]));
+        if (FAST) {
+          psum += __shfl_xor_sync(0xffffffffu, psum, 1);
+          psum += __shfl_xor_sync(0xffffffffu, psum, 2);
+          if ((j & 3) == 0) store_group_sum(j >> 2, psum);
+        }
+      }
+    }
+  }
+
   // (one K block in this case: the staged row is complete before the loop, the kept registers end here)
   if (PRO == kPrologueRmsNorm && rms_one_pass) {
     const int words = p.kblk >> 3;
@@ -684,7 +787,9 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
     const int k_hi = min(p.K, k_lo + p.kblk);
     // ---- stage x[:, k_lo .. k_lo + kblk) permuted per 8 k; zero beyond K and beyond M --------------
     if (kb > 0) bar_sync(1, kConsumers);         // everyone is done reading the previous block
-    if (FAST && !(PRO == kPrologueRmsNorm && rms_one_pass)) {
+    if (PRO == kPrologueNormStats) {
+      // (staged above)
+    } else if (FAST && !(PRO == kPrologueRmsNorm && rms_one_pass)) {
       // one batch column: a thread takes a whole scale group (four words, 64 contiguous bytes), so its offset sum
       // needs no exchange; all loads of a thread are issued before the first use
       const int groups = p.kblk >> 5;
@@ -920,10 +1025,12 @@ struct Prologue {
   const __half* norm_w = nullptr;
   __half* x_out = nullptr;
   float eps = 0.f;
+  const float* stats_in = nullptr;
+  float* stats_out = nullptr;
   RopeOut rope;          // rotary embedding + KV append in the epilogue (qkv matmul of a batch-1 step)
 };
 
-template <int NC, int CW, int CH, int PRO, bool FAST, bool GU>
+template <int NC, int CW, int CH, int PRO, bool FAST, int EPI>
 int launch_pipe(const __half* x, const uint32_t* wq, const __half* scales, __half* y, int M, int N, int K,
                 cudaStream_t stream, const Prologue& pro, const PeerReduce& red) {
   constexpr int MT = (NC + 7) / 8;
@@ -931,6 +1038,7 @@ int launch_pipe(const __half* x, const uint32_t* wq, const __half* scales, __hal
   constexpr int KC = 256 * CH;
   constexpr int kStageBytes = CH * kRows * (128 + 16);
   constexpr int kThreads = (CW + 2) * 32;
+  constexpr bool GU = EPI == kEpilogueGateUp;
   using XL = XLayout<NC>;
   PipeParams p;
   p.rope = pro.rope;
@@ -977,13 +1085,14 @@ int launch_pipe(const __half* x, const uint32_t* wq, const __half* scales, __hal
   p.x = x; p.y = y;
   p.M = M; p.N = N; p.K = K;
   p.delta = pro.delta; p.norm_w = pro.norm_w; p.x_out = pro.x_out; p.eps = pro.eps;
+  p.stats_in = pro.stats_in; p.stats_out = pro.stats_out;
   p.red = red;
   p.paired = current_layout() == kLayoutPaired;
   p.ntiles = (N + kRows - 1) / kRows;
   const int kpad = ((K + KC - 1) / KC) * KC;
   const int stages_per_tile = kpad / KC;
   const int sms = sm_count();
-  auto kern = q4f16_gemv_pipe_kernel<NC, CW, CH, PRO, FAST, GU>;
+  auto kern = q4f16_gemv_pipe_kernel<NC, CW, CH, PRO, FAST, EPI>;
   // Ask for the largest shared-memory carve-out: the default picks the smallest that fits ONE CTA,
   // which would keep further CTAs (or the next dependent launch) off the SM.
   cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
@@ -1077,7 +1186,7 @@ int launch_pipe(const __half* x, const uint32_t* wq, const __half* scales, __hal
   if (int rc = raise_smem_limit(limit, func, need, "gemv")) return rc;
   p.nstages = stages;
   p.kblk = kblk;
-  if (pro.rope.on && kblk < kpad) return B200_ENOTREADY;   // (K cut into blocks: the rotary epilogue takes one)
+  if ((pro.rope.on || PRO == kPrologueNormStats) && kblk < kpad) return B200_ENOTREADY;   // (K cut into blocks: these take one)
 
   cudaError_t e;
   cudaLaunchConfig_t cfg = {};
@@ -1121,7 +1230,7 @@ bool half_stages(int n, int k) {
   return NC >= 8 || pair || !two_long || (k <= 12288 && n <= 2 * sm_count() * kRows);
 }
 
-template <int CW, int CH, int PRO, bool GU>
+template <int CW, int CH, int PRO, int EPI>
 int launch_pipe_m(const __half* x, const uint32_t* wq, const __half* scales, __half* y, int m, int n, int k,
                   cudaStream_t stream, const Prologue& pro, const PeerReduce& red) {
   if (m == 1) {
@@ -1140,35 +1249,40 @@ int launch_pipe_m(const __half* x, const uint32_t* wq, const __half* scales, __h
     // returns, is 0-2 % faster back to back (N = 2048, K = 4096 3.84 / 3.79, N = 4736 4.97 / 4.88, 40 of N = K = 4096 183.3 / 182.4).
     // But it is a kernel of its own, and inside a decode step, where other kernels run in between, the o projection took
     // 0.3 us longer with it (a step of the 7B shape 1646 / 1656): one form for every K.
-    if (fast) return launch_pipe<1, CW, CW, PRO, true, GU>(x, wq, scales, y, m, n, k, stream, pro, red);
-    return launch_pipe<1, CW, CH, PRO, false, GU>(x, wq, scales, y, m, n, k, stream, pro, red);
+    if (fast) return launch_pipe<1, CW, CW, PRO, true, EPI>(x, wq, scales, y, m, n, k, stream, pro, red);
+    return launch_pipe<1, CW, CH, PRO, false, EPI>(x, wq, scales, y, m, n, k, stream, pro, red);
   }
   if (m == 2)
-    return half_stages<2>(n, k) ? launch_pipe<2, CW, CW, PRO, false, GU>(x, wq, scales, y, m, n, k, stream, pro, red)
-                             : launch_pipe<2, CW, CH, PRO, false, GU>(x, wq, scales, y, m, n, k, stream, pro, red);
+    return half_stages<2>(n, k) ? launch_pipe<2, CW, CW, PRO, false, EPI>(x, wq, scales, y, m, n, k, stream, pro, red)
+                             : launch_pipe<2, CW, CH, PRO, false, EPI>(x, wq, scales, y, m, n, k, stream, pro, red);
   if (m <= 4)
-    return half_stages<4>(n, k) ? launch_pipe<4, CW, CW, PRO, false, GU>(x, wq, scales, y, m, n, k, stream, pro, red)
-                             : launch_pipe<4, CW, CH, PRO, false, GU>(x, wq, scales, y, m, n, k, stream, pro, red);
+    return half_stages<4>(n, k) ? launch_pipe<4, CW, CW, PRO, false, EPI>(x, wq, scales, y, m, n, k, stream, pro, red)
+                             : launch_pipe<4, CW, CH, PRO, false, EPI>(x, wq, scales, y, m, n, k, stream, pro, red);
   if (m <= 8)
-    return half_stages<8>(n, k) ? launch_pipe<8, CW, CW, PRO, false, GU>(x, wq, scales, y, m, n, k, stream, pro, red)
-                             : launch_pipe<8, CW, CH, PRO, false, GU>(x, wq, scales, y, m, n, k, stream, pro, red);
-  return launch_pipe<16, CW, CH, PRO, false, GU>(x, wq, scales, y, m, n, k, stream, pro, red);
+    return half_stages<8>(n, k) ? launch_pipe<8, CW, CW, PRO, false, EPI>(x, wq, scales, y, m, n, k, stream, pro, red)
+                             : launch_pipe<8, CW, CH, PRO, false, EPI>(x, wq, scales, y, m, n, k, stream, pro, red);
+  if constexpr (PRO == kPrologueNormStats || EPI == kEpilogueAdd) return B200_ENOTREADY;
+  else return launch_pipe<16, CW, CH, PRO, false, EPI>(x, wq, scales, y, m, n, k, stream, pro, red);
 }
 
-template <int PRO, bool GU = false>
+template <int PRO, int EPI>
 int dispatch_form(const __half* x, const uint32_t* wq, const __half* scales, __half* y, int m, int n, int k,
                   cudaStream_t stream, const Prologue& pro, const PeerReduce& red) {
-  return launch_pipe_m<8, 16, PRO, GU>(x, wq, scales, y, m, n, k, stream, pro, red);
+  return launch_pipe_m<8, 16, PRO, EPI>(x, wq, scales, y, m, n, k, stream, pro, red);
 }
 
-template <bool GU = false>
+template <int EPI = kEpilogueStore>
 int dispatch_pipe(const __half* x, const uint32_t* wq, const __half* scales, __half* y, int64_t M, int64_t N, int64_t K,
                   cudaStream_t stream, const Prologue& pro, const PeerReduce& red) {
   if (K % 256 != 0 || (reinterpret_cast<uintptr_t>(scales) & 15u)) return B200_ENOTREADY;
   int m = (int)M, n = (int)N, k = (int)K;
-  if (pro.kind == kPrologueRmsNorm) return dispatch_form<kPrologueRmsNorm, GU>(x, wq, scales, y, m, n, k, stream, pro, red);
-  if (!GU && pro.kind == kPrologueSwiGLU) return dispatch_form<kPrologueSwiGLU>(x, wq, scales, y, m, n, k, stream, pro, red);
-  return dispatch_form<kPrologueNone, GU>(x, wq, scales, y, m, n, k, stream, pro, red);
+  if constexpr (EPI != kEpilogueAdd) {
+    if (pro.kind == kPrologueRmsNorm) return dispatch_form<kPrologueRmsNorm, EPI>(x, wq, scales, y, m, n, k, stream, pro, red);
+    if (pro.kind == kPrologueNormStats) return dispatch_form<kPrologueNormStats, EPI>(x, wq, scales, y, m, n, k, stream, pro, red);
+  }
+  if constexpr (EPI != kEpilogueGateUp)
+    if (pro.kind == kPrologueSwiGLU) return dispatch_form<kPrologueSwiGLU, EPI>(x, wq, scales, y, m, n, k, stream, pro, red);
+  return dispatch_form<kPrologueNone, EPI>(x, wq, scales, y, m, n, k, stream, pro, red);
 }
 
 // The sum over tensor-parallel ranks as a kernel of its own, for partial results that another kernel produced
@@ -1289,12 +1403,14 @@ int launch_gemv_pipe_rmsnorm(const __half* x, const __half* delta, const __half*
 // qkv = rmsnorm(x + delta) . decode(W)^T for ONE row, with the rotary embedding and the KV append in the epilogue:
 // writes the rotated query to q_out and the new token's rotated key and value into the caches at *pos; no qkv
 // buffer.  B200_ENOTREADY when the launch would not use the fast form (the epilogue is written for its layout).
+// stats_in: the statistics that b200_q4f16_gemv_add or b200_embed_rows_stats left (then no delta and no x_out).
 int launch_gemv_pipe_rmsnorm_rope(const __half* x, const __half* delta, const __half* norm_w, __half* x_out, float eps,
-                                  const uint32_t* wq, const __half* scales, const float* cos_t, const float* sin_t,
+                                  const float* stats_in, const uint32_t* wq, const __half* scales, const float* cos_t, const float* sin_t,
                                   const int* pos, __half* q_out, __half* k_cache, __half* v_cache, int64_t nh, int64_t K,
                                   cudaStream_t stream) {
   Prologue pro;
   pro.kind = kPrologueRmsNorm; pro.delta = delta; pro.norm_w = norm_w; pro.x_out = x_out; pro.eps = eps;
+  if (stats_in) { pro.kind = kPrologueNormStats; pro.stats_in = stats_in; }
   pro.rope.cos_t = cos_t; pro.rope.sin_t = sin_t; pro.rope.pos = pos;
   pro.rope.q_out = q_out; pro.rope.k_cache = k_cache; pro.rope.v_cache = v_cache;
   pro.rope.nh = (int)nh; pro.rope.on = 1;
@@ -1306,13 +1422,31 @@ int launch_gemv_pipe_rmsnorm_rope(const __half* x, const __half* delta, const __
 // weight is given.  The product is formed once per output in the epilogue; as a prologue of the next matmul every CTA
 // forms all of it again.
 int launch_gemv_pipe_gate_up(const __half* x, const __half* delta, const __half* norm_w, __half* x_out, float eps,
-                             const uint32_t* wq, const __half* scales, __half* act, int64_t M, int64_t I, int64_t K,
+                             const float* stats_in, const uint32_t* wq, const __half* scales, __half* act, int64_t M, int64_t I, int64_t K,
                              cudaStream_t stream) {
   Prologue pro;
   if (norm_w) {
     pro.kind = kPrologueRmsNorm; pro.delta = delta; pro.norm_w = norm_w; pro.x_out = x_out; pro.eps = eps;
   }
-  return dispatch_pipe<true>(x, wq, scales, act, M, 2 * I, K, stream, pro, PeerReduce{});
+  if (stats_in) { pro.kind = kPrologueNormStats; pro.stats_in = stats_in; }
+  return dispatch_pipe<kEpilogueGateUp>(x, wq, scales, act, M, 2 * I, K, stream, pro, PeerReduce{});
+}
+
+// y = (x * rsqrt(mean(x^2) + eps) * norm_w) . decode(W)^T with the statistics of stats_in (up to eight rows).
+int launch_gemv_pipe_norm(const __half* x, const float* stats_in, const __half* norm_w, float eps, const uint32_t* wq, const __half* scales,
+                          __half* y, int64_t M, int64_t N, int64_t K, cudaStream_t stream) {
+  Prologue pro;
+  pro.kind = kPrologueNormStats; pro.norm_w = norm_w; pro.eps = eps; pro.stats_in = stats_in;
+  return dispatch_pipe(x, wq, scales, y, M, N, K, stream, pro, PeerReduce{});
+}
+
+// y += x . decode(W)^T, and the new values' sums of squares by row and tile of 16 columns (up to eight rows, N % 16 == 0).
+int launch_gemv_pipe_add(const __half* x, const uint32_t* wq, const __half* scales, __half* y, float* stats_out, int64_t M, int64_t N,
+                         int64_t K, int swiglu, cudaStream_t stream) {
+  Prologue pro;
+  pro.kind = swiglu ? kPrologueSwiGLU : kPrologueNone;
+  pro.stats_out = stats_out;
+  return dispatch_pipe<kEpilogueAdd>(x, wq, scales, y, M, N, K, stream, pro, PeerReduce{});
 }
 
 // y = (silu(gu[:, :K]) * gu[:, K:]) . decode(W)^T

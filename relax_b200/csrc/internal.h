@@ -59,12 +59,16 @@ int launch_gemv_pipe_rmsnorm(const __half* x, const __half* delta, const __half*
                              const uint32_t* wq, const __half* scales, __half* y, int64_t M, int64_t N, int64_t K,
                              cudaStream_t stream);
 int launch_gemv_pipe_rmsnorm_rope(const __half* x, const __half* delta, const __half* norm_w, __half* x_out, float eps,
-                                  const uint32_t* wq, const __half* scales, const float* cos_t, const float* sin_t,
+                                  const float* stats_in, const uint32_t* wq, const __half* scales, const float* cos_t, const float* sin_t,
                                   const int* pos, __half* q_out, __half* k_cache, __half* v_cache, int64_t nh, int64_t K,
                                   cudaStream_t stream);
 int launch_gemv_pipe_gate_up(const __half* x, const __half* delta, const __half* norm_w, __half* x_out, float eps,
-                             const uint32_t* wq, const __half* scales, __half* act, int64_t M, int64_t I, int64_t K,
+                             const float* stats_in, const uint32_t* wq, const __half* scales, __half* act, int64_t M, int64_t I, int64_t K,
                              cudaStream_t stream);
+int launch_gemv_pipe_norm(const __half* x, const float* stats_in, const __half* norm_w, float eps, const uint32_t* wq, const __half* scales,
+                          __half* y, int64_t M, int64_t N, int64_t K, cudaStream_t stream);
+int launch_gemv_pipe_add(const __half* x, const uint32_t* wq, const __half* scales, __half* y, float* stats_out, int64_t M, int64_t N,
+                         int64_t K, int swiglu, cudaStream_t stream);
 int launch_gemv_pipe_swiglu(const __half* gu, const uint32_t* wq, const __half* scales, __half* y, int64_t M, int64_t N,
                             int64_t K, cudaStream_t stream);
 int launch_gemv_pipe_allreduce(const __half* x, const uint32_t* wq, const __half* scales, __half* y, int64_t M, int64_t N,
@@ -79,7 +83,8 @@ int launch_gemm(const __half* x, const uint32_t* wq, const __half* scales, __hal
 
 // fp16 output projection of a decode step (1 <= B <= 16) with optional greedy sampling; B200_ENOTREADY when the
 // activations do not fit in shared memory.
-int launch_lm_head(const __half* x, const __half* w, __half* logits, int* tokens, float* scratch, int64_t B, int64_t V,
+// With stats: x is the residual stream, its rows are normalised on the way in (B <= 8).
+int launch_lm_head(const __half* x, const float* stats, const __half* norm_w, float eps, __half* h_out, const __half* w, __half* logits, int* tokens, float* scratch, int64_t B, int64_t V,
                    int64_t H, int64_t token_offset, cudaStream_t stream);
 int64_t lm_head_scratch_bytes();
 

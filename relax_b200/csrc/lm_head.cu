@@ -40,10 +40,12 @@ __device__ __forceinline__ Best better(Best a, Best b) {
   return (b.v > a.v || (b.v == a.v && b.i < a.i)) ? b : a;
 }
 
-// NCB: column blocks of 8 batch rows (1 or 2).
-template <int NCB>
+// NCB: column blocks of 8 batch rows (1 or 2).  NORM (one block): x is the residual stream and stats [B][H / 16] holds the partial
+// sums of squares of its rows; the rows are normalised (RMSNorm, one fp16 rounding) as they are staged (and stored to h_out, if given).
+template <int NCB, bool NORM>
 __global__ void __launch_bounds__(warps_of(NCB) * 32, NCB == 1 ? 2 : 1)
-f16_lm_head_kernel(const __half* __restrict__ x, const __half* __restrict__ w, __half* __restrict__ logits,
+f16_lm_head_kernel(const __half* __restrict__ x, const float* __restrict__ stats, const __half* __restrict__ norm_w, float eps,
+                   __half* __restrict__ h_out, const __half* __restrict__ w, __half* __restrict__ logits,
                    int* __restrict__ tokens, float* __restrict__ scratch, int B, int V, int H, int token_offset) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int pitch = H * 2 + kPadBytes;                       // bytes per staged activation row
@@ -57,10 +59,28 @@ f16_lm_head_kernel(const __half* __restrict__ x, const __half* __restrict__ w, _
 
   pdl_launch_dependents();
   pdl_wait();                                                // x is the previous kernel's output
+  __shared__ float s_inv[8];
+  if (NORM) {
+    if (warp < B) {                                          // (eight warps, up to eight rows)
+      float tot = 0.f;
+      for (int i = lane * 4; i < H / 16; i += 128) {
+        const float4 v = *reinterpret_cast<const float4*>(stats + (int64_t)warp * (H / 16) + i);
+        tot += (v.x + v.y) + (v.z + v.w);
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
+      if (lane == 0) s_inv[warp] = rsqrtf(tot / (float)H + eps);
+    }
+    __syncthreads();
+  }
   for (int i = tid; i < NC * (H / 8); i += kThreads) {
     const int m = i / (H / 8), j = i - m * (H / 8);
     uint4 v = make_uint4(0, 0, 0, 0);
     if (m < B) v = *reinterpret_cast<const uint4*>(x + (int64_t)m * H + j * 8);
+    if (NORM && m < B) {
+      v = skinny::scale_f16x8(v, s_inv[m], *reinterpret_cast<const uint4*>(norm_w + j * 8));
+      if (h_out && blockIdx.x == 0) *reinterpret_cast<uint4*>(h_out + (int64_t)m * H + j * 8) = v;
+    }
     *reinterpret_cast<uint4*>(xs + (size_t)m * pitch + j * 16) = v;
   }
   __syncthreads();
@@ -178,7 +198,7 @@ f16_lm_head_kernel(const __half* __restrict__ x, const __half* __restrict__ w, _
 
 int64_t lm_head_scratch_bytes() { return ((int64_t)sm_count() * 2 * 16 * 2 + 4) * (int64_t)sizeof(float); }
 
-int launch_lm_head(const __half* x, const __half* w, __half* logits, int* tokens, float* scratch, int64_t B, int64_t V,
+int launch_lm_head(const __half* x, const float* stats, const __half* norm_w, float eps, __half* h_out, const __half* w, __half* logits, int* tokens, float* scratch, int64_t B, int64_t V,
                    int64_t H, int64_t token_offset, cudaStream_t stream) {
   const int ncb = B <= 8 ? 1 : 2;
   const size_t smem = (size_t)8 * ncb * (H * 2 + kPadBytes) + (size_t)warps_of(ncb) * 16 * 8 * ncb * sizeof(float);
@@ -196,10 +216,10 @@ int launch_lm_head(const __half* x, const __half* w, __half* logits, int* tokens
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = options().gemv_pdl ? 1 : 0;
-  auto kern = ncb == 1 ? f16_lm_head_kernel<1> : f16_lm_head_kernel<2>;
-  static SmemLimit limits[2];
-  if (int rc = raise_smem_limit(limits[ncb - 1], reinterpret_cast<const void*>(kern), smem, "lm_head")) return rc;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, x, w, logits, tokens, scratch, (int)B, (int)V, (int)H, (int)token_offset);
+  auto kern = stats ? f16_lm_head_kernel<1, true> : ncb == 1 ? f16_lm_head_kernel<1, false> : f16_lm_head_kernel<2, false>;
+  static SmemLimit limits[3];
+  if (int rc = raise_smem_limit(limits[stats ? 2 : ncb - 1], reinterpret_cast<const void*>(kern), smem, "lm_head")) return rc;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, x, stats, norm_w, eps, h_out, w, logits, tokens, scratch, (int)B, (int)V, (int)H, (int)token_offset);
   if (e != cudaSuccess) return fail(B200_ELAUNCH, "lm_head launch: %s", cudaGetErrorString(e));
   count_launch();
   return B200_OK;

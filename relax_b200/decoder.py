@@ -125,6 +125,10 @@ class DecodeEngine:
         # the separate kernels are faster (measured per layer at context 2000: 80 against 88 us at batch 2, 124 against
         # 176 at batch 8, 174 against 291 at batch 16).
         self.fused = (B == 1) if fused is None else (bool(fused) and B <= 16)
+        # chained: up to 8 rows, o and down add their product to the residual stream themselves and leave the sums of squares of its
+        # rows behind, from which qkv, gate|up and the output projection normalise it while they stage it: no launch for the norms.
+        # The default where it applies; `fused` = True or False select the two forms that form the statistics afresh.
+        self.chained = fused is None and world == 1 and not layer_kernel and B <= 8 and cfg.hidden % 256 == 0
         # rotary embedding, KV append and attention are one launch; True and "rope" take the entry points whose loads all wait for
         # the qkv matmul, False the one whose first loads of older cache entries run beside it
         self.fused_attention = "rope" if fused_attention == "rope" else bool(fused_attention)
@@ -135,12 +139,13 @@ class DecodeEngine:
         self.q = torch.zeros((B, self.nh_local, 128), **f16)
         self.attn = torch.zeros((B, hl), **f16)
         self.o = torch.zeros((B, H), **f16)
-        self.gu = None if self.fused else torch.zeros((B, 2 * il_max), **f16)       # (where SwiGLU is a launch of its own)
+        self.gu = torch.zeros((B, 2 * il_max), **f16)   # (where SwiGLU is a launch of its own)
         self.act = torch.zeros((B, il_max), **f16)
         self.down = torch.zeros((B, H), **f16)
         self.kc = [torch.zeros((B, max_ctx, self.nh_local, 128), **f16) for _ in layers]
         self.vc = [torch.zeros((B, max_ctx, self.nh_local, 128), **f16) for _ in layers]
         self.scratch = torch.zeros((4,), dtype=torch.float32, device=self.device)     # (the attention entry points ask for one)
+        self.stats = torch.zeros((B, max(H // 16, 1)), dtype=torch.float32, device=self.device)   # chained: sums of squares of x
         self.pos = torch.zeros((1,), dtype=torch.int32, device=self.device)
         self.tokens = torch.zeros((B,), dtype=torch.int32, device=self.device)
         self.cos, self.sin = rope_tables(max_ctx, 128, cfg.theta, self.device)
@@ -260,7 +265,89 @@ class DecodeEngine:
     def _gate_up_in_one(self, w) -> bool:
         """Whether SwiGLU runs in the epilogue of the gate|up matmul: with fused prologues, else where the library would
         take that matmul through the kernel that has the epilogue (asked anew each time: options may change)."""
-        return self.fused or bool(self.L.b200_q4f16_gemv_gate_up_applies(w["gu"][1].data_ptr(), self.batch, w["inter_local"], self.cfg.hidden))
+        return (self.fused and not self.chained) or bool(self.L.b200_q4f16_gemv_gate_up_applies(w["gu"][1].data_ptr(), self.batch, w["inter_local"], self.cfg.hidden))
+
+    def _in_skinny(self, w, n, k) -> bool:
+        """Whether the chained forms, which the skinny kernel has, are the ones for this matmul (asked anew each time, as below)."""
+        return bool(self.L.b200_q4f16_gemv_add_applies(w[1].data_ptr(), self.batch, n, k))
+
+    def _add(self, x, w, out, k, sp, swiglu=False):
+        """The residual stream += x . W^T, statistics included: None.  Or, where the chained form does not apply, `out` with the
+        product still to be added.  `swiglu`: x is gate | up, SwiGLU is applied first."""
+        H = self.cfg.hidden
+        if self._in_skinny(w, H, k):
+            self._check(self.L.b200_q4f16_gemv_add(x.data_ptr(), w[0].data_ptr(), w[1].data_ptr(), self.x.data_ptr(),
+                                                   self.stats.data_ptr(), self.batch, H, k, int(swiglu), sp))
+            return None
+        if swiglu:
+            self._check(self.L.b200_silu_mul_early_release(x.data_ptr(), self.act.data_ptr(), self.batch, k, sp))
+            x = self.act
+        self._matmul(x, w, out, H, k, sp)
+        return out
+
+    def _norm(self, delta, norm, sp):
+        """h = rmsnorm(x += delta) as a launch of its own."""
+        self._check(self.L.b200_rmsnorm_early_release(self.x.data_ptr(), delta.data_ptr() if delta is not None else None, norm.data_ptr(),
+                                                      self.h.data_ptr(), self.batch, self.cfg.hidden, self.cfg.eps, sp))
+
+    def _chained_layer(self, i: int, delta, sp: int):
+        """One layer in the chained form: qkv, attention, o, gate|up, down.  `delta` as in :meth:`layer_step`; None: the residual
+        stream is complete and has its statistics."""
+        cfg, L, B, w = self.cfg, self.L, self.batch, self.layers[i]
+        H, il = cfg.hidden, w["inter_local"]
+        roped = False
+        if delta is None and self.rope_epilogue:
+            rc = L.b200_q4f16_gemv_norm_rope(self.x.data_ptr(), self.stats.data_ptr(), w["norm1"].data_ptr(), cfg.eps,
+                                             w["qkv"][0].data_ptr(), w["qkv"][1].data_ptr(), self.cos.data_ptr(), self.sin.data_ptr(),
+                                             self.pos.data_ptr(), self.q.data_ptr(), self.kc[i].data_ptr(), self.vc[i].data_ptr(),
+                                             self.nh_local, H, sp)
+            if rc != _lib.ENOTREADY:        # (else the exact form is selected)
+                self._check(rc)
+                roped = True
+        if not roped and delta is None and self._in_skinny(w["qkv"], 3 * H, H):
+            self._check(L.b200_q4f16_gemv_norm(self.x.data_ptr(), self.stats.data_ptr(), w["norm1"].data_ptr(), cfg.eps,
+                                               w["qkv"][0].data_ptr(), w["qkv"][1].data_ptr(), self.qkv.data_ptr(), B, 3 * H, H, sp))
+        elif not roped:
+            self._norm(delta, w["norm1"], sp)
+            self._matmul(self.h, w["qkv"], self.qkv, 3 * H, H, sp)
+        self._attention(i, roped, sp)
+        delta = self._add(self.attn, w["o"], self.o, H, sp)
+        if not self._gate_up_in_one(w):
+            self._norm(delta, w["norm2"], sp)
+            self._matmul(self.h, w["gu"], self.gu, 2 * il, H, sp)
+            return self._add(self.gu, w["down"], self.down, il, sp, swiglu=True)
+        if delta is None:
+            self._check(L.b200_q4f16_gemv_norm_gate_up(self.x.data_ptr(), self.stats.data_ptr(), w["norm2"].data_ptr(), cfg.eps,
+                                                       w["gu"][0].data_ptr(), w["gu"][1].data_ptr(), self.act.data_ptr(), B, il, H, sp))
+        else:
+            self._norm(delta, w["norm2"], sp)
+            self._check(L.b200_q4f16_gemv_gate_up(self.h.data_ptr(), None, None, None, 0.0, w["gu"][0].data_ptr(), w["gu"][1].data_ptr(),
+                                                  self.act.data_ptr(), B, il, H, sp))
+        return self._add(self.act, w["down"], self.down, il, sp)
+
+    def _attention(self, i: int, roped: bool, sp: int):
+        """`roped`: the qkv matmul has rotated q and appended k and v, else all of that is done here.
+
+        Early loads: the position and the older cache entries are final before any kernel of a step but its first can begin.
+        A kernel begins only after the one in front of it has begun, embed_rows lets its successor begin only after it
+        has waited for everything in front of it, and every kernel waits for its predecessor before it ends."""
+        L, B = self.L, self.batch
+        if roped:
+            self._check(L.b200_attn_decode_early_release(self.q.data_ptr(), self.kc[i].data_ptr(), self.vc[i].data_ptr(),
+                                                         self.pos.data_ptr(), self.attn.data_ptr(), self.scratch.data_ptr(), B,
+                                                         self.nh_local, self.max_ctx, _lib.ATTN_EARLY_KV_LOADS, sp))
+        elif self.fused_attention == "rope":
+            self._check(L.b200_attn_decode_rope(self.qkv.data_ptr(), self.cos.data_ptr(), self.sin.data_ptr(), self.pos.data_ptr(),
+                                                self.kc[i].data_ptr(), self.vc[i].data_ptr(), self.attn.data_ptr(),
+                                                self.scratch.data_ptr(), B, self.nh_local, self.max_ctx, sp))
+        elif self.fused_attention:
+            self._check(L.b200_attn_decode_fused(self.qkv.data_ptr(), self.cos.data_ptr(), self.sin.data_ptr(), self.pos.data_ptr(),
+                                                 self.kc[i].data_ptr(), self.vc[i].data_ptr(), self.attn.data_ptr(),
+                                                 self.scratch.data_ptr(), B, self.nh_local, self.max_ctx, sp))
+        else:
+            self._check(L.b200_attn_decode_step(self.qkv.data_ptr(), self.cos.data_ptr(), self.sin.data_ptr(), self.pos.data_ptr(),
+                                                self.kc[i].data_ptr(), self.vc[i].data_ptr(), self.attn.data_ptr(), B, self.nh_local,
+                                                self.max_ctx, _lib.ATTN_EARLY_KV_LOADS | _lib.ATTN_EARLY_RELEASE, sp))
 
     def _allreduce(self, t):
         if self.world > 1:
@@ -298,28 +385,7 @@ class DecodeEngine:
             self._check(L.b200_rmsnorm_early_release(self.x.data_ptr(), dptr, w["norm1"].data_ptr(), self.h.data_ptr(), B, H,
                                                      cfg.eps, sp))
             self._matmul(self.h, w["qkv"], self.qkv, 3 * hl, H, sp)
-        if roped:
-            # The position and the older cache entries were final before the matmul in front began (the position was
-            # advanced two launches before this step's first kernel, each of which waits before it lets the next
-            # one start; the matmul's epilogue writes only the new token's slot, which the attention reads after
-            # its own wait)
-            self._check(L.b200_attn_decode_early_release(self.q.data_ptr(), self.kc[i].data_ptr(), self.vc[i].data_ptr(),
-                                                         self.pos.data_ptr(), self.attn.data_ptr(), self.scratch.data_ptr(), B,
-                                                         self.nh_local, self.max_ctx, _lib.ATTN_EARLY_KV_LOADS, sp))
-        elif self.fused_attention == "rope":
-            self._check(L.b200_attn_decode_rope(self.qkv.data_ptr(), self.cos.data_ptr(), self.sin.data_ptr(), self.pos.data_ptr(),
-                                                self.kc[i].data_ptr(), self.vc[i].data_ptr(), self.attn.data_ptr(),
-                                                self.scratch.data_ptr(), B, self.nh_local, self.max_ctx, sp))
-        elif self.fused_attention:
-            self._check(L.b200_attn_decode_fused(self.qkv.data_ptr(), self.cos.data_ptr(), self.sin.data_ptr(), self.pos.data_ptr(),
-                                                 self.kc[i].data_ptr(), self.vc[i].data_ptr(), self.attn.data_ptr(),
-                                                 self.scratch.data_ptr(), B, self.nh_local, self.max_ctx, sp))
-        else:
-            # rotary embedding + KV append + attention in one launch.  Early loads as above: no kernel of a step begins before
-            # embed_rows has waited for all of the step before
-            self._check(L.b200_attn_decode_step(self.qkv.data_ptr(), self.cos.data_ptr(), self.sin.data_ptr(), self.pos.data_ptr(),
-                                                self.kc[i].data_ptr(), self.vc[i].data_ptr(), self.attn.data_ptr(), B, self.nh_local,
-                                                self.max_ctx, _lib.ATTN_EARLY_KV_LOADS | _lib.ATTN_EARLY_RELEASE, sp))
+        self._attention(i, roped, sp)
         if self.peer is not None and B <= self.PEER_FUSED_MAX_ROWS:
             d = self._reduce_desc(0, i, self.o)
             self._check(L.b200_q4f16_gemv_allreduce(self.attn.data_ptr(), w["o"][0].data_ptr(), w["o"][1].data_ptr(),
@@ -364,8 +430,12 @@ class DecodeEngine:
         if self.guard is not None and not torch.cuda.is_current_stream_capturing():
             self.guard.check()
         sp = torch.cuda.current_stream(self.device).cuda_stream
-        self._check(L.b200_embed_rows(self.embed.data_ptr(), self.tokens.data_ptr(), self.x.data_ptr(), B, cfg.hidden,
-                                      self.embed.shape[0], sp))
+        if self.chained:
+            self._check(L.b200_embed_rows_stats(self.embed.data_ptr(), self.tokens.data_ptr(), self.x.data_ptr(), self.stats.data_ptr(), B,
+                                                cfg.hidden, self.embed.shape[0], sp))
+        else:
+            self._check(L.b200_embed_rows(self.embed.data_ptr(), self.tokens.data_ptr(), self.x.data_ptr(), B, cfg.hidden,
+                                          self.embed.shape[0], sp))
         delta = None
         xlast = self.x
         if self.layer_kernel:
@@ -375,10 +445,16 @@ class DecodeEngine:
                 delta, xlast = self.down, self.x_last
         else:
             for i in range(len(self.layers)):
-                delta = self.layer_step(i, delta, sp)
-        self._check(L.b200_rmsnorm_early_release(xlast.data_ptr(), delta.data_ptr() if delta is not None else None,
-                                                 self.final_norm.data_ptr(), self.h.data_ptr(), B, cfg.hidden, cfg.eps, sp))
-        if self.lm_head is not None:
+                delta = self._chained_layer(i, delta, sp) if self.chained else self.layer_step(i, delta, sp)
+        normed = not (self.chained and delta is None and self.lm_head is not None)
+        if normed:
+            self._check(L.b200_rmsnorm_early_release(xlast.data_ptr(), delta.data_ptr() if delta is not None else None,
+                                                     self.final_norm.data_ptr(), self.h.data_ptr(), B, cfg.hidden, cfg.eps, sp))
+        if not normed:
+            self._check(L.b200_lm_head_norm(self.x.data_ptr(), self.stats.data_ptr(), self.final_norm.data_ptr(), cfg.eps,
+                                            self.h.data_ptr(), self.lm_head.data_ptr(), self.logits_local.data_ptr(), self.tokens.data_ptr(),
+                                            self.lm_scratch.data_ptr(), B, self.lm_head.shape[0], cfg.hidden, 0, sp))
+        elif self.lm_head is not None:
             own = B <= 16                       # the library's output projection takes up to 16 rows; above that a library GEMM
             if own:
                 toks = self.tokens.data_ptr() if self.world == 1 else None
@@ -401,6 +477,19 @@ class DecodeEngine:
         head = 1 if self.lm_head is not None and self.batch <= 16 else 0
         if self.layer_kernel:
             return 1 + len(self.layers) + 1 + head + 2
+        if self.chained:
+            ready, norms = True, 0          # the residual stream has its statistics; norms as launches of their own
+            per_layer = 0
+            for w in self.layers:
+                per_layer += 5
+                roped = self.rope_epilogue and ready
+                norms += not (ready and (roped or self._in_skinny(w["qkv"], 3 * self.cfg.hidden, self.cfg.hidden)))
+                ready = self._in_skinny(w["o"], self.cfg.hidden, self.cfg.hidden)
+                one = self._gate_up_in_one(w)
+                norms += not (ready and one)
+                ready = self._in_skinny(w["down"], self.cfg.hidden, w["inter_local"])
+                per_layer += 0 if one or ready else 1          # (SwiGLU as a launch of its own)
+            return 1 + per_layer + norms + (0 if ready and head else 1) + head + 2
         peer_sums = 2 if self.peer is not None and self.batch > self.PEER_FUSED_MAX_ROWS else 0
         per_layer = 0
         for w in self.layers:
