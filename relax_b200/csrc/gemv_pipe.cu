@@ -122,6 +122,22 @@ struct PipeParams {
   PeerReduce red;
 };
 
+// The staged block of x: 16-byte slots, one per word of eight values, one of padding behind every eight (a lane reads words 8 t + i
+// of its column g).  Up to two batch columns they lie side by side.  From four on every column is a row of slots of its own,
+// whose pitch is 4 more than a multiple of eight: the eight lanes of a quarter warp then hit different banks, whether two columns
+// are read (g, t) or one is written word by word.
+template <int NC>
+struct XRows {
+  static constexpr bool kOwnRows = NC > 2;
+  static constexpr int kWord = kOwnRows ? 1 : NC;      // slots from a word to the next
+  static constexpr int kChunk = 36 * kWord;            // ... of 256 k
+  __host__ __device__ static constexpr int pitch(int k) { return kOwnRows ? k / 256 * 36 + (k / 256 % 2 == 0 ? 4 : 0) : 1; }
+  __host__ __device__ static constexpr size_t bytes(int k) {                                 // k: a multiple of 256
+    return (size_t)16 * (kOwnRows ? NC * pitch(k) : k / 256 * kChunk);
+  }
+  __device__ __forceinline__ static int slot(int jw, int col, int pitch) { return kWord * (jw + (jw >> 3)) + col * pitch; }
+};
+
 // The arithmetic of the fast form over a warp's U chunks of one stage (see the comment at its call site in the kernel).
 template <int U, int MT, int kXUnit, int kCUnit>
 __device__ __forceinline__ void fast_stage_fn(float (&acc)[2][MT][4], const uint4 (&w)[U][2][2], const uint2 (&sc)[U][2],
@@ -185,14 +201,14 @@ __device__ __forceinline__ void fast_stage_fn(float (&acc)[2][MT][4], const uint
 // Shared memory carve-up (after rounding the base up to 1024 bytes):
 //   ring:  nstages * kStageBytes
 //   bars:  full[kMaxStages] empty[kMaxStages] red_full[kMaxStages+1] red_empty[kMaxStages+1]
-//   xs:    XLayout::bytes(kblk)     permuted x block
+//   xs:    XRows::bytes(kblk)       permuted x block
 //   corr:  (fast form) 32 floats per 256-k chunk: minus the offset sum of each group, see corr_index()
 //   red:   (nstages+1) * CW * kOut * 4   per-warp partial sums of a tile, one buffer per tile in flight
 //   accs:  tiles_per_cta * kOut * 4 (only when K is cut into several blocks)
 //
 // Warps: CW consumers, then one TMA warp (two issuing lanes), then one epilogue warp.
 template <int NC, int CW, int CH, int PRO, bool FAST, int EPI>
-__global__ void __launch_bounds__((CW + 2) * 32, FAST ? 2 : 1)
+__global__ void __launch_bounds__((CW + 2) * 32, FAST || CH == CW ? 2 : 1)
 q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
   constexpr int MT = (NC + 7) / 8;
   constexpr bool GU = EPI == kEpilogueGateUp, ADD = EPI == kEpilogueAdd;
@@ -207,7 +223,7 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
   constexpr int kSBytes = CH * kRows * 16;            // [chunk][row][8 scales = 16 B]
   constexpr int kStageBytes = kWBytes + kSBytes;      // a multiple of 1024, as the swizzle needs
   constexpr int U = CH / CW;                          // chunks per warp per stage
-  using XL = XLayout<NC>;
+  using XL = XRows<NC>;
   static_assert(CH % CW == 0 && U >= 1, "each consumer warp takes whole chunks");
   static_assert(kStageBytes % 1024 == 0, "stage alignment");
   extern __shared__ unsigned char smem_unaligned[];
@@ -496,9 +512,10 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
   // Lanes whose batch column does not exist (g >= NC) read column 0: what they feed into the MMA only
   // reaches output columns >= NC, which are never stored.  (Fast form: see x_own below.)
   const int xcol = NC >= 8 ? g : (g < NC ? g : 0);
-  const uint4* x_thr = xs + (NC >= 8 ? (warp * 32 + 8 * t) * NC + (g ^ (2 * t)) : NC * (warp * 36 + 9 * t) + xcol);
-  constexpr int kXStage = CH * XL::kSlotsPerChunk;   // slots per stage
-  constexpr int kXUnit = CW * XL::kSlotsPerChunk;    // slots between this warp's chunks
+  const int xpitch = XL::pitch(p.kblk);
+  const uint4* x_thr = xs + xcol * xpitch + warp * XL::kChunk + 9 * t * XL::kWord;
+  constexpr int kXStage = CH * XL::kChunk;           // slots per stage
+  constexpr int kXUnit = CW * XL::kChunk;            // slots between this warp's chunks
   // fast form: column c of the MMA is the group that lane t = c holds, so the activation goes into the B
   // fragment of the lanes with g == t only (B[k slots of lane t][column g]); every other lane feeds zeros
   const bool x_own = g == t;
@@ -530,7 +547,7 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
       for (int wd = 0; wd < 4; ++wd) {
         uint4 b[MT];
 #pragma unroll
-        for (int mt = 0; mt < MT; ++mt) b[mt] = xu[(4 * h + wd) * NC + 8 * mt];
+        for (int mt = 0; mt < MT; ++mt) b[mt] = xu[(4 * h + wd) * XL::kWord + 8 * mt * xpitch];
         uint32_t a_lo[4], a_hi[4];
         q4_dequant_pairs(wr0[wd], s0, a_lo, qc);
         q4_dequant_pairs(wr1[wd], s1, a_hi, qc);
@@ -594,7 +611,7 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
   // Stores one staged word (eight activations of one batch column) in the permuted order the unpack
   // produces; the fast form also returns its offset sum.
   auto stage_word = [&](int j, int m, const uint4& v) -> float {
-    xs[XL::slot(j, m)] = staged_order(v, p.paired != 0);
+    xs[XL::slot(j, m, xpitch)] = staged_order(v, p.paired != 0);
     return FAST ? offset_sum_f16x8(v, p.paired != 0) : 0.f;
   };
   // Fast form (one batch column): minus the offset sum of scale group `grp`, twice (rows g and g+8 of the
@@ -603,6 +620,37 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
     const int ci = corr_index(grp);
     negcorr[ci] = -psum;
     negcorr[ci + 2] = -psum;
+  };
+
+  // From four columns on a warp stages the chunks that it multiplies itself (warp, warp + CW, .. of the block), lane = word of eight
+  // values: nobody waits for another warp's share, and columns past M are left out.  The items of a warp are its chunks by the
+  // rows of x, kItems of them in flight.  Dealt out over all threads of the CTA, eight columns whatever M is and a barrier
+  // behind, a launch took, us, before / now: M x N x K 5 x 2048 x 5632 7.1 / 5.5, 8 x 1024 x 3072 5.3 / 4.3, 8 x 4096 x 4096 7.8 / 6.6,
+  // 8 x 22016 x 4096 17.5 / 16.5, 4 x 4096 x 4096 6.0 / 5.5; up to two columns it is the faster way (2 x 4096 x 4096 5.1 / 5.3).
+  constexpr int kItems = PRO == kPrologueNone || PRO == kPrologueNormStats ? 8 : 4;
+  auto next_item = [&](int& c, int& m) {
+    if (++m == p.M) {
+      m = 0;
+      c += CW;
+    }
+  };
+  auto load_items = [&](int c, int m, int k_lo, int nch, uint4 (&a)[kItems], uint4 (&b)[kItems], uint4 (&w)[kItems]) {
+#pragma unroll
+    for (int r = 0; r < kItems; ++r) {
+      a[r] = b[r] = w[r] = make_uint4(0, 0, 0, 0);
+      if (c < nch) {
+        const int k = k_lo + c * 256 + lane * 8;
+        if (PRO == kPrologueSwiGLU) {               // x is [M, 2K] = gate | up
+          a[r] = *reinterpret_cast<const uint4*>(p.x + (int64_t)m * 2 * p.K + k);
+          b[r] = *reinterpret_cast<const uint4*>(p.x + (int64_t)m * 2 * p.K + p.K + k);
+        } else {
+          a[r] = *reinterpret_cast<const uint4*>(p.x + (int64_t)m * p.K + k);
+          if (PRO == kPrologueRmsNorm && p.delta) b[r] = *reinterpret_cast<const uint4*>(p.delta + (int64_t)m * p.K + k);
+          if (PRO == kPrologueRmsNorm) w[r] = *reinterpret_cast<const uint4*>(p.norm_w + k);
+        }
+        next_item(c, m);
+      }
+    }
   };
 
   int s = 0;                                     // ring slot of the current stage
@@ -615,14 +663,13 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
   uint4 fw[U][2][2];
   uint2 fsc[U][2];
   if (FAST) fast_load(0, 0, fw, fsc);
-  // NormStats: the items (words of eight values) that a thread stages at a time; the norm weights of the first ones are
-  // here when the wait returns
-  constexpr int kNormItems = NC >= 8 ? 4 : 2;
-  uint4 nw[kNormItems];
+  // NormStats: the first norm weights are here when the wait returns: of this thread's first items, or of this warp's first
+  // two chunks
+  uint4 nw[2];
   if (PRO == kPrologueNormStats) {
 #pragma unroll
-    for (int r = 0; r < kNormItems; ++r) {
-      const int k = (tid + r * kConsumers) / NC * 8;
+    for (int r = 0; r < (int)(sizeof(nw) / sizeof(nw[0])); ++r) {
+      const int k = XL::kOwnRows ? (warp + r * CW) * 256 + lane * 8 : (tid + r * kConsumers) / NC * 8;
       nw[r] = k < p.K ? *reinterpret_cast<const uint4*>(p.norm_w + k) : make_uint4(0, 0, 0, 0);
     }
   }
@@ -716,10 +763,31 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
   }
 
   // ---- RMSNorm with the statistics of the kernel that wrote x (one K block: checked by the launcher) ----------------
-  // The first loads of x and the partial sums travel together; warp m adds up row m's.
-  if (PRO == kPrologueNormStats) {
+  // The partial sums and the first loads of x travel together; warp m adds up row m's.
+  float4 part[2];
+  auto load_stats = [&]() {
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const int i = lane * 4 + 128 * r;
+      part[r] = warp < p.M && i < p.K >> 4 ? *reinterpret_cast<const float4*>(p.stats_in + (int64_t)warp * (p.K >> 4) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  };
+  auto add_stats = [&]() {
+    if (warp < p.M) {
+      float tot = ((part[0].x + part[0].y) + (part[0].z + part[0].w)) + ((part[1].x + part[1].y) + (part[1].z + part[1].w));
+      for (int i = lane * 4 + 256; i < p.K >> 4; i += 128) {          // (K > 4096)
+        const float4 v = *reinterpret_cast<const float4*>(p.stats_in + (int64_t)warp * (p.K >> 4) + i);
+        tot += (v.x + v.y) + (v.z + v.w);
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
+      if (lane == 0) s_inv[warp] = rsqrtf(tot / (float)p.K + p.eps);
+    }
+    bar_sync(1, kConsumers);
+  };
+  if (PRO == kPrologueNormStats && !XL::kOwnRows) {
+    constexpr int kNormItems = 2;
     const int items = (p.kblk >> 3) * NC;        // a multiple of kConsumers
-    const int parts = p.K >> 4;
     uint4 a[kNormItems];
     auto load = [&](int i0) {
 #pragma unroll
@@ -728,18 +796,9 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
         a[r] = m < p.M && j * 8 < p.K ? *reinterpret_cast<const uint4*>(p.x + (int64_t)m * p.K + j * 8) : make_uint4(0, 0, 0, 0);
       }
     };
+    load_stats();
     load(tid);
-    if (warp < p.M) {
-      float tot = 0.f;
-      for (int i = lane * 4; i < parts; i += 128) {
-        const float4 v = *reinterpret_cast<const float4*>(p.stats_in + (int64_t)warp * parts + i);
-        tot += (v.x + v.y) + (v.z + v.w);
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
-      if (lane == 0) s_inv[warp] = rsqrtf(tot / (float)p.K + p.eps);
-    }
-    bar_sync(1, kConsumers);
+    add_stats();
     for (int i0 = tid; i0 < items; i0 += kNormItems * kConsumers) {
       if (i0 != tid) {
         load(i0);
@@ -785,10 +844,47 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
   for (int kb = 0; kb < nkb; ++kb) {
     const int k_lo = kb * p.kblk;
     const int k_hi = min(p.K, k_lo + p.kblk);
-    // ---- stage x[:, k_lo .. k_lo + kblk) permuted per 8 k; zero beyond K and beyond M --------------
-    if (kb > 0) bar_sync(1, kConsumers);         // everyone is done reading the previous block
-    if (PRO == kPrologueNormStats) {
+    // ---- stage x[:, k_lo .. k_lo + kblk) permuted per 8 k --------------------------------------------------------
+    if (XL::kOwnRows) {
+      const int nch = (k_hi - k_lo) >> 8;
+      if (kb > 0) __syncwarp();                  // all lanes are done reading the previous block
+      if (PRO == kPrologueNormStats) load_stats();
+#pragma unroll 1
+      for (int c = warp, m = 0; c < nch;) {
+        uint4 a[kItems], b[kItems], w[kItems];
+        load_items(c, m, k_lo, nch, a, b, w);
+#pragma unroll
+        for (int r = 0; r < kItems; ++r)
+          if (c < nch) {
+            uint4 v = a[r];
+            if (PRO == kPrologueSwiGLU) v = silu_mul_f16x8(a[r], b[r]);           // fp32 inside, one fp16 rounding
+            if (PRO == kPrologueRmsNorm && p.delta) v = add_f16x8(v, b[r]);
+            if (PRO == kPrologueRmsNorm) v = scale_f16x8(v, s_inv[m], w[r]);
+            stage_word(c * 32 + lane, m, v);
+            next_item(c, m);
+          }
+      }
+      if (PRO == kPrologueNormStats) {
+        // as it came so far; every lane scales its own words in place (little code: it is fetched anew in every launch)
+        add_stats();
+#pragma unroll 1
+        for (int c = warp; c < nch; c += CW) {
+          const uint4 w = staged_order(nw[0], p.paired != 0);
+          nw[0] = nw[1];
+          if (c + 2 * CW < nch) nw[1] = *reinterpret_cast<const uint4*>(p.norm_w + (c + 2 * CW) * 256 + lane * 8);
+          uint4* x = xs + XL::slot(c * 32 + lane, 0, xpitch);
+#pragma unroll 2
+          for (int m = 0; m < p.M; ++m, x += xpitch) *x = scale_f16x8(*x, s_inv[m], w);
+        }
+      }
+      __syncwarp();
+    } else if (PRO == kPrologueNormStats) {
       // (staged above)
+      bar_sync(1, kConsumers);
+    } else if (kb > 0) {
+      bar_sync(1, kConsumers);                   // everyone is done reading the previous block
+    }
+    if (XL::kOwnRows || PRO == kPrologueNormStats) {
     } else if (FAST && !(PRO == kPrologueRmsNorm && rms_one_pass)) {
       // one batch column: a thread takes a whole scale group (four words, 64 contiguous bytes), so its offset sum
       // needs no exchange; all loads of a thread are issued before the first use
@@ -834,7 +930,7 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
       const int words = p.kblk >> 3;
       const int items = words * NC;              // a multiple of 32: a warp's 32 items are all inside or all outside
       // (registers: small batches keep two CTAs per SM; without a prologue only one array is live)
-      constexpr int R = NC >= 8 ? 4 : (PRO == kPrologueNone ? 4 : (NC == 1 ? 2 : 1));
+      constexpr int R = PRO == kPrologueNone ? 4 : (NC == 1 ? 2 : 1);
       for (int i0 = tid; i0 < items; i0 += kConsumers * R) {
         uint4 a[R], b[R], c[R];
         bool live[R];
@@ -877,7 +973,7 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
         }
       }
     }
-    bar_sync(1, kConsumers);
+    if (!XL::kOwnRows && PRO != kPrologueNormStats) bar_sync(1, kConsumers);
     for (int tile = blockIdx.x; tile < p.ntiles; tile += gridDim.x) {
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt)
@@ -1039,7 +1135,7 @@ int launch_pipe(const __half* x, const uint32_t* wq, const __half* scales, __hal
   constexpr int kStageBytes = CH * kRows * (128 + 16);
   constexpr int kThreads = (CW + 2) * 32;
   constexpr bool GU = EPI == kEpilogueGateUp;
-  using XL = XLayout<NC>;
+  using XL = XRows<NC>;
   PipeParams p;
   p.rope = pro.rope;
   if (GU) {
@@ -1221,7 +1317,7 @@ template <int NC>
 bool half_stages(int n, int k) {
   constexpr size_t kRing = 8 * kRows * (128 + 16);                            // a short stage
   constexpr size_t kRest = 3 * 8 * 128 * sizeof(float) + 2048;                // partial sums, barriers, alignment
-  const size_t x_short = XLayout<NC>::bytes((k + 2047) / 2048 * 2048), x_long = XLayout<NC>::bytes((k + 4095) / 4096 * 4096);
+  const size_t x_short = XRows<NC>::bytes((k + 2047) / 2048 * 2048), x_long = XRows<NC>::bytes((k + 4095) / 4096 * 4096);
   const bool pair = 2 * kRing + kRest + x_short <= kExclusiveSmem - 1024;
   const int tail = k % 4096;
   if (tail == 0 || tail > 2048) return NC <= 4 && pair && n > sm_count() * kRows * 3 / 2;
