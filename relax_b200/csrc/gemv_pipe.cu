@@ -208,7 +208,7 @@ __device__ __forceinline__ void fast_stage_fn(float (&acc)[2][MT][4], const uint
 //
 // Warps: CW consumers, then one TMA warp (two issuing lanes), then one epilogue warp.
 template <int NC, int CW, int CH, int PRO, bool FAST, int EPI>
-__global__ void __launch_bounds__((CW + 2) * 32, FAST || CH == CW ? 2 : 1)
+__global__ void __launch_bounds__((CW + 2) * 32, FAST || (CH == CW && CW == 8) ? 2 : 1)
 q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
   constexpr int MT = (NC + 7) / 8;
   constexpr bool GU = EPI == kEpilogueGateUp, ADD = EPI == kEpilogueAdd;
@@ -1277,7 +1277,7 @@ int launch_pipe(const __half* x, const uint32_t* wq, const __half* scales, __hal
   // 3.0 / 2.8, M = 4 N = 2048, K = 4096 5.7 / 4.5.  (Not the fast form up to K = 4096 on more than half of the SMs: the next
   // launch's first copies, which need a place beside this one, are worth as much there: 3.84 / 3.89 at N = 2048, K = 4096; at
   // N = 1024 3.46 / 3.23.  Not the longer stages of 2..8 rows, which mostly fill an SM by themselves.)
-  const bool alone = p.ntiles <= sms && (FAST ? K > 4096 || 2 * p.ntiles <= sms : NC == 1 || CH < 16);
+  const bool alone = p.ntiles <= sms && (FAST ? K > 4096 || 2 * p.ntiles <= sms : NC == 1 || CH < 16 || CW > 8);
   if (alone && need < kExclusiveSmem) need = kExclusiveSmem;
   if (int rc = raise_smem_limit(limit, func, need, "gemv")) return rc;
   p.nstages = stages;
@@ -1351,12 +1351,18 @@ int launch_pipe_m(const __half* x, const uint32_t* wq, const __half* scales, __h
   if (m == 2)
     return half_stages<2>(n, k) ? launch_pipe<2, CW, CW, PRO, false, EPI>(x, wq, scales, y, m, n, k, stream, pro, red)
                              : launch_pipe<2, CW, CH, PRO, false, EPI>(x, wq, scales, y, m, n, k, stream, pro, red);
+  // Sixteen consumer warps where one CTA fills an SM anyway and a tile has chunks for them: eight are too few to hide their own
+  // latencies.  3 or 4 rows with no more tiles than SMs and K > 4096: 8 / 16 warps, us, 4 x 2048 x 5632 5.5 / 5.1, 3 x 1024 x 8192
+  // 5.8 / 5.2, 4 x 1280 x 6912 5.7 / 5.0, but 4 x 2048 x 4096 4.1 / 4.2; 2 x 2048 x 5632 4.7 / 4.9.  5..8 rows with the long stages:
+  // 8 x 4096 x 4096 6.5 / 6.0, 7 x 7680 x 2560 7.4 / 7.1, 8 x 22016 x 4096 15.9 / 15.2, 8 x 3072 x 3072 5.4 / 5.0.
+  if (m > 2 && m <= 4 && k > 4096 && n <= sm_count() * kRows)
+    return launch_pipe<4, 2 * CW, CH, PRO, false, EPI>(x, wq, scales, y, m, n, k, stream, pro, red);
   if (m <= 4)
     return half_stages<4>(n, k) ? launch_pipe<4, CW, CW, PRO, false, EPI>(x, wq, scales, y, m, n, k, stream, pro, red)
                              : launch_pipe<4, CW, CH, PRO, false, EPI>(x, wq, scales, y, m, n, k, stream, pro, red);
   if (m <= 8)
     return half_stages<8>(n, k) ? launch_pipe<8, CW, CW, PRO, false, EPI>(x, wq, scales, y, m, n, k, stream, pro, red)
-                             : launch_pipe<8, CW, CH, PRO, false, EPI>(x, wq, scales, y, m, n, k, stream, pro, red);
+                             : launch_pipe<8, 2 * CW, CH, PRO, false, EPI>(x, wq, scales, y, m, n, k, stream, pro, red);
   if constexpr (PRO == kPrologueNormStats || EPI == kEpilogueAdd) return B200_ENOTREADY;
   else return launch_pipe<16, CW, CH, PRO, false, EPI>(x, wq, scales, y, m, n, k, stream, pro, red);
 }
