@@ -236,6 +236,13 @@ B200_API int b200_q4f16_gemv_rmsnorm_rope(const void* x, const void* delta, cons
 B200_API int b200_q4f16_gemv_swiglu(const void* gu, const void* wq, const void* scales, void* y, int64_t M, int64_t N,
                                     int64_t K, void* cuda_stream);
 
+/* The same (x is the normalised activation) in the kernel that the automatic dispatch takes for more rows: act = silu(x . Wg^T) *
+ * (x . Wu^T) for 1 <= M <= 128, any I and any K that b200_q4f16_matmul takes.  _applies: 1 where the automatic dispatch gives the
+ * gate|up matmul to that kernel. */
+B200_API int b200_q4f16_gate_up_applies(const void* scales, int64_t M, int64_t I, int64_t K);
+B200_API int b200_q4f16_gate_up(const void* x, const void* wq, const void* scales, void* act, int64_t M, int64_t I, int64_t K,
+                                void* cuda_stream);
+
 /* ---- the residual stream with its statistics (up to eight rows) -----------------------------------
  * b200_q4f16_gemv_add: y += x . W^T (y is the residual stream, fp16 [M,N], N % 16 == 0; the product is rounded to fp16, then the
  * sum, as the matmul and the residual add in b200_rmsnorm do), and stats, fp32 [M][N / 16], receives the sums of squares of the new

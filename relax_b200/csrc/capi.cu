@@ -529,6 +529,25 @@ int b200_q4f16_gemv_gate_up(const void* x, const void* delta, const void* norm_w
   return rc;
 }
 
+// SwiGLU in the epilogue of the weight-stationary kernel, for the rows that the automatic dispatch gives to it.
+int b200_q4f16_gate_up_applies(const void* scales, int64_t M, int64_t I, int64_t K) {
+  if (M < 1 || M > 128 || I < 1 || I > 0x3fffffffLL / 32 || K < 32 || K % 32 != 0 || !scales) return 0;
+  return weight_stationary_first(M, 2 * I, K, K % 256 != 0 || !aligned16(scales));
+}
+
+int b200_q4f16_gate_up(const void* x, const void* wq, const void* scales, void* act, int64_t M, int64_t I, int64_t K, void* stream) {
+  const char* who = "q4f16_gate_up";
+  if (I < 1 || I > 0x3fffffffLL / 32) return fail(B200_EINVAL, "%s: needs I >= 1, got %lld", who, (long long)I);
+  int rc = check_matmul(who, x, wq, scales, act, M, 2 * I, K);
+  if (rc) return rc;
+  if (M < 1 || M > 128 || K < 32) return fail(B200_EINVAL, "%s: takes 1 <= M <= 128 and K >= 32", who);
+  if ((rc = ensure_device())) return rc;
+  rc = launch_gemm_ws(static_cast<const __half*>(x), static_cast<const uint32_t*>(wq), static_cast<const __half*>(scales),
+                      static_cast<__half*>(act), M, 2 * I, K, static_cast<cudaStream_t>(stream), true);
+  if (rc == B200_ENOTREADY) return fail(rc, "%s: shape outside the fused kernel's domain", who);
+  return rc;
+}
+
 // ---- the residual stream with its statistics -------------------------------------------------------------------
 // Common to the forms that normalise x by statistics left behind: up to eight rows.
 static int check_norm_stats(const char* who, const void* stats, const void* norm_w, const void* scales, int64_t M, int64_t K) {

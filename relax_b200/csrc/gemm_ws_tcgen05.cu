@@ -78,7 +78,7 @@ struct WsParams {
   CUtensorMap tm_x;    // fp16   {64, M, K/64},    box {64, NB, SKB},  SWIZZLE_128B: [K block][batch row][128 B]
   CUtensorMap tm_w;    // uint32 {K/8, N},         box {32, 128},      SWIZZLE_128B: [row][128 B] (whole lines: 64-byte pieces
                        //                                                    halve the rate the weights arrive at)
-  CUtensorMap tm_s;    // fp16   {K/32, N},        box {8, 128}
+  CUtensorMap tm_s;    // fp16   {K/32, N},        box {8, 128}        (GU: rows as {N/2, 2}, boxes of 64 gate rows and their 64 up rows)
   const __half* scales;
   __half* y;
   int M, N, K;
@@ -87,7 +87,7 @@ struct WsParams {
   int x_resident;      // the x ring holds a whole slice: loaded once, kept for every tile
   int ksplit;          // CTAs per cluster = K slices
   int mt;              // token tiles of NB rows of x: tile t is row tile t / mt, token tile t % mt
-  int tiles;           // ceil(N / 128) * mt
+  int tiles;           // ceil(N / 128) * mt   (GU: ceil(N / 2 / 64) * mt)
   int cw;              // batch columns per owner: NB / ksplit, a multiple of 4
 };
 
@@ -150,7 +150,11 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const void* tmap, in
 // memory one trip ahead, and x comes one K block per load through a map that ends at K.  What lies past K is zero
 // on both sides (packed words, scales and x).  SKB: K blocks per x stage and A slot: 2 up to 128 batch
 // columns (fewer waits and arrivals), 1 above (tensor memory holds two accumulators of 192 columns and four slots of 32).
-template <bool PAIRED, int SKB, bool RAGGED>
+// GU: W's rows are [gate: N / 2 | up: N / 2]; a tile takes 64 of each and silu(gate) * up is stored, [M, N / 2], formed as the
+// separate kernel does from the fp16-rounded sums.  The two rows of a product are 64 apart in tensor memory, out of each other's warp's
+// reach, so the sums travel through the inbox with one slice too.  A layer's step without the launch for SwiGLU and without the trip
+// of gate | up to memory: 64 rows of hidden 1024 33.2 -> @GU1@ us, 16 of 2560 41.8 -> @GU2@, 16 of 4096 at 2012 133.1 -> @GU3@.
+template <bool PAIRED, int SKB, bool RAGGED, bool GU>
 __global__ void __launch_bounds__(kNumThreads, 1)
 q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
   extern __shared__ unsigned char smem_unaligned[];
@@ -161,7 +165,8 @@ q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
   unsigned char* raw_ring = x_ring + (size_t)p.SX * xstage;
   unsigned char* sc_ring = raw_ring + (size_t)p.SR * kRawBytes;
   float* inbox = reinterpret_cast<float*>(sc_ring + (size_t)p.SR * kScBytes);
-  Bars& bar = *reinterpret_cast<Bars*>(inbox + (p.ksplit > 1 ? (size_t)BR * p.NB : 0));
+  const bool exchange = GU || p.ksplit > 1;
+  Bars& bar = *reinterpret_cast<Bars*>(inbox + (exchange ? (size_t)BR * p.NB : 0));
   volatile int* abort_flag = &bar.abort_flag;
   cg::cluster_group cluster = cg::this_cluster();
 
@@ -177,6 +182,10 @@ q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
   const int nspans = ubase + (krank < uextra ? 1 : 0);
   const int nunits = 4 / SKB * nspans;                  // x stages = A slots of a tile
 
+  auto load_rows = [](void* dst, const void* map, int col, int row_tile, uint64_t* full) {
+    if (GU) tma_load_3d(dst, map, col, row_tile * (BR / 2), 0, full);
+    else tma_load_2d(dst, map, col, row_tile * BR, full);
+  };
   if (tid == 0) {
     bar.abort_flag = 0;
     for (int i = 0; i < p.SX; ++i) { mbar_init(&bar.x_full[i], 1); mbar_init(&bar.x_empty[i], 1); }
@@ -193,10 +202,10 @@ q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
     mbar_fence_init();
     for (int i = 0; i < p.SR && i < nspans; ++i) {
       mbar_arrive_expect_tx(&bar.r_full[i], kRawBytes);
-      tma_load_2d(raw_ring + (size_t)i * kRawBytes, &p.tm_w, (span0 + i) * 32, tile0 / p.mt * BR, &bar.r_full[i]);
+      load_rows(raw_ring + (size_t)i * kRawBytes, &p.tm_w, (span0 + i) * 32, tile0 / p.mt, &bar.r_full[i]);
       if (!RAGGED) {
         mbar_arrive_expect_tx(&bar.r_full[i], kScBytes);
-        tma_load_2d(sc_ring + (size_t)i * kScBytes, &p.tm_s, (span0 + i) * 8, tile0 / p.mt * BR, &bar.r_full[i]);
+        load_rows(sc_ring + (size_t)i * kScBytes, &p.tm_s, (span0 + i) * 8, tile0 / p.mt, &bar.r_full[i]);
       }
     }
   }
@@ -241,17 +250,17 @@ q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
       const int first = min(p.SR, nspans);            // requested during set-up
       Ring rr;
       for (int tile = tile0; tile < p.tiles; tile += tstep) {
-        const int row0 = tile / p.mt * BR;
+        const int row_tile = tile / p.mt;
         for (int sp = 0; sp < nspans; ++sp, rr.next(p.SR)) {
           if (tile == tile0 && sp < first) continue;
           const int s = rr.s;
           if (rr.wrapped) wait_or_abort(&bar.r_empty[s], rr.phase ^ 1, abort_flag, 3);
           if (warp == 2) {
             mbar_arrive_expect_tx(&bar.r_full[s], kRawBytes);
-            tma_load_2d(raw_ring + (size_t)s * kRawBytes, &p.tm_w, (span0 + sp) * 32, row0, &bar.r_full[s]);
+            load_rows(raw_ring + (size_t)s * kRawBytes, &p.tm_w, (span0 + sp) * 32, row_tile, &bar.r_full[s]);
           } else {
             mbar_arrive_expect_tx(&bar.r_full[s], kScBytes);
-            tma_load_2d(sc_ring + (size_t)s * kScBytes, &p.tm_s, (span0 + sp) * 8, row0, &bar.r_full[s]);
+            load_rows(sc_ring + (size_t)s * kScBytes, &p.tm_s, (span0 + sp) * 8, row_tile, &bar.r_full[s]);
           }
         }
       }
@@ -322,7 +331,12 @@ q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
     uint32_t phase = 0, use = 0;
     const int groups = p.K >> 5;
     auto global_scales = [&](uint32_t i, uint32_t (&out)[SKB]) {       // of the span with running index i
-      const int row = (tile0 + (int)(i / (uint32_t)nspans) * tstep) / p.mt * BR + r;
+      const int row_tile = (tile0 + (int)(i / (uint32_t)nspans) * tstep) / p.mt;
+      int row = row_tile * BR + r;
+      if (GU) {
+        row = row_tile * (BR / 2) + (r & 63);
+        row = row < p.N / 2 ? row + (r >> 6) * (p.N / 2) : p.N;
+      }
       const int g0 = (span0 + (int)(i % (uint32_t)nspans)) * 8 + 2 * SKB * part;
       const __half* src = p.scales + (int64_t)row * groups + g0;
 #pragma unroll
@@ -390,12 +404,13 @@ q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
     uint32_t it = 0, inbox_phase = 0;
     for (int tile = tile0; tile < p.tiles; tile += tstep, ++it) {
       const uint32_t buf = it & 1;
-      const int row = tile / p.mt * BR + r;
+      const int row = GU ? tile / p.mt * (BR / 2) + (r & 63) : tile / p.mt * BR + r;
+      const int out_rows = GU ? p.N / 2 : p.N;           // pitch of y
       const int tok0 = tile % p.mt * p.NB;
       const int ntok = min(p.NB, p.M - tok0);          // tokens of this tile
       const int ntok4 = (ntok + 3) & ~3;               // columns that are exchanged
       const int own = max(0, min(p.cw, ntok4 - krank * p.cw));     // columns that this CTA adds up and stores
-      __half* yt = p.y + (int64_t)tok0 * p.N + row;
+      __half* yt = p.y + (int64_t)tok0 * out_rows + row;
       // The owners have read what this CTA sent for the tile before.  This CTA is an owner itself: the two warps of a
       // quadrant send and sum different columns of the same rows, so without its own eight warps among the arrivals
       // the faster of the two could overwrite what the slower one has yet to add up.
@@ -405,12 +420,13 @@ q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
       if (p.ksplit > 1 && own > 0 && warp == 4 && lane == 0) mbar_arrive_expect_tx(&bar.inbox_full, (uint32_t)(p.ksplit * BR * own * 4));
       wait_or_abort(&bar.acc_full[buf], (it >> 1) & 1, abort_flag, 7);
       tc_fence_after_sync();
+      if (GU && p.ksplit == 1 && it > 0) bar_sync(2, 256);     // (the tile before has been read)
       const uint32_t taddr = tmem_base + ((uint32_t)(ew * 32) << 16) + buf * kAccPitch;
       for (int c0 = 16 * set; c0 < ntok; c0 += 32) {
         uint32_t v[16];
         tmem_ld_32x32b_x16(taddr + c0, v);
         tmem_ld_wait();
-        if (p.ksplit == 1) {
+        if (!exchange) {
           if (row < p.N) {
             __half* dst_y = yt + (int64_t)c0 * p.N;
             if (c0 + 16 <= ntok) {
@@ -422,6 +438,10 @@ q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
                 if (c0 + q < ntok) *dst_y = __float2half_rn(__uint_as_float(v[q]));
             }
           }
+        } else if (GU && p.ksplit == 1) {
+#pragma unroll
+          for (int q = 0; q < 16; q += 4)                      // (columns past the tokens too: there is room for NB)
+            *reinterpret_cast<uint4*>(inbox + (c0 + q) * BR + r * 4) = make_uint4(v[q], v[q + 1], v[q + 2], v[q + 3]);
         } else {
 #pragma unroll
           for (int q = 0; q < 16; q += 4) {
@@ -436,13 +456,22 @@ q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(&bar.acc_empty[buf]);
-      if (p.ksplit == 1) continue;
+      if (!exchange) continue;
       // ---- this CTA's columns: sum over the K slices in rank order
-      if (own > 0) wait_or_abort_cluster(&bar.inbox_full, inbox_phase, abort_flag, 11);
+      if (GU && p.ksplit == 1) bar_sync(2, 256);
+      else if (own > 0) wait_or_abort_cluster(&bar.inbox_full, inbox_phase, abort_flag, 11);
       inbox_phase ^= (uint32_t)(own > 0);            // (a CTA without columns in a tile's last tokens sits that phase out)
-      for (int l = 4 * set; l < own; l += 8) {
-        const int col = krank * p.cw + l;
-        const float* src = inbox + l * BR + r * 4;
+      auto total = [&](int l, int rr) {                // of columns l .. l + 3, row rr of the tile
+        const float* src = inbox + l * BR + rr * 4;
+        if (GU) {                                     // (one sum after the other: registers)
+          float4 sum = *reinterpret_cast<const float4*>(src);
+#pragma unroll 1
+          for (int q = 1; q < p.ksplit; ++q) {
+            const float4 v = *reinterpret_cast<const float4*>(src + (size_t)q * p.cw * BR);
+            sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+          }
+          return sum;
+        }
         float4 v[8];
 #pragma unroll
         for (int q = 0; q < 8; ++q)
@@ -451,17 +480,33 @@ q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
 #pragma unroll
         for (int q = 1; q < 8; ++q)
           if (q < p.ksplit) { sum.x += v[q].x; sum.y += v[q].y; sum.z += v[q].z; sum.w += v[q].w; }
-        if (row < p.N) {
-          __half* dst_y = yt + (int64_t)col * p.N;
+        return sum;
+      };
+      // GU: the four warps that hold rows of one half of the tile share the columns of both halves
+      const int first = GU ? 4 * (2 * set + (ew >> 1)) : 4 * set;
+      for (int l = first; l < own; l += GU ? 16 : 8) {
+        const int col = krank * p.cw + l;
+        float4 sum = total(l, GU ? r & 63 : r);
+        if (GU) {
+          const float4 up = total(l, (r & 63) + 64);
+          auto act = [](float g, float u) {
+            g = __half2float(__float2half_rn(g));
+            u = __half2float(__float2half_rn(u));
+            return g / (1.f + __expf(-g)) * u;
+          };
+          sum = make_float4(act(sum.x, up.x), act(sum.y, up.y), act(sum.z, up.z), act(sum.w, up.w));
+        }
+        if (row < out_rows) {
+          __half* dst_y = yt + (int64_t)col * out_rows;
           dst_y[0] = __float2half_rn(sum.x);
-          if (col + 1 < ntok) dst_y[p.N] = __float2half_rn(sum.y);
-          if (col + 2 < ntok) dst_y[2 * (int64_t)p.N] = __float2half_rn(sum.z);
-          if (col + 3 < ntok) dst_y[3 * (int64_t)p.N] = __float2half_rn(sum.w);
+          if (col + 1 < ntok) dst_y[out_rows] = __float2half_rn(sum.y);
+          if (col + 2 < ntok) dst_y[2 * (int64_t)out_rows] = __float2half_rn(sum.z);
+          if (col + 3 < ntok) dst_y[3 * (int64_t)out_rows] = __float2half_rn(sum.w);
         }
       }
       // Not after the last tile: the arrival's release would wait for the stores to y.
       __syncwarp();
-      if (tile + tstep < p.tiles && lane < p.ksplit) mbar_arrive_cluster(map_to_rank(free_addr, lane));
+      if (p.ksplit > 1 && tile + tstep < p.tiles && lane < p.ksplit) mbar_arrive_cluster(map_to_rank(free_addr, lane));
     }
   }
 
@@ -485,11 +530,12 @@ q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
 
 using WsKernel = void (*)(const WsParams);
 template <bool RAGGED>
-WsKernel kernel_of(int nb, bool paired) {
-  return nb <= 128 ? (paired ? q4f16_gemm_ws_tcgen05_kernel<true, 2, RAGGED> : q4f16_gemm_ws_tcgen05_kernel<false, 2, RAGGED>)
-                   : (paired ? q4f16_gemm_ws_tcgen05_kernel<true, 1, RAGGED> : q4f16_gemm_ws_tcgen05_kernel<false, 1, RAGGED>);
+WsKernel kernel_of(int nb, bool paired, bool gu) {
+  if (gu) return paired ? q4f16_gemm_ws_tcgen05_kernel<true, 2, RAGGED, true> : q4f16_gemm_ws_tcgen05_kernel<false, 2, RAGGED, true>;
+  return nb <= 128 ? (paired ? q4f16_gemm_ws_tcgen05_kernel<true, 2, RAGGED, false> : q4f16_gemm_ws_tcgen05_kernel<false, 2, RAGGED, false>)
+                   : (paired ? q4f16_gemm_ws_tcgen05_kernel<true, 1, RAGGED, false> : q4f16_gemm_ws_tcgen05_kernel<false, 1, RAGGED, false>);
 }
-WsKernel kernel_for(int nb, bool paired, bool ragged) { return ragged ? kernel_of<true>(nb, paired) : kernel_of<false>(nb, paired); }
+WsKernel kernel_for(int nb, bool paired, bool ragged, bool gu) { return ragged ? kernel_of<true>(nb, paired, gu) : kernel_of<false>(nb, paired, gu); }
 
 constexpr size_t kSmemCap = 227 * 1024;
 // More than half of an SM: one such CTA per SM, whatever its rings would need.  (It takes all of tensor memory; two
@@ -527,9 +573,11 @@ int max_clusters(int ksplit, const void* kern) {
 
 }  // namespace
 
-// Returns B200_ENOTREADY when the shape is outside what this kernel takes, or one for the prefill kernel.
+// Returns B200_ENOTREADY when the shape is outside what this kernel takes, or one for the prefill kernel.  gate_up: SwiGLU in the
+// epilogue (up to 128 rows, N even).
 int launch_gemm_ws(const __half* x, const uint32_t* wq, const __half* scales, __half* y, int64_t M, int64_t N,
-                   int64_t K, cudaStream_t stream) {
+                   int64_t K, cudaStream_t stream, bool gate_up) {
+  if (gate_up && (M > 128 || N % 2 != 0)) return B200_ENOTREADY;
   if (M < 1 || K < 32 || K % 32 != 0) return B200_ENOTREADY;
   const bool ragged = K % 256 != 0 || (reinterpret_cast<uintptr_t>(scales) & 15u) != 0;
   WsParams p;
@@ -539,15 +587,15 @@ int launch_gemm_ws(const __half* x, const uint32_t* wq, const __half* scales, __
   p.y = y;
   p.M = (int)M; p.N = (int)N; p.K = (int)K;
   const int units = (int)((K + 255) / 256);
-  const int64_t row_tiles = (N + BR - 1) / BR;
+  const int64_t row_tiles = gate_up ? (N / 2 + BR / 2 - 1) / (BR / 2) : (N + BR - 1) / BR;
   if (row_tiles * ((M + 15) / 16) > 0x3fffffff) return B200_ENOTREADY;      // (tile numbers are 32-bit)
   int clusters_of[4];
-  for (int i = 0; i < 4; ++i) clusters_of[i] = max_clusters(1 << i, reinterpret_cast<const void*>(kernel_for(16, paired, ragged)));
+  for (int i = 0; i < 4; ++i) clusters_of[i] = max_clusters(1 << i, reinterpret_cast<const void*>(kernel_for(16, paired, ragged, false)));
   const WsSplit split = choose_ws_split(M, row_tiles, units, (int)options().gemm_ws_ksplit, clusters_of);
   if (options().gemm_ws_ksplit == 0 && prefill_kernel_is_ahead(M, N, K, split, row_tiles, clusters_of[0])) return B200_ENOTREADY;
   const int ksplit = split.ksplit, nb16 = split.nb;
   const int skb = nb16 <= 128 ? 2 : 1;
-  auto kern = kernel_for(nb16, paired, ragged);
+  auto kern = kernel_for(nb16, paired, ragged, gate_up);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemCap);
   if (e != cudaSuccess) return fail(B200_ELAUNCH, "gemm_ws: cudaFuncSetAttribute(%zu): %s", kSmemCap, cudaGetErrorString(e));
   // an owner's columns are exchanged four at a time
@@ -563,7 +611,7 @@ int launch_gemm_ws(const __half* x, const uint32_t* wq, const __half* scales, __
   // Shared memory: the inbox, four packed spans (72 KB in flight cover HBM's latency at one SM's share of its
   // rate), then x: the whole slice if it fits (it is then loaded once for all tiles), else up to six stages; what
   // is left goes to the packed ring.
-  const size_t inbox = ksplit > 1 ? (size_t)BR * p.NB * sizeof(float) : 0;
+  const size_t inbox = ksplit > 1 || gate_up ? (size_t)BR * p.NB * sizeof(float) : 0;
   const size_t xstage = (size_t)skb * p.NB * 128;
   const size_t span = kRawBytes + kScBytes;
   const size_t fixed = 1024 + inbox + sizeof(Bars) + 256;
@@ -599,17 +647,21 @@ int launch_gemm_ws(const __half* x, const uint32_t* wq, const __half* scales, __
     const uint32_t b[3] = {BK, (uint32_t)p.NB, (uint32_t)skb};
     if ((rc = make_tmap(&p.tm_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, x, d, s, b, CU_TENSOR_MAP_SWIZZLE_128B))) return rc;
   }
+  // rows of W and of the scales: {N}, or gate and up rows {N / 2, 2} with boxes of 64 of each
+  const int rank = gate_up ? 3 : 2;
+  const uint64_t rows = (uint64_t)(gate_up ? N / 2 : N);
+  const uint32_t box_rows = gate_up ? BR / 2 : BR;
   {
-    const uint64_t d[2] = {(uint64_t)(K / 8), (uint64_t)N};
-    const uint64_t s[1] = {(uint64_t)(K / 2)};
-    const uint32_t b[2] = {32, BR};
-    if ((rc = make_tmap(&p.tm_w, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, wq, d, s, b, CU_TENSOR_MAP_SWIZZLE_128B))) return rc;
+    const uint64_t d[3] = {(uint64_t)(K / 8), rows, 2};
+    const uint64_t s[2] = {(uint64_t)(K / 2), (uint64_t)(K / 2) * rows};
+    const uint32_t b[3] = {32, box_rows, 2};
+    if ((rc = make_tmap(&p.tm_w, CU_TENSOR_MAP_DATA_TYPE_UINT32, rank, wq, d, s, b, CU_TENSOR_MAP_SWIZZLE_128B))) return rc;
   }
   if (!ragged) {
-    const uint64_t d[2] = {(uint64_t)(K / 32), (uint64_t)N};
-    const uint64_t s[1] = {(uint64_t)(K / 32) * 2};
-    const uint32_t b[2] = {8, BR};
-    if ((rc = make_tmap(&p.tm_s, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, scales, d, s, b, CU_TENSOR_MAP_SWIZZLE_NONE))) return rc;
+    const uint64_t d[3] = {(uint64_t)(K / 32), rows, 2};
+    const uint64_t s[2] = {(uint64_t)(K / 32) * 2, (uint64_t)(K / 32) * 2 * rows};
+    const uint32_t b[3] = {8, box_rows, 2};
+    if ((rc = make_tmap(&p.tm_s, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, rank, scales, d, s, b, CU_TENSOR_MAP_SWIZZLE_NONE))) return rc;
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)ksplit, (unsigned)clusters);

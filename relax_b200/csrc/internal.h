@@ -77,7 +77,7 @@ int launch_gemv_pipe_allreduce(const __half* x, const uint32_t* wq, const __half
 // (protocol of B200PeerReduce).
 int launch_peer_allreduce(int64_t count, const B200PeerReduce* red, cudaStream_t stream);
 int launch_gemm_ws(const __half* x, const uint32_t* wq, const __half* scales, __half* y, int64_t M, int64_t N,
-                   int64_t K, cudaStream_t stream);
+                   int64_t K, cudaStream_t stream, bool gate_up = false);
 int launch_gemm(const __half* x, const uint32_t* wq, const __half* scales, __half* y, int64_t M, int64_t N,
                 int64_t K, cudaStream_t stream);
 

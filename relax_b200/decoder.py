@@ -267,6 +267,10 @@ class DecodeEngine:
         take that matmul through the kernel that has the epilogue (asked anew each time: options may change)."""
         return (self.fused and not self.chained) or bool(self.L.b200_q4f16_gemv_gate_up_applies(w["gu"][1].data_ptr(), self.batch, w["inter_local"], self.cfg.hidden))
 
+    def _gate_up_wide(self, w) -> bool:
+        """Whether the gate|up matmul goes to the kernel for more rows, which has SwiGLU in its epilogue too."""
+        return bool(self.L.b200_q4f16_gate_up_applies(w["gu"][1].data_ptr(), self.batch, w["inter_local"], self.cfg.hidden))
+
     def _in_skinny(self, w, n, k) -> bool:
         """Whether the chained forms, which the skinny kernel has, are the ones for this matmul (asked anew each time, as below)."""
         return bool(self.L.b200_q4f16_gemv_add_applies(w[1].data_ptr(), self.batch, n, k))
@@ -403,7 +407,9 @@ class DecodeEngine:
             self._check(L.b200_rmsnorm_early_release(self.x.data_ptr(), self.o.data_ptr(), w["norm2"].data_ptr(), self.h.data_ptr(),
                                                      B, H, cfg.eps, sp))
             rc = _lib.ENOTREADY
-            if self._gate_up_in_one(w):
+            if self._gate_up_wide(w):
+                rc = L.b200_q4f16_gate_up(self.h.data_ptr(), w["gu"][0].data_ptr(), w["gu"][1].data_ptr(), self.act.data_ptr(), B, il, H, sp)
+            elif self._gate_up_in_one(w):
                 rc = L.b200_q4f16_gemv_gate_up(self.h.data_ptr(), None, None, None, 0.0, w["gu"][0].data_ptr(),
                                                w["gu"][1].data_ptr(), self.act.data_ptr(), B, il, H, sp)
             if rc == _lib.ENOTREADY:
@@ -493,7 +499,7 @@ class DecodeEngine:
         peer_sums = 2 if self.peer is not None and self.batch > self.PEER_FUSED_MAX_ROWS else 0
         per_layer = 0
         for w in self.layers:
-            mlp = 2 if self.fused else 3 if self._gate_up_in_one(w) else 4        # (norm,) gate|up (, SwiGLU), down
+            mlp = 2 if self.fused else 3 if self._gate_up_in_one(w) or self._gate_up_wide(w) else 4        # (norm,) gate|up (, SwiGLU), down
             per_layer += (1 if self.fused else 2) + 2 + mlp + peer_sums           # (norm,) qkv, attention, o
         return 1 + per_layer + 1 + head + 2
 
