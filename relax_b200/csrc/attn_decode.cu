@@ -46,9 +46,6 @@ struct AttnParams {
   int early_release;                     // the next launch may begin in the first instruction
 };
 
-__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) {
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
 }
@@ -100,7 +97,7 @@ attn_decode_kernel(const AttnParams p) {
   const int h = blockIdx.y, b = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int half = lane >> 4, d0 = (lane & 15) * 8;
-  if (c > 1) cluster_arrive_relaxed();                   // (every CTA of the cluster runs before anything is stored in it)
+  if (c > 1) ptx::cluster_arrive_relaxed();                   // (every CTA of the cluster runs before anything is stored in it)
 
   // early_loads: the caller promises that the position and the cache entries older than the new token were complete before the
   // launch in front of this one began.  Without the promise nothing is read before the wait.
@@ -269,7 +266,7 @@ attn_decode_kernel(const AttnParams p) {
     return;
   }
   const int per = 128 / c;                                         // dims of an owner
-  cluster_wait();                                                  // (the one at the start)
+  ptx::cluster_wait();                                             // (the one at the start)
   if (d < 128) {
     const int owner = d / per;
     st_cluster_f32(ptx::map_to_rank(ptx::smem_u32(&in_acc[rank][d - owner * per]), owner), A);
@@ -278,8 +275,8 @@ attn_decode_kernel(const AttnParams p) {
       st_cluster_f32(ptx::map_to_rank(ptx::smem_u32(&in_l[rank]), d), L);
     }
   }
-  cluster_arrive();
-  cluster_wait();
+  ptx::cluster_arrive();
+  ptx::cluster_wait();
   if (d < per) {
     M = -INFINITY;
     for (int r = 0; r < c; ++r) M = fmaxf(M, in_m[r]);

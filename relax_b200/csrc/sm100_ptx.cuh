@@ -75,6 +75,11 @@ __device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t pa
       : "memory");
   return ok != 0;
 }
+// Barrier of all threads of the cluster in two halves.  The relaxed arrival orders no memory accesses: the releasing one waits
+// for every store of the thread, to global memory too, to be performed, which takes a microsecond or two.
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // 16 bytes into the shared memory of any CTA of the cluster; their arrival is counted on a barrier of that CTA (both
 // addresses from map_to_rank), so the sender needs no release fence.
 __device__ __forceinline__ void st_async_v4(uint32_t addr, uint32_t bar_addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
