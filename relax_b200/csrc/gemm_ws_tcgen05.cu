@@ -153,7 +153,8 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const void* tmap, in
 // GU: W's rows are [gate: N / 2 | up: N / 2]; a tile takes 64 of each and silu(gate) * up is stored, [M, N / 2], formed as the
 // separate kernel does from the fp16-rounded sums.  The two rows of a product are 64 apart in tensor memory, out of each other's warp's
 // reach, so the sums travel through the inbox with one slice too.  A layer's step without the launch for SwiGLU and without the trip
-// of gate | up to memory: 64 rows of hidden 1024 33.2 -> @GU1@ us, 16 of 2560 41.8 -> @GU2@, 16 of 4096 at 2012 133.1 -> @GU3@.
+// of gate | up to memory: 64 rows of hidden 1024 33.2 -> 32.6 us, 24 of 4096 at 401 89.8 -> 85.8, 16
+// of 4096 at 2012 133.0 -> 130.3, 16 of 2560 the same.
 template <bool PAIRED, int SKB, bool RAGGED, bool GU>
 __global__ void __launch_bounds__(kNumThreads, 1)
 q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
@@ -598,7 +599,7 @@ int launch_gemm_ws(const __half* x, const uint32_t* wq, const __half* scales, __
   if (row_tiles * ((M + 15) / 16) > 0x3fffffff) return B200_ENOTREADY;      // (tile numbers are 32-bit)
   int clusters_of[4];
   for (int i = 0; i < 4; ++i) clusters_of[i] = max_clusters(1 << i, reinterpret_cast<const void*>(kernel_for(16, paired, ragged, false)));
-  const WsSplit split = choose_ws_split(M, row_tiles, units, (int)options().gemm_ws_ksplit, clusters_of);
+  const WsSplit split = choose_ws_split(M, row_tiles, units, (int)options().gemm_ws_ksplit, clusters_of, kWsClusterCosts);
   if (options().gemm_ws_ksplit == 0 && prefill_kernel_is_ahead(M, N, K, split, row_tiles, clusters_of[0])) return B200_ENOTREADY;
   const int ksplit = split.ksplit, nb16 = split.nb;
   const int skb = nb16 <= 128 ? 2 : 1;

@@ -13,6 +13,16 @@ struct WsSplit {
   int tried;    // combinations looked at
 };
 
+// What a cluster of CTAs costs over single ones, ns: the start of one of two, four and eight CTAs, and the last exchange beside
+// its 35 ns a column.  The defaults were fitted to the kernel when the cluster barriers of its set-up and teardown waited for memory;
+// kWsClusterCosts is the kernel as it is (chosen / best of the slices 1.011 -> 1.005 on average over 140 shapes of 16 to 128 rows,
+// M x N x K, us: 16 x 2560 x 4096 6.6 -> 5.4, 64 x 2560 x 2560 7.0 -> 6.0, 40 x 12288 x 8192 21.5 -> 19.6, 129 x 1024 x 4096 7.8 -> 6.6).
+struct WsClusterCosts {
+  int64_t start[3] = {500, 2800, 3500};
+  int64_t tail = 1000;
+};
+constexpr WsClusterCosts kWsClusterCosts = {{500, 1000, 3500}, 600};
+
 // A model of the time in nanoseconds, fitted to measurements at N = 4096, 12288 and 22016,
 // K = 4096 and 11008 and batches of 16, 64 and 128, and at 129..2048 tokens.  A 256-k span takes a CTA 0.53-0.65 us (up
 // to 128 columns) or 0.9-0.95 us; with many CTAs at work, what they fetch from L2 at about 14 TB/s if that is more.
@@ -26,7 +36,8 @@ struct WsSplit {
 // M rows of x, row_tiles tiles of 128 weight rows, units spans of 256 k; forced: the largest power of two of slices up to
 // it (0 = by the model); clusters[i]: clusters of 2^i CTAs that run at once.  Every width of a token tile is looked at
 // once, so at most 12 x 4 combinations whatever M is.
-inline WsSplit choose_ws_split(int64_t M, int64_t row_tiles, int units, int forced, const int (&clusters)[4]) {
+inline WsSplit choose_ws_split(int64_t M, int64_t row_tiles, int units, int forced, const int (&clusters)[4],
+                               const WsClusterCosts& costs = {}) {
   WsSplit best = {0, 1, 0};
   int64_t best_cost = 0;
   const int64_t mt0 = (M + kWsMaxNB - 1) / kWsMaxNB;
@@ -46,8 +57,8 @@ inline WsSplit choose_ws_split(int64_t M, int64_t row_tiles, int units, int forc
       const int64_t tile = (int64_t)((units + c - 1) / c) * (span > l2 ? span : l2);   // a tile's MMAs
       const int64_t drain = c == 1 ? 300 + 12 * nb : 800 + 50 * nb;              // ... and what the next tile must hide
       const bool room = M <= 128 && c >= 4 && 2 * tiles <= clusters[i] + (c == 8 ? 2 : 0);
-      const int64_t tail = c == 1 ? drain : room ? 900 + 38 * nb : 1000 + 35 * nb;   // the last tile's drain
-      const int64_t start = room ? (c == 8 && tiles > 4 ? 1600 - 8 * nb : 0) : c == 1 ? 0 : c == 2 ? 500 : c == 4 ? 2800 : 3500;
+      const int64_t tail = c == 1 ? drain : room ? 900 + 38 * nb : costs.tail + 35 * nb;   // the last tile's drain
+      const int64_t start = room ? (c == 8 && tiles > 4 ? 1600 - 8 * nb : 0) : c == 1 ? 0 : costs.start[i - 1];
       const int64_t cost = start + tile + (rounds - 1) * (tile > drain ? tile : drain) + tail;
       ++best.tried;
       if (best_cost == 0 || cost < best_cost) { best_cost = cost; best.ksplit = c; best.nb = nb; }
