@@ -15,6 +15,7 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libb200_q4f16.so")
+TORCH_CALL = os.path.join(HERE, "_torch_call.so")          # CPython extension: torch tensors to the library's C ABI
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 
 SOURCES = ["capi.cu", "tmap.cu", "dequant.cu", "gemv.cu", "gemv_pipe.cu", "gemm_tcgen05.cu", "gemm_ws_tcgen05.cu", "decoder_ops.cu", "attn_decode.cu", "decode_layer.cu", "lm_head.cu"]
@@ -45,7 +46,41 @@ def _stale() -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def _torch_call_command() -> list:
+    import sysconfig
+
+    import torch
+
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(_nvcc())) if os.path.isabs(_nvcc()) else "/usr/local/cuda"
+    include = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+               sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
+    lib = os.path.join(root, "lib")
+    return ["/usr/bin/g++" if os.path.exists("/usr/bin/g++") else "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *[f"-I{d}" for d in include],
+            os.path.join(CSRC, "torch_call.cpp"), "-o", TORCH_CALL, f"-L{lib}", f"-Wl,-rpath,{lib}",
+            "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
+
+
+def _torch_call_stale() -> bool:
+    deps = [os.path.join(CSRC, "torch_call.cpp"), os.path.join(INCLUDE, "b200_q4f16.h"), os.path.abspath(__file__)]
+    return not os.path.exists(TORCH_CALL) or any(os.path.getmtime(d) > os.path.getmtime(TORCH_CALL) for d in deps)
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
+    extension = None
+    if force or _torch_call_stale():
+        extension = subprocess.Popen(_torch_call_command(), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    try:
+        return _build_library(force, verbose)
+    finally:
+        if extension is not None:
+            out, _ = extension.communicate()
+            if extension.returncode != 0:
+                raise RuntimeError("g++ failed for torch_call.cpp:\n" + out)
+
+
+def _build_library(force: bool, verbose: bool) -> str:
     if not force and not _stale():
         return LIB
     objs = []

@@ -604,8 +604,9 @@ int launch_gemm_ws(const __half* x, const uint32_t* wq, const __half* scales, __
   const int ksplit = split.ksplit, nb16 = split.nb;
   const int skb = nb16 <= 128 ? 2 : 1;
   auto kern = kernel_for(nb16, paired, ragged, gate_up);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemCap);
-  if (e != cudaSuccess) return fail(B200_ELAUNCH, "gemm_ws: cudaFuncSetAttribute(%zu): %s", kSmemCap, cudaGetErrorString(e));
+  static SmemLimit limits[12];                           // (one per kernel variant)
+  if ((rc = raise_smem_limit(limits[(gate_up ? 2 : nb16 <= 128) * 4 + ragged * 2 + paired], reinterpret_cast<const void*>(kern), kSmemCap, "gemm_ws")))
+    return rc;
   // an owner's columns are exchanged four at a time
   if (ksplit == 8 || (ksplit > 1 && (nb16 / ksplit) % 4 != 0)) p.NB = (nb16 + 4 * ksplit - 1) / (4 * ksplit) * (4 * ksplit);
   else p.NB = nb16;
@@ -685,7 +686,7 @@ int launch_gemm_ws(const __half* x, const uint32_t* wq, const __half* scales, __
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = options().gemv_pdl ? 2 : 1;
-  e = cudaLaunchKernelEx(&cfg, kern, p);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, p);
   if (e != cudaSuccess) return fail(B200_ELAUNCH, "gemm_ws launch: %s", cudaGetErrorString(e));
   count_launch();
   return B200_OK;

@@ -1191,7 +1191,13 @@ int launch_pipe(const __half* x, const uint32_t* wq, const __half* scales, __hal
   auto kern = q4f16_gemv_pipe_kernel<NC, CW, CH, PRO, FAST, EPI>;
   // Ask for the largest shared-memory carve-out: the default picks the smallest that fits ONE CTA,
   // which would keep further CTAs (or the next dependent launch) off the SM.
-  cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+  // (Once per device: the attribute is the kernel's, and a call of the runtime on every launch is 0.3 us of the host's time.)
+  static SmemLimit carveout;
+  int dev = -1;
+  if (cudaGetDevice(&dev) == cudaSuccess)
+    carveout.raise(dev, 1, [&](size_t) {
+      return (int)cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    });
   auto fixed_bytes = [&](int stages) {
     return (size_t)1024 /* base alignment slack */ + (4 * kMaxStages + 2) * sizeof(uint64_t) + (size_t)stages * kStageBytes +
            (size_t)(stages + 1) * CW * kOut * sizeof(float);

@@ -139,6 +139,24 @@ def _dequantize_by_pointer(L, wq, scales, out) -> bool:
     return L.b200_q4f16_dequantize(wq.data_ptr(), scales.data_ptr(), out.data_ptr(), n, k, stream) == 0
 
 
+_native = None      # the extension module, bound to the loaded library; False: not built (the checks run in Python then)
+
+
+def _torch_call():
+    global _native
+    if _native is None:
+        try:
+            from . import _torch_call as module
+        except ImportError:
+            _native = False
+        else:
+            L = _lib.lib()
+            module.bind(*(ctypes.cast(fn, ctypes.c_void_p).value
+                          for fn in (L.b200_set_stream, L.b200_q4f16_matmul, L.b200_q4f16_matmul_layout, L.b200_q4f16_dequantize)))
+            _native = module
+    return _native
+
+
 def q4f16_matmul(x: torch.Tensor, wq: torch.Tensor, scales: torch.Tensor, out: torch.Tensor | None = None,
                  family: str = "auto", layout=None) -> torch.Tensor:
     """y[M,N] fp16 = x[M,K] . decode(wq[N,K/8], scales[N,K/32])^T, through the DLPack entry point
@@ -147,6 +165,10 @@ def q4f16_matmul(x: torch.Tensor, wq: torch.Tensor, scales: torch.Tensor, out: t
     of ``wq`` for this call; None takes the library's option "weights.layout"."""
     if out is None:
         out = torch.empty((x.shape[0], wq.shape[0]), dtype=torch.float16, device=x.device)
+    if family == "auto":
+        native = _native or _torch_call()
+        if native and native.matmul(x, wq, scales, out, -1 if layout is None else _layout_code(layout)):
+            return out
     L = _lib.lib()
     if family == "auto":
         if _matmul_by_pointer(L, x, wq, scales, out, layout):
@@ -202,6 +224,10 @@ def q4f16_dequantize(wq: torch.Tensor, scales: torch.Tensor, out: torch.Tensor |
     """w[N,K] fp16 = decode(wq, scales); bit-exact with the reference's decode stage."""
     if out is None:
         out = torch.empty((wq.shape[0], wq.shape[1] * 8), dtype=torch.float16, device=wq.device)
+    if layout is None:
+        native = _native or _torch_call()
+        if native and native.dequantize(wq, scales, out):
+            return out
     L = _lib.lib()
     if layout is not None:
         N, K = wq.shape[0], wq.shape[1] * 8
