@@ -220,17 +220,25 @@ using namespace b200;
 // Measured, a call among others in us with one CTA per 16 KB / one per 4 KB / the same up to eight: 1 x 4096 x 4096
 // 14.0 / 12.4 / 12.3, 3 x 8640 x 3200 22.6 / 20.3 / 20.4, 4 x 12288 x 4096 21.0 / 23.8 / 21.8, 6 x 4096 x 8192 20.6 / 22.4 / 20.5,
 // 16 x 4096 x 4096 24.7 / 22.1 / 20.6, 16 x 8192 x 8192 34.9 / 32.0 / 30.8; waited for, 8 x 4096 x 11008 33.6 / 34.9 / 30.6.
-// The copy lets the matmul start beside it (the matmul reads only weights before its own wait), and the result copy is
-// launched as a programmatic dependent of the matmul.  Pageable host memory and larger transfers use cudaMemcpyAsync.
+// The copies are launched as programmatic dependents.  A copy lets the next launch begin once it has waited itself: the matmul
+// then starts beside it (it reads only weights before its own wait), but not beside the call in front, whose matmul it
+// would take the SMs from.  Without the attribute on the copy of x / with it, us a call among others: 1 x 4096 x 4096 12.4 / 11.1,
+// 1 x 8192 x 8192 18.2 / 16.4, 4 x 22016 x 4096 28.0 / 25.9, 6 x 4096 x 4096 17.2 / 14.4, 16 x 4096 x 4096 19.2 / 18.3.
+// Up to kHostDirectRows rows the skinny matmul stores its result to the host buffer itself, next to y_dev, in pieces of 32 bytes (one
+// row) or 16: a launch less.  With more rows the small writes take the bus longer than a copy takes: copy / direct,
+// 1 x 4096 x 4096 11.1 / 10.4, 1 x 22016 x 4096 19.1 / 18.2, 2 x 16384 x 4096 19.9 / 19.3, 3 x 12288 x 4096 18.7 / 17.9, 4 x 22016 x 4096 25.9 / 25.5,
+// 6 x 4096 x 4096 14.4 / 14.4, 8 x 16384 x 4096 28.7 / 34.8 (both without the attribute); few outputs 1 x 1024 x 2048 8.3 / 9.3.
+// Pageable host memory and larger transfers use cudaMemcpyAsync.
 namespace b200 {
 namespace {
 constexpr size_t kHostKernelBytes = 256 * 1024;
 constexpr size_t kHostCopyCtas = 8;
+constexpr int64_t kHostDirectRows = 4, kHostDirectN = 4096;
 
 __global__ void __launch_bounds__(256) host_copy_kernel(const unsigned char* __restrict__ src, unsigned char* __restrict__ dst,
-                                                        size_t bytes, int wait_for_primary) {
+                                                        size_t bytes) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  if (wait_for_primary) asm volatile("griddepcontrol.wait;" ::: "memory");
   const size_t n16 = bytes >> 4;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n16; i += (size_t)gridDim.x * blockDim.x)
     reinterpret_cast<uint4*>(dst)[i] = reinterpret_cast<const uint4*>(src)[i];
@@ -249,9 +257,9 @@ void* mapped_host_pointer(const void* host) {
   return a.devicePointer;
 }
 
-// dst <- src (one of them a mapped host buffer) on `s`; dependent = launch as a programmatic dependent
-// of the kernel before it in the stream (the copy waits for that kernel's completion itself).
-int host_copy(const void* src, void* dst, size_t bytes, bool dependent, cudaStream_t s) {
+// dst <- src (one of them a mapped host buffer) on `s`, a programmatic dependent of the kernel before it in the stream (the copy
+// waits for that kernel's completion itself).
+int host_copy(const void* src, void* dst, size_t bytes, cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
   const size_t ctas = (bytes + 4095) / 4096;
   cfg.gridDim = dim3((unsigned)(ctas < kHostCopyCtas ? ctas : kHostCopyCtas));
@@ -261,9 +269,9 @@ int host_copy(const void* src, void* dst, size_t bytes, bool dependent, cudaStre
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = dependent ? 1 : 0;
+  cfg.numAttrs = 1;
   cudaError_t e = cudaLaunchKernelEx(&cfg, host_copy_kernel, static_cast<const unsigned char*>(src),
-                                     static_cast<unsigned char*>(dst), bytes, dependent ? 1 : 0);
+                                     static_cast<unsigned char*>(dst), bytes);
   if (e != cudaSuccess) return fail(B200_ELAUNCH, "q4f16_matmul_host: copy kernel: %s", cudaGetErrorString(e));
   count_launch();
   return B200_OK;
@@ -710,18 +718,24 @@ int b200_q4f16_matmul_host(const void* x_host, void* x_dev, const void* wq, cons
   if (xb > 0) {
     void* xm = xb <= kHostKernelBytes && !(reinterpret_cast<uintptr_t>(x_host) & 15) ? mapped_host_pointer(x_host) : nullptr;
     if (xm) {
-      if ((rc = host_copy(xm, x_dev, xb, false, s))) return rc;
+      if ((rc = host_copy(xm, x_dev, xb, s))) return rc;
     } else {
       e = cudaMemcpyAsync(x_dev, x_host, xb, cudaMemcpyHostToDevice, s);
       if (e != cudaSuccess) return fail(B200_ELAUNCH, "q4f16_matmul_host: H2D copy: %s", cudaGetErrorString(e));
     }
   }
+  void* ym = yb > 0 && yb <= kHostKernelBytes && !(reinterpret_cast<uintptr_t>(y_host) & 15) ? mapped_host_pointer(y_host) : nullptr;
+  if (ym && xb > 0 && M <= kHostDirectRows && N >= kHostDirectN && options().gemv_variant != 1 && K % 256 == 0 && aligned16(scales) &&
+      !weight_stationary_first(M, N, K, false)) {
+    rc = launch_gemv_pipe_twice(static_cast<const __half*>(x_dev), static_cast<const uint32_t*>(wq), static_cast<const __half*>(scales),
+                                static_cast<__half*>(y_dev), static_cast<__half*>(ym), M, N, K, s);
+    if (rc != B200_ENOTREADY) return rc;
+  }
   rc = matmul_impl(kAuto, "q4f16_matmul_host", x_dev, wq, scales, y_dev, M, N, K, stream);
   if (rc) return rc;
   if (yb > 0) {
-    void* ym = yb <= kHostKernelBytes && !(reinterpret_cast<uintptr_t>(y_host) & 15) ? mapped_host_pointer(y_host) : nullptr;
     if (ym) {
-      if ((rc = host_copy(y_dev, ym, yb, true, s))) return rc;
+      if ((rc = host_copy(y_dev, ym, yb, s))) return rc;
     } else {
       e = cudaMemcpyAsync(y_host, y_dev, yb, cudaMemcpyDeviceToHost, s);
       if (e != cudaSuccess) return fail(B200_ELAUNCH, "q4f16_matmul_host: D2H copy: %s", cudaGetErrorString(e));

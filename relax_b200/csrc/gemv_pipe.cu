@@ -82,7 +82,8 @@ enum { kPrologueNone = 0, kPrologueRmsNorm = 1, kPrologueSwiGLU = 2, kPrologueNo
 // silu(gate) * up is stored, [M, N / 2].  kEpilogueAdd: y += the product (y is the residual stream), and the sum of squares of the
 // new values goes to stats_out[row of x][tile] for the norm that comes next.  Forms of their own: as a run-time flag the first
 // cost the plain batch-1 matmul 2.9 % (182.5 -> 187.8 us for 40 of N = K = 4096).
-enum { kEpilogueStore = 0, kEpilogueGateUp = 1, kEpilogueAdd = 2 };
+// kEpilogueStoreTwice: y goes to a second place too, a host buffer mapped into the device's address space.
+enum { kEpilogueStore = 0, kEpilogueGateUp = 1, kEpilogueAdd = 2, kEpilogueStoreTwice = 3 };
 
 // Rotary embedding + KV append in the epilogue of the qkv matmul (batch 1, fast form).  The weight rows are then
 // fetched through a 5-D tensor map whose 16-row tile is dims d0..d0+7 of one 128-wide head AND their rotate-half
@@ -115,6 +116,7 @@ struct PipeParams {
   const __half* norm_w;      // RmsNorm: weight [K]
   __half* x_out;             // RmsNorm: fp16(x + delta) is written here by CTA 0 (or null)
   float eps;
+  __half* y2;                // kEpilogueStoreTwice
   const float* stats_in;     // NormStats: [M][K / 16] partial sums of squares of x's rows
   float* stats_out;          // kEpilogueAdd: [M][ntiles]
   int paired;                // nibble order of the packed words: 0 reference, 1 paired (q4_common.cuh)
@@ -438,6 +440,7 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
               }
             } else if (row < p.N && col < p.M) {
               p.y[(int64_t)col * p.N + row] = __float2half_rn(sum);
+              if (EPI == kEpilogueStoreTwice) p.y2[(int64_t)col * p.N + row] = __float2half_rn(sum);
             }
           }
         }
@@ -1123,6 +1126,7 @@ struct Prologue {
   float eps = 0.f;
   const float* stats_in = nullptr;
   float* stats_out = nullptr;
+  __half* y2 = nullptr;
   RopeOut rope;          // rotary embedding + KV append in the epilogue (qkv matmul of a batch-1 step)
 };
 
@@ -1181,7 +1185,7 @@ int launch_pipe(const __half* x, const uint32_t* wq, const __half* scales, __hal
   p.x = x; p.y = y;
   p.M = M; p.N = N; p.K = K;
   p.delta = pro.delta; p.norm_w = pro.norm_w; p.x_out = pro.x_out; p.eps = pro.eps;
-  p.stats_in = pro.stats_in; p.stats_out = pro.stats_out;
+  p.stats_in = pro.stats_in; p.stats_out = pro.stats_out; p.y2 = pro.y2;
   p.red = red;
   p.paired = current_layout() == kLayoutPaired;
   p.ntiles = (N + kRows - 1) / kRows;
@@ -1369,7 +1373,7 @@ int launch_pipe_m(const __half* x, const uint32_t* wq, const __half* scales, __h
   if (m <= 8)
     return half_stages<8>(n, k) ? launch_pipe<8, CW, CW, PRO, false, EPI>(x, wq, scales, y, m, n, k, stream, pro, red)
                              : launch_pipe<8, 2 * CW, CH, PRO, false, EPI>(x, wq, scales, y, m, n, k, stream, pro, red);
-  if constexpr (PRO == kPrologueNormStats || EPI == kEpilogueAdd) return B200_ENOTREADY;
+  if constexpr (PRO == kPrologueNormStats || EPI == kEpilogueAdd || EPI == kEpilogueStoreTwice) return B200_ENOTREADY;
   else return launch_pipe<16, CW, CH, PRO, false, EPI>(x, wq, scales, y, m, n, k, stream, pro, red);
 }
 
@@ -1384,11 +1388,11 @@ int dispatch_pipe(const __half* x, const uint32_t* wq, const __half* scales, __h
                   cudaStream_t stream, const Prologue& pro, const PeerReduce& red) {
   if (K % 256 != 0 || (reinterpret_cast<uintptr_t>(scales) & 15u)) return B200_ENOTREADY;
   int m = (int)M, n = (int)N, k = (int)K;
-  if constexpr (EPI != kEpilogueAdd) {
+  if constexpr (EPI == kEpilogueStore || EPI == kEpilogueGateUp) {
     if (pro.kind == kPrologueRmsNorm) return dispatch_form<kPrologueRmsNorm, EPI>(x, wq, scales, y, m, n, k, stream, pro, red);
     if (pro.kind == kPrologueNormStats) return dispatch_form<kPrologueNormStats, EPI>(x, wq, scales, y, m, n, k, stream, pro, red);
   }
-  if constexpr (EPI != kEpilogueGateUp)
+  if constexpr (EPI == kEpilogueStore || EPI == kEpilogueAdd)
     if (pro.kind == kPrologueSwiGLU) return dispatch_form<kPrologueSwiGLU, EPI>(x, wq, scales, y, m, n, k, stream, pro, red);
   return dispatch_form<kPrologueNone, EPI>(x, wq, scales, y, m, n, k, stream, pro, red);
 }
@@ -1538,6 +1542,14 @@ int launch_gemv_pipe_gate_up(const __half* x, const __half* delta, const __half*
   }
   if (stats_in) { pro.kind = kPrologueNormStats; pro.stats_in = stats_in; }
   return dispatch_pipe<kEpilogueGateUp>(x, wq, scales, act, M, 2 * I, K, stream, pro, PeerReduce{});
+}
+
+// y = x . decode(W)^T, stored to y and to y2 (up to eight rows).
+int launch_gemv_pipe_twice(const __half* x, const uint32_t* wq, const __half* scales, __half* y, __half* y2, int64_t M, int64_t N,
+                           int64_t K, cudaStream_t stream) {
+  Prologue pro;
+  pro.y2 = y2;
+  return dispatch_pipe<kEpilogueStoreTwice>(x, wq, scales, y, M, N, K, stream, pro, PeerReduce{});
 }
 
 // y = (x * rsqrt(mean(x^2) + eps) * norm_w) . decode(W)^T with the statistics of stats_in (up to eight rows).
