@@ -161,6 +161,8 @@ B200_API int b200_lm_head(const void* h, const void* w, void* logits, int32_t* t
 B200_API int b200_lm_head_norm(const void* x, const void* stats, const void* norm_w, float eps, void* h_out, const void* w,
                                void* logits, int32_t* tokens, void* scratch, int64_t B, int64_t V, int64_t H, int64_t token_offset,
                                void* cuda_stream);
+/* tokens[b] = index of the largest of logits[b, 0..V), fp16: the lowest of equal ones; a NaN counts as the largest. */
+B200_API int b200_argmax_rows(const void* logits, int32_t* tokens, int64_t B, int64_t V, void* cuda_stream);
 
 /* ---- offline weight repack --------------------------------------------------------------
  * The reference binds weights into the executable as constants when it builds

@@ -105,6 +105,7 @@ PROTOTYPES = {
     "b200_lm_head_scratch_bytes": (_i64, []),
     "b200_lm_head": (_ci, [_vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _vp]),
     "b200_lm_head_norm": (_ci, [_vp, _vp, _vp, ctypes.c_float, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _vp]),
+    "b200_argmax_rows": (_ci, [_vp, _vp, _i64, _i64, _vp]),
     "b200_q4f16_repack": (_ci, [_vp, _vp, _i64, _i64, ctypes.c_int32, _vp]),
     "b200_q4f16_unpack": (_ci, [_vp, _vp, _i64, _i64, ctypes.c_int32, _vp]),
     "b200_q4f16_matmul_layout": (_ci, [_vp, _vp, _vp, _vp, _i64, _i64, _i64, ctypes.c_int32, _vp]),

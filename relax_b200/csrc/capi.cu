@@ -425,6 +425,15 @@ int b200_lm_head_norm(const void* x, const void* stats, const void* norm_w, floa
   return lm_head_impl(x, stats, norm_w, eps, h_out, w, logits, tokens, scratch, B, V, H, token_offset, stream);
 }
 
+int b200_argmax_rows(const void* logits, int32_t* tokens, int64_t B, int64_t V, void* stream) {
+  if (B < 0 || B > 0x7fffffffLL || V < 1 || V > 0x7ffffff0LL) return fail(B200_EINVAL, "argmax_rows: need B >= 0 and 1 <= V < 2^31");
+  if (B == 0) return B200_OK;
+  if (!logits || !tokens || (reinterpret_cast<uintptr_t>(logits) & 1u) || (reinterpret_cast<uintptr_t>(tokens) & 3u))
+    return fail(B200_EINVAL, "argmax_rows: null or misaligned pointer");
+  if (int rc = ensure_device()) return rc;
+  return launch_argmax_rows(static_cast<const __half*>(logits), tokens, B, V, static_cast<cudaStream_t>(stream));
+}
+
 int b200_q4f16_repack(const void* wq, void* packed_out, int64_t N, int64_t K, int32_t layout, void* stream) {
   return repack_impl("q4f16_repack", wq, packed_out, N, K, layout, true, stream);
 }

@@ -89,6 +89,7 @@ int launch_gemm(const __half* x, const uint32_t* wq, const __half* scales, __hal
 int launch_lm_head(const __half* x, const float* stats, const __half* norm_w, float eps, __half* h_out, const __half* w, __half* logits, int* tokens, float* scratch, int64_t B, int64_t V,
                    int64_t H, int64_t token_offset, cudaStream_t stream);
 int64_t lm_head_scratch_bytes();
+int launch_argmax_rows(const __half* logits, int* tokens, int64_t B, int64_t V, cudaStream_t stream);
 
 // Reads and clears the per-kernel device error words (bit 0-7: skinny pipeline, 8-15: tensor-core GEMM, 16-23: weight-stationary GEMM,
 // 24-30: decoder-layer kernel).

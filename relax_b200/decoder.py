@@ -3,8 +3,7 @@ matmul (RMSNorm, RoPE + KV cache, attention, SwiGLU) wired to the C-ABI kernels,
 tensor-parallel with one NCCL all-reduce after each row-parallel matmul.
 
 torch is used for device memory, streams, CUDA graphs and the NCCL process group; every kernel of a step is
-this library's for batches of up to 16 (above that the fp16 output projection is a plain library GEMM, and under
-tensor parallelism the sampling over the gathered vocabulary slices is torch's argmax).
+this library's for batches of up to 16 (above that the fp16 output projection is a plain library GEMM).
 
 Layout per rank (world size t, hidden H, heads nh, head dim 128, intermediate I):
 
@@ -473,16 +472,22 @@ class DecodeEngine:
                 torch.distributed.all_gather_into_tensor(self.gathered, self.logits_local, group=self.group)
                 self.logits.view(B, self.world, -1).copy_(self.gathered.permute(1, 0, 2))
             if not own or self.world > 1:
-                self.tokens.copy_(torch.argmax(self.logits, dim=1).to(torch.int32))
+                self._check(L.b200_argmax_rows(self.logits.data_ptr(), self.tokens.data_ptr(), B, self.logits.shape[1], sp))
         self._check(L.b200_advance_pos(self.pos.data_ptr(), 1, sp))
-        self._check(L.b200_advance_pos(self.epoch.data_ptr(), 1, sp))
+        if self._counts_steps():
+            self._check(L.b200_advance_pos(self.epoch.data_ptr(), 1, sp))
+
+    def _counts_steps(self) -> bool:
+        """Whether something in a step reads the step counter (flags of the sums over ranks, arrival counters of the layer kernel)."""
+        return self.peer is not None or self.layer_kernel
 
     def kernels_per_step(self) -> int:
         """Kernels of this library launched by one step: embed, 5 to 10 per layer, final norm, output projection for up to
-        16 rows, two counters."""
-        head = 1 if self.lm_head is not None and self.batch <= 16 else 0
+        16 rows, sampling where it is not part of that, one or two counters."""
+        head = int(self.lm_head is not None and self.batch <= 16)
+        tail = 1 + int(self._counts_steps()) + int(self.lm_head is not None and (self.batch > 16 or self.world > 1))
         if self.layer_kernel:
-            return 1 + len(self.layers) + 1 + head + 2
+            return 1 + len(self.layers) + 1 + head + tail
         if self.chained:
             ready, norms = True, 0          # the residual stream has its statistics; norms as launches of their own
             per_layer = 0
@@ -495,13 +500,13 @@ class DecodeEngine:
                 norms += not (ready and one)
                 ready = self._in_skinny(w["down"], self.cfg.hidden, w["inter_local"])
                 per_layer += 0 if one or ready else 1          # (SwiGLU as a launch of its own)
-            return 1 + per_layer + norms + (0 if ready and head else 1) + head + 2
+            return 1 + per_layer + norms + (0 if ready and head else 1) + head + tail
         peer_sums = 2 if self.peer is not None and self.batch > self.PEER_FUSED_MAX_ROWS else 0
         per_layer = 0
         for w in self.layers:
             mlp = 2 if self.fused else 3 if self._gate_up_in_one(w) or self._gate_up_wide(w) else 4        # (norm,) gate|up (, SwiGLU), down
             per_layer += (1 if self.fused else 2) + 2 + mlp + peer_sums           # (norm,) qkv, attention, o
-        return 1 + per_layer + 1 + head + 2
+        return 1 + per_layer + 1 + head + tail
 
     def capture(self, stream):
         """Captures one step into a CUDA graph on `stream` (after one eager warm-up step, which

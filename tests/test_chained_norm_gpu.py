@@ -131,6 +131,21 @@ def test_embed_rows_stats(cuda_lib):
     np.testing.assert_allclose(stats.sum(dim=1).cpu().numpy(), (table[[0, 39, 7]].astype(np.float64) ** 2).sum(axis=1), rtol=1e-5)
 
 
+@pytest.mark.parametrize("B,V", [(1, 1), (3, 7), (17, 8), (2, 1000), (64, 32000), (5, 8191), (20, 8200)])
+def test_argmax_rows(cuda_lib, B, V):
+    rng = np.random.default_rng(V)
+    a = rng.integers(-50, 50, (B, V)).astype(np.float16)               # many ties
+    a[0, V // 2:] = np.inf
+    if B > 2:
+        a[1, V - 1] = np.nan
+        a[2] = -np.inf
+    t, toks = _t(a), torch.full((B,), -7, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    assert cuda_lib.b200_argmax_rows(t.data_ptr(), toks.data_ptr(), B, V, 0) == 0, _lib.last_error()
+    torch.cuda.synchronize()
+    assert (toks.cpu().numpy() == a.argmax(axis=1)).all()              # (numpy: the first of equal ones, the first NaN)
+
+
 def test_refusals(cuda_lib):
     t = torch.zeros(1 << 16, dtype=torch.float16, device="cuda")
     p, q = t.data_ptr(), t.data_ptr() + 65536
@@ -144,6 +159,7 @@ def test_refusals(cuda_lib):
     assert L.b200_q4f16_gemv_norm(p, p, p, EPS, p, p, q, 1, 64, 288, 0) == _lib.EINVAL
     assert L.b200_q4f16_gemv_norm_gate_up(p, p, p, EPS, p, p, q, 1, 12, 256, 0) == _lib.EINVAL
     assert L.b200_lm_head_norm(p, p, p, EPS, None, p, q, None, None, 9, 64, 256, 0, 0) == _lib.EINVAL
+    assert L.b200_argmax_rows(p, None, 1, 8, 0) == _lib.EINVAL and L.b200_argmax_rows(p, p, 1, 0, 0) == _lib.EINVAL
     assert L.b200_embed_rows_stats(p, p, q, None, 1, 64, 4, 0) == _lib.EINVAL
     assert L.b200_q4f16_gemv_add_applies(p, 9, 64, 256) == 0 and L.b200_q4f16_gemv_add_applies(p, 1, 64, 288) == 0
     assert L.b200_q4f16_gemv_add_applies(p, 8, 4096, 8192) == 0 and L.b200_q4f16_gemv_add_applies(p, 8, 4096, 4096) == 1
