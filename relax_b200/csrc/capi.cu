@@ -141,6 +141,16 @@ bool weight_stationary_first(int64_t M, int64_t N, int64_t K, bool ragged) {
   return ahead && M <= options().gemm_ws_max_m && (M > 16 || options().gemv_variant == 0);
 }
 
+// Of that, the skinny kernel's form for a ragged K takes two to four rows of the weight-stationary kernel's share and up to eight of the
+// streaming kernel's where K is long enough for its start-up.  Weight-stationary / skinny in us: 2 x 8640 x 3200 11.0 / 7.4,
+// 3 x 8640 x 3200 9.7 / 7.6, 4 x 12288 x 1056 6.3 / 6.0, 4 x 5120 x 5152 11.1 / 9.6, 2 x 4096 x 9248 12.3 / 9.8, 4 x 4096 x 11040 13.2 / 13.3,
+// but 5 x 4096 x 4128 8.4 / 8.3, 8 x 22016 x 2080 13.8 / 15.3, 8 x 4096 x 7200 11.1 / 12.8, 6 x 2560 x 6944 8.3 / 11.2; streaming / skinny:
+// 3 x 2048 x 5152 9.5 / 5.1, 8 x 512 x 2080 4.9 / 3.8, 4 x 4096 x 2080 5.1 / 4.9, but 2 x 4096 x 1056 3.1 / 3.4, 8 x 4096 x 1056 4.4 / 4.5.
+bool skinny_ragged(int64_t M, int64_t N, int64_t K) {
+  if (M < 2 || M > 8 || options().gemv_variant != 0) return false;
+  return weight_stationary_first(M, N, K, true) ? M <= 4 : K >= 2048;
+}
+
 int matmul_impl(Family fam, const char* who, const void* x, const void* wq, const void* scales, void* y, int64_t M,
                 int64_t N, int64_t K, void* stream) {
   int rc = check_matmul(who, x, wq, scales, y, M, N, K);
@@ -158,6 +168,10 @@ int matmul_impl(Family fam, const char* who, const void* x, const void* wq, cons
   auto sh = static_cast<const __half*>(scales);
   auto yh = static_cast<__half*>(y);
   const bool ragged = K % 256 != 0 || !aligned16(scales);
+  if (fam == kAuto && ragged && skinny_ragged(M, N, K)) {
+    rc = launch_gemv_pipe_ragged(xh, wh, sh, yh, M, N, K, s);
+    if (rc != B200_ENOTREADY) return rc;
+  }
   if (fam == kGemmWs || (fam == kAuto && weight_stationary_first(M, N, K, ragged))) {
     rc = fam == kGemmWs && (M > 128 || ragged) ? B200_ENOTREADY : launch_gemm_ws(xh, wh, sh, yh, M, N, K, s);
     if (rc != B200_ENOTREADY) return rc;

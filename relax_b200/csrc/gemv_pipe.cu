@@ -77,7 +77,10 @@ constexpr uint64_t kProducerWaitNs = 30000000000ull;    // 30 s: may span the pr
 
 // What happens to x on its way into shared memory.  kPrologueNormStats: RMSNorm whose statistics the kernel that produced x has
 // left behind (kEpilogueAdd): no pass over the row, no residual add.
-enum { kPrologueNone = 0, kPrologueRmsNorm = 1, kPrologueSwiGLU = 2, kPrologueNormStats = 3 };
+// kPrologueRagged: x as it is, but K a multiple of 32 only (or scales off 16 bytes), which a row of scales in a tensor map cannot be.
+// The packed words come chunk by chunk through a 2-D map that ends at K, and every lane fetches its scales from global memory a stage
+// ahead.  What lies past K in the last chunk has a zero scale and a zero x.
+enum { kPrologueNone = 0, kPrologueRmsNorm = 1, kPrologueSwiGLU = 2, kPrologueNormStats = 3, kPrologueRagged = 4 };
 // What happens to a finished tile.  kEpilogueGateUp: W's rows are [gate: N / 2 | up: N / 2]; a tile takes eight of each and
 // silu(gate) * up is stored, [M, N / 2].  kEpilogueAdd: y += the product (y is the residual stream), and the sum of squares of the
 // new values goes to stats_out[row of x][tile] for the norm that comes next.  Forms of their own: as a run-time flag the first
@@ -117,6 +120,7 @@ struct PipeParams {
   __half* x_out;             // RmsNorm: fp16(x + delta) is written here by CTA 0 (or null)
   float eps;
   __half* y2;                // kEpilogueStoreTwice
+  const __half* scales;      // Ragged
   const float* stats_in;     // NormStats: [M][K / 16] partial sums of squares of x's rows
   float* stats_out;          // kEpilogueAdd: [M][ntiles]
   int paired;                // nibble order of the packed words: 0 reference, 1 paired (q4_common.cuh)
@@ -214,6 +218,7 @@ __global__ void __launch_bounds__((CW + 2) * 32, FAST || (CH == CW && CW == 8) ?
 q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
   constexpr int MT = (NC + 7) / 8;
   constexpr bool GU = EPI == kEpilogueGateUp, ADD = EPI == kEpilogueAdd;
+  constexpr bool RAG = PRO == kPrologueRagged;
   static_assert(!FAST || NC == 1, "the fast form is the batch-1 kernel");
   static_assert(MT == 1 || (!ADD && PRO != kPrologueNormStats), "up to eight rows");
   // outputs per row tile as one consumer warp leaves them: the exact form stores whole MMA fragments,
@@ -254,7 +259,7 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
     s_abort = 0;
     s_zero = make_uint4(0, 0, 0, 0);
     for (int s = 0; s < p.nstages; ++s) {
-      mbar_init(&full[s], 2);
+      mbar_init(&full[s], RAG ? 1 : 2);
       mbar_init(&empty[s], CW);
     }
     for (int s = 0; s < nred; ++s) {
@@ -271,7 +276,7 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
     // lane 0 loads the packed weights, lane 1 the scales: one tiled load per stage each (the two
     // lanes run as independent threads; one thread issuing both would halve the issue rate).
     const bool is_w = lane == 0;
-    if (lane < 2) {
+    if (lane < (RAG ? 1 : 2)) {
       prefetch_tmap(is_w ? &p.tm_w : &p.tm_s);
       const uint64_t policy = policy_evict_first();
       int s = 0;
@@ -309,6 +314,11 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
               // tile = 8 gate rows and the 8 up rows that they are multiplied with
               mbar_arrive_expect_tx(&full[s], is_w ? kWBytes : kSBytes);
               tma_load_4d_hint(is_w ? st : st + kWBytes, is_w ? &p.tm_w : &p.tm_s, 0, tile * 8, 0, k0 >> 8, &full[s], policy);
+            } else if (RAG) {
+              const int n = min(CH, (k_hi - k0 + 255) >> 8);
+              mbar_arrive_expect_tx(&full[s], (uint32_t)n * (kRows * 128));
+              for (int c = 0; c < n; ++c)
+                tma_load_2d_hint(st + c * (kRows * 128), &p.tm_w, ((k0 >> 8) + c) * 32, row0, &full[s], policy);
             } else if (is_w) {
               mbar_arrive_expect_tx(&full[s], kWBytes);
               tma_load_3d_hint(st, &p.tm_w, 0, row0, k0 >> 8, &full[s], policy);
@@ -630,7 +640,7 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
   // rows of x, kItems of them in flight.  Dealt out over all threads of the CTA, eight columns whatever M is and a barrier
   // behind, a launch took, us, before / now: M x N x K 5 x 2048 x 5632 7.1 / 5.5, 8 x 1024 x 3072 5.3 / 4.3, 8 x 4096 x 4096 7.8 / 6.6,
   // 8 x 22016 x 4096 17.5 / 16.5, 4 x 4096 x 4096 6.0 / 5.5; up to two columns it is the faster way (2 x 4096 x 4096 5.1 / 5.3).
-  constexpr int kItems = PRO == kPrologueNone || PRO == kPrologueNormStats ? 8 : 4;
+  constexpr int kItems = PRO == kPrologueNone || PRO == kPrologueNormStats || RAG ? 8 : 4;
   auto next_item = [&](int& c, int& m) {
     if (++m == p.M) {
       m = 0;
@@ -643,7 +653,8 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
       a[r] = b[r] = w[r] = make_uint4(0, 0, 0, 0);
       if (c < nch) {
         const int k = k_lo + c * 256 + lane * 8;
-        if (PRO == kPrologueSwiGLU) {               // x is [M, 2K] = gate | up
+        if (RAG && k >= p.K) {                      // (past the end of the last chunk: zeros)
+        } else if (PRO == kPrologueSwiGLU) {        // x is [M, 2K] = gate | up
           a[r] = *reinterpret_cast<const uint4*>(p.x + (int64_t)m * 2 * p.K + k);
           b[r] = *reinterpret_cast<const uint4*>(p.x + (int64_t)m * 2 * p.K + p.K + k);
         } else {
@@ -666,6 +677,25 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
   uint4 fw[U][2][2];
   uint2 fsc[U][2];
   if (FAST) fast_load(0, 0, fw, fsc);
+  // Ragged: the scales (groups 2t, 2t+1 of rows g and g+8) of this warp's chunks of the stage at `k0` of `tile`; zero past the ends
+  uint32_t next_sc[U][2];
+  auto ragged_scales = [&](int tile, int k0) {
+    const int groups = p.K >> 5;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int grp = ((k0 >> 8) + warp + u * CW) * 8 + 2 * t;
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const int row = tile * kRows + g + 8 * r;
+        const __half* src = p.scales + (int64_t)row * groups + grp;
+        uint32_t lo = 0, hi = 0;
+        if (row < p.N && grp < groups) lo = __half_as_ushort(__ldg(src));
+        if (row < p.N && grp + 1 < groups) hi = __half_as_ushort(__ldg(src + 1));
+        next_sc[u][r] = lo | (hi << 16);
+      }
+    }
+  };
+  if (RAG) ragged_scales(blockIdx.x, 0);
   // NormStats: the first norm weights are here when the wait returns: of this thread's first items, or of this warp's first
   // two chunks
   uint4 nw[2];
@@ -849,7 +879,7 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
     const int k_hi = min(p.K, k_lo + p.kblk);
     // ---- stage x[:, k_lo .. k_lo + kblk) permuted per 8 k --------------------------------------------------------
     if (XL::kOwnRows) {
-      const int nch = (k_hi - k_lo) >> 8;
+      const int nch = (k_hi - k_lo + 255) >> 8;
       if (kb > 0) __syncwarp();                  // all lanes are done reading the previous block
       if (PRO == kPrologueNormStats) load_stats();
 #pragma unroll 1
@@ -933,7 +963,7 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
       const int words = p.kblk >> 3;
       const int items = words * NC;              // a multiple of 32: a warp's 32 items are all inside or all outside
       // (registers: small batches keep two CTAs per SM; without a prologue only one array is live)
-      constexpr int R = PRO == kPrologueNone ? 4 : (NC == 1 ? 2 : 1);
+      constexpr int R = PRO == kPrologueNone || RAG ? 4 : (NC == 1 ? 2 : 1);
       for (int i0 = tid; i0 < items; i0 += kConsumers * R) {
         uint4 a[R], b[R], c[R];
         bool live[R];
@@ -1011,8 +1041,13 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
           w[u][1][0] = *reinterpret_cast<const uint4*>(su + w_off + 1024);
           w[u][1][1] = *reinterpret_cast<const uint4*>(su + (w_off ^ 16u) + 1024);
           const unsigned char* ss = st + u * (CW * kRows * 16);
-          sc[u][0] = *reinterpret_cast<const uint32_t*>(ss + s_off);
-          sc[u][1] = *reinterpret_cast<const uint32_t*>(ss + s_off + 128);
+          sc[u][0] = RAG ? next_sc[u][0] : *reinterpret_cast<const uint32_t*>(ss + s_off);
+          sc[u][1] = RAG ? next_sc[u][1] : *reinterpret_cast<const uint32_t*>(ss + s_off + 128);
+        }
+        if (RAG) {
+          // (one K block: checked by the launcher)
+          const bool same = k0 + KC < k_hi;
+          if (same || tile + (int)gridDim.x < p.ntiles) ragged_scales(same ? tile : tile + (int)gridDim.x, same ? k0 + KC : 0);
         }
         // the loads must have returned before the stage goes back to the producer
 #pragma unroll
@@ -1155,6 +1190,12 @@ int launch_pipe(const __half* x, const uint32_t* wq, const __half* scales, __hal
     const uint32_t sb[4] = {8, 8, 2, CH};
     rc = make_tmap(&p.tm_s, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, scales, sd, ss, sb, CU_TENSOR_MAP_SWIZZLE_NONE);
     if (rc) return rc;
+  } else if (PRO == kPrologueRagged) {
+    const uint64_t wd[2] = {(uint64_t)(K / 8), (uint64_t)N};
+    const uint64_t ws[1] = {(uint64_t)K / 2};
+    const uint32_t wb[2] = {32, kRows};
+    int rc = make_tmap(&p.tm_w, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, wq, wd, ws, wb, CU_TENSOR_MAP_SWIZZLE_128B);
+    if (rc) return rc;
   } else if (pro.rope.on) {
     // the fast form's epilogue layout, one K block, whole 128-row units
     if (!FAST || NC != 1 || M != 1 || N % 128 != 0 || N != 3 * pro.rope.nh * 128) return B200_ENOTREADY;
@@ -1185,7 +1226,7 @@ int launch_pipe(const __half* x, const uint32_t* wq, const __half* scales, __hal
   p.x = x; p.y = y;
   p.M = M; p.N = N; p.K = K;
   p.delta = pro.delta; p.norm_w = pro.norm_w; p.x_out = pro.x_out; p.eps = pro.eps;
-  p.stats_in = pro.stats_in; p.stats_out = pro.stats_out; p.y2 = pro.y2;
+  p.stats_in = pro.stats_in; p.stats_out = pro.stats_out; p.y2 = pro.y2; p.scales = scales;
   p.red = red;
   p.paired = current_layout() == kLayoutPaired;
   p.ntiles = (N + kRows - 1) / kRows;
@@ -1292,7 +1333,7 @@ int launch_pipe(const __half* x, const uint32_t* wq, const __half* scales, __hal
   if (int rc = raise_smem_limit(limit, func, need, "gemv")) return rc;
   p.nstages = stages;
   p.kblk = kblk;
-  if ((pro.rope.on || PRO == kPrologueNormStats) && kblk < kpad) return B200_ENOTREADY;   // (K cut into blocks: these take one)
+  if ((pro.rope.on || PRO == kPrologueNormStats || PRO == kPrologueRagged) && kblk < kpad) return B200_ENOTREADY;   // (K cut into blocks: these take one)
 
   cudaError_t e;
   cudaLaunchConfig_t cfg = {};
@@ -1339,7 +1380,9 @@ bool half_stages(int n, int k) {
 template <int CW, int CH, int PRO, int EPI>
 int launch_pipe_m(const __half* x, const uint32_t* wq, const __half* scales, __half* y, int m, int n, int k,
                   cudaStream_t stream, const Prologue& pro, const PeerReduce& red) {
-  if (m == 1) {
+  if constexpr (PRO == kPrologueRagged) {
+    if (m < 2 || m > 8) return B200_ENOTREADY;
+  } else if (m == 1) {
     // batch 1: the fast form unless the caller asks for the reference's rounding of every weight (gemv.exact = 1)
     // or, by default (gemv.exact = 0), K is short.  The line was drawn when the fast form had stages of 4096 k, which a short
     // K fills poorly: exact / fast at N = 4096 2.96 / 3.17 us at K = 512, 3.70 / 3.79 at 2048, 4.09 / 4.09 at 2560, 4.42 / 4.33 at
@@ -1373,7 +1416,7 @@ int launch_pipe_m(const __half* x, const uint32_t* wq, const __half* scales, __h
   if (m <= 8)
     return half_stages<8>(n, k) ? launch_pipe<8, CW, CW, PRO, false, EPI>(x, wq, scales, y, m, n, k, stream, pro, red)
                              : launch_pipe<8, 2 * CW, CH, PRO, false, EPI>(x, wq, scales, y, m, n, k, stream, pro, red);
-  if constexpr (PRO == kPrologueNormStats || EPI == kEpilogueAdd || EPI == kEpilogueStoreTwice) return B200_ENOTREADY;
+  if constexpr (PRO == kPrologueNormStats || PRO == kPrologueRagged || EPI == kEpilogueAdd || EPI == kEpilogueStoreTwice) return B200_ENOTREADY;
   else return launch_pipe<16, CW, CH, PRO, false, EPI>(x, wq, scales, y, m, n, k, stream, pro, red);
 }
 
@@ -1542,6 +1585,12 @@ int launch_gemv_pipe_gate_up(const __half* x, const __half* delta, const __half*
   }
   if (stats_in) { pro.kind = kPrologueNormStats; pro.stats_in = stats_in; }
   return dispatch_pipe<kEpilogueGateUp>(x, wq, scales, act, M, 2 * I, K, stream, pro, PeerReduce{});
+}
+
+// Two to eight rows with K % 32 == 0 or scales that are only 2-byte aligned.
+int launch_gemv_pipe_ragged(const __half* x, const uint32_t* wq, const __half* scales, __half* y, int64_t M, int64_t N, int64_t K,
+                            cudaStream_t stream) {
+  return dispatch_form<kPrologueRagged, kEpilogueStore>(x, wq, scales, y, (int)M, (int)N, (int)K, stream, Prologue{}, PeerReduce{});
 }
 
 // y = x . decode(W)^T, stored to y and to y2 (up to eight rows).

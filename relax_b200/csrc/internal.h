@@ -65,6 +65,8 @@ int launch_gemv_pipe_rmsnorm_rope(const __half* x, const __half* delta, const __
 int launch_gemv_pipe_gate_up(const __half* x, const __half* delta, const __half* norm_w, __half* x_out, float eps,
                              const float* stats_in, const uint32_t* wq, const __half* scales, __half* act, int64_t M, int64_t I, int64_t K,
                              cudaStream_t stream);
+int launch_gemv_pipe_ragged(const __half* x, const uint32_t* wq, const __half* scales, __half* y, int64_t M, int64_t N, int64_t K,
+                            cudaStream_t stream);
 int launch_gemv_pipe_twice(const __half* x, const uint32_t* wq, const __half* scales, __half* y, __half* y2, int64_t M, int64_t N,
                            int64_t K, cudaStream_t stream);
 int launch_gemv_pipe_norm(const __half* x, const float* stats_in, const __half* norm_w, float eps, const uint32_t* wq, const __half* scales,

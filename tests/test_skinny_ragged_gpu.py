@@ -1,0 +1,42 @@
+"""Two to eight rows with a K of whole scale groups only, or scales off 16 bytes: the skinny kernel's form for them against the oracle at
+the ends of its chunks (256 k), stages and row tiles, both layouts; nothing past the ends may be used."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from oracle import q4f16
+from relax_b200 import _lib, ops, synth
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M", [2, 3, 4, 5, 8])
+@pytest.mark.parametrize("N,K", [(1, 32), (16, 96), (17, 224), (33, 288), (2400, 480), (640, 2016), (257, 2080), (8640, 3200), (100, 4128),
+                                 (2380, 4352), (48, 6176), (96, 8160)])
+def test_ragged_rows(cuda_lib, M, N, K):
+    rng = np.random.default_rng(M + N + K)
+    wq, s = synth.make_weights(N, K, rng)
+    w = q4f16.dequantize(wq, s).astype(np.float64)
+    x = rng.standard_normal((M, K)).astype(np.float16)
+    paired = (M + N) % 2 == 1
+    # guard values behind every operand: NaN scales and activations, all-ones words
+    fx, fs = np.full(M * K + 512, np.nan, np.float16), np.full(s.size + 513, np.nan, np.float16)
+    fw = np.full(wq.size + 256, 0xffffffff, np.uint32)
+    off = int(K % 256 == 0)                                 # scales off 16 bytes where K alone is not ragged
+    fx[:M * K], fs[off:off + s.size], fw[:wq.size] = x.ravel(), s.ravel(), wq.ravel()
+    tx, ts, tw = (torch.from_numpy(a).cuda() for a in (fx, fs, fw))
+    twq = tw[:wq.size].view(N, K // 8)
+    if paired:
+        tw[:wq.size] = ops.q4f16_repack(twq.contiguous(), "paired").view(-1)
+    y = torch.full((M + 1, N), float("nan"), dtype=torch.float16, device="cuda")
+    torch.cuda.synchronize()
+    before = cuda_lib.b200_launch_count()
+    assert cuda_lib.b200_q4f16_matmul_layout(tx.data_ptr(), tw.data_ptr(), ts.data_ptr() + 2 * off, y.data_ptr(), M, N, K, int(paired), 0) == 0, _lib.last_error()
+    torch.cuda.synchronize()
+    assert cuda_lib.b200_launch_count() == before + 1 and cuda_lib.b200_device_error_flags() == 0
+    got, xf = y.cpu().numpy()[:M].astype(np.float64), x.astype(np.float64)
+    ref = xf @ w.T
+    # the bound of the parity tests: fp32 sums and one fp16 rounding
+    assert (np.abs(got - ref) <= 2.0 ** -10 * np.abs(ref) + 8e-6 * (np.abs(xf) @ np.abs(w).T)).all(), np.abs(got - ref).max()
+    assert bool(torch.isnan(y[M]).all())
