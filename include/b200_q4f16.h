@@ -357,7 +357,7 @@ B200_API int b200_decode_layer(const B200DecodeLayer* layer, void* cuda_stream);
 B200_API int b200_rmsnorm(void* x, const void* delta, const void* w, void* y, int64_t B, int64_t H, float eps,
                           void* cuda_stream);
 
-/* Early-release forms.  b200_rmsnorm, b200_silu_mul and the merge inside b200_attn_decode let the next programmatic
+/* Early-release forms.  b200_rmsnorm, b200_silu_mul and b200_attn_decode let the next programmatic
  * dependent launch begin once everything in front of them is complete (griddepcontrol.wait, then
  * griddepcontrol.launch_dependents).  The three *_early_release entry points compute the same and let it begin
  * in their first instruction, so that the set-up and first weight loads of a matmul of this library behind them run

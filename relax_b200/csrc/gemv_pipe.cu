@@ -1355,15 +1355,17 @@ int launch_pipe(const __half* x, const uint32_t* wq, const __half* scales, __hal
 // Stages of 2048 k instead of 4096 for 2..8 rows.  They waste less of a K that ends in the first half of a 4096-k stage;
 // and they leave room for a second CTA on the SM, which is worth it where there are tiles for two and both copies of x fit too
 // (up to four columns; with eight the arithmetic fills the SM either way).  4096-k / 2048-k stages in us:
-//   K ends in a first half   M = 2 N = 12288, K = 1024 6.3 / 4.9; M = 4 N = 12288, K = 2048 8.1 / 6.6, K = 6144 15.4 / 14.0; M = 8 N = 4096,
-//                            K = 2048 5.7 / 5.0, K = 9216 17.2 / 14.3
-//   ... one CTA either way   M = 4: the shorter ones where two long ones do not fit beside x (N = 5120, K = 13824 20.7 / 18.6) and
-//                            up to two tiles an SM (N = 4736, K = 9216 11.3 / 10.9; N = 4752 12.6 / 13.3, N = 12288 21.3 / 22.8), not
+//   K ends in a first half   M = 2 N = 12288, K = 1024 6.3 / 4.9; M = 4 N = 12288, K = 2048 7.5 / 6.6, K = 6144 14.7 / 13.4; M = 8 N = 4096,
+//                            K = 2048 4.6 / 4.2, N = 12288, K = 1024 7.1 / 6.0
+//   ... one CTA either way   M = 4: the shorter ones where two long ones do not fit beside x (N = 5120, K = 13824 21.0 / 18.7) and
+//                            up to two tiles an SM (N = 4736, K = 9216 10.9 / 11.0; N = 4752 12.3 / 13.2, N = 12288 20.6 / 22.9), not
 //                            for long K, of which a stage is little (M = 2 K = 17920 N = 4096 15.1 / 15.6, N = 12288 34.6 / 38.3)
-//   ... no two fit beside x  the longer ones, and K cut into blocks (M = 4 N = 4096, K = 21504 25.0 / 29.6, N = 8192, K = 26624 45 / 64;
-//                            M = 8 N = 5120, K = 13824 26.9 / 34.5)
-//   two CTAs of the shorter  M = 2 N = 12288, K = 4096 10.0 / 9.3, K = 14336 28.1 / 26.7; M = 4 N = 12288, K = 4096 10.9 / 10.3, but 160 tiles
-//                            (N = 2560) 5.5 / 5.8 and 32 tiles 4.24 / 4.35; M = 8 N = 12288, K = 3072 10.9 / 11.1
+//   ... no two fit beside x  the longer ones, and K cut into blocks (M = 4 N = 4096, K = 21504 25.0 / 29.6, N = 8192, K = 26624 45 / 64)
+//   two CTAs of the shorter  M = 2 N = 12288, K = 4096 10.0 / 9.3, K = 14336 28.1 / 26.7; M = 4 N = 12288, K = 4096 10.4 / 9.8, but 160 tiles
+//                            (N = 2560) 5.0 / 5.2 and 32 tiles 3.7 / 3.8
+//   eight columns            above one long stage always the shorter ones, whose eight warps share 256 k each, against sixteen that share
+//                            what is left of a long one: 8 x 5120 x 5120 11.3 / 9.3, 8 x 27648 x 5120 33.5 / 24.9, 7 x 7680 x 6144 14.6 / 12.0,
+//                            6 x 2560 x 6912 9.0 / 8.6, 5 x 4096 x 7680 10.0 / 9.5; 8 x 12288 x 3072 9.3 / 10.2
 template <int NC>
 bool half_stages(int n, int k) {
   constexpr size_t kRing = 8 * kRows * (128 + 16);                            // a short stage
@@ -1371,6 +1373,7 @@ bool half_stages(int n, int k) {
   const size_t x_short = XRows<NC>::bytes((k + 2047) / 2048 * 2048), x_long = XRows<NC>::bytes((k + 4095) / 4096 * 4096);
   const bool pair = 2 * kRing + kRest + x_short <= kExclusiveSmem - 1024;
   const int tail = k % 4096;
+  if (NC >= 8 && k > 4096) return 2 * kRing + kRest + x_short <= kMaxSmem;
   if (tail == 0 || tail > 2048) return NC <= 4 && pair && n > sm_count() * kRows * 3 / 2;
   if (2 * kRing + kRest + x_short > kMaxSmem) return false;
   const bool two_long = 4 * kRing + kRest + x_long <= kMaxSmem;
