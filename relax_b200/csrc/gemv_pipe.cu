@@ -816,7 +816,6 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
       for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
       if (lane == 0) s_inv[warp] = rsqrtf(tot / (float)p.K + p.eps);
     }
-    bar_sync(1, kConsumers);
   };
   if (PRO == kPrologueNormStats && !XL::kOwnRows) {
     constexpr int kNormItems = 2;
@@ -832,6 +831,7 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
     load_stats();
     load(tid);
     add_stats();
+    bar_sync(1, kConsumers);
     for (int i0 = tid; i0 < items; i0 += kNormItems * kConsumers) {
       if (i0 != tid) {
         load(i0);
@@ -886,6 +886,7 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
       for (int c = warp, m = 0; c < nch;) {
         uint4 a[kItems], b[kItems], w[kItems];
         load_items(c, m, k_lo, nch, a, b, w);
+        if (PRO == kPrologueNormStats && c == warp && m == 0) add_stats();       // (while the first loads are on their way)
 #pragma unroll
         for (int r = 0; r < kItems; ++r)
           if (c < nch) {
@@ -899,7 +900,8 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
       }
       if (PRO == kPrologueNormStats) {
         // as it came so far; every lane scales its own words in place (little code: it is fetched anew in every launch)
-        add_stats();
+        if (warp >= nch) add_stats();            // (a warp without chunks)
+        bar_sync(1, kConsumers);
 #pragma unroll 1
         for (int c = warp; c < nch; c += CW) {
           const uint4 w = staged_order(nw[0], p.paired != 0);
