@@ -9,6 +9,8 @@
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
+#include <cstdint>
+
 #include <ATen/PythonTorchFunctionTLS.h>
 #include <ATen/core/Tensor.h>
 #include <c10/cuda/CUDAFunctions.h>
@@ -52,8 +54,11 @@ PyObject* matmul(PyObject*, PyObject* const* args, Py_ssize_t n) {
     PyErr_SetString(PyExc_TypeError, "matmul(x, wq, scales, out, layout)");
     return nullptr;
   }
-  const long layout = PyLong_AsLong(args[4]);
+  // -1: no layout given.  Any other number that is no layout is for the general path, which refuses it.
+  int overflow = 0;
+  const long layout = PyLong_AsLongAndOverflow(args[4], &overflow);
   if (layout == -1 && PyErr_Occurred()) return nullptr;
+  if (overflow != 0 || layout < -1 || layout > INT32_MAX) Py_RETURN_FALSE;
   try {
     if (!g_entry.matmul || at::impl::torch_function_mode_enabled()) Py_RETURN_FALSE;
     const at::Tensor *x = plain_matrix(args[0], at::kHalf), *wq = plain_matrix(args[1], at::kUInt32),

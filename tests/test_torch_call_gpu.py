@@ -63,3 +63,17 @@ def test_plain_tensors_are_taken_and_others_are_not(cuda_lib):
     with pytest.raises(_lib.B200Error):
         ops.q4f16_matmul(wide[:, :256], wq, s)
     assert np.isfinite(ops.q4f16_matmul(x, wq, s).float().cpu().numpy()).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("layout", [-2, -3, -256, 2, 7, -2 ** 40])
+def test_numbers_that_are_no_layout_are_refused(cuda_lib, layout):
+    x, wq, s = (torch.from_numpy(a).cuda() for a in synth.make_case(2, 64, 256, seed=9))
+    out = torch.full((2, 64), float("nan"), dtype=torch.float16, device="cuda")
+    before = cuda_lib.b200_launch_count()
+    assert _native().matmul(x, wq, s, out, layout) is False
+    assert cuda_lib.b200_launch_count() == before and torch.isnan(out).all()
+    if -2 ** 31 <= layout:                                  # (the general path hands the number on as 32 bits)
+        with pytest.raises(_lib.B200Error):
+            ops.q4f16_matmul(x, wq, s, layout=layout)
+        assert cuda_lib.b200_launch_count() == before
