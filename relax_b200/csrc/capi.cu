@@ -592,7 +592,7 @@ static int check_norm_stats(const char* who, const void* stats, const void* norm
 
 int b200_q4f16_gemv_add_applies(const void* scales, int64_t M, int64_t N, int64_t K) {
   if (M < 1 || M > 8 || N < 16 || N % 16 != 0 || N > 0x7fffffffLL / 32 || K < 256 || K % 256 != 0 || !scales || !aligned16(scales)) return 0;
-  return !weight_stationary_first(M, N, K, false);
+  return options().gemv_variant != 1 && !weight_stationary_first(M, N, K, false);
 }
 
 int b200_q4f16_gemv_add(const void* x, const void* wq, const void* scales, void* y, void* stats, int64_t M, int64_t N, int64_t K,

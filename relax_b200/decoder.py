@@ -299,7 +299,8 @@ class DecodeEngine:
         cfg, L, B, w = self.cfg, self.L, self.batch, self.layers[i]
         H, il = cfg.hidden, w["inter_local"]
         roped = False
-        if delta is None and self.rope_epilogue:
+        skinny = delta is None and self._in_skinny(w["qkv"], 3 * H, H)
+        if skinny and self.rope_epilogue:
             rc = L.b200_q4f16_gemv_norm_rope(self.x.data_ptr(), self.stats.data_ptr(), w["norm1"].data_ptr(), cfg.eps,
                                              w["qkv"][0].data_ptr(), w["qkv"][1].data_ptr(), self.cos.data_ptr(), self.sin.data_ptr(),
                                              self.pos.data_ptr(), self.q.data_ptr(), self.kc[i].data_ptr(), self.vc[i].data_ptr(),
@@ -307,7 +308,7 @@ class DecodeEngine:
             if rc != _lib.ENOTREADY:        # (else the exact form is selected)
                 self._check(rc)
                 roped = True
-        if not roped and delta is None and self._in_skinny(w["qkv"], 3 * H, H):
+        if skinny and not roped:
             self._check(L.b200_q4f16_gemv_norm(self.x.data_ptr(), self.stats.data_ptr(), w["norm1"].data_ptr(), cfg.eps,
                                                w["qkv"][0].data_ptr(), w["qkv"][1].data_ptr(), self.qkv.data_ptr(), B, 3 * H, H, sp))
         elif not roped:
@@ -493,8 +494,7 @@ class DecodeEngine:
             per_layer = 0
             for w in self.layers:
                 per_layer += 5
-                roped = self.rope_epilogue and ready
-                norms += not (ready and (roped or self._in_skinny(w["qkv"], 3 * self.cfg.hidden, self.cfg.hidden)))
+                norms += not (ready and self._in_skinny(w["qkv"], 3 * self.cfg.hidden, self.cfg.hidden))
                 ready = self._in_skinny(w["o"], self.cfg.hidden, self.cfg.hidden)
                 one = self._gate_up_in_one(w)
                 norms += not (ready and one)

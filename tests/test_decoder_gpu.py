@@ -258,15 +258,18 @@ def test_decoder_steps_match_oracle(cuda_lib, B, fused):
 
 
 def test_decoder_follows_the_matmul_options(cuda_lib):
-    """At 2..8 rows gate|up goes where b200_q4f16_matmul would take it: with SwiGLU in the epilogue, or as the kernel that an option
-    asks for and a SwiGLU launch behind it; scales that come to lie off 16 bytes after the engine was built take that way too."""
+    """At 2..8 rows every matmul of a step goes where b200_q4f16_matmul would take it: with the norm, the residual add and SwiGLU in the
+    skinny kernel, or as the kernel that an option asks for with launches of their own for those; so does gate|up where its
+    scales come to lie off 16 bytes after the engine was built."""
     cfg, B = SMALL, 5
     rng = np.random.default_rng(17)
     layers = [decoder.to_device(tp.shard_layer(decoder.synth_layer_numpy(cfg, 40 + i), 0, 1, cfg.hidden, cfg.inter), "cuda") for i in range(cfg.layers)]
-    eng = decoder.DecodeEngine(cfg, layers, dev((0.5 * rng.standard_normal((cfg.vocab, cfg.hidden))).astype(F16)), dev(np.ones(cfg.hidden, F16)),
-                               dev((0.05 * rng.standard_normal((cfg.vocab, cfg.hidden))).astype(F16)), B, 16, "cuda")
+    made = (dev((0.5 * rng.standard_normal((cfg.vocab, cfg.hidden))).astype(F16)), dev(np.ones(cfg.hidden, F16)),
+            dev((0.05 * rng.standard_normal((cfg.vocab, cfg.hidden))).astype(F16)), B, 16, "cuda")
+    eng = decoder.DecodeEngine(cfg, layers, *made)
+    apart = decoder.DecodeEngine(cfg, layers, *made, fused=False)            # a launch of its own for everything but the matmuls
 
-    def step():
+    def step(eng=eng):
         eng.set_position(0)
         eng.tokens.copy_(torch.arange(B, dtype=torch.int32))
         before = cuda_lib.b200_launch_count()
@@ -279,9 +282,14 @@ def test_decoder_follows_the_matmul_options(cuda_lib):
     try:
         _lib.set_option("gemv.variant", 1)
         count1, out1 = step()
+        assert count1 == eng.kernels_per_step()
+        # the same kernels in both engines (the streaming one for all four matmuls), so the same bits
+        assert (out1 == step(apart)[1]).all()
     finally:
         _lib.set_option("gemv.variant", 0)
-    assert count1 == count + cfg.layers
+    # two norms and SwiGLU a layer, and the last norm
+    assert count1 == count + 3 * cfg.layers + 1
+    assert (step(apart)[1] != out1).any(), "the two kernels differ in the order of their sums"
     close(out1, ref, 1e-2, 1e-2 * scale, "streaming kernel")
     for w in layers:
         off = torch.empty(w["gu"][1].numel() + 1, dtype=torch.float16, device="cuda")[1:].view(w["gu"][1].shape)

@@ -1,0 +1,72 @@
+"""CPU tests of which entry points a decode step asks for: the engine on the host, with a library that only writes down the calls
+(what it is asked about sizes and options, the real one answers)."""
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from relax_b200 import _lib, decoder
+
+
+class Recorder:
+    """The library with every launch replaced by a note of it; `refuse`: entry points that answer B200_ENOTREADY."""
+
+    def __init__(self, refuse=()):
+        self.real, self.calls, self.refuse = _lib.lib(), [], refuse
+
+    def __getattr__(self, name):
+        fn = getattr(self.real, name)
+        if name.endswith(("_applies", "_bytes")):
+            return fn
+
+        def note(*args):
+            self.calls.append((name, args))
+            return _lib.ENOTREADY if name in self.refuse else _lib.OK
+
+        return note
+
+    def names(self):
+        return [name.removeprefix("b200_") for name, _ in self.calls]
+
+
+def engine(hidden, batch, inter=768, layers=2, **kw):
+    cfg = decoder.DecoderConfig(hidden=hidden, heads=hidden // 128, inter=inter, layers=layers, vocab=64)
+    # (nothing reads the weights here: sixteen aligned bytes of each will do)
+    w = dict.fromkeys(("qkv", "o", "gu", "down"), (torch.zeros(8, dtype=torch.int32), torch.zeros(8, dtype=torch.float16)))
+    w |= {"norm1": torch.zeros(8, dtype=torch.float16), "norm2": torch.zeros(8, dtype=torch.float16), "inter_local": inter}
+    eng = decoder.DecodeEngine(cfg, [dict(w) for _ in range(layers)], torch.zeros((64, 8), dtype=torch.float16),
+                               torch.zeros(8, dtype=torch.float16), torch.zeros((64, 8), dtype=torch.float16), batch, 16, "cpu", **kw)
+    eng.L = Recorder()
+    return eng
+
+
+@pytest.fixture
+def option():
+    before = {name: _lib.get_option(name) for name in ("gemv.variant", "gemm.ws_max_m")}
+    yield _lib.set_option
+    for name, value in before.items():
+        _lib.set_option(name, value)
+
+
+def layers(eng):
+    """The calls of all layers and what is left to add behind the last."""
+    delta = None
+    for i in range(len(eng.layers)):
+        delta = eng._chained_layer(i, delta, 0)
+    return eng.L.names(), delta
+
+
+CHAINED = ["q4f16_gemv_norm", "attn_decode_step", "q4f16_gemv_add", "q4f16_gemv_norm_gate_up", "q4f16_gemv_add"]
+APART = ["rmsnorm_early_release", "q4f16_matmul", "attn_decode_step", "q4f16_matmul", "rmsnorm_early_release", "q4f16_matmul",
+         "silu_mul_early_release", "q4f16_matmul"]
+
+
+@pytest.mark.parametrize("batch", [1, 2, 5, 8])
+def test_matmuls_of_a_step_follow_the_option(option, batch):
+    eng = engine(512, batch, rope_epilogue=False)
+    assert eng.chained
+    assert layers(eng) == (2 * CHAINED, None)
+    option("gemv.variant", 1)                               # the register-streaming kernel: no prologue, no epilogue
+    eng = engine(512, batch)
+    names, delta = layers(eng)
+    assert names == 2 * APART and delta is eng.down
+    assert eng.kernels_per_step() == 1 + len(names) + 1 + 1 + 1
