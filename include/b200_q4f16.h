@@ -253,8 +253,10 @@ B200_API int b200_q4f16_gate_up(const void* x, const void* wq, const void* scale
  * read before the kernel has synchronised with the launch in front, as weights and scales are.  K % 256 == 0, scales 16-byte aligned.
  * B200_ENOTREADY, and nothing launched: a shape that the skinny kernel does not take in one piece (a long K), for _norm_rope
  * also one that would not use the fast form; b200_rmsnorm and the plain matmul take those.
- * b200_q4f16_gemv_add_applies: 1 where, under the present options, b200_q4f16_matmul would take the matmul through the skinny kernel. */
+ * b200_q4f16_gemv_add_applies: 1 where, under the present options, b200_q4f16_matmul would take the matmul through the skinny kernel.
+ * b200_q4f16_gemv_norm_applies: the same, and x fits in one piece, so that _norm and (N = 2 I) _norm_gate_up do not answer B200_ENOTREADY. */
 B200_API int b200_q4f16_gemv_add_applies(const void* scales, int64_t M, int64_t N, int64_t K);
+B200_API int b200_q4f16_gemv_norm_applies(const void* scales, int64_t M, int64_t N, int64_t K);
 B200_API int b200_q4f16_gemv_add(const void* x, const void* wq, const void* scales, void* y, void* stats, int64_t M, int64_t N,
                                  int64_t K, int32_t swiglu, void* cuda_stream);
 B200_API int b200_q4f16_gemv_norm(const void* x, const void* stats, const void* norm_w, float eps, const void* wq,

@@ -119,6 +119,7 @@ PROTOTYPES = {
     "b200_q4f16_gate_up_applies": (_ci, [_vp, _i64, _i64, _i64]),
     "b200_q4f16_gate_up": (_ci, [_vp, _vp, _vp, _vp, _i64, _i64, _i64, _vp]),
     "b200_q4f16_gemv_add_applies": (_ci, [_vp, _i64, _i64, _i64]),
+    "b200_q4f16_gemv_norm_applies": (_ci, [_vp, _i64, _i64, _i64]),
     "b200_q4f16_gemv_add": (_ci, [_vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, ctypes.c_int32, _vp]),
     "b200_q4f16_gemv_norm": (_ci, [_vp, _vp, _vp, ctypes.c_float, _vp, _vp, _vp, _i64, _i64, _i64, _vp]),
     "b200_q4f16_gemv_norm_gate_up": (_ci, [_vp, _vp, _vp, ctypes.c_float, _vp, _vp, _vp, _i64, _i64, _i64, _vp]),

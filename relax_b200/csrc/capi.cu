@@ -613,6 +613,11 @@ int b200_q4f16_gemv_add(const void* x, const void* wq, const void* scales, void*
   return rc;
 }
 
+int b200_q4f16_gemv_norm_applies(const void* scales, int64_t M, int64_t N, int64_t K) {
+  if (M < 1 || M > 8 || N < 1 || N > 0x7fffffffLL / 32 || K < 256 || K % 256 != 0 || K > 0x3fffffffLL || !scales || !aligned16(scales)) return 0;
+  return options().gemv_variant != 1 && !weight_stationary_first(M, N, K, false) && gemv_pipe_norm_fits(M, N, K);
+}
+
 int b200_q4f16_gemv_norm(const void* x, const void* stats, const void* norm_w, float eps, const void* wq, const void* scales, void* y,
                          int64_t M, int64_t N, int64_t K, void* stream) {
   const char* who = "q4f16_gemv_norm";

@@ -1167,16 +1167,32 @@ struct Prologue {
   RopeOut rope;          // rotary embedding + KV append in the epilogue (qkv matmul of a batch-1 step)
 };
 
-template <int NC, int CW, int CH, int PRO, bool FAST, int EPI>
+// One form of the kernel: NC columns of x staged, CW consumer warps, CH chunks of 256 k a stage.
+template <int NC_, int CW_, int CH_, bool FAST_>
+struct PipeForm {
+  static constexpr int NC = NC_, CW = CW_, CH = CH_;
+  static constexpr bool FAST = FAST_;
+  static constexpr int kOut = FAST ? kRows * 2 : (NC + 7) / 8 * 128;
+  static constexpr int kStageBytes = CH * kRows * (128 + 16);
+  // Shared memory: everything but the staged x (see the carve-up above the kernel), and a block of x of k values a row
+  static constexpr size_t fixed_bytes(int stages) {
+    return (size_t)1024 /* base alignment slack */ + (4 * kMaxStages + 2) * sizeof(uint64_t) + (size_t)stages * kStageBytes +
+           (size_t)(stages + 1) * CW * kOut * sizeof(float);
+  }
+  static constexpr size_t block_bytes(int k) { return XRows<NC>::bytes(k) + (FAST ? (size_t)(k / 256) * 32 * sizeof(float) : 0); }
+  static constexpr int padded(int k) { return (k + 256 * CH - 1) / (256 * CH) * (256 * CH); }
+  // All of x beside one stage
+  static constexpr bool one_block(int k) { return fixed_bytes(1) + block_bytes(padded(k)) <= kMaxSmem; }
+};
+
+template <class Form, int PRO, int EPI>
 int launch_pipe(const __half* x, const uint32_t* wq, const __half* scales, __half* y, int M, int N, int K,
                 cudaStream_t stream, const Prologue& pro, const PeerReduce& red) {
-  constexpr int MT = (NC + 7) / 8;
-  constexpr int kOut = FAST ? kRows * 2 : MT * 128;
+  constexpr int NC = Form::NC, CW = Form::CW, CH = Form::CH, kOut = Form::kOut;
+  constexpr bool FAST = Form::FAST;
   constexpr int KC = 256 * CH;
-  constexpr int kStageBytes = CH * kRows * (128 + 16);
   constexpr int kThreads = (CW + 2) * 32;
   constexpr bool GU = EPI == kEpilogueGateUp;
-  using XL = XRows<NC>;
   PipeParams p;
   p.rope = pro.rope;
   if (GU) {
@@ -1232,7 +1248,7 @@ int launch_pipe(const __half* x, const uint32_t* wq, const __half* scales, __hal
   p.red = red;
   p.paired = current_layout() == kLayoutPaired;
   p.ntiles = (N + kRows - 1) / kRows;
-  const int kpad = ((K + KC - 1) / KC) * KC;
+  const int kpad = Form::padded(K);
   const int stages_per_tile = kpad / KC;
   const int sms = sm_count();
   auto kern = q4f16_gemv_pipe_kernel<NC, CW, CH, PRO, FAST, EPI>;
@@ -1245,11 +1261,8 @@ int launch_pipe(const __half* x, const uint32_t* wq, const __half* scales, __hal
     carveout.raise(dev, 1, [&](size_t) {
       return (int)cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     });
-  auto fixed_bytes = [&](int stages) {
-    return (size_t)1024 /* base alignment slack */ + (4 * kMaxStages + 2) * sizeof(uint64_t) + (size_t)stages * kStageBytes +
-           (size_t)(stages + 1) * CW * kOut * sizeof(float);
-  };
-  auto block_bytes = [&](int k) { return XL::bytes(k) + (FAST ? (size_t)(k / 256) * 32 * sizeof(float) : 0); };
+  auto fixed_bytes = Form::fixed_bytes;
+  auto block_bytes = Form::block_bytes;
   static SmemLimit limit;                            // (one per kernel variant, for all threads)
   const void* const func = reinterpret_cast<const void*>(kern);
   size_t need = 0;
@@ -1382,12 +1395,10 @@ bool half_stages(int n, int k) {
   return NC >= 8 || pair || !two_long || (k <= 12288 && n <= 2 * sm_count() * kRows);
 }
 
-template <int CW, int CH, int PRO, int EPI>
-int launch_pipe_m(const __half* x, const uint32_t* wq, const __half* scales, __half* y, int m, int n, int k,
-                  cudaStream_t stream, const Prologue& pro, const PeerReduce& red) {
-  if constexpr (PRO == kPrologueRagged) {
-    if (m < 2 || m > 8) return B200_ENOTREADY;
-  } else if (m == 1) {
+// The form for m rows of k values and n outputs, handed to f.
+template <int CW, int CH, class F>
+auto with_form(int m, int n, int k, F f) {
+  if (m == 1) {
     // batch 1: the fast form unless the caller asks for the reference's rounding of every weight (gemv.exact = 1)
     // or, by default (gemv.exact = 0), K is short.  The line was drawn when the fast form had stages of 4096 k, which a short
     // K fills poorly: exact / fast at N = 4096 2.96 / 3.17 us at K = 512, 3.70 / 3.79 at 2048, 4.09 / 4.09 at 2560, 4.42 / 4.33 at
@@ -1403,32 +1414,40 @@ int launch_pipe_m(const __half* x, const uint32_t* wq, const __half* scales, __h
     // returns, is 0-2 % faster back to back (N = 2048, K = 4096 3.84 / 3.79, N = 4736 4.97 / 4.88, 40 of N = K = 4096 183.3 / 182.4).
     // But it is a kernel of its own, and inside a decode step, where other kernels run in between, the o projection took
     // 0.3 us longer with it (a step of the 7B shape 1646 / 1656): one form for every K.
-    if (fast) return launch_pipe<1, CW, CW, PRO, true, EPI>(x, wq, scales, y, m, n, k, stream, pro, red);
-    return launch_pipe<1, CW, CH, PRO, false, EPI>(x, wq, scales, y, m, n, k, stream, pro, red);
+    if (fast) return f(PipeForm<1, CW, CW, true>{});
+    return f(PipeForm<1, CW, CH, false>{});
   }
   if (m == 2)
-    return half_stages<2>(n, k) ? launch_pipe<2, CW, CW, PRO, false, EPI>(x, wq, scales, y, m, n, k, stream, pro, red)
-                             : launch_pipe<2, CW, CH, PRO, false, EPI>(x, wq, scales, y, m, n, k, stream, pro, red);
+    return half_stages<2>(n, k) ? f(PipeForm<2, CW, CW, false>{}) : f(PipeForm<2, CW, CH, false>{});
   // Sixteen consumer warps where one CTA fills an SM anyway and a tile has chunks for them: eight are too few to hide their own
   // latencies.  3 or 4 rows with no more tiles than SMs and K > 4096: 8 / 16 warps, us, 4 x 2048 x 5632 5.5 / 5.1, 3 x 1024 x 8192
   // 5.8 / 5.2, 4 x 1280 x 6912 5.7 / 5.0, but 4 x 2048 x 4096 4.1 / 4.2; 2 x 2048 x 5632 4.7 / 4.9.  5..8 rows with the long stages:
   // 8 x 4096 x 4096 6.5 / 6.0, 7 x 7680 x 2560 7.4 / 7.1, 8 x 22016 x 4096 15.9 / 15.2, 8 x 3072 x 3072 5.4 / 5.0.
   if (m > 2 && m <= 4 && k > 4096 && n <= sm_count() * kRows)
-    return launch_pipe<4, 2 * CW, CH, PRO, false, EPI>(x, wq, scales, y, m, n, k, stream, pro, red);
+    return f(PipeForm<4, 2 * CW, CH, false>{});
   if (m <= 4)
-    return half_stages<4>(n, k) ? launch_pipe<4, CW, CW, PRO, false, EPI>(x, wq, scales, y, m, n, k, stream, pro, red)
-                             : launch_pipe<4, CW, CH, PRO, false, EPI>(x, wq, scales, y, m, n, k, stream, pro, red);
+    return half_stages<4>(n, k) ? f(PipeForm<4, CW, CW, false>{}) : f(PipeForm<4, CW, CH, false>{});
   if (m <= 8)
-    return half_stages<8>(n, k) ? launch_pipe<8, CW, CW, PRO, false, EPI>(x, wq, scales, y, m, n, k, stream, pro, red)
-                             : launch_pipe<8, 2 * CW, CH, PRO, false, EPI>(x, wq, scales, y, m, n, k, stream, pro, red);
-  if constexpr (PRO == kPrologueNormStats || PRO == kPrologueRagged || EPI == kEpilogueAdd || EPI == kEpilogueStoreTwice) return B200_ENOTREADY;
-  else return launch_pipe<16, CW, CH, PRO, false, EPI>(x, wq, scales, y, m, n, k, stream, pro, red);
+    return half_stages<8>(n, k) ? f(PipeForm<8, CW, CW, false>{}) : f(PipeForm<8, 2 * CW, CH, false>{});
+  return f(PipeForm<16, CW, CH, false>{});
+}
+
+// Whether x of m rows stays in one piece beside a stage, as kPrologueNormStats and kPrologueRagged need it.
+bool one_block(int m, int n, int k) {
+  return with_form<8, 16>(m, n, k, [&](auto form) { return decltype(form)::one_block(k); });
 }
 
 template <int PRO, int EPI>
 int dispatch_form(const __half* x, const uint32_t* wq, const __half* scales, __half* y, int m, int n, int k,
                   cudaStream_t stream, const Prologue& pro, const PeerReduce& red) {
-  return launch_pipe_m<8, 16, PRO, EPI>(x, wq, scales, y, m, n, k, stream, pro, red);
+  return with_form<8, 16>(m, n, k, [&](auto form) -> int {
+    using Form = decltype(form);
+    // (forms that no caller asks for are not built)
+    constexpr int kMaxNC = PRO == kPrologueNormStats || PRO == kPrologueRagged || EPI == kEpilogueAdd || EPI == kEpilogueStoreTwice ? 8 : 16;
+    constexpr int kMinNC = PRO == kPrologueRagged ? 2 : 1;
+    if constexpr (Form::NC < kMinNC || Form::NC > kMaxNC) return B200_ENOTREADY;
+    else return launch_pipe<Form, PRO, EPI>(x, wq, scales, y, m, n, k, stream, pro, red);
+  });
 }
 
 template <int EPI = kEpilogueStore>
@@ -1605,6 +1624,9 @@ int launch_gemv_pipe_twice(const __half* x, const uint32_t* wq, const __half* sc
   pro.y2 = y2;
   return dispatch_pipe<kEpilogueStoreTwice>(x, wq, scales, y, M, N, K, stream, pro, PeerReduce{});
 }
+
+// Whether the forms with stats_in take these sizes.
+bool gemv_pipe_norm_fits(int64_t M, int64_t N, int64_t K) { return M <= 8 && one_block((int)M, (int)N, (int)K); }
 
 // y = (x * rsqrt(mean(x^2) + eps) * norm_w) . decode(W)^T with the statistics of stats_in (up to eight rows).
 int launch_gemv_pipe_norm(const __half* x, const float* stats_in, const __half* norm_w, float eps, const uint32_t* wq, const __half* scales,

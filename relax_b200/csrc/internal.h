@@ -69,6 +69,7 @@ int launch_gemv_pipe_ragged(const __half* x, const uint32_t* wq, const __half* s
                             cudaStream_t stream);
 int launch_gemv_pipe_twice(const __half* x, const uint32_t* wq, const __half* scales, __half* y, __half* y2, int64_t M, int64_t N,
                            int64_t K, cudaStream_t stream);
+bool gemv_pipe_norm_fits(int64_t M, int64_t N, int64_t K);
 int launch_gemv_pipe_norm(const __half* x, const float* stats_in, const __half* norm_w, float eps, const uint32_t* wq, const __half* scales,
                           __half* y, int64_t M, int64_t N, int64_t K, cudaStream_t stream);
 int launch_gemv_pipe_add(const __half* x, const uint32_t* wq, const __half* scales, __half* y, float* stats_out, int64_t M, int64_t N,

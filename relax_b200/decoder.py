@@ -274,6 +274,10 @@ class DecodeEngine:
         """Whether the chained forms, which the skinny kernel has, are the ones for this matmul (asked anew each time, as below)."""
         return bool(self.L.b200_q4f16_gemv_add_applies(w[1].data_ptr(), self.batch, n, k))
 
+    def _norm_in_skinny(self, w, n, k) -> bool:
+        """The same for a matmul that normalises the residual stream on its way in, all of which has to fit beside it."""
+        return bool(self.L.b200_q4f16_gemv_norm_applies(w[1].data_ptr(), self.batch, n, k))
+
     def _add(self, x, w, out, k, sp, swiglu=False):
         """The residual stream += x . W^T, statistics included: None.  Or, where the chained form does not apply, `out` with the
         product still to be added.  `swiglu`: x is gate | up, SwiGLU is applied first."""
@@ -299,7 +303,7 @@ class DecodeEngine:
         cfg, L, B, w = self.cfg, self.L, self.batch, self.layers[i]
         H, il = cfg.hidden, w["inter_local"]
         roped = False
-        skinny = delta is None and self._in_skinny(w["qkv"], 3 * H, H)
+        skinny = delta is None and self._norm_in_skinny(w["qkv"], 3 * H, H)
         if skinny and self.rope_epilogue:
             rc = L.b200_q4f16_gemv_norm_rope(self.x.data_ptr(), self.stats.data_ptr(), w["norm1"].data_ptr(), cfg.eps,
                                              w["qkv"][0].data_ptr(), w["qkv"][1].data_ptr(), self.cos.data_ptr(), self.sin.data_ptr(),
@@ -320,7 +324,7 @@ class DecodeEngine:
             self._norm(delta, w["norm2"], sp)
             self._matmul(self.h, w["gu"], self.gu, 2 * il, H, sp)
             return self._add(self.gu, w["down"], self.down, il, sp, swiglu=True)
-        if delta is None:
+        if delta is None and self._norm_in_skinny(w["gu"], 2 * il, H):
             self._check(L.b200_q4f16_gemv_norm_gate_up(self.x.data_ptr(), self.stats.data_ptr(), w["norm2"].data_ptr(), cfg.eps,
                                                        w["gu"][0].data_ptr(), w["gu"][1].data_ptr(), self.act.data_ptr(), B, il, H, sp))
         else:
@@ -494,10 +498,10 @@ class DecodeEngine:
             per_layer = 0
             for w in self.layers:
                 per_layer += 5
-                norms += not (ready and self._in_skinny(w["qkv"], 3 * self.cfg.hidden, self.cfg.hidden))
+                norms += not (ready and self._norm_in_skinny(w["qkv"], 3 * self.cfg.hidden, self.cfg.hidden))
                 ready = self._in_skinny(w["o"], self.cfg.hidden, self.cfg.hidden)
                 one = self._gate_up_in_one(w)
-                norms += not (ready and one)
+                norms += not (ready and one and self._norm_in_skinny(w["gu"], 2 * w["inter_local"], self.cfg.hidden))
                 ready = self._in_skinny(w["down"], self.cfg.hidden, w["inter_local"])
                 per_layer += 0 if one or ready else 1          # (SwiGLU as a launch of its own)
             return 1 + per_layer + norms + (0 if ready and head else 1) + head + tail

@@ -7,7 +7,7 @@ torch = pytest.importorskip("torch")
 
 from oracle import decoder as odec
 from oracle import q4f16
-from relax_b200 import _lib, synth
+from relax_b200 import _lib, decoder, synth
 
 pytestmark = pytest.mark.gpu
 EPS = 1e-5
@@ -163,3 +163,61 @@ def test_refusals(cuda_lib):
     assert L.b200_embed_rows_stats(p, p, q, None, 1, 64, 4, 0) == _lib.EINVAL
     assert L.b200_q4f16_gemv_add_applies(p, 9, 64, 256) == 0 and L.b200_q4f16_gemv_add_applies(p, 1, 64, 288) == 0
     assert L.b200_q4f16_gemv_add_applies(p, 8, 4096, 8192) == 0 and L.b200_q4f16_gemv_add_applies(p, 8, 4096, 4096) == 1
+
+
+@pytest.mark.parametrize("variant", [0, 1, 2])
+def test_the_question_about_the_fit_is_answered_as_the_launch_answers(cuda_lib, variant):
+    K = [256, 2304, 2560, 4096, 4352, 6144, 7936, 8192, 8448, 8704, 9216, 12288, 16384]
+    t = torch.zeros(64 * 16384 // 8, dtype=torch.int32, device="cuda")
+    h = torch.zeros(64 * 16384, dtype=torch.float16, device="cuda")
+    y, stats = torch.empty((8, 64), dtype=torch.float16, device="cuda"), torch.zeros(8 * 1024, dtype=torch.float32, device="cuda")
+    _lib.set_option("gemv.variant", variant)
+    try:
+        for M in range(1, 9):
+            for k in K:
+                rc = cuda_lib.b200_q4f16_gemv_norm(h.data_ptr(), stats.data_ptr(), h.data_ptr(), 1e-5, t.data_ptr(), h.data_ptr(), y.data_ptr(), M, 64, k, 0)
+                fits = rc != _lib.ENOTREADY
+                assert rc == 0 or not fits
+                ours = variant == 2 or (variant == 0 and not (M >= 5 and k >= 8192))          # (the rest: weight-stationary, streaming)
+                assert cuda_lib.b200_q4f16_gemv_norm_applies(h.data_ptr(), M, 64, k) == int(fits and ours), (M, k)
+    finally:
+        _lib.set_option("gemv.variant", 0)
+    torch.cuda.synchronize()
+    assert cuda_lib.b200_device_error_flags() == 0
+
+
+@pytest.mark.parametrize("B,option", [(5, ("gemv.variant", 2)), (8, ("gemv.variant", 2)), (8, ("gemm.ws_max_m", 4))])
+def test_step_of_a_model_too_wide_for_the_normalising_forms(cuda_lib, B, option):
+    """Against the engine that has a launch for every norm: the appended keys and values have its bits."""
+    cfg = decoder.DecoderConfig(hidden=9216, heads=72, inter=1024, layers=2, vocab=320)
+    layers = []
+    for i in range(cfg.layers):
+        layer = decoder.synth_layer_torch(cfg, 31 + i, "cuda")
+        layer |= {name: (layer[name][0], layer[name][1] * 0.1) for name in ("qkv", "o", "gu", "down")}
+        layers.append(layer | {"inter_local": cfg.inter})
+    embed = torch.randn((cfg.vocab, cfg.hidden), dtype=torch.float16, device="cuda") * 0.1
+    norm = torch.ones(cfg.hidden, dtype=torch.float16, device="cuda")
+    before = _lib.get_option(option[0])
+    out = []
+    try:
+        _lib.set_option(*option)
+        for kw in ({}, dict(fused=False)):
+            eng = decoder.DecodeEngine(cfg, layers, embed, norm, embed, B, 16, "cuda", **kw)
+            assert eng.chained == (not kw)
+            for _ in range(2):
+                eng.tokens.copy_(torch.arange(B, dtype=torch.int32))
+                launches = cuda_lib.b200_launch_count()
+                eng.step()
+                torch.cuda.synchronize()
+                assert cuda_lib.b200_launch_count() - launches == eng.kernels_per_step()
+            out.append(eng)
+    finally:
+        _lib.set_option(option[0], before)
+    a, b = out
+    for i in range(cfg.layers):
+        assert torch.equal(a.kc[i][:, :2], b.kc[i][:, :2]) and torch.equal(a.vc[i][:, :2], b.vc[i][:, :2])
+    assert float(a.kc[-1][:, :2].abs().max()) > 0
+    # (the statistics of the last norm are added up in another order)
+    scale = float(b.logits.abs().max())
+    assert torch.isfinite(a.logits).all() and float((a.logits - b.logits).abs().max()) <= 4e-3 * scale
+    assert cuda_lib.b200_device_error_flags() == 0

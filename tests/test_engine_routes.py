@@ -70,3 +70,27 @@ def test_matmuls_of_a_step_follow_the_option(option, batch):
     names, delta = layers(eng)
     assert names == 2 * APART and delta is eng.down
     assert eng.kernels_per_step() == 1 + len(names) + 1 + 1 + 1
+
+
+@pytest.mark.parametrize("batch", [5, 8])
+@pytest.mark.parametrize("name,value", [("gemv.variant", 2), ("gemm.ws_max_m", 4)])
+def test_a_row_that_does_not_fit_is_normalised_by_itself(option, batch, name, value):
+    """5..8 rows of a wide model stay in the skinny kernel only where an option asks for it; all of x beside a stage ends between
+    8192 and 9216 values a row.  The forms without a norm cut K and go on."""
+    option(name, value)
+    scales = 1 << 20                                        # (only its alignment is looked at)
+    applies = [_lib.lib().b200_q4f16_gemv_norm_applies(scales, batch, 3 * k, k) for k in (256, 4096, 8192, 9216, 16384)]
+    assert applies == [1, 1, 1, 0, 0]
+    assert _lib.lib().b200_q4f16_gemv_add_applies(scales, batch, 9216, 9216) == 1
+    eng = engine(9216, batch)
+    assert eng.chained
+    names, delta = layers(eng)
+    assert names == 2 * ["rmsnorm_early_release", "q4f16_matmul", "attn_decode_step", "q4f16_gemv_add", "rmsnorm_early_release",
+                         "q4f16_gemv_gate_up", "q4f16_gemv_add"] and delta is None
+    assert eng.kernels_per_step() == 1 + len(names) + 1 + 1
+
+
+def test_up_to_four_rows_of_every_width_fit():
+    for batch in (1, 2, 3, 4):
+        for hidden in range(256, 16384 + 1, 256):
+            assert _lib.lib().b200_q4f16_gemv_norm_applies(1 << 20, batch, 3 * hidden, hidden) == 1
