@@ -333,17 +333,18 @@ class DecodeEngine:
                                                   self.act.data_ptr(), B, il, H, sp))
         return self._add(self.act, w["down"], self.down, il, sp)
 
-    def _attention(self, i: int, roped: bool, sp: int):
+    def _attention(self, i: int, roped: bool, sp: int, early: bool = True):
         """`roped`: the qkv matmul has rotated q and appended k and v, else all of that is done here.
 
-        Early loads: the position and the older cache entries are final before any kernel of a step but its first can begin.
+        `early` (loads): the position and the older cache entries are final before any kernel of a step but its first can begin.
         A kernel begins only after the one in front of it has begun, embed_rows lets its successor begin only after it
         has waited for everything in front of it, and every kernel waits for its predecessor before it ends."""
         L, B = self.L, self.batch
+        loads = _lib.ATTN_EARLY_KV_LOADS if early else 0
         if roped:
             self._check(L.b200_attn_decode_early_release(self.q.data_ptr(), self.kc[i].data_ptr(), self.vc[i].data_ptr(),
                                                          self.pos.data_ptr(), self.attn.data_ptr(), self.scratch.data_ptr(), B,
-                                                         self.nh_local, self.max_ctx, _lib.ATTN_EARLY_KV_LOADS, sp))
+                                                         self.nh_local, self.max_ctx, loads, sp))
         elif self.fused_attention == "rope":
             self._check(L.b200_attn_decode_rope(self.qkv.data_ptr(), self.cos.data_ptr(), self.sin.data_ptr(), self.pos.data_ptr(),
                                                 self.kc[i].data_ptr(), self.vc[i].data_ptr(), self.attn.data_ptr(),
@@ -355,15 +356,18 @@ class DecodeEngine:
         else:
             self._check(L.b200_attn_decode_step(self.qkv.data_ptr(), self.cos.data_ptr(), self.sin.data_ptr(), self.pos.data_ptr(),
                                                 self.kc[i].data_ptr(), self.vc[i].data_ptr(), self.attn.data_ptr(), B, self.nh_local,
-                                                self.max_ctx, _lib.ATTN_EARLY_KV_LOADS | _lib.ATTN_EARLY_RELEASE, sp))
+                                                self.max_ctx, loads | _lib.ATTN_EARLY_RELEASE, sp))
 
     def _allreduce(self, t):
         if self.world > 1:
             torch.distributed.all_reduce(t, group=self.group)
 
-    def layer_step(self, i: int, delta, sp: int):
+    def layer_step(self, i: int, delta, sp: int, within_step: bool = False):
         """One layer; `delta` is the tensor still to be added to the residual stream (or None).
         Returns the layer's MLP output (to be added by whoever consumes the stream next).
+
+        Outside a step (`within_step` False) whatever the caller launched in front may have written the position and the
+        caches, and no kernel between it and the attention waits before it lets the next one begin: no early loads then.
 
         The early-release forms: behind every one of them is a matmul (or the output projection), which reads nothing
         but weights before it has waited for the kernel in front."""
@@ -393,7 +397,7 @@ class DecodeEngine:
             self._check(L.b200_rmsnorm_early_release(self.x.data_ptr(), dptr, w["norm1"].data_ptr(), self.h.data_ptr(), B, H,
                                                      cfg.eps, sp))
             self._matmul(self.h, w["qkv"], self.qkv, 3 * hl, H, sp)
-        self._attention(i, roped, sp)
+        self._attention(i, roped, sp, early=within_step)
         if self.peer is not None and B <= self.PEER_FUSED_MAX_ROWS:
             d = self._reduce_desc(0, i, self.o)
             self._check(L.b200_q4f16_gemv_allreduce(self.attn.data_ptr(), w["o"][0].data_ptr(), w["o"][1].data_ptr(),
@@ -455,7 +459,7 @@ class DecodeEngine:
                 delta, xlast = self.down, self.x_last
         else:
             for i in range(len(self.layers)):
-                delta = self._chained_layer(i, delta, sp) if self.chained else self.layer_step(i, delta, sp)
+                delta = self._chained_layer(i, delta, sp) if self.chained else self.layer_step(i, delta, sp, within_step=True)
         normed = not (self.chained and delta is None and self.lm_head is not None)
         if normed:
             self._check(L.b200_rmsnorm_early_release(xlast.data_ptr(), delta.data_ptr() if delta is not None else None,

@@ -94,3 +94,20 @@ def test_up_to_four_rows_of_every_width_fit():
     for batch in (1, 2, 3, 4):
         for hidden in range(256, 16384 + 1, 256):
             assert _lib.lib().b200_q4f16_gemv_norm_applies(1 << 20, batch, 3 * hidden, hidden) == 1
+
+
+@pytest.mark.parametrize("batch,kw", [(1, dict(fused=True)), (1, dict(fused=False)), (3, dict(fused=True)), (3, dict(fused=False)), (12, {}), (1, {}), (3, {})])
+def test_only_a_step_promises_the_attention_a_finished_cache(monkeypatch, batch, kw):
+    """A layer by itself stands behind whatever the caller launched, which may have written the position and the caches."""
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: type("S", (), {"cuda_stream": 0}))
+    eng = engine(2560, batch, **kw)
+
+    def flags():
+        out = [args[-2] & _lib.ATTN_EARLY_KV_LOADS for name, args in eng.L.calls if name.startswith("b200_attn_decode")]
+        eng.L.calls.clear()
+        return out
+
+    eng.layer_step(1, None, 0)
+    assert flags() == [0]
+    eng.step()
+    assert flags() == [_lib.ATTN_EARLY_KV_LOADS] * len(eng.layers)
