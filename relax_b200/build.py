@@ -11,6 +11,8 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+import sysconfig
+import warnings
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -46,11 +48,7 @@ def _stale() -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
-def _torch_call_command() -> list:
-    import sysconfig
-
-    import torch
-
+def _torch_call_command(torch) -> list:
     root = os.path.dirname(torch.__file__)
     cuda = os.path.dirname(os.path.dirname(_nvcc())) if os.path.isabs(_nvcc()) else "/usr/local/cuda"
     include = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
@@ -62,22 +60,39 @@ def _torch_call_command() -> list:
             "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
 
 
-def _torch_call_stale() -> bool:
+def _torch_call_stale(path: str) -> bool:
     deps = [os.path.join(CSRC, "torch_call.cpp"), os.path.join(INCLUDE, "b200_q4f16.h"), os.path.abspath(__file__)]
-    return not os.path.exists(TORCH_CALL) or any(os.path.getmtime(d) > os.path.getmtime(TORCH_CALL) for d in deps)
+    return not os.path.exists(path) or any(os.path.getmtime(d) > os.path.getmtime(path) for d in deps)
+
+
+def _start_torch_call(force: bool):
+    """The compiler of the extension, started; None: it is there, or there is no torch to build it for.  Raises where it cannot run."""
+    try:
+        import torch
+    except ImportError:
+        return None
+    if not force and not _torch_call_stale(TORCH_CALL):
+        return None
+    return subprocess.Popen(_torch_call_command(torch), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    extension = None
-    if force or _torch_call_stale():
-        extension = subprocess.Popen(_torch_call_command(), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    """The library, and the extension beside it.  The library needs nvcc only; without the extension the operators make
+    its checks in Python, so what keeps it from being built is a warning."""
+    compiler, why = None, ""
+    try:
+        compiler = _start_torch_call(force)
+    except Exception as e:
+        why = f"{type(e).__name__}: {e}"
     try:
         return _build_library(force, verbose)
     finally:
-        if extension is not None:
-            out, _ = extension.communicate()
-            if extension.returncode != 0:
-                raise RuntimeError("g++ failed for torch_call.cpp:\n" + out)
+        if compiler is not None:
+            out, _ = compiler.communicate()
+            if compiler.returncode != 0:
+                why = out
+        if why:
+            warnings.warn("torch_call.cpp was not built, operator calls on torch tensors take longer: " + why, RuntimeWarning, stacklevel=2)
 
 
 def _build_library(force: bool, verbose: bool) -> str:
