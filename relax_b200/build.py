@@ -17,7 +17,6 @@ import warnings
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libb200_q4f16.so")
-TORCH_CALL = os.path.join(HERE, "_torch_call.so")          # CPython extension: torch tensors to the library's C ABI
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 
 SOURCES = ["capi.cu", "tmap.cu", "dequant.cu", "gemv.cu", "gemv_pipe.cu", "gemm_tcgen05.cu", "gemm_ws_tcgen05.cu", "decoder_ops.cu", "attn_decode.cu", "decode_layer.cu", "lm_head.cu"]
@@ -48,6 +47,12 @@ def _stale() -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def torch_call_path(torch_version: str) -> str:
+    """The CPython extension (torch tensors to the library's C ABI) for this interpreter and that torch.  It is compiled against
+    the insides of torch's tensors, so one that was built for another torch or Python is never looked at."""
+    return os.path.join(HERE, f"_torch_call.{sysconfig.get_config_var('SOABI')}.torch-{torch_version}.so")
+
+
 def _torch_call_command(torch) -> list:
     root = os.path.dirname(torch.__file__)
     cuda = os.path.dirname(os.path.dirname(_nvcc())) if os.path.isabs(_nvcc()) else "/usr/local/cuda"
@@ -56,7 +61,7 @@ def _torch_call_command(torch) -> list:
     lib = os.path.join(root, "lib")
     return ["/usr/bin/g++" if os.path.exists("/usr/bin/g++") else "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
             f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *[f"-I{d}" for d in include],
-            os.path.join(CSRC, "torch_call.cpp"), "-o", TORCH_CALL, f"-L{lib}", f"-Wl,-rpath,{lib}",
+            os.path.join(CSRC, "torch_call.cpp"), "-o", torch_call_path(torch.__version__), f"-L{lib}", f"-Wl,-rpath,{lib}",
             "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
 
 
@@ -71,7 +76,7 @@ def _start_torch_call(force: bool):
         import torch
     except ImportError:
         return None
-    if not force and not _torch_call_stale(TORCH_CALL):
+    if not force and not _torch_call_stale(torch_call_path(torch.__version__)):
         return None
     return subprocess.Popen(_torch_call_command(torch), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
 

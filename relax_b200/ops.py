@@ -8,10 +8,11 @@ torch is used only for device memory and streams.
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 
 import torch
 
-from . import _lib
+from . import _lib, build
 from ._lib import B200Error, DLDataType, DLDevice, DLTensor  # noqa: F401
 
 
@@ -139,15 +140,17 @@ def _dequantize_by_pointer(L, wq, scales, out) -> bool:
     return L.b200_q4f16_dequantize(wq.data_ptr(), scales.data_ptr(), out.data_ptr(), n, k, stream) == 0
 
 
-_native = None      # the extension module, bound to the loaded library; False: not built (the checks run in Python then)
+_native = None      # the extension module, bound to the loaded library; False: not built for this torch (the checks run in Python then)
 
 
 def _torch_call():
     global _native
     if _native is None:
+        path = build.torch_call_path(torch.__version__)
         try:
-            from . import _torch_call as module
-        except ImportError:
+            spec = importlib.util.spec_from_file_location(__package__ + "._torch_call", path)
+            module = importlib.util.module_from_spec(spec)
+        except ImportError:                 # (no such file, or one that does not load)
             _native = False
         else:
             L = _lib.lib()
