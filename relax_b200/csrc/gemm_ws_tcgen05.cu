@@ -599,7 +599,7 @@ int launch_gemm_ws(const __half* x, const uint32_t* wq, const __half* scales, __
   if (row_tiles * ((M + 15) / 16) > 0x3fffffff) return B200_ENOTREADY;      // (tile numbers are 32-bit)
   int clusters_of[4];
   for (int i = 0; i < 4; ++i) clusters_of[i] = max_clusters(1 << i, reinterpret_cast<const void*>(kernel_for(16, paired, ragged, false)));
-  const WsSplit split = choose_ws_split(M, row_tiles, units, (int)options().gemm_ws_ksplit, clusters_of, kWsClusterCosts);
+  const WsSplit split = choose_ws_split(M, row_tiles, units, (int)options().gemm_ws_ksplit, clusters_of);
   if (options().gemm_ws_ksplit == 0 && prefill_kernel_is_ahead(M, N, K, split, row_tiles, clusters_of[0])) return B200_ENOTREADY;
   const int ksplit = split.ksplit, nb16 = split.nb;
   const int skb = nb16 <= 128 ? 2 : 1;

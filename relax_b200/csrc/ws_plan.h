@@ -13,31 +13,25 @@ struct WsSplit {
   int tried;    // combinations looked at
 };
 
-// What a cluster of CTAs costs over single ones, ns: the start of one of two, four and eight CTAs, and the last exchange beside
-// its 35 ns a column.  The defaults were fitted to the kernel when the cluster barriers of its set-up and teardown waited for memory;
-// kWsClusterCosts is the kernel as it is (chosen / best of the slices 1.011 -> 1.005 on average over 140 shapes of 16 to 128 rows,
-// M x N x K, us: 16 x 2560 x 4096 6.6 -> 5.4, 64 x 2560 x 2560 7.0 -> 6.0, 40 x 12288 x 8192 21.5 -> 19.6, 129 x 1024 x 4096 7.8 -> 6.6).
-struct WsClusterCosts {
-  int64_t start[3] = {500, 2800, 3500};
-  int64_t tail = 1000;
-};
-constexpr WsClusterCosts kWsClusterCosts = {{500, 1000, 3500}, 600};
-
 // A model of the time in nanoseconds, fitted to measurements at N = 4096, 12288 and 22016,
 // K = 4096 and 11008 and batches of 16, 64 and 128, and at 129..2048 tokens.  A 256-k span takes a CTA 0.53-0.65 us (up
-// to 128 columns) or 0.9-0.95 us; with many CTAs at work, what they fetch from L2 at about 14 TB/s if that is more.
+// to 128 columns) or 0.9-0.95 us; with many CTAs at work, what they fetch from L2 at about 14 TB/s (13 in clusters) if that is more.
 // Draining a tile is cheap with one slice (stores to y, behind the next tile's MMAs) and costs the exchange of the
-// partial tiles with several, which the next tile hides only as far as its own MMAs last; a larger cluster starts
-// later, unless (one token tile, four or eight CTAs) the clusters at work leave room for as many again: the set-up of a
-// launch then runs beside the launch before it; in part for more than four clusters of eight.  M = 64, K = 4096, 1 / 2 / 4 / 8 slices: N = 4096 11.0 / 8.7 / 9.0 / 10.8 us, N = 12288 12.9 / 14.3 / 15.6 / 23.2,
+// partial tiles with several, which the next tile hides only as far as its own MMAs last.  A larger cluster starts
+// later: up to 128 rows by as much as the clusters of the last round leave too little room for the first ones of the next launch, whose
+// set-up runs beside them where there is room (in part for more than four clusters of eight).  One figure for every
+// launch without room made 16 x 4096 x 2080 take four slices, 6.8 us where two take 5.2, and 96 x 8192 x 2560 two, 9.8 / 8.8; above 128 rows
+// 777 x 12288 x 7168 took two, 135 / 111.  Chosen / best of the slices over 2200 shapes, up to 128 rows 1.012 -> 1.0045 on average
+// and at most 1.31 -> 1.14, above 1.006 -> 1.003 and 1.21 -> 1.17.  Measured first: M = 64, K = 4096, 1 / 2 / 4 / 8 slices: N = 4096 11.0 / 8.7 / 9.0 / 10.8 us, N = 12288 12.9 / 14.3 / 15.6 / 23.2,
 // N = 22016 22.1 / 20.5 / 24.0 / 40.3; N = 4096 and K = 11008: 26.4 / 16.4 / 13.5 / 14.6.  M = 300, N = 12288, K = 4096 in 2 / 3 / 4
 // token tiles: 31.7 / 29.5 / 34.8.  Few row tiles, M = 64, K = 2048, N = 512: 6.7 / 6.3 / 5.1 / 4.9, N = 1024: 6.7 / 6.3 / 5.2 / 5.8,
 // N = 2048: 6.8 / 6.5 / 5.1 / 7.3; N = 1024, K = 8192: 20.0 / 13.0 / 8.4 / 7.6.
 // M rows of x, row_tiles tiles of 128 weight rows, units spans of 256 k; forced: the largest power of two of slices up to
 // it (0 = by the model); clusters[i]: clusters of 2^i CTAs that run at once.  Every width of a token tile is looked at
 // once, so at most 12 x 4 combinations whatever M is.
-inline WsSplit choose_ws_split(int64_t M, int64_t row_tiles, int units, int forced, const int (&clusters)[4],
-                               const WsClusterCosts& costs = {}) {
+inline WsSplit choose_ws_split(int64_t M, int64_t row_tiles, int units, int forced, const int (&clusters)[4]) {
+  constexpr int64_t kCrowdedStart[4] = {0, 1800, 3000, 4300};        // up to 128 rows, no room at all beside the last round
+  constexpr int64_t kManyRowsStart[4] = {0, 0, 600, 1900};
   WsSplit best = {0, 1, 0};
   int64_t best_cost = 0;
   const int64_t mt0 = (M + kWsMaxNB - 1) / kWsMaxNB;
@@ -52,13 +46,17 @@ inline WsSplit choose_ws_split(int64_t M, int64_t row_tiles, int units, int forc
       if (forced > 0 && !(c <= forced && (c * 2 > forced || c * 2 > units || c == 8))) continue;
       const int64_t rounds = (tiles + clusters[i] - 1) / clusters[i];
       const int64_t busy = tiles * c / rounds;                                   // CTAs at work, on average
-      const int64_t l2 = busy * (nb * 512 + kWsSpanBytes) / 14000;
+      const int64_t l2 = busy * (nb * 512 + kWsSpanBytes) / (c == 1 ? 14000 : 13000);
       const int64_t span = nb <= 128 ? 520 + nb : 760 + nb;
       const int64_t tile = (int64_t)((units + c - 1) / c) * (span > l2 ? span : l2);   // a tile's MMAs
       const int64_t drain = c == 1 ? 300 + 12 * nb : 800 + 50 * nb;              // ... and what the next tile must hide
-      const bool room = M <= 128 && c >= 4 && 2 * tiles <= clusters[i] + (c == 8 ? 2 : 0);
-      const int64_t tail = c == 1 ? drain : room ? 900 + 38 * nb : costs.tail + 35 * nb;   // the last tile's drain
-      const int64_t start = room ? (c == 8 && tiles > 4 ? 1600 - 8 * nb : 0) : c == 1 ? 0 : costs.start[i - 1];
+      // clusters of the next launch's first round that find no place beside this one's last
+      const int64_t all = clusters[i], excess = tiles - (rounds - 1) * all + (tiles < all ? tiles : all) - all - (c == 8 ? 2 : 0);
+      const int64_t crowd = excess > 0 ? excess : 0;
+      const bool room = M <= 128 && c >= 4 && crowd == 0;
+      const int64_t tail = c == 1 ? drain : room ? 900 + 38 * nb : (M <= 128 ? 600 : 400) + 35 * nb;   // the last tile's drain
+      const int64_t start = M > 128 ? kManyRowsStart[i] : room ? (c == 8 && tiles > 4 ? 1600 - 8 * nb : 0)
+                                                               : (c == 2 ? 500 : 0) + kCrowdedStart[i] * crowd / all;
       const int64_t cost = start + tile + (rounds - 1) * (tile > drain ? tile : drain) + tail;
       ++best.tried;
       if (best_cost == 0 || cost < best_cost) { best_cost = cost; best.ksplit = c; best.nb = nb; }
