@@ -217,10 +217,14 @@ q4f16_gemm_ws_tcgen05_kernel(const __grid_constant__ WsParams p) {
   __syncwarp();
   tc_fence_before_sync();
   // The peers' barriers are initialised before anything arrives on them: the fence above orders the initialisation, so the
-  // arrival need not (a releasing one, with the weight loads just requested, took 1.8 us).
-  if (p.ksplit > 1) cluster_arrive_relaxed();
+  // arrival need not (a releasing one, with the weight loads just requested, took 1.8 us).  One branch around both halves: with the
+  // block's barrier between them a run of single CTAs was 1.5-2.8 % slower (us, this / that: 512 x 12288 x 11008 117.0 / 119.6,
+  // 1024 x 16384 x 8192 242.5 / 248.5, 2048 x 11008 x 4096 156.7 / 158.8), and clusters no faster.
+  if (p.ksplit > 1) {
+    cluster_arrive_relaxed();
+    cluster_wait();
+  }
   __syncthreads();
-  if (p.ksplit > 1) cluster_wait();
   tc_fence_after_sync();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, bar.tmem_base, 0);
   pdl_launch_dependents();
