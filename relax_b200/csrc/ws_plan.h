@@ -21,8 +21,9 @@ struct WsSplit {
 // later: up to 128 rows by as much as the clusters of the last round leave too little room for the first ones of the next launch, whose
 // set-up runs beside them where there is room (in part for more than four clusters of eight).  One figure for every
 // launch without room made 16 x 4096 x 2080 take four slices, 6.8 us where two take 5.2, and 96 x 8192 x 2560 two, 9.8 / 8.8; above 128 rows
-// 777 x 12288 x 7168 took two, 135 / 111.  Chosen / best of the slices over 2200 shapes, up to 128 rows 1.012 -> 1.0045 on average
-// and at most 1.31 -> 1.14, above 1.006 -> 1.003 and 1.21 -> 1.17.  Measured first: M = 64, K = 4096, 1 / 2 / 4 / 8 slices: N = 4096 11.0 / 8.7 / 9.0 / 10.8 us, N = 12288 12.9 / 14.3 / 15.6 / 23.2,
+// 777 x 12288 x 7168 took two, 135 / 111.  Chosen / best of the slices over 2200 shapes on a GPU that holds 74, 33 and 15 clusters
+// at once, up to 128 rows 1.012 -> 1.0045 on average and at most 1.31 -> 1.15, above 1.006 -> 1.004.  (That number differs from GPU to GPU: 36 and 16
+// were seen too.)  Measured first: M = 64, K = 4096, 1 / 2 / 4 / 8 slices: N = 4096 11.0 / 8.7 / 9.0 / 10.8 us, N = 12288 12.9 / 14.3 / 15.6 / 23.2,
 // N = 22016 22.1 / 20.5 / 24.0 / 40.3; N = 4096 and K = 11008: 26.4 / 16.4 / 13.5 / 14.6.  M = 300, N = 12288, K = 4096 in 2 / 3 / 4
 // token tiles: 31.7 / 29.5 / 34.8.  Few row tiles, M = 64, K = 2048, N = 512: 6.7 / 6.3 / 5.1 / 4.9, N = 1024: 6.7 / 6.3 / 5.2 / 5.8,
 // N = 2048: 6.8 / 6.5 / 5.1 / 7.3; N = 1024, K = 8192: 20.0 / 13.0 / 8.4 / 7.6.
@@ -30,7 +31,7 @@ struct WsSplit {
 // it (0 = by the model); clusters[i]: clusters of 2^i CTAs that run at once.  Every width of a token tile is looked at
 // once, so at most 12 x 4 combinations whatever M is.
 inline WsSplit choose_ws_split(int64_t M, int64_t row_tiles, int units, int forced, const int (&clusters)[4]) {
-  constexpr int64_t kCrowdedStart[4] = {0, 1800, 3000, 4300};        // up to 128 rows, no room at all beside the last round
+  constexpr int64_t kStart[4] = {0, 500, 0, 3000}, kCrowdedStart[4] = {0, 2000, 2400, 1300};     // up to 128 rows; more where there is no room at all
   constexpr int64_t kManyRowsStart[4] = {0, 0, 600, 1900};
   WsSplit best = {0, 1, 0};
   int64_t best_cost = 0;
@@ -53,10 +54,10 @@ inline WsSplit choose_ws_split(int64_t M, int64_t row_tiles, int units, int forc
       // clusters of the next launch's first round that find no place beside this one's last
       const int64_t all = clusters[i], excess = tiles - (rounds - 1) * all + (tiles < all ? tiles : all) - all - (c == 8 ? 2 : 0);
       const int64_t crowd = excess > 0 ? excess : 0;
-      const bool room = M <= 128 && c >= 4 && crowd == 0;
-      const int64_t tail = c == 1 ? drain : room ? 900 + 38 * nb : (M <= 128 ? 600 : 400) + 35 * nb;   // the last tile's drain
+      const bool room = M <= 128 && c >= 4 && rounds == 1 && crowd == 0;
+      const int64_t tail = c == 1 ? drain : room ? 900 + 38 * nb : (M <= 128 ? 300 + 38 * nb : 400 + 35 * nb);   // the last tile's drain
       const int64_t start = M > 128 ? kManyRowsStart[i] : room ? (c == 8 && tiles > 4 ? 1600 - 8 * nb : 0)
-                                                               : (c == 2 ? 500 : 0) + kCrowdedStart[i] * crowd / all;
+                                                               : kStart[i] + kCrowdedStart[i] * crowd / all;
       const int64_t cost = start + tile + (rounds - 1) * (tile > drain ? tile : drain) + tail;
       ++best.tried;
       if (best_cost == 0 || cost < best_cost) { best_cost = cost; best.ksplit = c; best.nb = nb; }

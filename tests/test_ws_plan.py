@@ -35,14 +35,14 @@ def exhaustive(m, row_tiles, units, forced, clusters):
             tile = -(-units // c) * span
             drain = 300 + 12 * nb if c == 1 else 800 + 50 * nb
             crowd = max(tiles - (rounds - 1) * clusters[i] + min(tiles, clusters[i]) - clusters[i] - (2 if c == 8 else 0), 0)
-            room = m <= 128 and c >= 4 and crowd == 0
+            room = m <= 128 and c >= 4 and rounds == 1 and crowd == 0
             if m > 128:
                 start = (0, 0, 600, 1900)[i]
             elif room:
                 start = 1600 - 8 * nb if c == 8 and tiles > 4 else 0
             else:
-                start = (0, 500, 0, 0)[i] + (0, 1800, 3000, 4300)[i] * crowd // clusters[i]
-            tail = drain if c == 1 else 900 + 38 * nb if room else (600 if m <= 128 else 400) + 35 * nb
+                start = (0, 500, 0, 3000)[i] + (0, 2000, 2400, 1300)[i] * crowd // clusters[i]
+            tail = drain if c == 1 else 900 + 38 * nb if room else 300 + 38 * nb if m <= 128 else 400 + 35 * nb
             cost = start + tile + (rounds - 1) * max(tile, drain) + tail
             if best is None or cost < best[0]:
                 best = (cost, nb, c)
@@ -65,7 +65,7 @@ def test_choice_equals_the_exhaustive_search(program):
     rng = random.Random(7)
     cases = [(m, rt, 16, 0, (148, 74, 36, 16)) for m in list(range(1, 700)) + [2047, 2048, 5000, 100000] for rt in (1, 32, 172)]
     cases += [(int(2 ** rng.uniform(0, 15)), rng.randint(1, 300), rng.randint(1, 64), rng.choice((0, 0, 1, 2, 4, 8)),
-               rng.choice(((148, 74, 36, 16), (132, 66, 33, 16), (8, 4, 2, 1)))) for _ in range(3000)]
+               rng.choice(((148, 74, 36, 16), (148, 74, 33, 15), (132, 66, 33, 16), (8, 4, 2, 1)))) for _ in range(3000)]
     for case, got in zip(cases, program(cases)):
         assert got[:2] == exhaustive(*case), case
 
@@ -87,9 +87,10 @@ def test_long_prompts_that_one_wave_of_the_prefill_kernel_holds(program):
 
 def test_slices_where_clusters_crowd_the_gpu(program):
     # as measured: the best number of slices (four, two or one were taken for them: 5-30 % slower)
-    for best, shapes in ((2, [(8, 4096, 2080), (16, 4096, 2080), (16, 4096, 2560), (12, 4096, 3200), (9, 22016, 3200)]),
+    for best, shapes in ((2, [(8, 4096, 2080), (16, 4096, 2080), (16, 4096, 2560), (9, 22016, 3200)]),
                          (1, [(64, 8192, 2080), (96, 8192, 2560), (96, 6144, 2560), (777, 12288, 7168), (777, 12288, 8192)]),
-                         (4, [(9, 10240, 5120), (33, 10240, 7168), (16, 2560, 4096), (64, 2560, 2560), (16, 4096, 11008), (24, 1024, 4096), (16, 2048, 11008)]),
+                         (4, [(9, 10240, 5120), (33, 10240, 7168), (16, 2560, 4096), (64, 2560, 2560), (16, 4096, 11008), (16, 4096, 5120), (24, 1024, 4096), (16, 2048, 11008)]),
                          (8, [(16, 512, 8192)])):
-        got = program([(m, -(-n // 128), -(-k // 256), 0, (148, 74, 36, 16)) for m, n, k in shapes])
-        assert [g[1] for g in got] == [best] * len(shapes), list(zip(shapes, got))
+        for clusters in ((148, 74, 36, 16), (148, 74, 33, 15)):                     # (two GPUs of one kind)
+            got = program([(m, -(-n // 128), -(-k // 256), 0, clusters) for m, n, k in shapes])
+            assert [g[1] for g in got] == [best] * len(shapes), (clusters, list(zip(shapes, got)))
