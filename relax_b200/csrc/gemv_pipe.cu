@@ -641,32 +641,6 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
   // behind, a launch took, us, before / now: M x N x K 5 x 2048 x 5632 7.1 / 5.5, 8 x 1024 x 3072 5.3 / 4.3, 8 x 4096 x 4096 7.8 / 6.6,
   // 8 x 22016 x 4096 17.5 / 16.5, 4 x 4096 x 4096 6.0 / 5.5; up to two columns it is the faster way (2 x 4096 x 4096 5.1 / 5.3).
   constexpr int kItems = PRO == kPrologueNone || PRO == kPrologueNormStats || RAG ? 8 : 4;
-  auto next_item = [&](int& c, int& m) {
-    if (++m == p.M) {
-      m = 0;
-      c += CW;
-    }
-  };
-  auto load_items = [&](int c, int m, int k_lo, int nch, uint4 (&a)[kItems], uint4 (&b)[kItems], uint4 (&w)[kItems]) {
-#pragma unroll
-    for (int r = 0; r < kItems; ++r) {
-      a[r] = b[r] = w[r] = make_uint4(0, 0, 0, 0);
-      if (c < nch) {
-        const int k = k_lo + c * 256 + lane * 8;
-        if (RAG && k >= p.K) {                      // (past the end of the last chunk: zeros)
-        } else if (PRO == kPrologueSwiGLU) {        // x is [M, 2K] = gate | up
-          a[r] = *reinterpret_cast<const uint4*>(p.x + (int64_t)m * 2 * p.K + k);
-          b[r] = *reinterpret_cast<const uint4*>(p.x + (int64_t)m * 2 * p.K + p.K + k);
-        } else {
-          a[r] = *reinterpret_cast<const uint4*>(p.x + (int64_t)m * p.K + k);
-          if (PRO == kPrologueRmsNorm && p.delta) b[r] = *reinterpret_cast<const uint4*>(p.delta + (int64_t)m * p.K + k);
-          if (PRO == kPrologueRmsNorm) w[r] = *reinterpret_cast<const uint4*>(p.norm_w + k);
-        }
-        next_item(c, m);
-      }
-    }
-  };
-
   int s = 0;                                     // ring slot of the current stage
   uint32_t round = 0;                            // how many times the ring has wrapped
   int rb = 0;                                    // reduction buffer of the current tile
@@ -882,20 +856,52 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
       const int nch = (k_hi - k_lo + 255) >> 8;
       if (kb > 0) __syncwarp();                  // all lanes are done reading the previous block
       if (PRO == kPrologueNormStats) load_stats();
+      // An item's places in x and in the staged block are stepped to with 32-bit numbers: a launch fetches the code anew, and with the places
+      // computed it is 0.2 us longer to run through (us, staged by all threads / computed / stepped to with 64 bits / as here:
+      // 3 x 512 x 1024 2.68 / 2.89 / 2.75 / 2.64, 3 x 5120 x 2048 4.37 / 4.93 / 4.22 / 4.12, 8 x 5120 x 4096 8.82 / 7.08 / 7.15 / 6.66,
+      // 8 x 22016 x 4096 17.6 / 15.4 / 15.7 / 15.2; four items instead of eight 3 x 5120 x 2048 4.61).
+      const uint32_t words = (uint32_t)p.K >> 3, x_row = PRO == kPrologueSwiGLU ? 2 * words : words;     // (SwiGLU: x is [M, 2K] = gate | up)
+      const uint32_t x_back = CW * 32 - (uint32_t)p.M * x_row;            // from behind the last row to the next chunk's first
+      const int s_back = CW * XL::kChunk - p.M * xpitch;
+      int load_m = 0, load_k = k_lo + warp * 256 + lane * 8;
+      uint32_t src = (uint32_t)load_k >> 3;
+      const uint4* const xg = reinterpret_cast<const uint4*>(p.x);
+      int m = 0, k0 = k_lo + warp * 256;
+      uint4* dst = xs + XL::slot(warp * 32 + lane, 0, xpitch);
 #pragma unroll 1
-      for (int c = warp, m = 0; c < nch;) {
+      while (k0 < k_hi) {
         uint4 a[kItems], b[kItems], w[kItems];
-        load_items(c, m, k_lo, nch, a, b, w);
-        if (PRO == kPrologueNormStats && c == warp && m == 0) add_stats();       // (while the first loads are on their way)
+#pragma unroll
+        for (int r = 0; r < kItems; ++r) {
+          a[r] = b[r] = w[r] = make_uint4(0, 0, 0, 0);
+          if (load_k < k_hi) {                    // (ragged K: what lies past the end of the last chunk stays zero)
+            a[r] = xg[src];
+            if (PRO == kPrologueSwiGLU) b[r] = xg[src + words];
+            if (PRO == kPrologueRmsNorm && p.delta) b[r] = reinterpret_cast<const uint4*>(p.delta)[src];
+            if (PRO == kPrologueRmsNorm) w[r] = *reinterpret_cast<const uint4*>(p.norm_w + load_k);
+          }
+          src += x_row;
+          if (++load_m == p.M) {
+            load_m = 0;
+            load_k += CW * 256;
+            src += x_back;
+          }
+        }
+        if (PRO == kPrologueNormStats && k0 == warp * 256 && m == 0) add_stats();       // (while the first loads are on their way)
 #pragma unroll
         for (int r = 0; r < kItems; ++r)
-          if (c < nch) {
+          if (k0 < k_hi) {
             uint4 v = a[r];
             if (PRO == kPrologueSwiGLU) v = silu_mul_f16x8(a[r], b[r]);           // fp32 inside, one fp16 rounding
             if (PRO == kPrologueRmsNorm && p.delta) v = add_f16x8(v, b[r]);
             if (PRO == kPrologueRmsNorm) v = scale_f16x8(v, s_inv[m], w[r]);
-            stage_word(c * 32 + lane, m, v);
-            next_item(c, m);
+            *dst = staged_order(v, p.paired != 0);
+            dst += xpitch;
+            if (++m == p.M) {
+              m = 0;
+              k0 += CW * 256;
+              dst += s_back;
+            }
           }
       }
       if (PRO == kPrologueNormStats) {
