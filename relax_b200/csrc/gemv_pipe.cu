@@ -671,8 +671,10 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
   };
   if (RAG) ragged_scales(blockIdx.x, 0);
   // NormStats: the first norm weights are here when the wait returns: of this thread's first items, or of this warp's first
-  // two chunks
-  uint4 nw[2];
+  // two chunks (with sixteen warps the first, which is all there is up to K = 4096, and registers are short: two / one, us,
+  // 5 x 7680 x 2560 8.8 / 8.3, 8 x 12288 x 4096 12.8 / 12.4)
+  constexpr int kNw = XL::kOwnRows && CW == 16 ? 1 : 2;
+  uint4 nw[kNw];
   if (PRO == kPrologueNormStats) {
 #pragma unroll
     for (int r = 0; r < (int)(sizeof(nw) / sizeof(nw[0])); ++r) {
@@ -911,8 +913,8 @@ q4f16_gemv_pipe_kernel(const __grid_constant__ PipeParams p) {
 #pragma unroll 1
         for (int c = warp; c < nch; c += CW) {
           const uint4 w = staged_order(nw[0], p.paired != 0);
-          nw[0] = nw[1];
-          if (c + 2 * CW < nch) nw[1] = *reinterpret_cast<const uint4*>(p.norm_w + (c + 2 * CW) * 256 + lane * 8);
+          nw[0] = nw[kNw - 1];
+          if (c + kNw * CW < nch) nw[kNw - 1] = *reinterpret_cast<const uint4*>(p.norm_w + (c + kNw * CW) * 256 + lane * 8);
           uint4* x = xs + XL::slot(c * 32 + lane, 0, xpitch);
 #pragma unroll 2
           for (int m = 0; m < p.M; ++m, x += xpitch) *x = scale_f16x8(*x, s_inv[m], w);
