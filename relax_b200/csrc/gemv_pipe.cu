@@ -1389,6 +1389,8 @@ int launch_pipe(const __half* x, const uint32_t* wq, const __half* scales, __hal
 //   eight columns            above one long stage always the shorter ones, whose eight warps share 256 k each, against sixteen that share
 //                            what is left of a long one: 8 x 5120 x 5120 11.3 / 9.3, 8 x 27648 x 5120 33.5 / 24.9, 7 x 7680 x 6144 14.6 / 12.0,
 //                            6 x 2560 x 6912 9.0 / 8.6, 5 x 4096 x 7680 10.0 / 9.5; 8 x 12288 x 3072 9.3 / 10.2
+//                            (eight warps on long stages, a form that is not built, had 6 x 28672 x 7168 33.0 where these take 34.1, and
+//                            6 x 16384 x 7168 21.4 / 20.7)
 template <int NC>
 bool half_stages(int n, int k) {
   constexpr size_t kRing = 8 * kRows * (128 + 16);                            // a short stage
@@ -1451,7 +1453,7 @@ int dispatch_form(const __half* x, const uint32_t* wq, const __half* scales, __h
   return with_form<8, 16>(m, n, k, [&](auto form) -> int {
     using Form = decltype(form);
     // (forms that no caller asks for are not built)
-    constexpr int kMaxNC = PRO == kPrologueNormStats || PRO == kPrologueRagged || EPI == kEpilogueAdd || EPI == kEpilogueStoreTwice ? 8 : 16;
+    constexpr int kMaxNC = EPI == kEpilogueStoreTwice ? 2 : PRO == kPrologueNormStats || PRO == kPrologueRagged || EPI == kEpilogueAdd ? 8 : 16;
     constexpr int kMinNC = PRO == kPrologueRagged ? 2 : 1;
     if constexpr (Form::NC < kMinNC || Form::NC > kMaxNC) return B200_ENOTREADY;
     else return launch_pipe<Form, PRO, EPI>(x, wq, scales, y, m, n, k, stream, pro, red);
@@ -1625,7 +1627,7 @@ int launch_gemv_pipe_ragged(const __half* x, const uint32_t* wq, const __half* s
   return dispatch_form<kPrologueRagged, kEpilogueStore>(x, wq, scales, y, (int)M, (int)N, (int)K, stream, Prologue{}, PeerReduce{});
 }
 
-// y = x . decode(W)^T, stored to y and to y2 (up to eight rows).
+// y = x . decode(W)^T, stored to y and to y2 (one or two rows).
 int launch_gemv_pipe_twice(const __half* x, const uint32_t* wq, const __half* scales, __half* y, __half* y2, int64_t M, int64_t N,
                            int64_t K, cudaStream_t stream) {
   Prologue pro;

@@ -11,7 +11,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("M", [1, 2, 3, 4, 5])
-@pytest.mark.parametrize("N,K", [(4096, 256), (4100, 2560), (4095, 512), (11008, 2048), (4096, 288)])
+@pytest.mark.parametrize("N,K", [(4096, 256), (4100, 2560), (4095, 512), (11008, 2048), (4096, 288), (1, 256), (17, 1024), (8192, 1024), (8200, 1024),
+                                 (16384, 1024), (16392, 1024), (12280, 4096), (12296, 4096)])
 def test_host_results(cuda_lib, M, N, K):
     wq, s = (torch.from_numpy(a).cuda() for a in synth.make_weights(N, K, np.random.default_rng(N + K)))
     gen = torch.Generator().manual_seed(M)
