@@ -143,12 +143,22 @@ bool weight_stationary_first(int64_t M, int64_t N, int64_t K, bool ragged) {
 
 // Of that, the skinny kernel's form for a ragged K takes two to four rows of the weight-stationary kernel's share and up to eight of the
 // streaming kernel's where K is long enough for its start-up.  Weight-stationary / skinny in us: 2 x 8640 x 3200 11.0 / 7.4,
-// 3 x 8640 x 3200 9.7 / 7.6, 4 x 12288 x 1056 6.3 / 6.0, 4 x 5120 x 5152 11.1 / 9.6, 2 x 4096 x 9248 12.3 / 9.8, 4 x 4096 x 11040 13.2 / 13.3,
-// but 5 x 4096 x 4128 8.4 / 8.3, 8 x 22016 x 2080 13.8 / 15.3, 8 x 4096 x 7200 11.1 / 12.8, 6 x 2560 x 6944 8.3 / 11.2; streaming / skinny:
-// 3 x 2048 x 5152 9.5 / 5.1, 8 x 512 x 2080 4.9 / 3.8, 4 x 4096 x 2080 5.1 / 4.9, but 2 x 4096 x 1056 3.1 / 3.4, 8 x 4096 x 1056 4.4 / 4.5.
+// 3 x 8640 x 3200 9.7 / 7.6, 4 x 12288 x 1056 6.3 / 6.0, 4 x 5120 x 5152 11.1 / 9.6, 2 x 4096 x 9248 12.3 / 9.8, 4 x 4096 x 7200 10.9 / 9.9,
+// but 5 x 4096 x 4128 8.4 / 8.6, 8 x 22016 x 2080 13.8 / 15.3, 8 x 4096 x 7200 11.1 / 12.8, 6 x 2560 x 6944 8.3 / 11.2; streaming / skinny:
+// 3 x 2048 x 5152 9.5 / 5.1, 8 x 512 x 2080 4.9 / 3.8, 4 x 4096 x 2080 5.2 / 4.7, but 2 x 4096 x 1056 3.1 / 3.4, 8 x 4096 x 1056 4.4 / 4.5.
+// Not from three rows on: few chunks of very many tiles (4 x 28672 x 1056 10.1 / 10.8, 4 x 24576 x 544 6.9 / 8.9), and a long K of one to two tiles an
+// SM (4 x 3072 x 9248 11.1 / 13.8, 3 x 4096 x 9248 12.5 / 13.6).  Not against the streaming kernel: where a wave of tiles leaves more than half of
+// the next one empty, with two rows (2 x 6144 x 2592 5.9 / 6.6) and for a short K (2 x 3072 x 2080 3.8 / 4.7, 3 x 6144 x 2080 5.7 / 6.5).
 bool skinny_ragged(int64_t M, int64_t N, int64_t K) {
   if (M < 2 || M > 8 || options().gemv_variant != 0) return false;
-  return weight_stationary_first(M, N, K, true) ? M <= 4 : K >= 2048;
+  const int64_t tiles = (N + 15) / 16, sms = sm_count();
+  if (weight_stationary_first(M, N, K, true)) {
+    if (M > 4) return false;
+    return M == 2 || !((K <= 1280 && N >= 14000) || (K > 8192 && tiles > sms && tiles <= 2 * sms));
+  }
+  const bool one_wave = 2 * tiles > 2 * sms && 2 * tiles < 3 * sms, two_waves = tiles > 2 * sms && tiles < 3 * sms;
+  if (M <= 4 && K < 2304 && (one_wave || two_waves)) return false;
+  return K >= 2048 && !(M == 2 && two_waves);
 }
 
 int matmul_impl(Family fam, const char* who, const void* x, const void* wq, const void* scales, void* y, int64_t M,
