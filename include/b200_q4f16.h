@@ -240,7 +240,7 @@ B200_API int b200_q4f16_gemv_swiglu(const void* gu, const void* wq, const void* 
 
 /* The same (x is the normalised activation) in the kernel that the automatic dispatch takes for more rows: act = silu(x . Wg^T) *
  * (x . Wu^T) for 1 <= M <= 128, any I and any K that b200_q4f16_matmul takes.  _applies: 1 where the automatic dispatch gives the
- * gate|up matmul to that kernel. */
+ * gate|up matmul to that kernel and SwiGLU in its epilogue is faster than a launch of its own. */
 B200_API int b200_q4f16_gate_up_applies(const void* scales, int64_t M, int64_t I, int64_t K);
 B200_API int b200_q4f16_gate_up(const void* x, const void* wq, const void* scales, void* act, int64_t M, int64_t I, int64_t K,
                                 void* cuda_stream);

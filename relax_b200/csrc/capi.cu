@@ -573,10 +573,11 @@ int b200_q4f16_gemv_gate_up(const void* x, const void* delta, const void* norm_w
   return rc;
 }
 
-// SwiGLU in the epilogue of the weight-stationary kernel, for the rows that the automatic dispatch gives to it.
+// SwiGLU in the epilogue of the weight-stationary kernel, where the automatic dispatch gives the matmul to it and that is the faster way.
 int b200_q4f16_gate_up_applies(const void* scales, int64_t M, int64_t I, int64_t K) {
   if (M < 1 || M > 128 || I < 1 || I > 0x3fffffffLL / 32 || K < 32 || K % 32 != 0 || !scales) return 0;
-  return weight_stationary_first(M, 2 * I, K, K % 256 != 0 || !aligned16(scales));
+  const bool ragged = K % 256 != 0 || !aligned16(scales);
+  return weight_stationary_first(M, 2 * I, K, ragged) && gemm_ws_gate_up_is_ahead(M, I, K, ragged);
 }
 
 int b200_q4f16_gate_up(const void* x, const void* wq, const void* scales, void* act, int64_t M, int64_t I, int64_t K, void* stream) {

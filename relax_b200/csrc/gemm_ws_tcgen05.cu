@@ -585,6 +585,20 @@ int max_clusters(int ksplit, const void* kern) {
 
 }  // namespace
 
+// Whether SwiGLU in the epilogue is faster than a launch of its own behind the matmul.  Up to 96 rows it is.  Above, the inbox
+// takes so much of a CTA's shared memory that a long run of one slice is slower, unless it is one that fills the SMs: separate / in the
+// epilogue in us, M x I x K 64 x 5632 x 4096 14.7 / 14.0, 96 x 11008 x 4096 27.7 / 26.4, 112 x 4096 x 5120 17.7 / 14.5 and 128 x 1024 x 4096
+// 11.6 / 9.9 (four slices), 128 x 8192 x 3072 16.7 / 16.2, but 128 x 1024 x 2048 10.1 / 11.2, 128 x 5632 x 5120 19.5 / 21.4,
+// 128 x 11008 x 1024 12.4 / 13.2, 112 x 8192 x 8192 31.1 / 34.4.
+bool gemm_ws_gate_up_is_ahead(int64_t M, int64_t I, int64_t K, bool ragged) {
+  if (M <= 96) return true;
+  const int64_t tiles = (I + BR / 2 - 1) / (BR / 2);
+  int clusters_of[4];
+  for (int i = 0; i < 4; ++i) clusters_of[i] = max_clusters(1 << i, reinterpret_cast<const void*>(kernel_for(16, false, ragged, false)));
+  if (tiles > 64) return 3 * tiles > 2 * clusters_of[0] && tiles <= clusters_of[0] && K <= 4096;
+  return choose_ws_split(M, tiles, (int)((K + 255) / 256), (int)options().gemm_ws_ksplit, clusters_of).ksplit > 1;
+}
+
 // Returns B200_ENOTREADY when the shape is outside what this kernel takes, or one for the prefill kernel.  gate_up: SwiGLU in the
 // epilogue (up to 128 rows, N even).
 int launch_gemm_ws(const __half* x, const uint32_t* wq, const __half* scales, __half* y, int64_t M, int64_t N,

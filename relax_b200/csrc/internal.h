@@ -81,6 +81,7 @@ int launch_gemv_pipe_allreduce(const __half* x, const uint32_t* wq, const __half
 // Sum over tensor-parallel ranks of `count` fp16 values whose per-rank partial results sit in peer-mapped buffers
 // (protocol of B200PeerReduce).
 int launch_peer_allreduce(int64_t count, const B200PeerReduce* red, cudaStream_t stream);
+bool gemm_ws_gate_up_is_ahead(int64_t M, int64_t I, int64_t K, bool ragged);
 int launch_gemm_ws(const __half* x, const uint32_t* wq, const __half* scales, __half* y, int64_t M, int64_t N,
                    int64_t K, cudaStream_t stream, bool gate_up = false);
 int launch_gemm(const __half* x, const uint32_t* wq, const __half* scales, __half* y, int64_t M, int64_t N,

@@ -52,3 +52,7 @@ def test_gate_up_refuses_and_applies(cuda_lib):
     assert cuda_lib.b200_q4f16_gate_up(p, None, p, p, 9, 8, 256, 0) == _lib.EINVAL
     assert cuda_lib.b200_q4f16_gate_up_applies(p, 9, 8, 256) == 1 and cuda_lib.b200_q4f16_gate_up_applies(p, 8, 8, 256) == 0
     assert cuda_lib.b200_q4f16_gate_up_applies(p, 129, 8, 256) == 0
+    # above 96 rows with several slices, or one round of single ones that fills the SMs
+    for M, I, K, one in ((96, 5632, 5120, 1), (97, 5632, 5120, 0), (128, 1024, 4096, 1), (128, 512, 512, 0), (128, 8192, 4096, 1), (128, 8192, 4352, 0),
+                         (128, 11008, 1024, 0)):
+        assert cuda_lib.b200_q4f16_gate_up_applies(p, M, I, K) == one, (M, I, K)
