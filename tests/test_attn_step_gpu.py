@@ -21,8 +21,8 @@ def _dev(a, offset):
     return out
 
 
-# (B, heads) by the warps that a pair gets: 64, 32, 16, 8, 4 (one wave), 8 (between one and two waves), 4 (more than two)
-SPLITS = [(1, 4), (2, 20), (5, 16), (5, 32), (10, 30), (21, 32), (40, 30)]
+# (B, heads) by the warps that a pair gets: 64, 32, 16, 8, 4 (one wave), 8 (a wave and a bit), 4 (most of two), 8 (two and a bit)
+SPLITS = [(1, 4), (2, 20), (5, 16), (5, 32), (10, 30), (21, 32), (32, 32), (40, 30)]
 
 
 @pytest.mark.parametrize("B,nh", SPLITS)
