@@ -257,6 +257,37 @@ def test_decoder_steps_match_oracle(cuda_lib, B, fused):
     assert cuda_lib.b200_device_error_flags() == 0
 
 
+# The default form of up to eight rows: chained throughout; with `down` in another kernel (a long K of 5..8 rows: weight-stationary; a K that is
+# no multiple of 256), so that its product is still to be added when the next layer, and the last norm, begin.
+@pytest.mark.parametrize("B,inter,chained_down", [(1, 768, True), (2, 768, True), (3, 768, True), (5, 768, True), (8, 768, True),
+                                                  (5, 8448, False), (8, 8448, False), (4, 8448, True), (1, 800, False), (3, 800, False), (8, 800, False)])
+def test_default_steps_match_oracle(cuda_lib, B, inter, chained_down):
+    cfg = decoder.DecoderConfig(hidden=512, heads=4, inter=inter, layers=3, vocab=500)
+    rng = np.random.default_rng(B + inter)
+    layers = [decoder.synth_layer_numpy(cfg, 300 + i) for i in range(cfg.layers)]
+    embed = (0.5 * rng.standard_normal((cfg.vocab, cfg.hidden))).astype(F16)
+    final_norm = (1 + 0.1 * rng.standard_normal(cfg.hidden)).astype(F16)
+    lm_head = (0.05 * rng.standard_normal((cfg.vocab, cfg.hidden))).astype(F16)
+    tokens = list(rng.integers(0, cfg.vocab, B))
+    max_ctx, steps = 32, 3
+    ref = oracle_steps(cfg, layers, embed, final_norm, lm_head, tokens, steps, max_ctx)
+    shards = [decoder.to_device(dict(l, inter_local=inter), "cuda") for l in layers]
+    eng = decoder.DecodeEngine(cfg, shards, dev(embed), dev(final_norm), dev(lm_head), B, max_ctx, "cuda")
+    assert eng.chained and all(eng._in_skinny(w["down"], cfg.hidden, inter) == chained_down for w in shards)
+    assert all(eng._in_skinny(w["o"], cfg.hidden, cfg.hidden) for w in shards)
+    for s in range(steps):
+        chosen = tokens if s == 0 else np.argmax(ref[s - 1][1].astype(np.float32), axis=1).astype(np.int32)
+        eng.tokens.copy_(torch.tensor(np.asarray(chosen), dtype=torch.int32))
+        launches = cuda_lib.b200_launch_count()
+        eng.step()
+        torch.cuda.synchronize()
+        assert cuda_lib.b200_launch_count() - launches == eng.kernels_per_step()
+        for got, want, what in ((eng.h, ref[s][0], "hidden state"), (eng.logits, ref[s][1], "logits")):
+            scale = np.abs(want.astype(np.float32)).max()
+            close(got.cpu().numpy(), want, 1e-2, 1e-2 * scale, f"{what} at step {s}")
+    assert cuda_lib.b200_device_error_flags() == 0
+
+
 def test_decoder_follows_the_matmul_options(cuda_lib):
     """At 2..8 rows every matmul of a step goes where b200_q4f16_matmul would take it: with the norm, the residual add and SwiGLU in the
     skinny kernel, or as the kernel that an option asks for with launches of their own for those; so does gate|up where its
