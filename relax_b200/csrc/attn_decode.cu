@@ -297,14 +297,16 @@ int launch_attn(const char* what, bool rope, AttnParams p, int64_t B, cudaStream
   const bool a16 = aligned(p.q, 16) && aligned(p.k_cache, 16) && aligned(p.v_cache, 16);
   // Warps per (head, batch): as many as the GPU holds at once, and no more than there are units.  64 only where half of the places
   // are enough (32 pairs at context 2012: 32 warps 51.6, 64 warps 52.4 us a layer of a step).  Above 592 pairs four warps each are
-  // more than one wave.  Where that leaves the last wave less than half full, eight warps each end sooner, unless the context is so short that
-  // they have little to do: 4 / 8 warps, us, 640 pairs at 1001 63.1 / 57.6, 800 at 2011 138.3 / 119.8, 1280 at 1501 156.3 / 145.2, 2048 at
-  // 1001 153.2 / 148.7, but 960 at 1001 74.2 / 79.1, 1024 at 130 14.4 / 18.9, 1536 at 1001 114.4 / 117.1, 640 at 130 12.4 / 13.5.  (A little
-  // more than a wave of pairs over a long context suits no split: 320 at 2011 60, where 128-token chunks in launches of their own took 56.)
+  // more than one wave; up to two waves of them leave too much of the second one empty (800 pairs at 1201: 4 warps 125, 8 warps
+  // 115 us), and so does a little more than two over a long context (1280 pairs at 1501 156.3 / 145.2; but at 301, inside a step, a layer took 114
+  // us with four and 117 with eight).  (A little more than one wave of pairs over a long context suits no split: 320 at 2011 60 us, where
+  // 128-token chunks in launches of their own took 56.)
   const int64_t pairs = B * p.nh;
   const int64_t slots = (int64_t)sm_count() * 16;
-  const int64_t last = pairs * 4 % slots;
-  int t = pairs * 4 > slots && last > 0 && 2 * last < slots && p.max_ctx > 16 * kUnit ? 8 : 4;
+  const int64_t last = pairs * 4 % slots;                  // of the last wave of four warps a pair
+  const bool second = pairs * 4 > slots && pairs * 2 < slots && p.max_ctx > 4 * kUnit;
+  const bool later = pairs * 2 >= slots && last > 0 && 2 * last < slots && p.max_ctx > 80 * kUnit;
+  int t = second || later ? 8 : 4;
   while (pairs * 2 * t <= (t == 32 ? slots / 2 : slots) && t < 64 && t * kUnit < p.max_ctx) t *= 2;
   const int w = t < 8 ? 4 : 8, c = t / w;
   auto pick = [&](auto k44, auto k48) { return w == 8 ? k48 : k44; };

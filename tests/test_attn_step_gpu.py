@@ -21,14 +21,14 @@ def _dev(a, offset):
     return out
 
 
-# (B, heads) by the warps that a pair gets: 64, 32, 16, 8, 4 (one wave), 8 (a wave and a bit), 4 (most of two), 8 (two and a bit)
-SPLITS = [(1, 4), (2, 20), (5, 16), (5, 32), (10, 30), (21, 32), (32, 32), (40, 30)]
+# (B, heads) by the warps that a pair gets: 64, 32, 16, 8, 4 (one wave), 8 (between one and two waves), 4 (more than two)
+SPLITS = [(1, 4), (2, 20), (5, 16), (5, 32), (10, 30), (21, 32), (40, 30)]
+LONG = (41, 29)                                          # (more than two waves, and a cache of more than 1280 tokens: 8)
 
 
-@pytest.mark.parametrize("B,nh", SPLITS)
-@pytest.mark.parametrize("ctx", [1, 2, 16, 17, 18, 33, 130, 515])
+@pytest.mark.parametrize("ctx,B,nh", [(ctx, *split) for ctx in (1, 2, 16, 17, 18, 33, 130, 515) for split in SPLITS] + [(17, *LONG), (515, *LONG)])
 def test_step_attention_against_the_oracle(cuda_lib, B, nh, ctx):
-    max_ctx = 1040 if B * nh < 200 else 528
+    max_ctx = 1040 if B * nh < 200 else 1296 if (B, nh) == LONG else 528
     offset = 4 if ctx in (17, 130) else 0                # 8-byte aligned only
     flags = 3 if ctx in (2, 33, 515) else 0              # (nothing that they may read early is written by the launch in front)
     pos = ctx - 1

@@ -31,19 +31,21 @@ def exhaustive(m, row_tiles, units, forced, clusters):
             if c > units or (forced and not (c <= forced and (c * 2 > forced or c * 2 > units or c == 8))):
                 continue
             rounds = -(-tiles // clusters[i])
-            span = max(520 + nb if nb <= 128 else 760 + nb, tiles * c // rounds * (nb * 512 + 18432) // (14000 if c == 1 else 13000))
+            span = max(520 + nb if nb <= 128 else 760 + nb, tiles * c // rounds * (nb * 512 + 18432) // 14000)
             tile = -(-units // c) * span
             drain = 300 + 12 * nb if c == 1 else 800 + 50 * nb
-            crowd = max(tiles - (rounds - 1) * clusters[i] + min(tiles, clusters[i]) - clusters[i] - (2 if c == 8 else 0), 0)
-            room = m <= 128 and c >= 4 and rounds == 1 and crowd == 0
-            if m > 128:
-                start = (0, 0, 600, 1900)[i]
-            elif room:
+            room = m <= 128 and c >= 4 and 2 * tiles <= clusters[i] + (2 if c == 8 else 0)
+            if room:
                 start = 1600 - 8 * nb if c == 8 and tiles > 4 else 0
             else:
-                start = (0, 500, 0, 3000)[i] + (0, 2000, 2400, 1300)[i] * crowd // clusters[i]
-            tail = drain if c == 1 else 900 + 38 * nb if room else 300 + 38 * nb if m <= 128 else 400 + 35 * nb
+                start = (0, 500, 1000, 3500)[i]
+                if m <= 128 and rounds == 1 and 2 * tiles > clusters[i]:
+                    crowd = (0, 500, 2400, 0)[i] * (2 * tiles - clusters[i]) // clusters[i]
+                    start = max(start, crowd) if c == 4 else start + crowd
+            tail = drain if c == 1 else 900 + 38 * nb if room else 600 + 35 * nb
             cost = start + tile + (rounds - 1) * max(tile, drain) + tail
+            if m > 128 and c > 1:
+                cost += cost * 15 // 1000
             if best is None or cost < best[0]:
                 best = (cost, nb, c)
     return best[1:]
@@ -87,7 +89,7 @@ def test_long_prompts_that_one_wave_of_the_prefill_kernel_holds(program):
 
 def test_slices_where_clusters_crowd_the_gpu(program):
     # as measured: the best number of slices (four, two or one were taken for them: 5-30 % slower)
-    for best, shapes in ((2, [(8, 4096, 2080), (16, 4096, 2080), (16, 4096, 2560), (9, 22016, 3200)]),
+    for best, shapes in ((2, [(8, 4096, 2080), (16, 4096, 2080), (16, 4096, 2560)]),
                          (1, [(64, 8192, 2080), (96, 8192, 2560), (96, 6144, 2560), (777, 12288, 7168), (777, 12288, 8192)]),
                          (4, [(9, 10240, 5120), (33, 10240, 7168), (16, 2560, 4096), (64, 2560, 2560), (16, 4096, 11008), (16, 4096, 5120), (24, 1024, 4096), (16, 2048, 11008)]),
                          (8, [(16, 512, 8192)])):
