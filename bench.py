@@ -375,11 +375,12 @@ def run_decode(args, world, rank, dev, batches):
             "bytes_per_step_per_gpu": per_rank,
             "hbm_frac_of_measured": per_rank / (ms / steps * 1e-3) / 1e9 / measured_peaks()["hbm_gbs"],
             "kernels_per_step": eng.kernels_per_step(), "engine": "one persistent kernel per layer" if eng.layer_kernel else
-            "fused prologues, skinny kernels" if eng.fused else
-            "separate RMSNorm/SwiGLU kernels, mid-batch tensor-core matmul",
+            "residual add, norms and SwiGLU inside the skinny matmuls" if eng.chained else
+            "norms and SwiGLU inside the skinny matmuls, residual stream by launches" if eng.fused else
+            "RMSNorm launches, SwiGLU in the epilogue of gate|up",
             "lm_head": ("fp16, tied to the embedding, vocabulary-sharded; this library's kernel (b200_lm_head)"
-                        + (", greedy token inside it" if world == 1 else ", torch argmax over the gathered slices")
-                        if batch <= 16 else "fp16, tied to the embedding, vocabulary-sharded (library GEMM + torch argmax above 16 rows)"),
+                        + (", greedy token inside it" if world == 1 else ", b200_argmax_rows over the gathered slices")
+                        if batch <= 16 else "fp16, tied to the embedding, vocabulary-sharded (library GEMM + b200_argmax_rows above 16 rows)"),
             "allreduce": (None if world == 1 else "NCCL fp16, 2 per layer" if eng.peer is None else
                           "fused into the o/down matmul kernels over NVLink peer memory (fp16 partials, rank-order sum)"
                           if batch <= eng.PEER_FUSED_MAX_ROWS else

@@ -16,8 +16,8 @@
 // memory, no counters, no second launch.  (Clusters of 16 CTAs were slower: one starts only where 16 places in a GPC are free at
 // once.)
 //
-// What bounds it: HBM from about 300 pairs on (64 x 32 heads at 1002: 150 us, 7.0 TB/s of the 6.45 a copy reaches; 16 x 32 at 2012
-// 76 us, 6.9), below that latency.  Against three launches (rotary + append, 128-token chunks, merge) a layer of a decode step
+// What bounds it: HBM from about 400 pairs on (64 x 32 heads at 1002: 150 us, reading 7.0 TB/s; 16 x 32 at 2012 76 us, 6.9; a copy, half
+// of it writes, moves 6.45), below that latency.  Against three launches (rotary + append, 128-token chunks, merge) a layer of a decode step
 // took, us, before / after: hidden 4096, 1 row at 2012 53.4 / 51.6, 2 at 1501 61.7 / 54.4, 8 at 151 71.5 / 65.7, 16 at 2012
 // 144.7 / 133.4, 64 at 1002 232.6 / 222; hidden 2048, 5 rows at 334 40.5 / 37.6; hidden 1024, 64 at 61 39.9 / 33.2.
 #include "internal.h"

@@ -18,10 +18,9 @@
 //                and feeds mma.sync m16n8k16 with x fragments read from a copy of x kept in
 //                shared memory in the matching permuted order.
 //   row tile   = 16 rows over the whole K range; each warp leaves its partial sums in shared
-//                memory and bumps a counter; the warp that arrives last adds them up (in warp
-//                order, so the result does not depend on who is last) and stores fp16.  Nobody
-//                waits at a tile boundary, so the warps drift apart and the shared-memory loads
-//                of one overlap the arithmetic of another.
+//                memory and arrives on a barrier; an epilogue warp adds them up in warp order and
+//                stores fp16.  No consumer waits at a tile boundary, so the warps drift apart and
+//                the shared-memory loads of one overlap the arithmetic of another.
 //   CTA        = row tiles blockIdx.x, blockIdx.x + gridDim.x, ...
 //
 // When x does not fit beside the ring (large M*K) the K range is cut into blocks: x is restaged
@@ -53,8 +52,8 @@
 //          |y - y_ref| <= 2^-11 * sum|x*w| (typically 3e-4 of the output's spread); an activation
 //          with a single 1.0 still reproduces the reference's weight bit for bit.
 //
-// Requires K % 256 == 0 and 16-byte aligned scales (tensor-map stride rules); other shapes use
-// the register-streaming kernel.
+// A row of scales can be a row of a tensor map only where K % 256 == 0 and the scales are 16-byte aligned.  Other shapes of two to
+// eight rows have a form that fetches its scales itself (kPrologueRagged); the rest goes to the register-streaming kernel.
 #include "internal.h"
 #include "q4_common.cuh"
 #include "skinny_common.cuh"

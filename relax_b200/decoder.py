@@ -119,10 +119,10 @@ class DecodeEngine:
         f16 = dict(dtype=torch.float16, device=self.device)
         hl = H // world
         il_max = max(l["inter_local"] for l in layers) if layers else cfg.inter
-        # fused: RMSNorm (+ residual add) runs inside the staging of the next skinny matmul; needs batch <= 16, the skinny
-        # kernel's range.  By default only at batch 1: every CTA of a fused kernel recomputes the statistics of all the batch's rows, and from two rows on
-        # the separate kernels are faster (measured per layer at context 2000: 80 against 88 us at batch 2, 124 against
-        # 176 at batch 8, 174 against 291 at batch 16).
+        # fused: RMSNorm (+ residual add) runs inside the staging of the next skinny matmul, which forms the statistics itself; needs
+        # batch <= 16, the skinny kernel's range.  Only on request, and at batch 1 where the chained form does not apply: every CTA
+        # of a fused kernel recomputes the statistics of all the batch's rows, and from two rows on separate norms are faster
+        # (when both forms had the same kernels besides, a layer at context 2000: 80 against 88 us at batch 2, 124 against 176 at batch 8).
         self.fused = (B == 1) if fused is None else (bool(fused) and B <= 16)
         # chained: up to 8 rows, o and down add their product to the residual stream themselves and leave the sums of squares of its
         # rows behind, from which qkv, gate|up and the output projection normalise it while they stage it: no launch for the norms.
@@ -155,13 +155,13 @@ class DecodeEngine:
         self.lm_scratch = torch.zeros((max(int(self.L.b200_lm_head_scratch_bytes()), 16) // 4,), dtype=torch.float32, device=self.device)
         self.graph = None
         self.launches_per_step = 0
-        # batch 1: one persistent kernel per layer (b200_decode_layer) instead of six launches.  Off by default:
-        # measured on B200 at the 7B shape it is slower (2.00 against 1.64 ms per token), because every stage boundary
+        # batch 1: one persistent kernel per layer (b200_decode_layer) instead of five launches.  Off by default:
+        # measured on B200 at the 7B shape it is slower (2.00 against 1.53 ms per token), because every stage boundary
         # inside it costs what a dependent launch costs, and its attention stage has only eight warps per SM with loads in
         # flight
         self.layer_kernel = False if layer_kernel is None else bool(layer_kernel)
-        # batch 1, fused prologues: rotary embedding + KV append run in the epilogue of the qkv matmul
-        # (b200_q4f16_gemv_rmsnorm_rope)
+        # batch 1: rotary embedding + KV append run in the epilogue of the qkv matmul (b200_q4f16_gemv_norm_rope, with fused
+        # prologues b200_q4f16_gemv_rmsnorm_rope)
         self.rope_epilogue = bool(rope_epilogue) and self.fused and B == 1 and not self.fused_attention and not self.layer_kernel
         if self.layer_kernel and B != 1:
             raise ValueError("the one-kernel-per-layer path is the batch-1 path")

@@ -162,8 +162,9 @@ def _torch_call():
 
 def q4f16_matmul(x: torch.Tensor, wq: torch.Tensor, scales: torch.Tensor, out: torch.Tensor | None = None,
                  family: str = "auto", layout=None) -> torch.Tensor:
-    """y[M,N] fp16 = x[M,K] . decode(wq[N,K/8], scales[N,K/32])^T, through the DLPack entry point
-    (all validation happens in the library).  ``family`` = "auto" | "gemv" | "gemm" picks the raw
+    """y[M,N] fp16 = x[M,K] . decode(wq[N,K/8], scales[N,K/32])^T.  Plain contiguous tensors on the current device go
+    straight to the raw-pointer entry point (through the extension, or with the same checks in Python); everything else goes
+    through the DLPack entry point, which validates it and names the error.  ``family`` = "auto" | "gemv" | "gemm" picks the raw
     entry point of one kernel family instead.  ``layout`` ("reference" | "paired") names the nibble order
     of ``wq`` for this call; None takes the library's option "weights.layout"."""
     if out is None:
