@@ -248,19 +248,32 @@ using namespace b200;
 // then starts beside it (it reads only weights before its own wait), but not beside the call in front, whose matmul it
 // would take the SMs from.  Without the attribute on the copy of x / with it, us a call among others: 1 x 4096 x 4096 12.4 / 11.1,
 // 1 x 8192 x 8192 18.2 / 16.4, 4 x 22016 x 4096 28.0 / 25.9, 6 x 4096 x 4096 17.2 / 14.4, 16 x 4096 x 4096 19.2 / 18.3.
-// A short call of one or two rows is bound by its launches, and there the skinny matmul stores the result to the host buffer itself, next
-// to y_dev, in pieces of 32 bytes (one row) or 16: a launch less.  A longer one is bound by the GPU, and those stores, most of
-// them at the end of the matmul, take the bus longer than a copy does, unless a CTA has several long tiles, beside which the stores of
-// the ones before go out.  Copy / direct, us a call among others, 1 x 512 x 1024 12.1 / 10.0,
-// 1 x 4096 x 4096 12.3 / 10.2, 2 x 2048 x 4096 12.1 / 10.6, 2 x 8192 x 1024 12.1 / 11.1, but 1 x 12288 x 2048 12.1 / 12.6, 1 x 4096 x 8192 12.2 / 12.8,
-// 1 x 4096 x 11008 14.3 / 15.3, 2 x 8192 x 2048 12.1 / 12.3, 2 x 22016 x 1024 14.2 / 16.1, 3 x 12288 x 2048 13.5 / 15.8, 4 x 4096 x 4096 12.5 / 13.3,
-// 4 x 22016 x 1024 16.4 / 23.3; 1 x 16384 x 4096 18.1 / 17.5, 2 x 22016 x 4096 22.5 / 21.4, 2 x 12288 x 8192 24.2 / 23.5, 1 x 22016 x 11008 35.5 / 35.5.
+// The skinny matmul can store the result to the host buffer itself, next to y_dev, in pieces of 32 bytes (one row) or 16: a launch less, but
+// most of those stores come at the end of the matmul and take the bus longer than a copy does.  Launched by the host, one or two rows of a
+// short call are bound by the launches, and a CTA with several long tiles sends the stores of the first beside the last; elsewhere the copy is
+// faster.  Copy / direct, us a call among others, 1 x 512 x 1024 12.1 / 10.0, 1 x 4096 x 4096 12.3 / 10.2, 2 x 2048 x 4096 12.1 / 10.6, 2 x 8192 x 1024
+// 12.1 / 11.1, 1 x 16384 x 4096 18.1 / 17.5, 2 x 22016 x 4096 22.5 / 21.4, but 1 x 12288 x 2048 12.1 / 12.6, 1 x 4096 x 8192 12.2 / 12.8, 1 x 4096 x 11008
+// 14.3 / 15.3, 2 x 8192 x 2048 12.1 / 12.3, 2 x 22016 x 1024 14.2 / 16.1, 3 x 12288 x 2048 13.5 / 15.8, 4 x 4096 x 4096 12.5 / 13.3, 4 x 22016 x 1024 16.4 / 23.3.
+// Replayed from a graph, where launches follow each other without the host, it is faster for up to four rows unless they have many outputs of
+// a short K: 1 x 512 x 1024 6.3 / 4.8, 1 x 4096 x 11008 11.8 / 10.9, 3 x 12288 x 4096 14.2 / 12.8, 4 x 22016 x 11008 45.8 / 42.4, but 3 x 12288 x 1024 9.0 / 9.9,
+// 4 x 22016 x 1024 12.4 / 17.7.
 // Pageable host memory and larger transfers use cudaMemcpyAsync.
 namespace b200 {
 namespace {
 constexpr size_t kHostKernelBytes = 256 * 1024;
 constexpr size_t kHostCopyCtas = 8;
-constexpr int64_t kHostDirectRows = 2, kHostDirectProducts = 1 << 24, kHostDirectN = 12288;
+
+// Whether the matmul stores its result to the host buffer itself.
+bool host_direct(int64_t M, int64_t N, int64_t K, cudaStream_t s) {
+  if (M > 4) return false;
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &status) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  if (status == cudaStreamCaptureStatusActive) return M <= 2 || K >= 4096 || M * N <= 12288 + 8 * K;
+  return M <= 2 && (M * N * K <= 1 << 24 || (N >= 12288 && K >= 4096));
+}
 
 __global__ void __launch_bounds__(256) host_copy_kernel(const unsigned char* __restrict__ src, unsigned char* __restrict__ dst,
                                                         size_t bytes) {
@@ -767,9 +780,8 @@ int b200_q4f16_matmul_host(const void* x_host, void* x_dev, const void* wq, cons
     }
   }
   void* ym = yb > 0 && yb <= kHostKernelBytes && !(reinterpret_cast<uintptr_t>(y_host) & 15) ? mapped_host_pointer(y_host) : nullptr;
-  if (ym && xb > 0 && M <= kHostDirectRows && (N * K <= kHostDirectProducts / M || (N >= kHostDirectN && K >= 4096)) &&
-      options().gemv_variant != 1 && K % 256 == 0 && aligned16(scales) &&
-      !weight_stationary_first(M, N, K, false)) {
+  if (ym && xb > 0 && options().gemv_variant != 1 && K % 256 == 0 && aligned16(scales) && !weight_stationary_first(M, N, K, false) &&
+      host_direct(M, N, K, s)) {
     rc = launch_gemv_pipe_twice(static_cast<const __half*>(x_dev), static_cast<const uint32_t*>(wq), static_cast<const __half*>(scales),
                                 static_cast<__half*>(y_dev), static_cast<__half*>(ym), M, N, K, s);
     if (rc != B200_ENOTREADY) return rc;

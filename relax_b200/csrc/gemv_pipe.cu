@@ -1452,7 +1452,7 @@ int dispatch_form(const __half* x, const uint32_t* wq, const __half* scales, __h
   return with_form<8, 16>(m, n, k, [&](auto form) -> int {
     using Form = decltype(form);
     // (forms that no caller asks for are not built)
-    constexpr int kMaxNC = EPI == kEpilogueStoreTwice ? 2 : PRO == kPrologueNormStats || PRO == kPrologueRagged || EPI == kEpilogueAdd ? 8 : 16;
+    constexpr int kMaxNC = EPI == kEpilogueStoreTwice ? 4 : PRO == kPrologueNormStats || PRO == kPrologueRagged || EPI == kEpilogueAdd ? 8 : 16;
     constexpr int kMinNC = PRO == kPrologueRagged ? 2 : 1;
     if constexpr (Form::NC < kMinNC || Form::NC > kMaxNC) return B200_ENOTREADY;
     else return launch_pipe<Form, PRO, EPI>(x, wq, scales, y, m, n, k, stream, pro, red);
@@ -1626,7 +1626,7 @@ int launch_gemv_pipe_ragged(const __half* x, const uint32_t* wq, const __half* s
   return dispatch_form<kPrologueRagged, kEpilogueStore>(x, wq, scales, y, (int)M, (int)N, (int)K, stream, Prologue{}, PeerReduce{});
 }
 
-// y = x . decode(W)^T, stored to y and to y2 (one or two rows).
+// y = x . decode(W)^T, stored to y and to y2 (up to four rows).
 int launch_gemv_pipe_twice(const __half* x, const uint32_t* wq, const __half* scales, __half* y, __half* y2, int64_t M, int64_t N,
                            int64_t K, cudaStream_t stream) {
   Prologue pro;
