@@ -23,12 +23,12 @@ def _dev(a, offset):
 
 # (B, heads) by the warps that a pair gets: 64, 32, 16, 8, 4 (one wave), 8 (between one and two waves), 4 (more than two)
 SPLITS = [(1, 4), (2, 20), (5, 16), (5, 32), (10, 30), (21, 32), (40, 30)]
-LONG = (41, 29)                                          # (more than two waves, and a cache of more than 1280 tokens: 8)
 
 
-@pytest.mark.parametrize("ctx,B,nh", [(ctx, *split) for ctx in (1, 2, 16, 17, 18, 33, 130, 515) for split in SPLITS] + [(17, *LONG), (515, *LONG)])
+@pytest.mark.parametrize("B,nh", SPLITS)
+@pytest.mark.parametrize("ctx", [1, 2, 16, 17, 18, 33, 130, 515])
 def test_step_attention_against_the_oracle(cuda_lib, B, nh, ctx):
-    max_ctx = 1040 if B * nh < 200 else 1296 if (B, nh) == LONG else 528
+    max_ctx = 1040 if B * nh < 200 else 528
     offset = 4 if ctx in (17, 130) else 0                # 8-byte aligned only
     flags = 3 if ctx in (2, 33, 515) else 0              # (nothing that they may read early is written by the launch in front)
     pos = ctx - 1
@@ -69,6 +69,31 @@ def test_step_attention_against_the_oracle(cuda_lib, B, nh, ctx):
                                      B, nh, max_ctx, flags & 1, 0) == 0, _lib.last_error()
     torch.cuda.synchronize()
     got = again.cpu().numpy()[rows].astype(np.float64)
+    assert (np.abs(got - ref) <= 2e-3 + 4e-3 * np.abs(ref)).all(), np.abs(got - ref).max()
+
+
+@pytest.mark.parametrize("ctx", [17, 515])
+def test_a_little_more_than_two_waves_over_a_long_cache(cuda_lib, ctx):
+    """Four warps a pair would leave a third wave nearly empty, and the cache has more than 1280 tokens: eight."""
+    B, nh, max_ctx, pos = 41, 29, 1296, ctx - 1
+    rng = np.random.default_rng(ctx)
+    kc, vc = (np.full((B, max_ctx, nh, D), np.nan, F16) for _ in "kv")
+    kc[:, :pos], vc[:, :pos] = (rng.standard_normal((B, pos, nh, D)).astype(F16) for _ in "kv")
+    qkv = rng.standard_normal((B, 3 * nh * D)).astype(F16)
+    cos, sin = odec.rope_tables(max_ctx, D)
+    tk, tv, tq = (_dev(a, 0) for a in (kc, vc, qkv))
+    tcos, tsin = (torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (cos, sin))
+    tpos = torch.tensor([pos], dtype=torch.int32, device="cuda")
+    out = torch.full((B, nh * D), float("nan"), dtype=torch.float16, device="cuda")
+    torch.cuda.synchronize()
+    assert cuda_lib.b200_attn_decode_step(tq.data_ptr(), tcos.data_ptr(), tsin.data_ptr(), tpos.data_ptr(), tk.data_ptr(), tv.data_ptr(),
+                                          out.data_ptr(), B, nh, max_ctx, 3, 0) == 0, _lib.last_error()
+    torch.cuda.synchronize()
+    rows = [0, B // 2, B - 1]
+    q = odec.rope(qkv[:, :nh * D].reshape(B, nh, D), cos[pos], sin[pos])
+    kc[:, pos], vc[:, pos] = tk.cpu().numpy()[:, pos], qkv[:, 2 * nh * D:].reshape(B, nh, D)
+    ref = odec.attention_decode(q[rows], kc[rows], vc[rows], ctx).astype(np.float64)
+    got = out.cpu().numpy()[rows].astype(np.float64)
     assert (np.abs(got - ref) <= 2e-3 + 4e-3 * np.abs(ref)).all(), np.abs(got - ref).max()
 
 

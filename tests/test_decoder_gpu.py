@@ -289,18 +289,15 @@ def test_default_steps_match_oracle(cuda_lib, B, inter, chained_down):
 
 
 def test_decoder_follows_the_matmul_options(cuda_lib):
-    """At 2..8 rows every matmul of a step goes where b200_q4f16_matmul would take it: with the norm, the residual add and SwiGLU in the
-    skinny kernel, or as the kernel that an option asks for with launches of their own for those; so does gate|up where its
-    scales come to lie off 16 bytes after the engine was built."""
+    """At 2..8 rows gate|up goes where b200_q4f16_matmul would take it: with SwiGLU in the epilogue, or as the kernel that an option
+    asks for and a SwiGLU launch behind it; scales that come to lie off 16 bytes after the engine was built take that way too."""
     cfg, B = SMALL, 5
     rng = np.random.default_rng(17)
     layers = [decoder.to_device(tp.shard_layer(decoder.synth_layer_numpy(cfg, 40 + i), 0, 1, cfg.hidden, cfg.inter), "cuda") for i in range(cfg.layers)]
-    made = (dev((0.5 * rng.standard_normal((cfg.vocab, cfg.hidden))).astype(F16)), dev(np.ones(cfg.hidden, F16)),
-            dev((0.05 * rng.standard_normal((cfg.vocab, cfg.hidden))).astype(F16)), B, 16, "cuda")
-    eng = decoder.DecodeEngine(cfg, layers, *made)
-    apart = decoder.DecodeEngine(cfg, layers, *made, fused=False)            # a launch of its own for everything but the matmuls
+    eng = decoder.DecodeEngine(cfg, layers, dev((0.5 * rng.standard_normal((cfg.vocab, cfg.hidden))).astype(F16)), dev(np.ones(cfg.hidden, F16)),
+                               dev((0.05 * rng.standard_normal((cfg.vocab, cfg.hidden))).astype(F16)), B, 16, "cuda")
 
-    def step(eng=eng):
+    def step():
         eng.set_position(0)
         eng.tokens.copy_(torch.arange(B, dtype=torch.int32))
         before = cuda_lib.b200_launch_count()
@@ -313,14 +310,9 @@ def test_decoder_follows_the_matmul_options(cuda_lib):
     try:
         _lib.set_option("gemv.variant", 1)
         count1, out1 = step()
-        assert count1 == eng.kernels_per_step()
-        # the same kernels in both engines (the streaming one for all four matmuls), so the same bits
-        assert (out1 == step(apart)[1]).all()
     finally:
         _lib.set_option("gemv.variant", 0)
-    # two norms and SwiGLU a layer, and the last norm
-    assert count1 == count + 3 * cfg.layers + 1
-    assert (step(apart)[1] != out1).any(), "the two kernels differ in the order of their sums"
+    assert count1 == count + 3 * cfg.layers + 1         # (two norms and SwiGLU a layer, and the last norm)
     close(out1, ref, 1e-2, 1e-2 * scale, "streaming kernel")
     for w in layers:
         off = torch.empty(w["gu"][1].numel() + 1, dtype=torch.float16, device="cuda")[1:].view(w["gu"][1].shape)
@@ -329,6 +321,36 @@ def test_decoder_follows_the_matmul_options(cuda_lib):
     count2, out2 = step()
     assert count2 == count + cfg.layers
     close(out2, ref, 1e-2, 1e-2 * scale, "scales off 16 bytes")
+    assert cuda_lib.b200_device_error_flags() == 0
+
+
+def test_every_matmul_of_a_step_follows_the_variant(cuda_lib):
+    """With gemv.variant = 1 the chained engine and the one with a launch for everything but the matmuls run the same kernels (the
+    streaming one for all four matmuls) and have the same bits."""
+    cfg, B = SMALL, 5
+    rng = np.random.default_rng(18)
+    layers = [decoder.to_device(tp.shard_layer(decoder.synth_layer_numpy(cfg, 40 + i), 0, 1, cfg.hidden, cfg.inter), "cuda") for i in range(cfg.layers)]
+    made = (dev((0.5 * rng.standard_normal((cfg.vocab, cfg.hidden))).astype(F16)), dev(np.ones(cfg.hidden, F16)),
+            dev((0.05 * rng.standard_normal((cfg.vocab, cfg.hidden))).astype(F16)), B, 16, "cuda")
+    eng, apart = decoder.DecodeEngine(cfg, layers, *made), decoder.DecodeEngine(cfg, layers, *made, fused=False)
+    assert eng.chained and not apart.chained
+
+    def logits(eng):
+        eng.set_position(0)
+        eng.tokens.copy_(torch.arange(B, dtype=torch.int32))
+        before = cuda_lib.b200_launch_count()
+        eng.step()
+        torch.cuda.synchronize()
+        assert cuda_lib.b200_launch_count() - before == eng.kernels_per_step()
+        return eng.logits.float().cpu().numpy()
+
+    try:
+        _lib.set_option("gemv.variant", 1)
+        streaming = logits(eng)
+        assert (streaming == logits(apart)).all()
+    finally:
+        _lib.set_option("gemv.variant", 0)
+    assert (logits(apart) != streaming).any(), "the two kernels differ in the order of their sums"
     assert cuda_lib.b200_device_error_flags() == 0
 
 

@@ -1,6 +1,5 @@
 """Two to eight rows with a K of whole scale groups only, or scales off 16 bytes: the skinny kernel's form for them against the oracle at
-the ends of its chunks (256 k), stages and row tiles, both layouts; nothing past the ends may be used.  (Of the small sizes those of a K
-below 2048 go to the streaming kernel, large products of five and eight rows to the weight-stationary one: the same holds for them.)"""
+the ends of its chunks (256 k), stages and row tiles, both layouts; nothing past the ends may be used."""
 import numpy as np
 import pytest
 
@@ -10,15 +9,6 @@ from oracle import q4f16
 from relax_b200 import _lib, ops, synth
 
 pytestmark = pytest.mark.gpu
-
-
-@pytest.mark.parametrize("M,N,K", [
-    # K within one stage, many tiles a CTA (smaller products of so short a K are the streaming kernel's)
-    (4, 12289, 1056), (3, 13985, 1248), (4, 8001, 1568), (3, 9440, 1824), (4, 6353, 2016),
-    # the ends of the dispatch's ranges: on the other side are the weight-stationary and the streaming kernel
-    (4, 14000, 1056), (4, 13999, 1056), (3, 2384, 8224), (3, 2368, 8224), (2, 4752, 2592), (2, 4736, 2592), (3, 2384, 2080), (3, 3552, 2080)])
-def test_short_k_and_dispatch(cuda_lib, M, N, K):
-    test_ragged_rows(cuda_lib, M, N, K)
 
 
 @pytest.mark.parametrize("M", [2, 3, 4, 5, 8])
@@ -50,3 +40,14 @@ def test_ragged_rows(cuda_lib, M, N, K):
     # the bound of the parity tests: fp32 sums and one fp16 rounding
     assert (np.abs(got - ref) <= 2.0 ** -10 * np.abs(ref) + 8e-6 * (np.abs(xf) @ np.abs(w).T)).all(), np.abs(got - ref).max()
     assert bool(torch.isnan(y[M]).all())
+
+
+# (Of the small sizes above those of a K below 2048 go to the streaming kernel, large products of five and eight rows to the
+# weight-stationary one: the same holds for them.)
+@pytest.mark.parametrize("M,N,K", [
+    # K within one stage, many tiles a CTA (smaller products of so short a K are the streaming kernel's)
+    (4, 12289, 1056), (3, 13985, 1248), (4, 8001, 1568), (3, 9440, 1824), (4, 6353, 2016),
+    # the ends of the dispatch's ranges: on the other side are the weight-stationary and the streaming kernel
+    (4, 14000, 1056), (4, 13999, 1056), (3, 2384, 8224), (3, 2368, 8224), (2, 4752, 2592), (2, 4736, 2592), (3, 2384, 2080), (3, 3552, 2080)])
+def test_short_k_and_dispatch(cuda_lib, M, N, K):
+    test_ragged_rows(cuda_lib, M, N, K)
