@@ -4,7 +4,7 @@
 // The reference has no attention op; the semantics are the composition of its elementwise ops, statistics in fp32,
 // one fp16 rounding of the rotated q and k and one of the result, which is what the oracle's restatement does too.
 //
-// Work: a cluster of 1, 2, 4 or 8 CTAs per (head, batch).  The cache entries older than the new token are cut into units of 16
+// Work: a cluster of 1, 2, 4 or 8 CTAs of four, five or eight warps per (head, batch).  The cache entries older than the new token are cut into units of 16
 // tokens that are dealt out over all warps of the cluster.  Lane l of a warp holds dims 8 (l % 16).. + 7 of token
 // 2 j + l / 16 of a unit, so that a load is 16 bytes a lane, a score takes four shuffles for two tokens, and the two halves of
 // a warp keep their own online softmax until the end.  The keys of the next unit are requested as soon as this one's scores are
@@ -88,7 +88,7 @@ __device__ __forceinline__ float dot8(const float (&q)[8], const uint4& k) {
   return s;
 }
 
-// W warps.  128 registers a thread, 16 warps an SM: each has 8 KB of keys and values in flight.
+// W warps.  At least 128 registers a thread, 16 (W = 5: 15) warps an SM: each has 8 KB of keys and values in flight.
 template <int W, bool ROPE, bool A16>
 __global__ void __launch_bounds__(W * 32, 16 / W)
 attn_decode_kernel(const AttnParams p) {
@@ -228,7 +228,8 @@ attn_decode_kernel(const AttnParams p) {
   }
 
   // ---- the two halves of the warp, the warps of the CTA, the CTAs of the cluster ------------------------------------
-  __shared__ float sm_m[W], sm_l[W], sm_acc[W][128];
+  __shared__ float sm_m[W], sm_l[W];
+  __shared__ __align__(16) float sm_acc[W][128];
   __shared__ float in_m[kMaxCluster], in_l[kMaxCluster], in_acc[kMaxCluster][128];     // from every rank: this owner's dims
   {
     const float mo = __shfl_xor_sync(0xffffffffu, m, 16);
@@ -299,8 +300,11 @@ int launch_attn(const char* what, bool rope, AttnParams p, int64_t B, cudaStream
   // are enough (32 pairs at context 2012: 32 warps 51.6, 64 warps 52.4 us a layer of a step).  Above 592 pairs four warps each are
   // more than one wave; up to two waves of them leave too much of the second one empty (800 pairs at 1201: 4 warps 125, 8 warps
   // 115 us), and so does a little more than two over a long context (1280 pairs at 1501 156.3 / 145.2; but at 301, inside a step, a layer took 114
-  // us with four and 117 with eight).  (A little more than one wave of pairs over a long context suits no split: 320 at 2011 60 us, where
-  // 128-token chunks in launches of their own took 56.)
+  // us with four and 117 with eight).
+  // Five warps are three CTAs an SM: from 297 to 444 pairs, where eight warps each are more than one wave and four leave places empty, one
+  // CTA of five, and from 593 to 666, over a cache of more than 640 tokens, two, which fill their last wave.  A layer of a step (hidden 4096,
+  // inter 2816), us, before / now: 320 pairs at 301 68.7 / 67.7, at 1001 89.3 / 84.8, at 2011 117.8 / 109.2; 416 70.7 / 70.0, 93.1 / 90.8, 124.1 / 120.5;
+  // 640 at 301 72.2 / 72.8, at 1001 108.3 / 105.3, at 2011 160.1 / 149.3; behind the lines, at 2011, 448 126.9 / 150.3, 672 163.4 / 166.0.
   const int64_t pairs = B * p.nh;
   const int64_t slots = (int64_t)sm_count() * 16;
   const int64_t last = pairs * 4 % slots;                  // of the last wave of four warps a pair
@@ -308,17 +312,20 @@ int launch_attn(const char* what, bool rope, AttnParams p, int64_t B, cudaStream
   const bool later = pairs * 2 >= slots && last > 0 && 2 * last < slots && p.max_ctx > 80 * kUnit;
   int t = second || later ? 8 : 4;
   while (pairs * 2 * t <= (t == 32 ? slots / 2 : slots) && t < 64 && t * kUnit < p.max_ctx) t *= 2;
-  const int w = t < 8 ? 4 : 8, c = t / w;
-  auto pick = [&](auto k44, auto k48) { return w == 8 ? k48 : k44; };
-  auto kern = rope ? (a16 ? pick(attn_decode_kernel<4, true, true>, attn_decode_kernel<8, true, true>)
-                          : pick(attn_decode_kernel<4, true, false>, attn_decode_kernel<8, true, false>))
-                   : (a16 ? pick(attn_decode_kernel<4, false, true>, attn_decode_kernel<8, false, true>)
-                          : pick(attn_decode_kernel<4, false, false>, attn_decode_kernel<8, false, false>));
+  const int64_t fives = (int64_t)sm_count() * 3;           // CTAs of five warps in a wave
+  if (pairs * 8 > slots && pairs <= fives && p.max_ctx > 4 * kUnit) t = 5;
+  if (pairs * 4 > slots && pairs * 2 <= 3 * fives && p.max_ctx > 40 * kUnit) t = 10;
+  const int w = t % 5 == 0 ? 5 : t < 8 ? 4 : 8, c = t / w;
+  auto pick = [&](auto k4, auto k5, auto k8) { return w == 8 ? k8 : w == 5 ? k5 : k4; };
+  auto kern = rope ? (a16 ? pick(attn_decode_kernel<4, true, true>, attn_decode_kernel<5, true, true>, attn_decode_kernel<8, true, true>)
+                          : pick(attn_decode_kernel<4, true, false>, attn_decode_kernel<5, true, false>, attn_decode_kernel<8, true, false>))
+                   : (a16 ? pick(attn_decode_kernel<4, false, true>, attn_decode_kernel<5, false, true>, attn_decode_kernel<8, false, true>)
+                          : pick(attn_decode_kernel<4, false, false>, attn_decode_kernel<5, false, false>, attn_decode_kernel<8, false, false>));
   // The keys and values in flight are lines of the L1 cache, so most of the SM's memory has to be cache: behind a matmul that
   // had it as shared memory, and without this, 16 warps were held to 25 KB in flight.  A layer of a step, us, before / after: 16 rows
   // at 2012 148 / 133, 5 rows at 2001 (hidden 5120) 141 / 117, 64 at 1002 (hidden 4096) 239 / 222.
-  static SmemLimit carveout[8];
-  const int variant = (w == 8) * 4 + rope * 2 + a16;
+  static SmemLimit carveout[12];
+  const int variant = (w == 8 ? 8 : w == 5 ? 4 : 0) + rope * 2 + a16;
   int dev = -1;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess)

@@ -72,10 +72,13 @@ def test_step_attention_against_the_oracle(cuda_lib, B, nh, ctx):
     assert (np.abs(got - ref) <= 2e-3 + 4e-3 * np.abs(ref)).all(), np.abs(got - ref).max()
 
 
-@pytest.mark.parametrize("ctx", [17, 515])
-def test_a_little_more_than_two_waves_over_a_long_cache(cuda_lib, ctx):
-    """Four warps a pair would leave a third wave nearly empty, and the cache has more than 1280 tokens: eight."""
-    B, nh, max_ctx, pos = 41, 29, 1296, ctx - 1
+# (B, heads, cache) by the warps: 8 (four would leave a third wave nearly empty); 5 from the first to the last pair (one wave); 4 (one wave);
+# 2 x 5 from the first to the last pair
+@pytest.mark.parametrize("B,nh,max_ctx", [(41, 29, 1296), (27, 11, 528), (37, 12, 80), (18, 28, 528), (593, 1, 656), (37, 18, 656)])
+@pytest.mark.parametrize("ctx", [1, 17, 81, 515])
+def test_splits_at_the_ends_of_a_wave(cuda_lib, B, nh, max_ctx, ctx):
+    ctx = min(ctx, max_ctx)
+    pos = ctx - 1
     rng = np.random.default_rng(ctx)
     kc, vc = (np.full((B, max_ctx, nh, D), np.nan, F16) for _ in "kv")
     kc[:, :pos], vc[:, :pos] = (rng.standard_normal((B, pos, nh, D)).astype(F16) for _ in "kv")
